@@ -17,7 +17,7 @@ from ixrun_b200.engine import StreamingLinear
 from ixrun_b200.gpu_pack import int8x_quantize_gpu, quantize_pack_gpu
 from ixrun_b200.hybrid27b import Hybrid27B, HybridConfig
 from ixrun_b200.kernels import decode_weight
-from ixrun_b200.llama_runner import BatchedGreedyDecoder, LlamaConfig, PackedLlama, Verifier, linear_shapes
+from ixrun_b200.llama_runner import BatchedGreedyDecoder, LlamaConfig, PackedLlama, Verifier
 from ixrun_b200.p6 import set_pdl
 
 BITS = 5.4428          # bits per weight of the packed format on this code distribution
@@ -99,17 +99,35 @@ def _weight(gen, out_f, in_f):
     return (c * 2.0 ** -9).bfloat16().view(out_f, in_f)
 
 
+def _llama_parameters(case, gen):
+    """the parameters as a checkpoint holds them: weight of every linear (all layers alike), embedding, head, norms"""
+    h, heads, ffn = case["hidden"], case["hidden"] // 128, case["ffn"]
+    w = {n: _weight(gen, *s) for n, s in
+         {"q_proj": (h, h), "k_proj": (heads // 2 * 128, h), "v_proj": (heads // 2 * 128, h), "o_proj": (h, h),
+          "gate_proj": (ffn, h), "up_proj": (ffn, h), "down_proj": (h, ffn)}.items()}
+    # a residual stream that the layers add to, as in a trained model: bf16 rounding does not pile up to the stream's own size
+    embed = torch.randn(case["vocab"], h, generator=gen, device="cuda").bfloat16()
+    head = (torch.randn(case["vocab"], h, generator=gen, device="cuda") * 0.02).bfloat16()
+    norm = [[(1 + 0.1 * torch.randn(h, generator=gen, device="cuda")).bfloat16() for _ in range(2)]
+            for _ in range(case["layers"])]
+    return w, embed, head, norm
+
+
+def _max_seq(case):
+    return case["context"] + (case["rows"] if case["kind"] != "batch" else 0) + 256
+
+
+def _batch_positions(case, gen):
+    """sequences of different lengths, from half of the context to all of it"""
+    return (case["context"] * (0.5 + 0.5 * torch.rand(case["rows"], generator=gen, device="cuda"))).to(torch.int32)
+
+
 def _llama_model(case, gen):
-    rows, ctx = case["rows"], case["context"]
     heads = case["hidden"] // 128
     cfg = LlamaConfig(n_layers=case["layers"], hidden=case["hidden"], intermediate=case["ffn"], n_heads=heads,
-                      n_kv_heads=heads // 2, vocab=case["vocab"], max_seq=ctx + (rows if case["kind"] != "batch" else 0) + 256)
-    one = {n: int8x_quantize_gpu(_weight(gen, *s)) for n, s in linear_shapes(cfg).items()}    # every layer its own device copy
-    # a residual stream that the layers add to, as in a trained model: bf16 rounding does not pile up to the stream's own size
-    embed = torch.randn(cfg.vocab, cfg.hidden, generator=gen, device="cuda").bfloat16()
-    head = (torch.randn(cfg.vocab, cfg.hidden, generator=gen, device="cuda") * 0.02).bfloat16()
-    norm = [[(1 + 0.1 * torch.randn(cfg.hidden, generator=gen, device="cuda")).bfloat16() for _ in range(2)]
-            for _ in range(cfg.n_layers)]
+                      n_kv_heads=heads // 2, vocab=case["vocab"], max_seq=_max_seq(case))
+    w, embed, head, norm = _llama_parameters(case, gen)
+    one = {n: int8x_quantize_gpu(t) for n, t in w.items()}         # every layer gets its own device copy
     return cfg, PackedLlama(cfg, [one] * cfg.n_layers, embed, head, norms=norm)
 
 
@@ -156,8 +174,7 @@ def prepare(case, seed):
     if kind == "batch":
         d = s["dec"] = BatchedGreedyDecoder(m, case["rows"])
         _fill(gen, d.k_cache, d.v_cache)
-        # sequences of different lengths, from half of the context to all of it
-        s["pos"] = (case["context"] * (0.5 + 0.5 * torch.rand(case["rows"], generator=gen, device="cuda"))).to(torch.int32)
+        s["pos"] = _batch_positions(case, gen)
         d.pos32.copy_(s["pos"])
         return _captured(s, d)
     _fill(gen, m.k_cache, m.v_cache)
@@ -254,3 +271,96 @@ def tolerance(case):
         return {"rel": 2e-3, "max": 0.03, "differ": 0.0}
     # bf16 activations through all layers: against the same weights in dense matmuls with eager glue rel 0.0084 and max 0.039
     return {"rel": 0.03, "max": 0.15}
+
+
+# ------------------------------------------------------------------------------------------------ the same in 64 bits
+def _codes(w):
+    """the quantiser's int8 codes and bf16 scale of a bf16 weight"""
+    scale = (w.abs().max().clamp_min(1e-8) / 127.0).bfloat16()
+    return (w.float() / scale.float()).round().clamp(-127, 127), scale
+
+
+def _dequantised(w):
+    codes, scale = _codes(w)
+    return (codes * scale.float()).bfloat16().double()             # the bf16 weight that the format stands for
+
+
+@torch.no_grad()
+def exact(case, seed):
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    kind = case["kind"]
+    if kind in ("linear", "deploy", "decode"):
+        out_f, in_f = case["out_f"], case["in_f"]
+        w = _weight(gen, out_f, in_f)
+        bias = (torch.randn(out_f, generator=gen, device="cuda") * 0.1).bfloat16() if case.get("bias") else None
+        if kind == "decode":
+            return _dequantised(w)
+        x = torch.randn(case.get("rows", 1), in_f, generator=gen, device="cuda").bfloat16()
+        y = x.double() @ _dequantised(w).t()
+        if bias is not None:
+            y = y + bias.double()
+        if kind == "linear":
+            return y
+        codes, scale = _codes(w)
+        return [y, codes.to(torch.int8), scale] + [None] * 5
+    if kind == "hybrid":
+        return None                                                # its weights are drawn inside the model
+    return _exact_llama(case, gen)
+
+
+def _exact_llama(case, gen):
+    """the decoder on the dequantised weights, every activation in 64 bits"""
+    kind, rows, hidden, d = case["kind"], case["rows"], case["hidden"], 128
+    heads, layers = hidden // d, case["layers"]
+    kvh, max_seq = heads // 2, _max_seq(case)
+    w, embed, head, norm = _llama_parameters(case, gen)
+    w = {n: _dequantised(t) for n, t in w.items()}
+    ids = torch.randint(0, case["vocab"], (rows,), generator=gen, device="cuda")
+    seqs = rows if kind == "batch" else 1
+    kc = torch.zeros(layers, seqs, max_seq, kvh, d, dtype=torch.bfloat16, device="cuda")
+    vc = torch.zeros_like(kc)
+    if kind != "prefill":
+        _fill(gen, kc, vc)
+    if kind == "batch":
+        pos = _batch_positions(case, gen).long()
+        seq = torch.arange(rows, device="cuda")
+    else:
+        pos = case["context"] + torch.arange(rows, device="cuda")
+        seq = torch.zeros(rows, dtype=torch.long, device="cuda")
+    half = d // 2
+    ang = pos[:, None].double() / 10000.0 ** (torch.arange(half, device="cuda").double() / half)
+    cos, sin = ang.cos()[:, None, :], ang.sin()[:, None, :]
+
+    def rope(t):
+        a, b = t[..., :half], t[..., half:]
+        return torch.cat([a * cos - b * sin, b * cos + a * sin], dim=-1)
+
+    def rms(t, g):
+        return t * torch.rsqrt(t.pow(2).mean(-1, keepdim=True) + 1e-5) * g
+
+    h = embed[ids].double()
+    ks, vs = [], []
+    n_ctx = int(pos.max().item()) + 1
+    mask = torch.arange(n_ctx, device="cuda")[None, :] <= pos[:, None]             # [rows, n_ctx]
+    for li in range(layers):
+        x = rms(h, norm[li][0].double())
+        q = rope((x @ w["q_proj"].t()).view(rows, heads, d))
+        k = rope((x @ w["k_proj"].t()).view(rows, kvh, d))
+        v = (x @ w["v_proj"].t()).view(rows, kvh, d)
+        kk, vv = kc[li].double(), vc[li].double()
+        kk[seq, pos], vv[seq, pos] = k, v
+        ks.append(kk if kind == "batch" else k)
+        vs.append(vv if kind == "batch" else v)
+        qg = q.view(rows, kvh, 2, d)
+        if kind == "batch":
+            s = torch.einsum("rghd,rsgd->rghs", qg, kk[:, :n_ctx])
+        else:
+            s = torch.einsum("rghd,sgd->rghs", qg, kk[0, :n_ctx])
+        p = (s * d ** -0.5).masked_fill(~mask[:, None, None, :], -torch.inf).softmax(-1)
+        a = torch.einsum("rghs,rsgd->rghd", p, vv[:, :n_ctx]) if kind == "batch" else torch.einsum("rghs,sgd->rghd", p, vv[0, :n_ctx])
+        h = h + a.reshape(rows, hidden) @ w["o_proj"].t()
+        x = rms(h, norm[li][1].double())
+        g = x @ w["gate_proj"].t()
+        h = h + (g * torch.sigmoid(g) * (x @ w["up_proj"].t())) @ w["down_proj"].t()
+    h = rms(h[-1:] if kind == "prefill" else h, 1.0)
+    return [h @ head.double().t(), torch.stack(ks), torch.stack(vs)]
