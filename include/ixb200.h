@@ -210,6 +210,10 @@ int ixb_p6_build(const int8_t *codes_device, const void *scale_device, int64_t s
                  void *plane_device,
                  int32_t *blk_off_device, void *esc_device, int64_t n_esc, void *ws_device, size_t ws_bytes,
                  ixb_stream_t stream);
+int ixb_p6_plane(const int8_t *codes_device, int64_t out_f, int64_t in_f, void *plane_device, int32_t *blk_off_device,
+                 int64_t *n_esc_host, void *ws_device, size_t ws_bytes, ixb_stream_t stream);
+int ixb_p6_entries(const int8_t *codes_device, const void *scale_device, int64_t scale_stride, int64_t out_f, int64_t in_f,
+                   const int32_t *blk_off_device, void *esc_device, int64_t n_esc, ixb_stream_t stream);
 int ixb_p6_decode(const ixb_p6 *t, void *out_device, int out_kind, ixb_stream_t stream);
 size_t ixb_p6_gemv_scratch_bytes(int64_t out_f, int64_t in_f, int64_t m_rows);
 int ixb_p6_gemv(const ixb_p6 *t, const void *x_device, int64_t m_rows, const void *bias_device,

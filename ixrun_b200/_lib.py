@@ -106,6 +106,10 @@ def lib():
     L.ixb_p6_blocks.argtypes = [i64, i64]
     L.ixb_p6_build.restype = C.c_int
     L.ixb_p6_build.argtypes = [vp, vp, i64, i64, i64, vp, vp, vp, i64, vp, sz, vp]
+    L.ixb_p6_plane.restype = C.c_int
+    L.ixb_p6_plane.argtypes = [vp, i64, i64, vp, vp, C.POINTER(i64), vp, sz, vp]
+    L.ixb_p6_entries.restype = C.c_int
+    L.ixb_p6_entries.argtypes = [vp, vp, i64, i64, i64, vp, vp, i64, vp]
     L.ixb_p6_decode.restype = C.c_int
     L.ixb_p6_decode.argtypes = [C.POINTER(P6Struct), vp, C.c_int, vp]
     L.ixb_p6_gemv_scratch_bytes.restype = sz

@@ -111,7 +111,41 @@ __device__ __forceinline__ uint32_t p6_get(const uint32_t (&w)[6], int p, int h)
 }
 
 // ------------------------------------------------------------------ build ---
-// codes [out_f, in_f] -> plane blocks and the number of outliers of every block (one warp per block)
+// the lane's 32 codes of block (R, kbi): out[0..3] row g, out[4..7] row g + 8, 16 consecutive columns each, as bytes;
+// elements beyond the tensor are 0.  Two 16-byte loads where rows and tensor allow.
+__device__ __forceinline__ void p6_load_codes(const int8_t *__restrict__ codes, uint32_t out_f, uint32_t in_f, uint32_t R,
+                                              uint32_t kbi, int lane, uint32_t (&out)[8])
+{
+    const uint32_t col0 = kbi * kTileCols + 16 * (lane & 3);
+    const bool vec = ((in_f & 15u) | ((uintptr_t)codes & 15u)) == 0;
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+        const uint32_t row = R * kTileRows + (lane >> 2) + 8 * s;
+        uint4 v = make_uint4(0, 0, 0, 0);
+        const int8_t *src = codes + (size_t)row * in_f + col0;
+        if (row < out_f && vec) {
+            if (col0 < in_f) v = __ldg((const uint4 *)src);             // in_f % 16 == 0: all 16 columns or none
+            out[4 * s] = v.x; out[4 * s + 1] = v.y; out[4 * s + 2] = v.z; out[4 * s + 3] = v.w;
+        } else {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                uint32_t u = 0;
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+                    if (row < out_f && col0 + 4 * k + c < in_f) u |= (uint32_t)(uint8_t)src[4 * k + c] << (8 * c);
+                out[4 * s + k] = u;
+            }
+        }
+    }
+}
+// element h of pair p out of them (column 4 (p >> 2) + 2 ((p & 3) >> 1) + h of row g + 8 (p & 1), see p6_elem)
+__device__ __forceinline__ int p6_code_of(const uint32_t (&cw)[8], int p, int h)
+{
+    return (int)(int8_t)(cw[4 * (p & 1) + (p >> 2)] >> (8 * (2 * ((p & 3) >> 1) + h)));
+}
+
+// codes [out_f, in_f] -> plane blocks and the number of outliers of every block (one warp per block).  Bound by memory:
+// 33 us for 5120 x 5120 with one byte per load, before.
 __global__ void __launch_bounds__(256)
 k_p6_plane(const int8_t *__restrict__ codes, uint32_t out_f, uint32_t in_f, uint32_t rt, uint32_t kb,
            unsigned char *plane, int32_t *blk_cnt)
@@ -120,16 +154,14 @@ k_p6_plane(const int8_t *__restrict__ codes, uint32_t out_f, uint32_t in_f, uint
     int lane = threadIdx.x & 31;
     if (b >= rt * kb) return;
     uint32_t R = b / kb, kbi = b - R * kb;
-    uint32_t w[6] = {0, 0, 0, 0, 0, 0};
+    uint32_t cw[8], w[6] = {0, 0, 0, 0, 0, 0};
     uint32_t n_out = 0;
+    p6_load_codes(codes, out_f, in_f, R, kbi, lane, cw);
 #pragma unroll
     for (int p = 0; p < 16; ++p) {
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            uint32_t r, c;
-            p6_elem(lane, p, h, r, c);
-            uint32_t row = R * kTileRows + r, col = kbi * kTileCols + c;
-            int code = (row < out_f && col < in_f) ? (int)codes[(size_t)row * in_f + col] : 0;
+            const int code = p6_code_of(cw, p, h);
             bool out = code > kP6CodeMax || code < kP6CodeMin;
             n_out += out;
             p6_put(w, p, h, p6_field(out ? 0 : code));
@@ -138,8 +170,8 @@ k_p6_plane(const int8_t *__restrict__ codes, uint32_t out_f, uint32_t in_f, uint
     unsigned char *blk = plane + (size_t)b * kP6BlockBytes;
     ((uint4 *)blk)[lane] = make_uint4(w[0], w[1], w[2], w[3]);
     ((uint2 *)(blk + 512))[lane] = make_uint2(w[4], w[5]);
-    n_out = warp_incl_scan(n_out, lane);
-    if (lane == 31) blk_cnt[b] = (int32_t)n_out;
+    n_out = __reduce_add_sync(0xffffffffu, n_out);
+    if (lane == 0) blk_cnt[b] = (int32_t)n_out;
 }
 
 // outlier entries of every block, in (lane, pair, half) order (one warp per block)
@@ -153,23 +185,22 @@ k_p6_esc(const int8_t *__restrict__ codes, uint32_t out_f, uint32_t in_f, uint32
     if (b >= rt * kb) return;
     uint32_t R = b / kb, kbi = b - R * kb;
     float sc = __bfloat162float(scale[R * scale_stride]);
-    int code[32];
+    uint32_t cw[8];
+    p6_load_codes(codes, out_f, in_f, R, kbi, lane, cw);
     uint32_t n_out = 0;
 #pragma unroll
     for (int i = 0; i < 32; ++i) {
-        uint32_t r, c;
-        p6_elem(lane, i >> 1, i & 1, r, c);
-        uint32_t row = R * kTileRows + r, col = kbi * kTileCols + c;
-        code[i] = (row < out_f && col < in_f) ? (int)codes[(size_t)row * in_f + col] : 0;
-        n_out += (code[i] > kP6CodeMax || code[i] < kP6CodeMin);
+        const int code = p6_code_of(cw, i >> 1, i & 1);
+        n_out += (code > kP6CodeMax || code < kP6CodeMin);
     }
     uint32_t at = (uint32_t)blk_off[b] + warp_incl_scan(n_out, lane) - n_out;
 #pragma unroll
     for (int i = 0; i < 32; ++i) {
-        if (code[i] > kP6CodeMax || code[i] < kP6CodeMin) {
+        const int code = p6_code_of(cw, i >> 1, i & 1);
+        if (code > kP6CodeMax || code < kP6CodeMin) {
             uint32_t r, c;
             p6_elem(lane, i >> 1, i & 1, r, c);
-            uint32_t wbits = __bfloat16_as_ushort(__float2bfloat16_rn((float)code[i] * sc));
+            uint32_t wbits = __bfloat16_as_ushort(__float2bfloat16_rn((float)code * sc));
             if (at < n_esc) esc[at] = (wbits << 16) | (r << 12) | ((b & 63u) << 6) | c;   // never beyond the caller's buffer
             ++at;
         }

@@ -71,24 +71,26 @@ class P6Packed:
         self.device, self.out_f, self.in_f, self.N = dev, int(out_f), int(in_f), int(out_f) * int(in_f)
         self.total_bytes = int(total_bytes)          # the reference format's byte count of this tensor
         c = codes.contiguous().reshape(-1)
-        n_esc = int(((c < CODE_MIN) | (c > CODE_MAX)).sum().item())
         L = _lib.lib()
         nb = int(L.ixb_p6_blocks(self.out_f, self.in_f))
         # sizes include the slack that the GEMV's prefetch may read
         self.plane = torch.empty((nb + SLACK_BLOCKS) * BLOCK_BYTES // 4, dtype=torch.int32, device=dev)
         self.blk_off = torch.empty(nb + 1, dtype=torch.int32, device=dev)
-        self.esc = torch.empty(n_esc + SLACK_ENTRIES, dtype=torch.int32, device=dev)
-        self.n_esc = n_esc
         self.scale = scale.detach().to(dev, torch.bfloat16).reshape(-1).contiguous()
         if self.scale.numel() not in (1, (self.out_f + 15) // 16):
             raise ValueError("scale must hold one value, or one per 16-row tile")
         stride = 0 if self.scale.numel() == 1 else 1
         self.sections = [(0, self.out_f)]            # (first row, rows) of every fused part
         ws = torch.empty((nb + 1) * 4, dtype=torch.uint8, device=dev)
+        count = C.c_int64()
         with torch.cuda.device(dev):
-            _lib.check(L.ixb_p6_build(c.data_ptr(), self.scale.data_ptr(), stride, self.out_f, self.in_f, self.plane.data_ptr(),
-                                      self.blk_off.data_ptr(), self.esc.data_ptr(), n_esc,
-                                      ws.data_ptr(), ws.numel(), _lib.stream_ptr(dev)))
+            st = _lib.stream_ptr(dev)
+            _lib.check(L.ixb_p6_plane(c.data_ptr(), self.out_f, self.in_f, self.plane.data_ptr(), self.blk_off.data_ptr(),
+                                      C.byref(count), ws.data_ptr(), ws.numel(), st))
+            self.n_esc = n_esc = int(count.value)
+            self.esc = torch.empty(n_esc + SLACK_ENTRIES, dtype=torch.int32, device=dev)
+            _lib.check(L.ixb_p6_entries(c.data_ptr(), self.scale.data_ptr(), stride, self.out_f, self.in_f,
+                                        self.blk_off.data_ptr(), self.esc.data_ptr(), n_esc, st))
         self.struct = _lib.P6Struct(self.plane.data_ptr(), self.blk_off.data_ptr(), self.esc.data_ptr(), n_esc,
                                     self.scale.data_ptr(), self.out_f, self.in_f, stride)
         self.resident_bytes = nb * BLOCK_BYTES + 4 * (nb + 1 + n_esc) + 2
