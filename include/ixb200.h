@@ -170,7 +170,7 @@ int ixb_group_scale(const int8_t *codes_device, const void *group_scales_fp16_de
  *   plane    a 6-bit field per element, blocks of 16 rows x 64 columns (ragged
  *            edges padded), 768 contiguous bytes per block, block b =
  *            row_tile * ceil(in_f / 64) + column_block.  The field is bits 7..2
- *            of the low byte of the bf16 number 1 + code / 32 (codes -16 .. 31),
+ *            of the low byte of the bf16 number 96 + code (codes -32 .. 31),
  *            so the GEMV needs a shift, a mask and ONE fused multiply-add per
  *            pair of weights to obtain bf16(code * scale) -- the reference's
  *            dequantised weight (ixrun/quantize.py:182, ixrun/fused.py:169-170),
@@ -178,16 +178,18 @@ int ixb_group_scale(const int8_t *codes_device, const void *group_scales_fp16_de
  *   esc      every other code as a uint32 entry: bf16(code * scale) in the high
  *            half, row in tile, block index mod 64 and column in block below;
  *            blk_off: int32 first entry of every block
- * about 6 + 32 * P(code outside -16 .. 31) bits per weight.  Buffer sizes
+ * about 6 + 32 * P(code outside -32 .. 31) bits per weight.  Buffer sizes
  * (B = ixb_p6_blocks): plane (B + 5) * 768 bytes, blk_off (B + 1) * 4 bytes,
  * esc (n_esc + 64) * 4 bytes; plane and esc 16-byte aligned.
  * ixb_p6_build: int8 codes [out_f, in_f] + the bf16 scale -> layout (n_esc =
- *   number of codes outside -16 .. 31; entries beyond n_esc are not written;
+ *   number of codes outside -32 .. 31, or more; entries beyond n_esc are not written;
  *   ws: (B + 1) * 4 bytes).
+ * ixb_p6_plane, ixb_p6_entries: the same in two steps, for a caller that does not know n_esc: the first writes plane and
+ *   blk_off and gives the number of outliers on the host (it synchronises the stream), the second writes esc.
  * ixb_p6_decode: layout -> int8 codes / bf16 weights (out_kind as ixb_decode).
  * ixb_p6_gemv: same result definition, bias and argument meaning as ixb_gemv,
- *   1..8 activation rows in one kernel: plane on the tensor cores (mma.sync,
- *   exact bf16 x bf16 products, fp32 accumulation), outliers on the CUDA cores;
+ *   1..8 activation rows in one kernel: plane and outliers on the tensor cores
+ *   (mma.sync, exact bf16 x bf16 products, fp32 accumulation);
  *   partial sums are added in a fixed order (reproducible, no floating-point
  *   atomics).  Scratch: ixb_p6_gemv_scratch_bytes bytes, 16-byte aligned, zero
  *   before the first call; every launch leaves it all zero again, so one buffer

@@ -4,17 +4,17 @@
 // reference's (3,5,8) streams decode to (ixrun/quantize.py:80-96), and keeps
 // those codes exactly.  Nothing in it is addressed by rank: every 1024-weight
 // block (16 rows x 64 columns, one warp) sits at a fixed address, and turning it
-// into tensor-core operands costs three instructions per PAIR of weights:
+// into tensor-core operands costs four instructions per PAIR of weights:
 //
-//   plane   every element owns a 6-bit field F that is bits 7..2 of the low
-//           byte of the bf16 number a = 1 + code / 32:
-//             code in [0, 31]    a in [1, 2)    F = 32 + code
-//             code in [-16, -1]  a in [0.5, 1)  F = 32 + 2 code
-//           so (F << 2) | 0x3F00 IS a, and one fused multiply-add
-//           fma(a, 32 s, -32 s) = bf16(code * s) rounds the exact product once:
-//           the reference's dequantised weight bf16(f32(code) * f32(scale))
-//           (ixrun/quantize.py:182, ixrun/fused.py:169-170), bit for bit, for any scale s.
-//           Other codes ("outliers") leave the placeholder F = 32 (weight 0).
+//   plane   every element of code -32 .. 31 owns a 6-bit field F = 32 + code; put at bits 6..1 of the low byte it makes
+//           a bf16 number of the binade [64, 128):
+//             (F << 1) | 0x4280 = 64 + F = 96 + code
+//           so a packed subtraction of 96 gives the code exactly, and the packed multiplication by the scale rounds the
+//           exact product once: the reference's dequantised weight bf16(f32(code) * f32(scale))
+//           (ixrun/quantize.py:182, ixrun/fused.py:169-170), bit for bit, for any scale.
+//           Other codes ("outliers") leave the placeholder F = 32 (weight 0).  (Before, F was part of 1 + code / 32 over
+//           two binades, one fused multiply-add per pair instead of two operations, but it held -16 .. 31 only: 1.2 % of
+//           the benchmark distribution were outliers, 4 bytes and an extra step each, against 0.07 % now.)
 //           Blocks of 16 rows x 64 columns, ragged edges padded with
 //           placeholders (p6_elem gives the element of lane / pair / half); a
 //           lane owns 32 fields in six 32-bit words,
@@ -30,15 +30,13 @@
 //           64 consecutive blocks of one row tile resolves its columns without
 //           knowing which block an entry came from.
 //
-// Size: 6 + 32 * P(outlier) bits per weight + 4 bytes per block (6.4 bpw for
+// Size: 6 + 32 * P(outlier) bits per weight + 4 bytes per block (6.05 bpw for
 // the benchmark distribution).
 //
 // y = W x is one kernel (k_p6_mma): per warp a ring of cp.async-staged blocks,
-// twelve shift/mask/fma triples and four five-instruction pairs per lane give
-// the A fragments of four mma.sync.m16n8k16 (bf16) with the activations as B;
-// the outliers of a warp's run of blocks are staged once in shared memory and
-// added on the CUDA cores (weight * x into per-row, per-lane sums) per row-tile
-// segment of the run, while the ring keeps fetching.  Products are exact, accumulation is fp32, and no
+// four instructions per pair of weights give the A fragments of four mma.sync.m16n8k16 (bf16) with the activations as B;
+// the outliers of a warp's run of blocks are staged once in shared memory and added per row-tile segment of the run as
+// the k index of further mmas, while the ring keeps fetching.  Products are exact, accumulation is fp32, and no
 // floating-point atomics are used: results are reproducible.
 #pragma once
 #include "ixb_common.cuh"
@@ -77,7 +75,7 @@ constexpr int kP6BlockBytes = 768;
 constexpr int kP6Slots = 4;                       // ring slots per warp; blocks are fetched three ahead
 constexpr int kP6SlackBlocks = 5;                 // readable blocks behind the plane (the ring fetches past a run end)
 constexpr int kP6SlackEntries = 64;               // readable entries behind the outlier list
-constexpr int kP6CodeMin = -16, kP6CodeMax = 31;  // codes that the plane holds
+constexpr int kP6CodeMin = -32, kP6CodeMax = 31;  // codes that the plane holds
 
 struct P6 {
     const unsigned char *plane;  // [(nb + slack) * 768]
@@ -89,8 +87,8 @@ struct P6 {
     uint32_t scale_stride;
 };
 
-__host__ __device__ __forceinline__ uint32_t p6_field(int code) { return (uint32_t)(code >= 0 ? 32 + code : 32 + 2 * code); }
-__host__ __device__ __forceinline__ int p6_code(uint32_t f) { return f >= 32u ? (int)f - 32 : ((int)f - 32) / 2; }
+__host__ __device__ __forceinline__ uint32_t p6_field(int code) { return (uint32_t)(32 + code); }
+__host__ __device__ __forceinline__ int p6_code(uint32_t f) { return (int)f - 32; }
 
 __device__ __forceinline__ void p6_put(uint32_t (&w)[6], int p, int h, uint32_t f)
 {
@@ -276,14 +274,21 @@ __global__ void __launch_bounds__(256) k_p6_decode_esc(P6 p, void *out)
 // ------------------------------------------------------------------ GEMV ----
 constexpr int kP6Threads = 768;
 constexpr int kP6Warps = kP6Threads / 32;
-constexpr int kP6StageEntries = 512;                                  // outlier entries a warp stages in shared memory
 constexpr int kP6RingBytes = kP6Slots * kP6BlockBytes;                // 3072
-// per warp: ring, per-row outlier sums [16][32] fp32, staged entries, two partial tiles [2][32] float4
-constexpr int kP6WarpSmem = kP6RingBytes + 16 * 32 * 4 + kP6StageEntries * 4 + 2 * 32 * 16;
 constexpr int kP6TailTiles = 32;                                      // row tiles per CTA that the barrier-free tail tracks
 constexpr int kP6TailBytes = kP6TailTiles * 12;                       // per tile: arrival counter + two words of plan
-constexpr int kP6SmemFixed = kP6Warps * kP6WarpSmem + kP6TailBytes;
-static_assert(kP6WarpSmem % 128 == 0, "per-warp shared memory keeps 128-byte alignment");
+// Shared memory of one warp: ring, an outlier step's operand tiles (A: 2 x 16 x 16 bf16, zero between steps; B: 2 x 8 x
+// 16), staged entries, two partial row tiles (16 sums at one activation row, else [32] float4).  A CTA: kP6Warps of
+// these, the tail's plan, the activations.
+template <bool MULTI>
+struct P6Smem {
+    static constexpr int kEntries = 128;                              // outlier entries a warp stages: five per block of a 24-block run
+    static constexpr int kTiles = kP6RingBytes, kStage = kTiles + 1024 + 512;
+    static constexpr int kParts = kStage + kEntries * 4, kPart = MULTI ? 32 * 16 : 16 * 4;
+    static constexpr int kWarp = kParts + 2 * kPart;
+    static constexpr int kFixed = kP6Warps * kWarp + kP6TailBytes;
+    static_assert(kWarp % 128 == 0 && kStage % 16 == 0, "per-warp shared memory keeps its alignment");
+};
 
 __device__ __forceinline__ void p6_cp16(uint32_t dst, const void *src)
 {
@@ -307,13 +312,43 @@ __device__ __forceinline__ uint2 p6_lds64(uint32_t addr)
     asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr) : "memory");
     return v;
 }
-// two fields at bits 7..2 / 23..18 of t -> the two bf16 numbers a = 1 + code / 32 -> the two weights
-__device__ __forceinline__ uint32_t p6_pair(uint32_t t, uint32_t e2, uint32_t b2, uint32_t c2)
+__device__ __forceinline__ uint32_t p6_lds32(uint32_t addr)
 {
-    uint32_t v, w;
-    asm("lop3.b32 %0, %1, 0x00FC00FC, %2, 0xEA;" : "=r"(v) : "r"(t), "r"(e2));
-    asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(w) : "r"(v), "r"(b2), "r"(c2));
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+    return v;
+}
+__device__ __forceinline__ void p6_ldmatrix(uint32_t (&r)[4], uint32_t addr)
+{
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+// two bf16 numbers 96 + code -> the two weights; s2: the scale in both halves
+__device__ __forceinline__ uint32_t p6_weights(uint32_t v, uint32_t s2)
+{
+    uint32_t w;
+    asm("{\n\t.reg .b32 c;\n\tadd.rn.bf16x2 c, %1, %2;\n\tmul.rn.bf16x2 %0, c, %3;\n\t}" : "=r"(w) : "r"(v), "r"(0xC2C0C2C0u), "r"(s2));
     return w;
+}
+// a lane's six plane words -> its 16 pairs of weights; e2 = 0x42804280 (kept in a register by the caller)
+__device__ __forceinline__ void p6_unpack(const uint32_t (&w)[6], uint32_t e2, uint32_t s2, uint32_t (&f)[16])
+{
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+        f[2 * k] = p6_weights(p6_and_or(w[k] << 1, 0x007E007Eu, e2), s2);
+        f[2 * k + 1] = p6_weights(p6_and_or(w[k] >> 5, 0x007E007Eu, e2), s2);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        uint32_t v = p6_and_or(w[i] >> 11, 0x001E001Eu, e2);
+        v = p6_and_or(w[4 + (i >> 1)] >> (7 + 2 * (i & 1)), 0x00600060u, v);
+        f[12 + i] = p6_weights(v, s2);
+    }
+}
+__device__ __forceinline__ uint32_t p6_scale2(const __nv_bfloat16 &s)
+{
+    const uint32_t b = (uint32_t)__bfloat16_as_ushort(s);
+    return b | b << 16;
 }
 
 // Where the outputs of a row-parallel shard go instead of y: into this rank's slot of EVERY rank's all-reduce buffer
@@ -391,7 +426,7 @@ __device__ __forceinline__ uint32_t p6_part_of(uint32_t pos, uint32_t q, uint32_
     return pos < big ? pos / (q + 1u) : r + (pos - big) / q;      // q > 0 whenever pos >= big
 }
 
-// layout -> bf16 weights in one pass, with the GEMV's own conversion (shift, mask, one fma per pair of elements): the
+// layout -> bf16 weights in one pass, with the GEMV's own conversion: the
 // block's outliers are dropped into a zeroed image of the lanes' registers in shared memory first and OR-ed over the
 // placeholders (+0.0), so every weight is stored once, in 16-byte pieces; needs in_f % 8 == 0 and a 16-byte aligned
 // output.  One warp per block.
@@ -401,6 +436,10 @@ __global__ void __launch_bounds__(256) k_p6_decode_bf16(P6 p, __nv_bfloat16 *out
     uint32_t b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     int lane = threadIdx.x & 31;
     if (b >= p.rt * p.kb) return;                    // whole warps leave together
+    // the plane first: the chain of offsets, entries and image below hides its way from memory
+    const unsigned char *blk = p.plane + (size_t)b * kP6BlockBytes;
+    const uint4 a = __ldg((const uint4 *)blk + lane);
+    const uint2 a2 = __ldg((const uint2 *)(blk + 512) + lane);
     uint4 *img = images + (threadIdx.x >> 5) * 128;
 #pragma unroll
     for (int q = 0; q < 4; ++q) img[q * 32 + lane] = make_uint4(0, 0, 0, 0);
@@ -420,25 +459,9 @@ __global__ void __launch_bounds__(256) k_p6_decode_bf16(P6 p, __nv_bfloat16 *out
     }
     __syncwarp();
     uint32_t R = b / p.kb, kbi = b - R * p.kb;
-    const float s32 = 32.f * __bfloat162float(p.scale[R * p.scale_stride]);
-    const uint32_t bb = (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(s32));
-    const uint32_t b2 = bb | (bb << 16), c2 = b2 ^ 0x80008000u, e2 = 0x3F003F00u;
-    const unsigned char *blk = p.plane + (size_t)b * kP6BlockBytes;
-    const uint4 a = ((const uint4 *)blk)[lane];
-    const uint2 a2 = ((const uint2 *)(blk + 512))[lane];
     const uint32_t w[6] = {a.x, a.y, a.z, a.w, a2.x, a2.y};
     uint32_t f[16];
-#pragma unroll
-    for (int k = 0; k < 6; ++k) {
-        f[2 * k] = p6_pair(w[k] << 2, e2, b2, c2);
-        f[2 * k + 1] = p6_pair(w[k] >> 4, e2, b2, c2);
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        uint32_t v = p6_and_or(w[i] >> 10, 0x003C003Cu, e2);
-        v = p6_and_or(w[4 + (i >> 1)] >> (6 + 2 * (i & 1)), 0x00C000C0u, v);
-        asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(f[12 + i]) : "r"(v), "r"(b2), "r"(c2));
-    }
+    p6_unpack(w, 0x42804280u, p6_scale2(p.scale[R * p.scale_stride]), f);
 #pragma unroll
     for (int q = 0; q < 4; ++q) {                    // placeholders are +0.0, so OR-ing the outlier weights in is exact
         const uint4 v = img[q * 32 + lane];
@@ -474,24 +497,22 @@ __global__ void __launch_bounds__(256) k_p6_decode_bf16(P6 p, __nv_bfloat16 *out
 // last arriver sums the slots in CTA order and clears them.  tickets[] (gridDim.x + 1 words) and cta_slots must be
 // zero before the first launch and are left zero, so one scratch buffer serves launches of any shape in turn.  XS = 1: activations staged in shared memory (bf16, padded rows); XS = 0: read from
 // global memory.
-
-template <int XS>
+template <int XS, bool MULTI>
 __global__ void __launch_bounds__(kP6Threads, 1)
 k_p6_mma(P6 p, const __nv_bfloat16 *__restrict__ x, uint32_t m_rows, const __nv_bfloat16 *__restrict__ bias, void *y,
          int y_f32, float4 *cta_slots, uint32_t *tickets, uint32_t nb, uint32_t xstride, uint32_t cq, uint32_t cr, uint32_t unit,
          P6Push push)
 {
     extern __shared__ __align__(128) unsigned char p6_smem[];
-    __nv_bfloat16 *xs = (__nv_bfloat16 *)(p6_smem + kP6SmemFixed);                       // [m_rows][xstride]
+    using SM = P6Smem<MULTI>;
+    __nv_bfloat16 *xs = (__nv_bfloat16 *)(p6_smem + SM::kFixed);                         // [m_rows][xstride]
 
     const int lane = threadIdx.x & 31;
     const int wid = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);   // the same in every lane, and known to be
     const int g = lane >> 2, t = lane & 3;
     const uint32_t KB = p.kb;
-    unsigned char *wsm = p6_smem + wid * kP6WarpSmem;
-    float *oacc = (float *)(wsm + kP6RingBytes);                       // [16 rows][32 lanes] outlier sums, zero between passes
-    uint32_t *estage = (uint32_t *)(wsm + kP6RingBytes + 2048);        // the run's first kP6StageEntries outlier entries
-    float4 *wparts = (float4 *)(wsm + kP6RingBytes + 4096);            // partial sums of the run's first / last row tile
+    unsigned char *wsm = p6_smem + wid * SM::kWarp;
+    uint32_t *estage = (uint32_t *)(wsm + SM::kStage);                 // the run's first SM::kEntries outlier entries
 
     const uint32_t cb0 = p6_begin(blockIdx.x, cq, cr) * unit, cb1 = p6_begin(blockIdx.x + 1, cq, cr) * unit;
     const uint32_t L = cb1 - cb0, wq = L / kP6Warps, wr = L - wq * kP6Warps;
@@ -500,7 +521,7 @@ k_p6_mma(P6 p, const __nv_bfloat16 *__restrict__ x, uint32_t m_rows, const __nv_
     // ---- plan of the tail, made while nothing else can run yet.  For every row tile R0 + i that this CTA touches
     // (fast path: at most kP6TailTiles): which warps' runs meet it, whether it lies inside the CTA's range, how many
     // partial sums will arrive (0: one run covers it and writes y itself), and the CTAs that share it.
-    uint32_t *tcnt = (uint32_t *)(p6_smem + kP6Warps * kP6WarpSmem);   // [kP6TailTiles] arrivals
+    uint32_t *tcnt = (uint32_t *)(p6_smem + kP6Warps * SM::kWarp);   // [kP6TailTiles] arrivals
     uint32_t *tplan = tcnt + kP6TailTiles;                             // [kP6TailTiles][2]
     const uint32_t Rc0 = cb0 / KB, Rc1 = L ? (cb1 - 1u) / KB : Rc0;
     const bool fast_tail = L != 0 && Rc1 - Rc0 < (uint32_t)kP6TailTiles;
@@ -543,11 +564,11 @@ k_p6_mma(P6 p, const __nv_bfloat16 *__restrict__ x, uint32_t m_rows, const __nv_
             pf_left -= more ? 1u : 0u;
         }
 #pragma unroll
-        for (int r = 0; r < 16; ++r) oacc[r * 32 + lane] = 0.f;
+        for (int k = 0; k < 3; ++k) ((uint4 *)(wsm + SM::kTiles))[k * 32 + lane] = make_uint4(0, 0, 0, 0);
     }
     // the scale of the run's first row tile and of the one after it (a fused tensor has one per row tile); the
     // walk below always holds the next tile's scale one segment ahead, so the load is never waited for
-    uint32_t e2, b2 = 0, c2 = 0;
+    uint32_t e2, s2 = 0;
     uint32_t sc_cur = 0, sc_next = 0;
     {
         if (p.scale_stride) {                                          // (uniform) a fused tensor: one scale per row tile
@@ -557,14 +578,9 @@ k_p6_mma(P6 p, const __nv_bfloat16 *__restrict__ x, uint32_t m_rows, const __nv_
         } else {
             sc_cur = (uint32_t)__bfloat16_as_ushort(p.scale[0]);
         }
-        asm volatile("mov.b32 %0, 0x3F003F00;" : "=r"(e2));            // opaque, so that it stays a register operand
+        asm volatile("mov.b32 %0, 0x42804280;" : "=r"(e2));            // opaque, so that it stays a register operand
     }
-    auto set_scale = [&](uint32_t bits) {
-        const float s32 = 32.f * __uint_as_float(bits << 16);
-        const uint32_t bb = (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(s32));    // exact: a power-of-two multiple
-        b2 = bb | (bb << 16);
-        c2 = b2 ^ 0x80008000u;
-    };
+    auto set_scale = [&](uint32_t bits) { s2 = bits | bits << 16; };
     set_scale(sc_cur);
     asm volatile("griddepcontrol.wait;" ::: "memory");
     // a pushing launch marks its words with the number of this all-reduce call: one more than the counter that the
@@ -599,9 +615,9 @@ k_p6_mma(P6 p, const __nv_bfloat16 *__restrict__ x, uint32_t m_rows, const __nv_
     if (active) {
         const uint32_t es = (uint32_t)__cvta_generic_to_shared(estage);
 #pragma unroll
-        for (int q = 0; q < kP6StageEntries / 128; ++q) {
+        for (int q = 0; q < (SM::kEntries + 127) / 128; ++q) {
             const int32_t ch = j_base + (q * 32 + lane) * 4;
-            if (ch < j_end) p6_cp16(es + (q * 32 + lane) * 16, p.esc + ch);
+            if (ch < j_end && (q * 32 + lane) * 4 < SM::kEntries) p6_cp16(es + (q * 32 + lane) * 16, p.esc + ch);
         }
     }
     cp_async_commit();
@@ -617,8 +633,14 @@ k_p6_mma(P6 p, const __nv_bfloat16 *__restrict__ x, uint32_t m_rows, const __nv_
             const uint32_t wb = p6_begin(w, wq, wr);
             if (wb == p6_begin(w + 1, wq, wr)) continue;                // a warp without blocks
             // the run of warp w meets tile R: R is its first tile unless the run began in the tile before
-            const float4 v = ((const float4 *)(p6_smem + w * kP6WarpSmem + kP6RingBytes + 4096))[(cb0 + wb >= t0 ? 0 : 32) + lane];
-            s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+            const unsigned char *part = p6_smem + w * SM::kWarp + SM::kParts + (cb0 + wb >= t0 ? 0 : SM::kPart);
+            if (MULTI) {
+                const float4 v = ((const float4 *)part)[lane];
+                s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+            } else {                                                    // only activation row 0 counts: lanes t == 0, c[0] and c[2]
+                s.x += ((const float *)part)[g];
+                s.z += ((const float *)part)[g + 8];
+            }
         }
         if (inside) {
             const float cc[4] = {s.x, s.y, s.z, s.w};
@@ -716,33 +738,22 @@ k_p6_mma(P6 p, const __nv_bfloat16 *__restrict__ x, uint32_t m_rows, const __nv_
                 cp_async_commit();
                 n16 += kP6BlockBytes;
                 pf_left -= more ? 1u : 0u;
+                uint4 x0, x1;
+                if (!XS) {                                        // requested ahead of the wait for the block
+                    x0 = *(const uint4 *)((const char *)xg + xo);
+                    x1 = *(const uint4 *)((const char *)xg + xo + 16);
+                }
                 cp_async_wait<3>();                               // this lane's chunks of the block have landed ...
                 __syncwarp();                                     // ... and so have the other lanes'
                 const uint4 a = p6_lds128(d16 + cs);
                 const uint2 a2 = p6_lds64(d8 + cs);
-                uint4 x0, x1;
                 if (XS) {
                     x0 = p6_lds128(xs_l + xo);
                     x1 = p6_lds128(xs_l + xo + 16u);
-                } else {
-                    x0 = *(const uint4 *)((const char *)xg + xo);
-                    x1 = *(const uint4 *)((const char *)xg + xo + 16);
                 }
+                const uint32_t w[6] = {a.x, a.y, a.z, a.w, a2.x, a2.y};
                 uint32_t f[16];
-                {
-                    const uint32_t w[6] = {a.x, a.y, a.z, a.w, a2.x, a2.y};
-#pragma unroll
-                    for (int k = 0; k < 6; ++k) {
-                        f[2 * k] = p6_pair(w[k] << 2, e2, b2, c2);
-                        f[2 * k + 1] = p6_pair(w[k] >> 4, e2, b2, c2);
-                    }
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        uint32_t v = p6_and_or(w[i] >> 10, 0x003C003Cu, e2);
-                        v = p6_and_or(w[4 + (i >> 1)] >> (6 + 2 * (i & 1)), 0x00C000C0u, v);
-                        asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(f[12 + i]) : "r"(v), "r"(b2), "r"(c2));
-                    }
-                }
+                p6_unpack(w, e2, s2, f);
                 p6_mma(c, f[0], f[1], f[2], f[3], x0.x, x0.y);
                 p6_mma(c1, f[4], f[5], f[6], f[7], x0.z, x0.w);
                 p6_mma(c, f[8], f[9], f[10], f[11], x1.x, x1.y);
@@ -753,41 +764,99 @@ k_p6_mma(P6 p, const __nv_bfloat16 *__restrict__ x, uint32_t m_rows, const __nv_
             }
         };
 
-        // Outliers of blocks [sb, sb + 64) at most, all in row tile R: entries [jlo, jhi).  Every lane multiplies
-        // its entries' weights with their activations into oacc[row][lane]; the rows are then summed across the
-        // lanes in a fixed order and added to the C fragment (row g -> c[0], c[1]; row g + 8 -> c[2], c[3]).
+        // Outliers of blocks [sb, sb + 64) at most, all in row tile R: entries [jlo, jhi), 32 per step, one per lane, as
+        // the k index of two more mmas.  A lane writes its weight into its column of A (at the entry's row) and the
+        // activations it meets into its column of B (one per activation row); ldmatrix turns the tiles into operands.
+        // So an entry is looked at once for all activation rows, every row of activations gets the same bits alone or
+        // beside others, and no sums over lanes are left.  (Products on the CUDA cores and sums over the lanes, row by
+        // row of activations: 17408 x 5120 19 us at two rows and 37 us at eight, against 17.4 and 18.4 us now; at one row,
+        // with as many outliers, the two forms differ by less than 10 %.)
+        // The zeros of A turn infinite and NaN activations into NaN in rows that they do not reach: if a sum is not finite
+        // afterwards, the steps are taken again with those activations as 0 in B and their products added one by one.
+        const uint32_t tiles = (uint32_t)__cvta_generic_to_shared(wsm + SM::kTiles);
+        const uint32_t my_a = tiles + (lane >> 4) * 512u + ((lane >> 3) & 1) * 256u + (lane & 7) * 2u;              // + row * 16
+        const uint32_t my_b = tiles + 1024u + (lane >> 4) * 256u + ((lane >> 3) & 1) * 128u + (lane & 7) * 2u;      // + m * 16
+        const uint32_t es = (uint32_t)__cvta_generic_to_shared(estage), pitch = XS ? xstride : p.in_f;
+        constexpr int MR = MULTI ? 8 : 1;
+        uint32_t at = my_a;                                               // where this lane's weight lies
+        auto outlier_steps = [&](uint32_t s64, const __nv_bfloat16 *xm, int32_t jlo, int32_t jhi, auto check) {
+            constexpr bool kCheck = decltype(check)::value;
+            unsigned short xv[MR];
+            auto fetch = [&](int32_t j) -> uint32_t {                     // a lane beyond the end: weight 0, row 0, column 0
+                uint32_t e = s64;
+                if (j < jhi) {
+                    const uint32_t rel = (uint32_t)(j - j_base);
+                    e = rel < (uint32_t)SM::kEntries ? p6_lds32(es + rel * 4u) : __ldg(p.esc + j);
+                }
+                const __nv_bfloat16 *xe = xm + (((e & 0xFFFu) - s64) & 0xFFFu);
+#pragma unroll
+                for (int m = 0; m < MR; ++m)
+                    if (!MULTI || (uint32_t)m < m_rows) xv[m] = __bfloat16_as_ushort(xe[(size_t)m * pitch]);
+                return e;
+            };
+            uint32_t e = fetch(jlo + lane);
+            for (int32_t j = jlo; j < jhi; j += 32) {
+                asm volatile("st.shared.u16 [%0], %1;" ::"r"(at), "h"((unsigned short)0) : "memory");
+                at = my_a + ((e >> 8) & 0xF0u);
+                asm volatile("st.shared.u16 [%0], %1;" ::"r"(at), "h"((unsigned short)(e >> 16)) : "memory");
+                bool bad = false;
+#pragma unroll
+                for (int m = 0; m < MR; ++m) {
+                    if (MULTI && (uint32_t)m >= m_rows) break;
+                    if (kCheck && (xv[m] & 0x7F80u) == 0x7F80u) {
+                        bad = true;
+                        xv[m] = 0;
+                    }
+                    asm volatile("st.shared.u16 [%0], %1;" ::"r"(my_b + m * 16u), "h"(xv[m]) : "memory");
+                }
+                if (kCheck) {
+                    for (uint32_t left = __ballot_sync(0xffffffffu, bad && j + lane < jhi); left; left &= left - 1u) {
+                        const uint32_t ek = __shfl_sync(0xffffffffu, e, __ffs((int)left) - 1), row = (ek >> 12) & 15u;
+                        const __nv_bfloat16 *xk = xm + (((ek & 0xFFFu) - s64) & 0xFFFu);
+#pragma unroll
+                        for (int i = 0; i < 2; ++i) {
+                            const uint32_t m = 2u * t + i;
+                            if (m >= m_rows || (row & 7u) != (uint32_t)g) continue;
+                            const float xf = __bfloat162float(xk[(size_t)m * pitch]);
+                            if ((__float_as_uint(xf) & 0x7F800000u) != 0x7F800000u) continue;
+                            const float v = __uint_as_float(ek & 0xFFFF0000u) * xf;
+                            if (row < 8u) c[i] += v;
+                            else c[2 + i] += v;
+                        }
+                        __syncwarp();
+                    }
+                }
+                __syncwarp();                                             // the step's tiles are written
+                e = fetch(j + 32 + lane);                                 // (the next step's loads are on their way)
+                uint32_t a0[4], a1[4], bf[4];
+                p6_ldmatrix(a0, tiles + lane * 16u);
+                p6_ldmatrix(a1, tiles + 512u + lane * 16u);
+                p6_ldmatrix(bf, tiles + 1024u + lane * 16u);
+                p6_mma(c, a0[0], a0[1], a0[2], a0[3], bf[0], bf[1]);
+                p6_mma(c1, a1[0], a1[1], a1[2], a1[3], bf[2], bf[3]);
+                __syncwarp();                                             // every lane has read them
+            }
+        };
         auto outlier_pass = [&](uint32_t sb, int32_t jlo, int32_t jhi) {
             if (jlo >= jhi) return;                                       // warp uniform
-            const uint32_t s64 = (sb & 63u) << 6, xcol0 = (sb - R * KB) * kTileCols;
-            for (uint32_t m = 0; m < m_rows; ++m) {
-                const __nv_bfloat16 *xm = (XS ? xs + (size_t)m * xstride : x + (size_t)m * p.in_f) + xcol0;
-                for (int32_t j = jlo + lane; j < jhi; j += 32) {
-                    const uint32_t rel = (uint32_t)(j - j_base);
-                    const uint32_t e = rel < (uint32_t)kP6StageEntries ? estage[rel] : __ldg(p.esc + j);
-                    const uint32_t idx = ((e & 0xFFFu) - s64) & 0xFFFu;   // column relative to block sb
-                    const float xv = __uint_as_float((uint32_t)__bfloat16_as_ushort(xm[idx]) << 16);
-                    const float wv = __uint_as_float(e & 0xFFFF0000u);
-                    float *a = oacc + ((e >> 12) & 15u) * 32u + lane;
-                    *a = fmaf(wv, xv, *a);
+            const uint32_t s64 = (sb & 63u) << 6;
+            const __nv_bfloat16 *xm = (XS ? xs : x) + (sb - R * KB) * kTileCols;
+            float before[8];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                before[i] = c[i];
+                before[4 + i] = c1[i];
+            }
+            outlier_steps(s64, xm, jlo, jhi, P6Flag<false>());
+            // the sum of the absolute values is NaN or infinite if one of the eight is
+            const float all = fabsf(c[0]) + fabsf(c[1]) + fabsf(c[2]) + fabsf(c[3]) + fabsf(c1[0]) + fabsf(c1[1]) + fabsf(c1[2]) + fabsf(c1[3]);
+            if (__any_sync(0xffffffffu, !(all < INFINITY))) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    c[i] = before[i];
+                    c1[i] = before[4 + i];
                 }
-                __syncwarp();
-                const uint32_t row = lane & 15, half = lane >> 4;
-                float v[16];
-#pragma unroll
-                for (int jj = 0; jj < 16; ++jj)                           // conflict free: rows rotate through the banks
-                    v[jj] = oacc[row * 32u + half * 16u + ((jj + row) & 15u)];
-#pragma unroll
-                for (int jj = 0; jj < 16; ++jj) oacc[row * 32u + half * 16u + ((jj + row) & 15u)] = 0.f;
-                float s = 0.f;
-#pragma unroll
-                for (int jj = 0; jj < 16; ++jj) s += v[jj];
-                s += __shfl_xor_sync(0xffffffffu, s, 16);
-                const float v0 = __shfl_sync(0xffffffffu, s, g), v1 = __shfl_sync(0xffffffffu, s, g + 8);
-                if ((uint32_t)t == (m >> 1)) {
-                    if (m & 1u) { c[1] += v0; c[3] += v1; }
-                    else { c[0] += v0; c[2] += v1; }
-                }
-                __syncwarp();
+                outlier_steps(s64, xm, jlo, jhi, P6Flag<true>());
             }
         };
 
@@ -822,7 +891,13 @@ k_p6_mma(P6 p, const __nv_bfloat16 *__restrict__ x, uint32_t m_rows, const __nv_
             }
             if (whole) p6_store_tile(push, push_e, p.out_f, R, lane, c, m_rows, bias, y, y_f32);
             else {
-                wparts[(R == R_first ? 0 : 32) + lane] = make_float4(c[0], c[1], c[2], c[3]);
+                unsigned char *part = wsm + SM::kParts + (R == R_first ? 0 : SM::kPart);
+                if (MULTI) {
+                    ((float4 *)part)[lane] = make_float4(c[0], c[1], c[2], c[3]);
+                } else if (t == 0) {
+                    ((float *)part)[g] = c[0];
+                    ((float *)part)[g + 8] = c[2];
+                }
                 if (fast_tail) tile_arrive(R);
             }
             c[0] = c[1] = c[2] = c[3] = 0.f;

@@ -210,14 +210,9 @@ k_p6_gemm(P6 p, const __nv_bfloat16 *__restrict__ x, uint32_t m_tok, float *__re
         const uint32_t b_first = (have ? R : 0u) * KB + kb0;         // block of i = 0
         constexpr uint32_t kStep = kPgPhases;                        // this warp's blocks are kStep apart
         const unsigned char *n16 = p.plane + (size_t)(b_first + ph3) * kP6BlockBytes + lane * 16;
-        uint32_t e2, b2, c2;
-        {
-            const float s32 = 32.f * __bfloat162float(p.scale[(have ? R : 0u) * p.scale_stride]);
-            const uint32_t bb = (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(s32));
-            b2 = bb | (bb << 16);
-            c2 = b2 ^ 0x80008000u;
-            asm volatile("mov.b32 %0, 0x3F003F00;" : "=r"(e2));
-        }
+        uint32_t e2;
+        const uint32_t s2 = p6_scale2(p.scale[(have ? R : 0u) * p.scale_stride]);
+        asm volatile("mov.b32 %0, 0x42804280;" : "=r"(e2));
         // outlier bookkeeping: lane l keeps blk_off[b_first + win + l]; a block's entries are requested two of this
         // warp's blocks ahead
         uint32_t win = 0;
@@ -272,17 +267,7 @@ k_p6_gemm(P6 p, const __nv_bfloat16 *__restrict__ x, uint32_t m_tok, float *__re
                 const uint4 a = p6_lds128(d16 + cs);
                 const uint2 a2 = p6_lds64(d8 + cs);
                 const uint32_t w[6] = {a.x, a.y, a.z, a.w, a2.x, a2.y};
-#pragma unroll
-                for (int k = 0; k < 6; ++k) {
-                    f[2 * k] = p6_pair(w[k] << 2, e2, b2, c2);
-                    f[2 * k + 1] = p6_pair(w[k] >> 4, e2, b2, c2);
-                }
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    uint32_t v = p6_and_or(w[q] >> 10, 0x003C003Cu, e2);
-                    v = p6_and_or(w[4 + (q >> 1)] >> (6 + 2 * (q & 1)), 0x00C000C0u, v);
-                    asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(f[12 + q]) : "r"(v), "r"(b2), "r"(c2));
-                }
+                p6_unpack(w, e2, s2, f);
                 is = cs;
                 cs = cs == (uint32_t)(3 * kP6BlockBytes) ? 0u : cs + (uint32_t)kP6BlockBytes;
             }

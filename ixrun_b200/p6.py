@@ -2,9 +2,9 @@
 
 The (3,5,8) streams remain the interchange format; ``P6Packed.from_packed``
 transcodes them on the GPU, keeping every int8 code.  P6 spends 6 plane bits per weight on a field that *is* part of the
-bf16 number ``1 + code/32`` (codes -16..31), so one fused multiply-add per pair
-of weights yields the reference's ``bf16(code * scale)``; every other code goes
-to a short list that the GEMV adds on the CUDA cores.
+bf16 number ``96 + code`` (codes -32..31), so a subtraction and a multiplication
+per pair of weights yield the reference's ``bf16(code * scale)``; every other code goes
+to a short list.
 """
 from __future__ import annotations
 
@@ -26,7 +26,7 @@ def set_pdl(on: bool) -> bool:
     the device has been synchronised: a layout still being built would be read too early."""
     return bool(_lib.lib().ixb_set_pdl(1 if on else 0))
 
-CODE_MIN, CODE_MAX = -16, 31     # codes that the plane holds
+CODE_MIN, CODE_MAX = -32, 31     # codes that the plane holds
 SLACK_BLOCKS, SLACK_ENTRIES, BLOCK_BYTES = 5, 64, 768
 
 

@@ -209,7 +209,7 @@ def test_p6_fused_tensor_gives_every_part_its_own_result(in_f, rows):
 @pytest.mark.parametrize("out_f,in_f,m", [(128, 512, 16), (16, 1024, 64), (40, 5120, 33), (100, 1024, 9), (300, 512, 64),
                                           (512, 5120, 64), (1000, 2176, 17), (3, 3072, 1), (2048, 2048, 32)])
 def test_p6_gemm_small_m_against_the_oracle(out_f, in_f, m):
-    """tcgen05 GEMM on the resident layout (1..64 rows) against the oracle's fp32 result; bias, bf16 output and
+    """GEMM on the resident layout (1..64 rows) against the oracle's fp32 result; bias, bf16 output and
     repeatability; within fp32 summation-order rounding of the GEMV for the rows both take."""
     codes, scale, p6 = make(out_f, in_f, out_f * 3 + m)
     sc_bits = int(scale.view(torch.int16).item()) & 0xFFFF
@@ -242,3 +242,47 @@ def test_p6_gemm_full_size(out_f, in_f, m):
     err = float((y.double() - ref).abs().max() / ref.abs().max())
     assert err < 2e-5, err
     assert torch.equal(p6.gemm(x), y.bfloat16())
+
+
+@pytest.mark.parametrize("out_f,in_f,dense", [(48, 6464, False), (48, 6464, True), (16, 64, True), (2500, 96, True), (5120, 320, False)])
+def test_p6_gemv_rows_get_the_bits_they_get_alone(out_f, in_f, dense):
+    """Outliers go through the tensor core 32 at a time for all activation rows: runs of more than 64 blocks, more steps
+    than blocks (every second code an outlier), segments shorter than the pipeline, several row tiles per run; up to 8
+    rows, with activations in shared memory and (wide rows) from global memory.  Against float64 sums of exact products."""
+    from ixrun_b200.p6 import P6Packed
+
+    gen = torch.Generator(device="cuda").manual_seed(out_f + in_f)
+    codes = (torch.randn(out_f, in_f, generator=gen, device="cuda") * (40 if dense else 12)).round().clamp(-127, 127).to(torch.int8)
+    p6 = P6Packed(codes, torch.tensor(0.007, dtype=torch.bfloat16), out_f, in_f)
+    x = torch.randn(8, in_f, generator=gen, device="cuda").bfloat16()
+    ref = x.double() @ (codes.float() * p6.scale.float()).bfloat16().double().t()
+    alone = torch.cat([p6.gemv(x[i:i + 1], out_dtype=torch.float32) for i in range(8)])
+    assert float((alone.double() - ref).abs().max() / ref.abs().max()) < 2e-5
+    for m in (2, 3, 7, 8):
+        assert torch.equal(p6.gemv(x[:m], out_dtype=torch.float32), alone[:m])
+
+
+def test_p6_gemv_infinite_activation_reaches_only_its_rows():
+    """An infinite activation in one of three rows: the other rows keep their bits, and a weight row without an outlier in
+    that column gets what the dense product gives (an infinity of the weight's sign, NaN for weight 0)."""
+    from ixrun_b200.p6 import P6Packed
+
+    gen = torch.Generator(device="cuda").manual_seed(2)
+    out_f, in_f, col = 64, 256, 77
+    codes = torch.randint(1, 32, (out_f, in_f), generator=gen, device="cuda").to(torch.int8)
+    codes[::2] = -torch.randint(1, 17, (out_f // 2, in_f), generator=gen, device="cuda").to(torch.int8)
+    codes[5, col], codes[21, col], codes[3, 5], codes[8, col] = 100, -90, 120, 0
+    p6 = P6Packed(codes, torch.tensor(0.01, dtype=torch.bfloat16), out_f, in_f)
+    x = torch.randn(3, in_f, generator=gen, device="cuda").bfloat16()
+    clean = p6.gemv(x)
+    x[1, col] = float("inf")
+    y = p6.gemv(x)
+    assert torch.equal(y[0], clean[0]) and torch.equal(y[2], clean[2])
+    for got in (y[1], p6.gemv(x[1:2])[0]):
+        for r in range(out_f):
+            if r in (5, 21):
+                assert not bool(torch.isfinite(got[r]))               # an outlier there: not finite either
+            elif r == 8:
+                assert bool(torch.isnan(got[r]))
+            else:
+                assert bool(torch.isinf(got[r])) and bool(got[r] > 0) == bool(codes[r, col] > 0), r
