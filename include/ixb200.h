@@ -358,6 +358,12 @@ int ixb_attn_decode(const void *q_device, const void *k_cache_device, const void
                     const void *gate_device, int64_t gate_stride, void *out_device, void *scratch_device, size_t scratch_bytes,
                     int64_t hq, int64_t hkv, int64_t head_dim, int64_t splits, float scale, int64_t batch, int64_t q_stride,
                     int64_t batch_stride, int64_t gate_row_stride, ixb_stream_t stream);
+/* Causal attention of `rows` new rows of one sequence (positions pos0 .. pos0 + rows - 1, keys and values already in the
+ * caches [max_seq][hkv][head_dim]): out [rows][hq][head_dim] = softmax(scale * q.k) v over positions 0 .. pos0 + row.
+ * q [rows] with row pitch q_stride elements (a multiple of 8), heads contiguous; head_dim 64 or 128; 16-byte aligned. */
+int ixb_attn_prefill(const void *q_device, const void *k_cache_device, const void *v_cache_device, void *out_device,
+                     int64_t rows, int64_t pos0, int64_t hq, int64_t hkv, int64_t head_dim, float scale, int64_t q_stride,
+                     int64_t max_seq, ixb_stream_t stream);
 int ixb_conv_update(const void *x_device, void *state_device, const void *w_device, const void *bias_device, void *y_device,
                     int64_t channels, int64_t k, ixb_stream_t stream);
 int ixb_gdn_step(const void *qkv_device, const void *z_device, const void *a_device, const void *b_device,

@@ -5,6 +5,7 @@
 #include <cuda_fp16.h>
 #include "ixb_common.cuh"
 #include "ixb_gemm_tc.cuh"
+#include "ixb_attn_prefill.cuh"
 #include "ixb_p6_gemm.cuh"
 #include "ixb_pack.cuh"
 #include "ixb_p6.cuh"
@@ -1386,6 +1387,44 @@ extern "C" int ixb_attn_decode(const void *q, const void *k_cache, const void *v
     IXB_GLUE("k_attn_combine", launch_glue(k_attn_combine, dim3((unsigned)hq, (unsigned)batch), dim3(threads), st, (const float *)scratch,
                                            (__nv_bfloat16 *)out, (const __nv_bfloat16 *)gate, (uint32_t)splits, (uint32_t)head_dim,
                                            (uint32_t)gate_stride, (uint32_t)gate_row_stride));
+}
+
+template <int D>
+static cudaError_t launch_attn_prefill(const void *q, const void *k_cache, const void *v_cache, void *out, int64_t rows,
+                                       int64_t pos0, int64_t hq, int64_t hkv, float scale, int64_t q_stride, cudaStream_t st)
+{
+    static bool attr_set[64] = {false};
+    cudaError_t e = opt_in_smem(k_attn_prefill<D>, attr_set, (int)ap_smem_bytes<D>());
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)((rows + kApRows - 1) / kApRows), (unsigned)hq);
+    cfg.blockDim = dim3(kApThreads);
+    cfg.dynamicSmemBytes = ap_smem_bytes<D>();
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = g_p6_pdl.load() ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, k_attn_prefill<D>, (const __nv_bfloat16 *)q, (const __nv_bfloat16 *)k_cache,
+                              (const __nv_bfloat16 *)v_cache, (__nv_bfloat16 *)out, (uint32_t)rows, (uint32_t)pos0, (uint32_t)hq,
+                              (uint32_t)hkv, scale, (uint32_t)q_stride);
+}
+
+extern "C" int ixb_attn_prefill(const void *q, const void *k_cache, const void *v_cache, void *out, int64_t rows, int64_t pos0,
+                                int64_t hq, int64_t hkv, int64_t head_dim, float scale, int64_t q_stride, int64_t max_seq,
+                                ixb_stream_t stream)
+{
+    if (!q || !k_cache || !v_cache || !out) return fail(IXB_E_ARG, "NULL pointer argument");
+    if (rows <= 0 || pos0 < 0 || pos0 + rows > max_seq || max_seq > 0x7fffffffLL || hq <= 0 || hq > 65535 || hkv <= 0 || hq % hkv)
+        return fail(IXB_E_ARG, "bad shape");
+    if (head_dim != 64 && head_dim != 128) return fail(IXB_E_UNSUPPORTED, "head_dim=%lld: 64 or 128", (long long)head_dim);
+    if (q_stride < hq * head_dim || q_stride > 0x7fffffffLL || (q_stride & 7)) return fail(IXB_E_ARG, "bad row pitch");
+    if (((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)out) & 15u)
+        return fail(IXB_E_ARG, "q, caches or output are not 16-byte aligned");
+    cudaStream_t st = (cudaStream_t)stream;
+    IXB_GLUE("k_attn_prefill", head_dim == 64 ? launch_attn_prefill<64>(q, k_cache, v_cache, out, rows, pos0, hq, hkv, scale, q_stride, st)
+                                              : launch_attn_prefill<128>(q, k_cache, v_cache, out, rows, pos0, hq, hkv, scale, q_stride, st));
 }
 
 extern "C" int ixb_conv_update(const void *x, void *state, const void *w, const void *bias, void *y, int64_t channels,

@@ -11,7 +11,7 @@ import torch
 
 from . import _lib
 
-__all__ = ["gdn_conv_step", "add_rmsnorm", "finish_add_rmsnorm", "swiglu", "rope_kv", "AttnDecode", "conv_update", "gdn_step", "rope_tables"]
+__all__ = ["gdn_conv_step", "add_rmsnorm", "finish_add_rmsnorm", "swiglu", "rope_kv", "AttnDecode", "attn_prefill", "conv_update", "gdn_step", "rope_tables"]
 
 
 def _st(t):
@@ -154,6 +154,27 @@ class AttnDecode:
                                                   self.splits, float(scale if scale is not None else self.d ** -0.5), b,
                                                   q_stride or 0, batch_stride, gate_row_stride, _st(q)))
         return out
+
+
+def attn_prefill(q, k_cache, v_cache, pos0: int, hq: int, hkv: int, head_dim: int, out=None, scale: float | None = None):
+    """Causal attention of the rows of q [rows, >= hq*head_dim] (column slices allowed), which sit at positions pos0 + row
+    of the sequence in the caches [max_seq, hkv, head_dim] (their keys and values are in them already); head_dim 64 or
+    128; returns out [rows, hq*head_dim]."""
+    _bf16(k_cache, v_cache)
+    rows, cols, pitch = _rows_view(q, "q")
+    if cols < hq * head_dim or k_cache.shape[-2:] != (hkv, head_dim) or k_cache.shape != v_cache.shape:
+        raise ValueError("q is [rows, >= hq*head_dim], caches are [max_seq, hkv, head_dim]")
+    if out is None:
+        out = torch.empty(rows, hq * head_dim, dtype=torch.bfloat16, device=q.device)
+    elif out.numel() != rows * hq * head_dim:
+        raise ValueError("out must be [rows, hq*head_dim]")
+    _bf16(out)
+    with torch.cuda.device(q.device):
+        _lib.check(_lib.lib().ixb_attn_prefill(q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(), rows,
+                                               int(pos0), hq, hkv, head_dim,
+                                               float(scale if scale is not None else head_dim ** -0.5), pitch,
+                                               k_cache.shape[-3], _st(q)))
+    return out
 
 
 def conv_update(x, state, w, bias=None, out=None):

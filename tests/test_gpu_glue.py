@@ -97,6 +97,30 @@ def test_rope_kv_and_attention(hq, hkv, d, rot, norm):
     close(out, vc[0].float().repeat_interleave(rep, dim=0).reshape(-1), BF16_ULP)
 
 
+@pytest.mark.parametrize("rows,pos0", [(1, 0), (1, 90), (63, 0), (64, 64), (65, 0), (200, 37)])
+@pytest.mark.parametrize("hq,hkv,d", [(4, 2, 64), (3, 3, 128), (6, 1, 128)])
+def test_attn_prefill(hq, hkv, d, rows, pos0):
+    """Row and key tiles of 64: one row, one short of a tile, a whole one, one more; from the start and behind a context.
+    Bound: the bf16 output is off by at most half a unit in the last place, 2^-8 of the value (8 significant bits; the
+    value may sit at the bottom of its binade); probabilities of 17 bits that sum to 1 add 2^-17 of the largest value, the
+    fp32 exponentials and sums less than 2^-17 of it."""
+    from ixrun_b200.glue import attn_prefill
+
+    max_seq, dev = pos0 + rows + 30, "cuda"
+    qkv = torch.randn(rows, (hq + 2 * hkv) * d, device=dev).bfloat16()        # q is a column slice of a wider matrix
+    kc = torch.randn(max_seq, hkv, d, device=dev).bfloat16()
+    vc = torch.randn(max_seq, hkv, d, device=dev).bfloat16()
+    out = attn_prefill(qkv[:, :hq * d], kc, vc, pos0, hq, hkv, d)
+    n = pos0 + rows
+    q = qkv[:, :hq * d].double().view(rows, hkv, hq // hkv, d)
+    s = torch.einsum("rghd,sgd->rghs", q, kc[:n].double()) * d ** -0.5
+    mask = torch.arange(n, device=dev)[None, :] <= pos0 + torch.arange(rows, device=dev)[:, None]
+    p = s.masked_fill(~mask[:, None, None, :], -torch.inf).softmax(-1)
+    ref = torch.einsum("rghs,sgd->rghd", p, vc[:n].double()).reshape(rows, hq * d)
+    err = (out.double() - ref).abs()
+    assert (err <= ref.abs() * BF16_ULP + 2.0 ** -16 * vc.abs().max()).all(), float(err.max())
+
+
 def test_conv_update():
     from ixrun_b200.glue import conv_update
 
