@@ -1385,7 +1385,7 @@ extern "C" int ixb_attn_decode(const void *q, const void *k_cache, const void *v
     if (rc) return rc;
     const unsigned threads = (unsigned)std::max<int64_t>(head_dim, (splits + 31) / 32 * 32);
     IXB_GLUE("k_attn_combine", launch_glue(k_attn_combine, dim3((unsigned)hq, (unsigned)batch), dim3(threads), st, (const float *)scratch,
-                                           (__nv_bfloat16 *)out, (const __nv_bfloat16 *)gate, (uint32_t)splits, (uint32_t)head_dim,
+                                           (__nv_bfloat16 *)out, (const __nv_bfloat16 *)gate, pos, (uint32_t)splits, (uint32_t)head_dim,
                                            (uint32_t)gate_stride, (uint32_t)gate_row_stride));
 }
 

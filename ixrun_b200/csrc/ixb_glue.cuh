@@ -286,11 +286,20 @@ k_rope_kv(__nv_bfloat16 *q, const __nv_bfloat16 *__restrict__ k, const __nv_bflo
 // ---------------------------------------------------------------- single-query attention over the static cache
 // grid (groups, splits), 256 threads (8 warps).  A group is G consecutive query heads that share one KV head
 // (G = query heads per KV head, or 1): the K and V rows of a position are loaded once and used for all G heads.
-// The context [0, n_ctx) (n_ctx = pos[0] + 1) is cut into `splits` contiguous ranges; a warp walks its share of a range
+// The context [0, n_ctx) (n_ctx = pos[0] + 1) is cut into contiguous ranges, one per CTA: at most `splits` of them, and
+// none shorter than kAttnMinRange positions (attn_ranges; the CTAs beyond have nothing to do).  A short range is all
+// fixed cost -- joining the CTA's partial states -- so forty sequences of 150 to 300 positions cut 18 ways took 84 us a
+// layer; the number of ranges depends on the sequence alone, so it gets the same bits alone or in a batch.  A warp walks its share of a range
 // PPW positions at a time: D / 8 lanes hold 8 elements each of a position's K and V rows (one 16-byte load each, the
 // next iteration's rows requested before this one's arithmetic), a shuffle tree gives the G scores, and every
 // lane keeps a running maximum, denominator and weighted V sum per head (online softmax).  The CTA's warps are joined
 // in shared memory; the split's (maximum, denominator, sum[D]) per head goes to `part`; k_attn_combine joins the splits.
+constexpr uint32_t kAttnMinRange = 64;                 // positions: what the 8 warps of a CTA have in flight for D = 128
+__device__ __forceinline__ uint32_t attn_ranges(uint32_t n_ctx, uint32_t splits)
+{
+    return min(splits, (n_ctx + kAttnMinRange - 1u) / kAttnMinRange);
+}
+
 template <int D, int G>
 __global__ void __launch_bounds__(256)
 k_attn_decode(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat16 *__restrict__ k_cache,
@@ -305,7 +314,7 @@ k_attn_decode(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat16 *__restri
     part += (size_t)blockIdx.z * hq * gridDim.y * (D + 2);
     constexpr int LPP = D / 8;                         // lanes per position
     constexpr int PPW = 32 / LPP;                      // positions per warp iteration
-    constexpr int NS = 8 * PPW;                        // partial states per head in the CTA
+    constexpr int NS = 8;                              // partial states per head in the CTA: one per warp
     __shared__ float sm_m[G][NS], sm_l[G][NS];
     __shared__ float sm_acc[NS][D];                    // one head at a time
     asm volatile("griddepcontrol.launch_dependents;");
@@ -314,8 +323,9 @@ k_attn_decode(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat16 *__restri
     const uint32_t kvh = head0 / (hq / hkv);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int sub = lane / LPP, li = lane % LPP;       // which of the warp's positions, which 8 elements
-    const uint32_t n_ctx = (uint32_t)pos[0] + 1u;
-    const uint32_t per = (n_ctx + splits - 1) / splits, p0 = split * per, p1 = min(p0 + per, n_ctx);
+    const uint32_t n_ctx = (uint32_t)pos[0] + 1u, used = attn_ranges(n_ctx, splits);
+    if (split >= used) return;
+    const uint32_t per = (n_ctx + used - 1) / used, p0 = split * per, p1 = min(p0 + per, n_ctx);
     float qv[G][8];
 #pragma unroll
     for (int h = 0; h < G; ++h) {
@@ -384,20 +394,33 @@ k_attn_decode(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat16 *__restri
             }
         }
     }
-    // join the NS partial states of the CTA, head by head
-    const int slot = wid * PPW + sub;
-    if (li == 0) {
+    // join the warp's PPW partial states in registers, then the NS states of the CTA, head by head
+#pragma unroll
+    for (int h = 0; h < G; ++h) {
+#pragma unroll
+        for (int d = LPP; d < 32; d <<= 1) {
+            const float mo = __shfl_xor_sync(0xffffffffu, m[h], d), mn = fmaxf(m[h], mo);
+            const float c = m[h] == -INFINITY ? 0.f : __expf(m[h] - mn), co = mo == -INFINITY ? 0.f : __expf(mo - mn);
+            l[h] = l[h] * c + __shfl_xor_sync(0xffffffffu, l[h], d) * co;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) acc[h][j] = acc[h][j] * c + __shfl_xor_sync(0xffffffffu, acc[h][j], d) * co;
+            m[h] = mn;
+        }
+    }
+    if (lane == 0) {
 #pragma unroll
         for (int h = 0; h < G; ++h) {
-            sm_m[h][slot] = m[h];
-            sm_l[h][slot] = l[h];
+            sm_m[h][wid] = m[h];
+            sm_l[h][wid] = l[h];
         }
     }
 #pragma unroll
     for (int h = 0; h < G; ++h) {
         __syncthreads();                               // sm_acc is free (and, first time, sm_m / sm_l are written)
+        if (sub == 0) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) sm_acc[slot][li * 8 + j] = acc[h][j];
+            for (int j = 0; j < 8; ++j) sm_acc[wid][li * 8 + j] = acc[h][j];
+        }
         __syncthreads();
         float M = -INFINITY;
 #pragma unroll
@@ -424,20 +447,21 @@ k_attn_decode(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat16 *__restri
 // The splits' maxima and denominators are fetched by one thread each, the weighted sums with independent loads.
 constexpr int kAttnMaxSplits = 256;
 __global__ void __launch_bounds__(256)
-k_attn_combine(const float *__restrict__ part, __nv_bfloat16 *out, const __nv_bfloat16 *__restrict__ gate, uint32_t splits,
-               uint32_t D, uint32_t gate_stride, uint32_t gate_row_stride)
+k_attn_combine(const float *__restrict__ part, __nv_bfloat16 *out, const __nv_bfloat16 *__restrict__ gate, const int32_t *pos,
+               uint32_t max_splits, uint32_t D, uint32_t gate_stride, uint32_t gate_row_stride)
 {
     __shared__ float wgt[kAttnMaxSplits], red[32];
     asm volatile("griddepcontrol.launch_dependents;");
     const uint32_t head = blockIdx.x, t = threadIdx.x;
     // blockIdx.y: the sequence
-    part += (size_t)blockIdx.y * gridDim.x * splits * (D + 2);
+    part += (size_t)blockIdx.y * gridDim.x * max_splits * (D + 2);
     out += (size_t)blockIdx.y * gridDim.x * D;
     if (gate) gate += (size_t)blockIdx.y * gate_row_stride;
     float gv = 0.f;
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (gate && t < D) gv = bf2f(gate[(size_t)head * gate_stride + t]);
-    const float *p = part + (size_t)head * splits * (D + 2);
+    const uint32_t splits = attn_ranges((uint32_t)pos[blockIdx.y] + 1u, max_splits);
+    const float *p = part + (size_t)head * max_splits * (D + 2);
     float ms = -INFINITY, ls = 0.f;
     if (t < splits) {
         const float2 ml = *(const float2 *)(p + (size_t)t * (D + 2));
