@@ -134,14 +134,15 @@ class StreamingLinear(nn.Module):
 
     def forward(self, x):
         rows = x.numel() // self.in_features
-        if self._res is not None and x.dtype == torch.bfloat16 and 1 <= rows <= FUSED_MAX_ROWS \
-                and x.shape[-1] == self.in_features:
-            y = self._res.gemv(x.reshape(rows, self.in_features), bias=self._bias_bf16)
-            return y.view(x.shape[:-1] + (self.out_features,))
-        if self._res is not None and self._use_p6_gemm and x.dtype == torch.bfloat16 and rows <= TC_MAX_ROWS \
-                and self.in_features % 64 == 0 and x.shape[-1] == self.in_features:
-            y = self._res.gemm(x.reshape(rows, self.in_features), bias=self._bias_bf16)
-            return y.view(x.shape[:-1] + (self.out_features,))
+        res = self._res
+        if res is not None and x.dtype == torch.bfloat16 and x.shape[-1] == self.in_features and rows <= TC_MAX_ROWS:
+            y = None
+            if 1 <= rows <= FUSED_MAX_ROWS:
+                y = res.gemv(x, bias=self._bias_bf16)
+            elif self._use_p6_gemm and self.in_features % 64 == 0:
+                y = res.gemm(x, bias=self._bias_bf16)
+            if y is not None:
+                return y if x.dim() == 2 else y.view(x.shape[:-1] + (self.out_features,))
         if self._use_fused and x.dtype == torch.bfloat16 and 1 <= rows <= FUSED_MAX_ROWS \
                 and x.shape[-1] == self.in_features:
             y = self._dp.gemv(x.reshape(rows, self.in_features), bias=self._bias_bf16)

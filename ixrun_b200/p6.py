@@ -93,6 +93,9 @@ class P6Packed:
                                         self.blk_off.data_ptr(), self.esc.data_ptr(), n_esc, st))
         self.struct = _lib.P6Struct(self.plane.data_ptr(), self.blk_off.data_ptr(), self.esc.data_ptr(), n_esc,
                                     self.scale.data_ptr(), self.out_f, self.in_f, stride)
+        self._ref = C.byref(self.struct)             # (keeps the struct alive)
+        self._index = dev.index
+        self._gemv_need = None
         self.resident_bytes = nb * BLOCK_BYTES + 4 * (nb + 1 + n_esc) + 2
         self.scratch = scratch if scratch is not None else GemvScratch.shared(dev)
 
@@ -144,33 +147,43 @@ class P6Packed:
         flat = out.reshape(-1)
         if flat.dtype != dtype or flat.numel() < self.N or not flat.is_contiguous():
             raise ValueError("decode output must be a contiguous tensor of the right dtype and size")
-        with torch.cuda.device(self.device):
-            _lib.check(_lib.lib().ixb_p6_decode(C.byref(self.struct), flat.data_ptr(), 0 if kind == "codes" else 1,
-                                                _lib.stream_ptr(self.device)))
+        with _lib.on_device(self._index) as stream:
+            _lib.check(_lib.lib().ixb_p6_decode(self._ref, flat.data_ptr(), 0 if kind == "codes" else 1, stream))
         return flat[: self.N].view(self.out_f, self.in_f)
+
+    def _rows(self, x: torch.Tensor) -> torch.Tensor:
+        """x as contiguous bf16 rows [M, in_f]"""
+        if x.dtype != torch.bfloat16:
+            raise ValueError("activations must be bf16")
+        if x.dim() != 2 or x.shape[1] != self.in_f:
+            x = x.reshape(-1, self.in_f)
+        return x if x.is_contiguous() else x.contiguous()
+
+    def _out(self, m: int, out, out_dtype, bias, what: str) -> torch.Tensor:
+        if bias is not None and (bias.dtype != torch.bfloat16 or bias.numel() != self.out_f):
+            raise ValueError("bias must be bf16 [out_f]")
+        if out is None:
+            return torch.empty(m, self.out_f, dtype=out_dtype, device=self.device)
+        if out.dtype not in (torch.bfloat16, torch.float32) or out.numel() != m * self.out_f or not out.is_contiguous():
+            raise ValueError(f"{what} output must be a contiguous bf16/fp32 tensor of M*out_f elements")
+        return out
 
     def gemv(self, x: torch.Tensor, bias: torch.Tensor | None = None, out: torch.Tensor | None = None,
              out_dtype=torch.bfloat16) -> torch.Tensor:
         """y[M, out_f] = x[M, in_f] @ W.T, 1 <= M <= 8."""
-        if x.dtype != torch.bfloat16:
-            raise ValueError("activations must be bf16")
-        x2 = x.reshape(-1, self.in_f)
-        if not x2.is_contiguous():
-            x2 = x2.contiguous()
+        x2 = self._rows(x)
         m = x2.shape[0]
-        if out is None:
-            out = torch.empty(m, self.out_f, dtype=out_dtype, device=self.device)
-        elif out.dtype not in (torch.bfloat16, torch.float32) or out.numel() != m * self.out_f or not out.is_contiguous():
-            raise ValueError("gemv output must be a contiguous bf16/fp32 tensor of M*out_f elements")
-        if bias is not None and (bias.dtype != torch.bfloat16 or bias.numel() != self.out_f):
-            raise ValueError("bias must be bf16 [out_f]")
+        out = self._out(m, out, out_dtype, bias, "gemv")
         L = _lib.lib()
-        with torch.cuda.device(self.device):
-            s = self.scratch.reserve(L.ixb_p6_gemv_scratch_bytes(self.out_f, self.in_f, m))
-            _lib.check(L.ixb_p6_gemv(C.byref(self.struct), x2.data_ptr(), m,
-                                     None if bias is None else bias.data_ptr(), out.data_ptr(),
-                                     1 if out.dtype == torch.float32 else 0, s.data_ptr(), s.numel(),
-                                     _lib.stream_ptr(self.device)))
+        with _lib.on_device(self._index) as stream:
+            # the plan, and with it the scratch, depends on the shape alone
+            if self._gemv_need is None:
+                self._gemv_need = int(L.ixb_p6_gemv_scratch_bytes(self.out_f, self.in_f, 1))
+            s = self.scratch.reserve(self._gemv_need)
+            rc = L.ixb_p6_gemv(self._ref, x2.data_ptr(), m, None if bias is None else bias.data_ptr(), out.data_ptr(),
+                               1 if out.dtype == torch.float32 else 0, s.data_ptr(), s.numel(), stream)
+        if rc:
+            _lib.check(rc)
         return out
 
     GEMM_MAX_ROWS = 64
