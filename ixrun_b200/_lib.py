@@ -142,6 +142,8 @@ def lib():
     L.ixb_allreduce_finish_add_rmsnorm.argtypes = [C.POINTER(C.c_void_p), C.c_int, C.c_int, i64, vp, vp, f32, vp, i64, i64, vp]
     L.ixb_p6_gemm_scratch_bytes.restype = sz
     L.ixb_p6_gemm_scratch_bytes.argtypes = [i64, i64, i64]
+    L.ixb_p6_rows.restype = C.c_int
+    L.ixb_p6_rows.argtypes = [C.POINTER(P6Struct), vp, i64, vp, vp, C.c_int, vp]
     L.ixb_p6_gemm.restype = C.c_int
     L.ixb_p6_gemm.argtypes = [C.POINTER(P6Struct), vp, i64, vp, vp, C.c_int, vp, sz, vp]
     L.ixb_tpab_decode.restype = C.c_int

@@ -6,7 +6,7 @@
 #include "ixb_common.cuh"
 #include "ixb_gemm_tc.cuh"
 #include "ixb_attn_prefill.cuh"
-#include "ixb_p6_gemm.cuh"
+#include "ixb_p6_rows.cuh"
 #include "ixb_pack.cuh"
 #include "ixb_p6.cuh"
 #include "ixb_allreduce.cuh"
@@ -1519,63 +1519,114 @@ extern "C" int ixb_gemm(const ixb_packed *w, const int32_t *blk_q1, const int32_
 }
 
 // ------------------------------------------------ small-M GEMM on the resident P6 layout
-static PgPlan make_pg_plan(uint32_t out_f, uint32_t in_f)
+// The kernel's variants: n-tiles of eight activation rows, parts of K and stages per CTA (ixb_p6_rows.cuh).  Up to 32 rows
+// four parts (16 warps) fit the registers, more rows need the accumulators of three parts' worth.
+struct PrVariant {
+    void (*kernel)(P6, const __nv_bfloat16 *, uint32_t, const __nv_bfloat16 *, void *, int, uint32_t);
+    uint32_t nt, parts, smem;
+};
+template <int NT, int PARTS, int STAGES>
+static constexpr PrVariant pr_variant() { return {k_p6_rows<NT, PARTS, STAGES>, NT, PARTS, PrSmem<NT, PARTS, STAGES>::kBytes}; }
+static const PrVariant kPrVariants[] = {pr_variant<2, 4, 4>(), pr_variant<3, 4, 4>(), pr_variant<4, 4, 4>(),
+                                        pr_variant<5, 3, 4>(), pr_variant<6, 3, 4>(), pr_variant<8, 3, 4>()};
+constexpr int kPrVariantCount = sizeof(kPrVariants) / sizeof(kPrVariants[0]);
+constexpr int kPrMaxSplits = 8;                          // CTAs of a portable cluster
+
+// CTAs of variant v that run at once in clusters of s, on the current device
+static int pr_resident(int v, int s, int *out)
 {
-    PgPlan p;
-    const uint32_t rt = (out_f + kTileRows - 1) / kTileRows, kb = (in_f + kTileCols - 1) / kTileCols;
-    p.groups = (rt + kPgConv - 1) / kPgConv;
-    int dev = 0, sms = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    // K is split only as far as it takes to give about every SM one CTA; a split keeps at least eight column blocks
-    uint32_t splits = std::max<uint32_t>(1u, (uint32_t)sms / p.groups);
-    splits = std::min<uint32_t>(splits, std::max<uint32_t>(1u, kb / 8u));
-    p.splits = std::min<uint32_t>(splits, 16u);
-    p.grid = p.groups * p.splits;
-    return p;
+    static std::atomic<int> cached[64][kPrVariantCount][kPrMaxSplits + 1];
+    static bool attr_set[kPrVariantCount][64];
+    int dev = 0;
+    IXB_CUDA(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64) return fail(IXB_E_UNSUPPORTED, "device ordinal %d outside 0..63", dev);
+    IXB_CUDA(opt_in_smem(kPrVariants[v].kernel, attr_set[v], (int)kPrVariants[v].smem));
+    int n = cached[dev][v][s].load();
+    if (!n) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)(s * 148));
+        cfg.blockDim = dim3(kPrVariants[v].parts * 128u);
+        cfg.dynamicSmemBytes = kPrVariants[v].smem;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)s;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int clusters = 0;
+        IXB_CUDA(cudaOccupancyMaxActiveClusters(&clusters, kPrVariants[v].kernel, &cfg));
+        n = std::max(1, clusters * s);
+        cached[dev][v][s].store(n);
+    }
+    *out = n;
+    return IXB_OK;
+}
+
+// K splits (CTAs of a cluster) for a row count: the fewest rounds of steps over the whole grid.  A step is one column block
+// per part, about 0.6 us; joining the splits' sums through distributed shared memory costs about two of them.
+static int pr_splits(const P6 &p, int v, uint32_t *splits)
+{
+    const uint32_t groups = (p.rt + kPrTiles - 1) / kPrTiles, parts = kPrVariants[v].parts;
+    uint32_t best = 0;
+    for (uint32_t s = 1; s <= (uint32_t)kPrMaxSplits && s <= p.kb; ++s) {
+        int resident = 0, rc = pr_resident(v, (int)s, &resident);
+        if (rc) return rc;
+        const uint32_t rounds = (groups * s + (uint32_t)resident - 1) / (uint32_t)resident;
+        const uint32_t steps = ((p.kb + s - 1) / s + parts - 1) / parts;
+        const uint32_t cost = rounds * (steps + 4u + (s > 1u ? 2u : 0u));
+        if (!best || cost < best) {
+            best = cost;
+            *splits = s;
+        }
+    }
+    return IXB_OK;
 }
 
 extern "C" size_t ixb_p6_gemm_scratch_bytes(int64_t out_f, int64_t in_f, int64_t m_rows)
 {
-    if (out_f <= 0 || in_f <= 0 || m_rows < 1 || m_rows > kPgTok || out_f * in_f > 800000000LL) return 0;
-    PgPlan p = make_pg_plan((uint32_t)out_f, (uint32_t)in_f);
-    return 256 + (size_t)p.splits * (size_t)m_rows * (size_t)out_f * sizeof(float);
+    if (out_f <= 0 || in_f <= 0 || m_rows < 1 || m_rows > kPrMaxRows || out_f * in_f > 800000000LL) return 0;
+    return 256;                                          // (sums of K splits stay in shared memory)
 }
 
 extern "C" int ixb_p6_gemm(const ixb_p6 *t, const void *x, int64_t m_rows, const void *bias, void *y, int y_is_f32,
                            void *scratch, size_t scratch_bytes, ixb_stream_t stream)
 {
+    if (!t || !x || !y || !scratch) return fail(IXB_E_ARG, "NULL pointer argument");
+    if (t->in_f % kTileCols) return fail(IXB_E_UNSUPPORTED, "in_f=%lld is not a multiple of %d", (long long)t->in_f, kTileCols);
+    if ((uintptr_t)scratch & 255u) return fail(IXB_E_ARG, "scratch is not 256-byte aligned");
+    if (scratch_bytes < 256u) return fail(IXB_E_SCRATCH, "gemm scratch too small");
+    return ixb_p6_rows(t, x, m_rows, bias, y, y_is_f32, stream);
+}
+
+extern "C" int ixb_p6_rows(const ixb_p6 *t, const void *x, int64_t m_rows, const void *bias, void *y, int y_is_f32,
+                           ixb_stream_t stream)
+{
     P6 p;
     int rc = to_p6(t, &p);
     if (rc) return rc;
-    if (!x || !y || !scratch) return fail(IXB_E_ARG, "NULL pointer argument");
-    if (m_rows < 1 || m_rows > kPgTok) return fail(IXB_E_UNSUPPORTED, "m_rows=%lld outside 1..%d", (long long)m_rows, kPgTok);
-    if (p.in_f % (uint32_t)kTileCols) return fail(IXB_E_UNSUPPORTED, "in_f=%u is not a multiple of %d", p.in_f, kTileCols);
+    if (!x || !y) return fail(IXB_E_ARG, "NULL pointer argument");
+    if (m_rows < 1 || m_rows > kPrMaxRows) return fail(IXB_E_UNSUPPORTED, "m_rows=%lld outside 1..%d", (long long)m_rows, kPrMaxRows);
+    if (p.in_f % 8u) return fail(IXB_E_UNSUPPORTED, "in_f=%u is not a multiple of 8", p.in_f);
     if ((uintptr_t)x & 15u) return fail(IXB_E_ARG, "x is not 16-byte aligned");
-    if ((uintptr_t)scratch & 255u) return fail(IXB_E_ARG, "scratch is not 256-byte aligned");
-    if (scratch_bytes < ixb_p6_gemm_scratch_bytes(p.out_f, p.in_f, m_rows)) return fail(IXB_E_SCRATCH, "gemm scratch too small");
-    PgPlan plan = make_pg_plan(p.out_f, p.in_f);
-    cudaStream_t st = (cudaStream_t)stream;
-    static bool attr_set[64] = {false};
-    IXB_CUDA(opt_in_smem(k_p6_gemm, attr_set, (int)kPgSmemBytes));
-    uint32_t *err = (uint32_t *)scratch;
-    float *part = (float *)((char *)scratch + 256);
+    int v = 0;
+    while (kPrVariants[v].nt * 8u < (uint32_t)m_rows) ++v;
+    uint32_t splits = 1;
+    if ((rc = pr_splits(p, v, &splits))) return rc;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(plan.grid);
-    cfg.blockDim = dim3(kPgThreads);
-    cfg.dynamicSmemBytes = kPgSmemBytes;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.gridDim = dim3((p.rt + kPrTiles - 1) / kPrTiles * splits);
+    cfg.blockDim = dim3(kPrVariants[v].parts * 128u);
+    cfg.dynamicSmemBytes = kPrVariants[v].smem;
+    cfg.stream = (cudaStream_t)stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = splits;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = g_p6_pdl.load() ? 1 : 0;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, k_p6_gemm, p, (const __nv_bfloat16 *)x, (uint32_t)m_rows, part, err, plan);
-    if (e != cudaSuccess) return fail(IXB_E_CUDA, "k_p6_gemm launch: %s", cudaGetErrorString(e));
-    if ((rc = launch_check("k_p6_gemm"))) return rc;
-    uint32_t total = (uint32_t)m_rows * p.out_f;
-    IXB_GLUE("k_gemm_finalize", launch_glue(k_gemm_finalize, dim3((total + 255) / 256), dim3(256), st, (const float *)part,
-                                            plan.splits, (uint32_t)m_rows, p.out_f, (const __nv_bfloat16 *)bias, y, y_is_f32,
-                                            (const uint32_t *)err));
+    cfg.numAttrs = g_p6_pdl.load() ? 2 : 1;
+    IXB_GLUE("k_p6_rows", cudaLaunchKernelEx(&cfg, kPrVariants[v].kernel, p, (const __nv_bfloat16 *)x, (uint32_t)m_rows,
+                                             (const __nv_bfloat16 *)bias, y, y_is_f32, splits));
 }
 
 // ------------------------------------------------ gemv without caller scratch

@@ -26,6 +26,8 @@ __all__ = ["Int8XEngine", "StreamingLinear", "GraphLinear", "ResourceScheduler",
 
 FUSED_MAX_ROWS = 8        # rows served by the CUDA-core fused kernel
 TC_MAX_ROWS = 64          # rows served by the tensor-core fused kernel (when enabled)
+# Rows served in passes of the same kernel, without a bias (decode + dense matmul adds it before the one rounding).
+PASSES_MAX_ROWS = 128
 
 
 class StreamingLinear(nn.Module):
@@ -135,12 +137,14 @@ class StreamingLinear(nn.Module):
     def forward(self, x):
         rows = x.numel() // self.in_features
         res = self._res
-        if res is not None and x.dtype == torch.bfloat16 and x.shape[-1] == self.in_features and rows <= TC_MAX_ROWS:
+        if res is not None and x.dtype == torch.bfloat16 and x.shape[-1] == self.in_features and rows <= PASSES_MAX_ROWS:
             y = None
             if 1 <= rows <= FUSED_MAX_ROWS:
                 y = res.gemv(x, bias=self._bias_bf16)
-            elif self._use_p6_gemm and self.in_features % 64 == 0:
+            elif self._use_p6_gemm and rows <= TC_MAX_ROWS and self.in_features % 64 == 0:
                 y = res.gemm(x, bias=self._bias_bf16)
+            elif self._use_p6_gemm and rows > FUSED_MAX_ROWS and self._bias is None and self.in_features % 8 == 0:
+                y = res.rows(x)
             if y is not None:
                 return y if x.dim() == 2 else y.view(x.shape[:-1] + (self.out_features,))
         if self._use_fused and x.dtype == torch.bfloat16 and 1 <= rows <= FUSED_MAX_ROWS \

@@ -191,30 +191,36 @@ class P6Packed:
     def gemm(self, x: torch.Tensor, bias: torch.Tensor | None = None, out: torch.Tensor | None = None,
              out_dtype=torch.bfloat16) -> torch.Tensor:
         """y[M, out_f] = x[M, in_f] @ W.T for 1 <= M <= 64 on the tensor cores, reading the resident layout once
-        (in_f a multiple of 64).  The scratch (split-K partial sums) is kept per tensor shape on this object."""
-        if x.dtype != torch.bfloat16:
-            raise ValueError("activations must be bf16")
-        x2 = x.reshape(-1, self.in_f)
-        if not x2.is_contiguous():
-            x2 = x2.contiguous()
+        (in_f a multiple of 64)."""
+        x2 = self._rows(x)
         m = x2.shape[0]
-        if out is None:
-            out = torch.empty(m, self.out_f, dtype=out_dtype, device=self.device)
-        elif out.dtype not in (torch.bfloat16, torch.float32) or out.numel() != m * self.out_f or not out.is_contiguous():
-            raise ValueError("gemm output must be a contiguous bf16/fp32 tensor of M*out_f elements")
-        if bias is not None and (bias.dtype != torch.bfloat16 or bias.numel() != self.out_f):
-            raise ValueError("bias must be bf16 [out_f]")
-        L = _lib.lib()
-        need = int(L.ixb_p6_gemm_scratch_bytes(self.out_f, self.in_f, m))
-        if need == 0:
+        out = self._out(m, out, out_dtype, bias, "gemm")
+        if not 1 <= m <= self.GEMM_MAX_ROWS:
             raise ValueError(f"unsupported GEMM shape: {m} rows")
-        ws = getattr(self, "_gemm_ws", None)
-        if ws is None or ws.numel() < need:
-            ws = self._gemm_ws = torch.empty(need, dtype=torch.uint8, device=self.device)
-        with torch.cuda.device(self.device):
-            _lib.check(L.ixb_p6_gemm(C.byref(self.struct), x2.data_ptr(), m, None if bias is None else bias.data_ptr(),
-                                     out.data_ptr(), 1 if out.dtype == torch.float32 else 0, ws.data_ptr(), ws.numel(),
-                                     _lib.stream_ptr(self.device)))
+        L = _lib.lib()
+        with _lib.on_device(self._index) as stream:
+            s = self.scratch.reserve(256)                # (checked, not used: the splits' sums stay in shared memory)
+            rc = L.ixb_p6_gemm(self._ref, x2.data_ptr(), m, None if bias is None else bias.data_ptr(), out.data_ptr(),
+                               1 if out.dtype == torch.float32 else 0, s.data_ptr(), s.numel(), stream)
+        if rc:
+            _lib.check(rc)
+        return out
+
+    def rows(self, x: torch.Tensor) -> torch.Tensor:
+        """y[M, out_f] = x[M, in_f] @ W.T in bf16 for any M >= 1 and in_f a multiple of 8, up to 64 rows per pass over the
+        resident layout."""
+        x2 = self._rows(x)
+        m = x2.shape[0]
+        out = self._out(m, None, torch.bfloat16, None, "gemm")
+        passes = -(-m // self.GEMM_MAX_ROWS)
+        step = -(-(-(-m // passes)) // 8) * 8            # even passes of whole groups of eight rows
+        L = _lib.lib()
+        with _lib.on_device(self._index) as stream:
+            for r in range(0, m, step):
+                rc = L.ixb_p6_rows(self._ref, x2.data_ptr() + 2 * r * self.in_f, min(step, m - r), None,
+                                   out.data_ptr() + 2 * r * self.out_f, 0, stream)
+                if rc:
+                    _lib.check(rc)
         return out
 
     def gemv_push(self, x: torch.Tensor, ar) -> int:

@@ -244,6 +244,30 @@ def test_p6_gemm_full_size(out_f, in_f, m):
     assert torch.equal(p6.gemm(x), y.bfloat16())
 
 
+@pytest.mark.parametrize("m", [9, 16, 17, 24, 25, 33, 40, 41, 48, 49, 64])
+@pytest.mark.parametrize("out_f,in_f,outliers", [(129, 64, False), (272, 192, True), (2064, 2240, False)])
+def test_p6_gemm_row_counts(out_f, in_f, outliers, m):
+    """Every variant of the kernel at the edges of its row counts; one column block, three (a part without work), 35 over
+    several splits; a last row group of one tile; blocks with up to 800 outliers.  fp32 against float64 sums of exact
+    products: the metric and bound of the tests above."""
+    from ixrun_b200.p6 import P6Packed
+
+    gen = torch.Generator(device="cuda").manual_seed(out_f + m)
+    if outliers:
+        codes = torch.randint(-127, 128, (out_f, in_f), generator=gen, device="cuda").to(torch.int8)
+    else:
+        codes = (torch.randn(out_f, in_f, generator=gen, device="cuda") * 12).round().clamp(-127, 127).to(torch.int8)
+    p6 = P6Packed(codes, torch.tensor(0.007, dtype=torch.bfloat16), out_f, in_f)
+    x = torch.randn(m, in_f, generator=gen, device="cuda").bfloat16()
+    w = p6.decode(kind="bf16").double()
+    assert torch.equal(w, (codes.float() * p6.scale.float()).bfloat16().double())
+    ref = x.double() @ w.t()
+    y = p6.gemm(x, out_dtype=torch.float32)
+    assert float((y.double() - ref).abs().max() / ref.abs().max()) < 2e-5
+    bias = torch.randn(out_f, generator=gen, device="cuda").bfloat16()
+    assert torch.equal(p6.gemm(x, bias=bias), y.bfloat16() + bias)
+
+
 @pytest.mark.parametrize("out_f,in_f,dense", [(48, 6464, False), (48, 6464, True), (16, 64, True), (2500, 96, True), (5120, 320, False)])
 def test_p6_gemv_rows_get_the_bits_they_get_alone(out_f, in_f, dense):
     """Outliers go through the tensor core 32 at a time for all activation rows: runs of more than 64 blocks, more steps
