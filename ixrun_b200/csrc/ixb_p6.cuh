@@ -367,6 +367,9 @@ struct P6Push {
     uint32_t *done;               // scratch word counting finished warps, zero between launches
 };
 
+template <bool V>
+struct P6Flag { static constexpr bool value = V; };
+
 // one output (activation row m, weight row `row`): to y (+ bias), or as a marked word to every rank
 __device__ __forceinline__ void p6_put_out(const P6Push &push, uint32_t e, uint32_t out_f, uint32_t m, uint32_t row, float v,
                                            const __nv_bfloat16 *__restrict__ bias, void *y, int y_f32)
