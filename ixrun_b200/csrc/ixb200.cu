@@ -1328,6 +1328,16 @@ extern "C" int ixb_rope_kv(void *q, const void *k, const void *v, const int32_t 
     if (rows <= 0 || hq <= 0 || hkv <= 0 || max_seq <= 0) return fail(IXB_E_ARG, "bad shape");
     if (head_dim != 64 && head_dim != 128 && head_dim != 256) return fail(IXB_E_UNSUPPORTED, "head_dim=%lld: 64, 128 or 256", (long long)head_dim);
     if (rot_dim <= 0 || rot_dim > head_dim || (rot_dim & 1)) return fail(IXB_E_ARG, "rot_dim must be even and at most head_dim");
+    if (!q_norm && !k_norm && rot_dim == head_dim && ((q_stride | kv_stride | batch_stride) & 7) == 0 &&
+        (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)cos_tab | (uintptr_t)sin_tab) & 15u) == 0 &&
+        rows * (hq + hkv) <= (1LL << 26)) {
+        const int64_t threads = rows * (hq + hkv) * (head_dim / 16);
+        IXB_GLUE("k_rope_kv8", launch_glue(k_rope_kv8, dim3((unsigned)((threads + 127) / 128)), dim3(128), (cudaStream_t)stream,
+                                           (__nv_bfloat16 *)q, (const __nv_bfloat16 *)k, (const __nv_bfloat16 *)v, pos,
+                                           (__nv_bfloat16 *)k_cache, (__nv_bfloat16 *)v_cache, cos_tab, sin_tab, (uint32_t)rows,
+                                           (uint32_t)hq, (uint32_t)hkv, (uint32_t)head_dim, (uint32_t)q_stride, (uint32_t)max_seq,
+                                           (uint32_t)kv_stride, (size_t)batch_stride));
+    }
     IXB_GLUE("k_rope_kv", launch_glue(k_rope_kv, dim3((unsigned)rows, (unsigned)(hq + hkv)), dim3((unsigned)(head_dim / 2)), (cudaStream_t)stream,
                                       (__nv_bfloat16 *)q, (const __nv_bfloat16 *)k, (const __nv_bfloat16 *)v, pos,
                                       (__nv_bfloat16 *)k_cache, (__nv_bfloat16 *)v_cache, (const __nv_bfloat16 *)q_norm,
@@ -1397,7 +1407,7 @@ static cudaError_t launch_attn_prefill(const void *q, const void *k_cache, const
     cudaError_t e = opt_in_smem(k_attn_prefill<D>, attr_set, (int)ap_smem_bytes<D>());
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)((rows + kApRows - 1) / kApRows), (unsigned)hq);
+    cfg.gridDim = dim3((unsigned)hq, (unsigned)((rows + kApRows - 1) / kApRows));
     cfg.blockDim = dim3(kApThreads);
     cfg.dynamicSmemBytes = ap_smem_bytes<D>();
     cfg.stream = st;
@@ -1416,7 +1426,7 @@ extern "C" int ixb_attn_prefill(const void *q, const void *k_cache, const void *
                                 ixb_stream_t stream)
 {
     if (!q || !k_cache || !v_cache || !out) return fail(IXB_E_ARG, "NULL pointer argument");
-    if (rows <= 0 || pos0 < 0 || pos0 + rows > max_seq || max_seq > 0x7fffffffLL || hq <= 0 || hq > 65535 || hkv <= 0 || hq % hkv)
+    if (rows <= 0 || pos0 < 0 || pos0 + rows > max_seq || max_seq > 0x7fffffffLL || rows > 65535LL * kApRows || hq <= 0 || hkv <= 0 || hq % hkv)
         return fail(IXB_E_ARG, "bad shape");
     if (head_dim != 64 && head_dim != 128) return fail(IXB_E_UNSUPPORTED, "head_dim=%lld: 64 or 128", (long long)head_dim);
     if (q_stride < hq * head_dim || q_stride > 0x7fffffffLL || (q_stride & 7)) return fail(IXB_E_ARG, "bad row pitch");

@@ -3,21 +3,23 @@
 // 0 .. pos0 + r.  The eager path runs this as fp32 matmuls around a masked softmax over the whole static cache.
 //
 // Bound: the tensor core (4 MMA steps of 16 x 8 x 16 per 16 x 8 scores and head dimension 16: one for Q K^T, two for
-// P V), far from it in practice because a 1000-row prompt has only 256 CTAs of work; the cache rows of a KV head come
-// from L2.  CTA = 64 rows of one query head, 4 warps of 16 rows; keys and values in tiles of 64 through two cp.async
-// stages; the row tiles with the longest contexts start first.  Q K^T: bf16 operands, fp32 sums.  The probabilities stay
-// fp32-like: p = hi + lo with two bf16 numbers (17 significant bits) and two MMAs, so nothing is lost against the fp32
-// path; the denominator is summed from the fp32 values.
-// Measured (1000 rows, 16 query / 8 KV heads of 128): see the figures at ixb_attn_prefill.
+// P V): a 1000-row prompt's 16 x 136 pairs of 64-row and 64-key tiles of 16 heads are 12.6 us at mma.sync's rate.  What it
+// has to fight is the chain of key tiles of the last rows and the uneven lengths: CTA = 64 rows of one query head, two
+// groups of four warps (16 rows a warp) take the even and the odd key tiles, each through its own two cp.async stages, and
+// join at the end; the row tiles with the longest contexts of all heads start first.  Q K^T: bf16 operands, fp32 sums.  The
+// probabilities stay fp32-like: p = hi + lo with two bf16 numbers (17 significant bits) and two MMAs, so nothing is lost
+// against the fp32 path; the denominator is summed from the fp32 values.
+// Measured (1000 rows, 16 query / 8 KV heads of 128, under the profiler): 50 us with one group per CTA and the heads one
+// after the other.
 #pragma once
 #include "ixb_p6.cuh"
 
 namespace ixb {
 
-constexpr int kApRows = 64, kApKeys = 64, kApThreads = 128;
+constexpr int kApRows = 64, kApKeys = 64, kApGroup = 128, kApThreads = 2 * kApGroup;
 
 template <int D>
-constexpr uint32_t ap_smem_bytes() { return (uint32_t)(kApRows + 4 * kApKeys) * (D + 8) * 2u; }   // Q, two stages of K and V
+constexpr uint32_t ap_smem_bytes() { return (uint32_t)(kApRows + 8 * kApKeys) * (D + 8) * 2u; }   // Q, two groups' two stages of K and V
 
 __device__ __forceinline__ void ap_ldmatrix_t(uint32_t (&r)[4], uint32_t addr)
 {
@@ -29,7 +31,7 @@ __device__ __forceinline__ uint32_t ap_pack(float lo, float hi)
     return (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(lo)) | (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(hi)) << 16;
 }
 
-// grid (row tiles, query heads)
+// grid (query heads, row tiles)
 template <int D>
 __global__ void __launch_bounds__(kApThreads)
 k_attn_prefill(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat16 *__restrict__ k_cache,
@@ -40,29 +42,31 @@ k_attn_prefill(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat16 *__restr
     constexpr int CH = D / 8;                          // 16-byte chunks per row
     extern __shared__ __align__(128) unsigned char ap_smem[];
     const uint32_t s0 = (uint32_t)__cvta_generic_to_shared(ap_smem);
-    const uint32_t sq = s0, sk = s0 + kApRows * PITCH * 2u, stage_bytes = 2u * kApKeys * PITCH * 2u, sv = sk + kApKeys * PITCH * 2u;
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, g = lane >> 2, t = lane & 3;
-    const uint32_t head = blockIdx.y, kvh = head / (hq / hkv);
-    const uint32_t r0 = (gridDim.x - 1u - blockIdx.x) * kApRows;       // longest contexts first
+    const uint32_t stage_bytes = 2u * kApKeys * PITCH * 2u;
+    const int tid = threadIdx.x & (kApGroup - 1), lane = tid & 31, wid = tid >> 5, g = lane >> 2, t = lane & 3;
+    const uint32_t kg = threadIdx.x / kApGroup;        // the group: key tiles kg, kg + 2, ...
+    const uint32_t sq = s0, sk = s0 + kApRows * PITCH * 2u + kg * 2u * stage_bytes, sv = sk + kApKeys * PITCH * 2u;
+    const uint32_t head = blockIdx.x, kvh = head / (hq / hkv);
+    const uint32_t r0 = (gridDim.y - 1u - blockIdx.y) * kApRows;       // longest contexts first
     asm volatile("griddepcontrol.launch_dependents;");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const uint32_t n_keys = pos0 + min(r0 + (uint32_t)kApRows, T);     // keys that any row of the tile sees
     const uint32_t n_tiles = (n_keys + kApKeys - 1) / kApKeys;
     const size_t row_stride = (size_t)hkv * D;
-    for (int c = tid; c < kApRows * CH; c += kApThreads) {
+    for (int c = threadIdx.x; c < kApRows * CH; c += kApThreads) {
         const uint32_t r = c / CH, ch = c % CH;
         p6_cp16(sq + (r * PITCH + ch * 8u) * 2u, q + (size_t)min(r0 + r, T - 1u) * q_stride + (size_t)head * D + ch * 8u);
     }
     auto fetch = [&](uint32_t kt) {                                     // rows beyond the last key repeat it (masked below)
-        const uint32_t st = (kt & 1u) * stage_bytes;
-        for (int c = tid; c < kApKeys * CH; c += kApThreads) {
+        const uint32_t st = (kt >> 1 & 1u) * stage_bytes;
+        for (int c = tid; c < kApKeys * CH; c += kApGroup) {
             const uint32_t r = c / CH, ch = c % CH;
             const size_t at = (size_t)min(kt * kApKeys + r, n_keys - 1u) * row_stride + (size_t)kvh * D + ch * 8u;
             p6_cp16(sk + st + (r * PITCH + ch * 8u) * 2u, k_cache + at);
             p6_cp16(sv + st + (r * PITCH + ch * 8u) * 2u, v_cache + at);
         }
     };
-    fetch(0);
+    if (kg < n_tiles) fetch(kg);
     cp_async_commit();
     cp_async_wait<0>();
     __syncthreads();
@@ -76,10 +80,10 @@ k_attn_prefill(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat16 *__restr
     float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
     const float sl2 = scale * 1.4426950408889634f;     // scores in units of log2: probabilities are powers of two
     const uint32_t p_lo = pos0 + r0 + wid * 16 + g;    // position of the lane's first row (the second is 8 further)
-    for (uint32_t kt = 0; kt < n_tiles; ++kt) {
-        if (kt + 1 < n_tiles) fetch(kt + 1);           // the other stage: its readers passed the barrier below
+    for (uint32_t kt = kg; kt < n_tiles; kt += 2) {
+        if (kt + 2 < n_tiles) fetch(kt + 2);           // the other stage: its readers passed the barrier below
         cp_async_commit();
-        const uint32_t st = (kt & 1u) * stage_bytes;
+        const uint32_t st = (kt >> 1 & 1u) * stage_bytes;
         float s[kApKeys / 8][4];
 #pragma unroll
         for (int n = 0; n < kApKeys / 8; ++n) s[n][0] = s[n][1] = s[n][2] = s[n][3] = 0.f;
@@ -147,18 +151,39 @@ k_attn_prefill(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat16 *__restr
             }
         }
         cp_async_wait<0>();
-        __syncthreads();                                // the next stage has landed, this one is free
+        asm volatile("bar.sync %0, %1;" ::"r"(kg + 1u), "n"(kApGroup) : "memory");    // the group's next stage has landed, this one is free
     }
+    // the odd tiles' group hands its sums over through its own stages
+    constexpr int OP = D + 4;                          // floats per row
+    float *xo = (float *)(ap_smem + kApRows * PITCH * 2 + 2 * stage_bytes), *xm = xo + kApRows * OP, *xl = xm + kApRows;
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
         l[h] += __shfl_xor_sync(0xffffffffu, l[h], 1);
         l[h] += __shfl_xor_sync(0xffffffffu, l[h], 2);
-        const uint32_t row = r0 + wid * 16 + g + 8 * h;
+        if (kg == 1) {
+            const uint32_t r = wid * 16 + g + 8 * h;
+#pragma unroll
+            for (int n = 0; n < D / 8; ++n) *(float2 *)(xo + r * OP + n * 8 + 2 * t) = make_float2(o[n][2 * h], o[n][2 * h + 1]);
+            if (t == 0) {
+                xm[r] = m[h];
+                xl[r] = l[h];
+            }
+        }
+    }
+    __syncthreads();
+    if (kg == 1) return;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const uint32_t r = wid * 16 + g + 8 * h, row = r0 + r;
         if (row >= T) continue;
-        const float inv = 1.f / l[h];
+        const float m1 = xm[r], mn = fmaxf(m[h], m1), mb = mn == -INFINITY ? 0.f : mn;
+        const float f0 = exp2f(m[h] - mb), f1 = exp2f(m1 - mb), inv = 1.f / (l[h] * f0 + xl[r] * f1);
         __nv_bfloat16 *dst = out + ((size_t)row * hq + head) * D + 2 * t;
 #pragma unroll
-        for (int n = 0; n < D / 8; ++n) *(uint32_t *)(dst + n * 8) = ap_pack(o[n][2 * h] * inv, o[n][2 * h + 1] * inv);
+        for (int n = 0; n < D / 8; ++n) {
+            const float2 v = *(const float2 *)(xo + r * OP + n * 8 + 2 * t);
+            *(uint32_t *)(dst + n * 8) = ap_pack((o[n][2 * h] * f0 + v.x * f1) * inv, (o[n][2 * h + 1] * f0 + v.y * f1) * inv);
+        }
     }
 }
 

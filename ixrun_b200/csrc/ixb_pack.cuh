@@ -48,11 +48,15 @@ __device__ __forceinline__ int code_level(int c)
     return a <= 3 ? 0 : (a <= 15 ? 1 : 2);
 }
 
-__device__ __forceinline__ int quantise_code(uint32_t bf16_bits, float sc)
+// code = clamp(rint(w / sc)), the division rounded to fp32 as the reference does.  w * (1 / sc) is within 2^-22 of the
+// quotient, which for |code| < 128 is 3e-5: away from the halves between two codes both round to the same code, and only
+// near them (or beyond 128, infinite, NaN, a scale without a reciprocal) the division itself is taken.
+__device__ __forceinline__ int quantise_code(uint32_t bf16_bits, float sc, float inv)
 {
-    float q = rintf(__fdiv_rn(__uint_as_float(bf16_bits << 16), sc));
-    q = fminf(fmaxf(q, -127.f), 127.f);
-    return (int)q;
+    const float w = __uint_as_float(bf16_bits << 16);
+    float q = w * inv, n = rintf(q);
+    if (!(fabsf(q - n) < 0.499f && fabsf(q) < 128.f)) n = rintf(__fdiv_rn(w, sc));
+    return (int)fminf(fmaxf(n, -127.f), 127.f);
 }
 
 // One warp per 1024-element block.  MODE 0: quantise from bf16 weights and write codes; MODE 1: read existing codes.
@@ -68,10 +72,11 @@ k_codes_and_counts(const uint16_t *__restrict__ w, const uint32_t *absmax_bits, 
     uint32_t b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     int lane = threadIdx.x & 31;
     if (b >= nb) return;
-    float sc = 1.f;
+    float sc = 1.f, inv = 1.f;
     if (MODE == 0) {
         __nv_bfloat16 s = scale_from_absmax(*absmax_bits);
         sc = __bfloat162float(s);
+        inv = __frcp_rn(sc);
         if (b == 0 && lane == 0) *scale_out = s;
     }
     uint32_t n1 = 0, n2 = 0;
@@ -94,7 +99,7 @@ k_codes_and_counts(const uint16_t *__restrict__ w, const uint32_t *absmax_bits, 
             for (int i = 0; i < 8; ++i) {
                 int c;
                 if (MODE == 0) {
-                    c = quantise_code((wr[i >> 1] >> (16 * (i & 1))) & 0xffffu, sc);
+                    c = quantise_code((wr[i >> 1] >> (16 * (i & 1))) & 0xffffu, sc, inv);
                     co[i >> 2] |= (uint32_t)(c & 0xff) << (8 * (i & 3));
                 } else {
                     c = (int)(int8_t)(cr[i >> 2] >> (8 * (i & 3)));
@@ -114,7 +119,7 @@ k_codes_and_counts(const uint16_t *__restrict__ w, const uint32_t *absmax_bits, 
         for (uint32_t i = 0; i < 32u && e0 + i < n; ++i) {
             int c;
             if (MODE == 0) {
-                c = quantise_code(w[e0 + i], sc);
+                c = quantise_code(w[e0 + i], sc, inv);
                 codes[e0 + i] = (int8_t)c;
             } else {
                 c = codes[e0 + i];
@@ -132,25 +137,19 @@ k_codes_and_counts(const uint16_t *__restrict__ w, const uint32_t *absmax_bits, 
     if (lane == 0) { cnt1[b] = (int32_t)n1; cnt2[b] = (int32_t)n2; }
 }
 
-// fields of one stream, put down one after the other into a warp's image of the stream's words: whole words and the two
-// ends that neighbouring lanes share go in with a shared-memory OR
-struct FieldWriter {
-    uint32_t *img;                // word of the next bit
-    uint64_t buf;
-    uint32_t fill;
-    __device__ __forceinline__ FieldWriter(uint32_t *image, uint32_t bit) : img(image + (bit >> 5)), buf(0), fill(bit & 31u) {}
-    __device__ __forceinline__ void put(uint32_t v, uint32_t width)
-    {
-        buf |= (uint64_t)v << fill;
-        fill += width;
-        if (fill >= 32u) {
-            atomicOr(img++, (uint32_t)buf);
-            buf >>= 32;
-            fill -= 32u;
-        }
+// a lane's bits of one stream (NW words, the first bit lowest, zero beyond its end) into the warp's image at bit `bit`
+template <int NW>
+__device__ __forceinline__ void or_bits(uint32_t *image, uint32_t bit, const uint32_t (&v)[NW])
+{
+    uint32_t *at = image + (bit >> 5);
+    uint32_t carry = 0;
+#pragma unroll
+    for (int k = 0; k <= NW; ++k) {
+        const uint32_t cur = k < NW ? v[k] : 0u, word = __funnelshift_l(carry, cur, bit & 31u);
+        if (word) atomicOr(at + k, word);
+        carry = cur;
     }
-    __device__ __forceinline__ void flush() { if (fill) atomicOr(img, (uint32_t)buf); }
-};
+}
 
 // The block's words of one stream (bits [bit0, bit1) of it, image word 0 = stream word bit0 / 32) to memory: the first and
 // the last may be shared with the neighbouring blocks.
@@ -164,9 +163,11 @@ __device__ __forceinline__ void write_image(uint32_t *stream, const uint32_t *im
     }
 }
 
-// Streams must be zero on entry.  One warp per block, lane = word of 32 elements; the block's part of every stream is put
-// together in shared memory and written in whole words (one global atomic per field, before: 104 us for 5120 x 5120).
-constexpr int kPackB2 = 0, kPackL1 = 34, kPackL2 = 132, kPackWords = 296;    // 33, 97 and 162 words at most
+// Streams must be zero on entry.  One warp per block, lane = word of 32 elements.  Bound by instructions: a lane runs its
+// elements backwards and shifts every field in at the low end of its own bits (3 words of level 1, 5 of level 2, one of
+// the second bitmap), with predicates and no branches but for the rare level 3; the lanes' bits meet in an image of the
+// block's words in shared memory, which is written in whole words.  5120 x 5120: 104 us with one global atomic per field.
+constexpr int kPackB2 = 0, kPackL1 = 36, kPackL2 = 140, kPackWords = 308;    // 33, 97 and 161 words at most
 __global__ void __launch_bounds__(256)
 k_pack(const int8_t *__restrict__ codes, uint32_t n, const int32_t *__restrict__ a_blk, const int32_t *__restrict__ c_blk,
        uint32_t *b2, uint32_t *l1, uint32_t *l2, uint8_t *l3)
@@ -199,6 +200,7 @@ k_pack(const int8_t *__restrict__ codes, uint32_t n, const int32_t *__restrict__
         m1 |= (uint32_t)(lv == 0) << i;
         e2 |= (uint32_t)(lv == 1) << i;
     }
+    const uint32_t nl = ~m1 & (valid == 32u ? 0xffffffffu : (1u << valid) - 1u);     // not level 1
     const uint32_t a0 = (uint32_t)a_blk[b], c0 = (uint32_t)c_blk[b], r0 = b * kBlk - a0;    // the block's first ranks
     const uint32_t i1 = warp_incl_scan(__popc(m1), lane), i2 = warp_incl_scan(__popc(e2), lane);
     const uint32_t a1 = a0 + __shfl_sync(0xffffffffu, i1, 31), c1 = c0 + __shfl_sync(0xffffffffu, i2, 31);
@@ -206,25 +208,30 @@ k_pack(const int8_t *__restrict__ codes, uint32_t n, const int32_t *__restrict__
     uint32_t a = a0 + i1 - __popc(m1), cc = c0 + i2 - __popc(e2);
     uint32_t r = min(e0, n) - a;  // rank among non-L1 elements
     uint32_t t = r - cc;
-    FieldWriter w1(img + kPackL1, 3u * a - (3u * a0 & ~31u)), w2(img + kPackL2, 5u * cc - (5u * c0 & ~31u)),
-        wb(img + kPackB2, r - (r0 & ~31u));
-    __syncwarp();                                        // the image is zero
+    // levels 1 and 2 and the second bitmap, from the last element to the first
+    uint32_t v1[3] = {0, 0, 0}, v2[5] = {0, 0, 0, 0, 0}, vb[1] = {0};
 #pragma unroll
-    for (int i = 0; i < 32; ++i) {
-        if ((uint32_t)i >= valid) break;
-        const int c = (int)(int8_t)(cw[i >> 2] >> (8 * (i & 3)));
+    for (int i = 31; i >= 0; --i) {
+        const uint32_t c = (cw[i >> 2] >> (8 * (i & 3))) & 0xffu;       // the code modulo 256
         if ((m1 >> i) & 1u) {
-            w1.put((uint32_t)(c + 3), 3u);
-        } else {
-            const uint32_t two = (e2 >> i) & 1u;
-            wb.put(two, 1u);
-            if (two) w2.put((uint32_t)(c + 15), 5u);
-            else l3[t++] = (uint8_t)(c + 127);
+            v1[2] = __funnelshift_l(v1[1], v1[2], 3);
+            v1[1] = __funnelshift_l(v1[0], v1[1], 3);
+            v1[0] = v1[0] << 3 | ((c + 3u) & 7u);
+        }
+        if ((nl >> i) & 1u) vb[0] = vb[0] << 1 | ((e2 >> i) & 1u);
+        if ((e2 >> i) & 1u) {
+            v2[4] = __funnelshift_l(v2[3], v2[4], 5);
+            v2[3] = __funnelshift_l(v2[2], v2[3], 5);
+            v2[2] = __funnelshift_l(v2[1], v2[2], 5);
+            v2[1] = __funnelshift_l(v2[0], v2[1], 5);
+            v2[0] = v2[0] << 5 | ((c + 15u) & 31u);
         }
     }
-    w1.flush();
-    w2.flush();
-    wb.flush();
+    __syncwarp();                                        // the image is zero
+    or_bits(img + kPackL1, 3u * a - (3u * a0 & ~31u), v1);
+    or_bits(img + kPackL2, 5u * cc - (5u * c0 & ~31u), v2);
+    or_bits(img + kPackB2, r - (r0 & ~31u), vb);
+    for (uint32_t left = nl & ~e2; left; left &= left - 1u) l3[t++] = (uint8_t)(codes[e0 + __ffs((int)left) - 1] + 127);
     __syncwarp();
     write_image(l1, img + kPackL1, 3u * a0, 3u * a1, lane);
     write_image(l2, img + kPackL2, 5u * c0, 5u * c1, lane);
