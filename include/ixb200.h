@@ -361,6 +361,14 @@ int ixb_attn_decode(const void *q_device, const void *k_cache_device, const void
                     const void *gate_device, int64_t gate_stride, void *out_device, void *scratch_device, size_t scratch_bytes,
                     int64_t hq, int64_t hkv, int64_t head_dim, int64_t splits, float scale, int64_t batch, int64_t q_stride,
                     int64_t batch_stride, int64_t gate_row_stride, ixb_stream_t stream);
+/* ixb_attn_decode in one launch: the last CTA of a head group joins the context's parts.  tickets: batch * hq words, zero
+ * before the first call, left zero by every call (a buffer of its own for launches that may overlap); max_seq: rows of
+ * every cache, whose contents beyond the position are read but not used. */
+int ixb_attn_decode_join(const void *q_device, const void *k_cache_device, const void *v_cache_device, const int32_t *pos_device,
+                         const void *gate_device, int64_t gate_stride, void *out_device, void *scratch_device,
+                         size_t scratch_bytes, void *tickets_device, int64_t hq, int64_t hkv, int64_t head_dim, int64_t splits,
+                         float scale, int64_t batch, int64_t q_stride, int64_t batch_stride, int64_t gate_row_stride,
+                         int64_t max_seq, ixb_stream_t stream);
 /* Causal attention of `rows` new rows of one sequence (positions pos0 .. pos0 + rows - 1, keys and values already in the
  * caches [max_seq][hkv][head_dim]): out [rows][hq][head_dim] = softmax(scale * q.k) v over positions 0 .. pos0 + row.
  * q [rows] with row pitch q_stride elements (a multiple of 8), heads contiguous; head_dim 64 or 128; 16-byte aligned. */

@@ -158,6 +158,8 @@ def lib():
     L.ixb_attn_scratch_bytes.argtypes = [i64, i64, i64]
     L.ixb_attn_decode.restype = C.c_int
     L.ixb_attn_decode.argtypes = [vp, vp, vp, vp, vp, i64, vp, vp, sz, i64, i64, i64, i64, f32, i64, i64, i64, i64, vp]
+    L.ixb_attn_decode_join.restype = C.c_int
+    L.ixb_attn_decode_join.argtypes = [vp, vp, vp, vp, vp, i64, vp, vp, sz, vp, i64, i64, i64, i64, f32, i64, i64, i64, i64, i64, vp]
     L.ixb_attn_prefill.restype = C.c_int
     L.ixb_attn_prefill.argtypes = [vp, vp, vp, vp, i64, i64, i64, i64, i64, f32, i64, i64, vp]
     L.ixb_conv_update.restype = C.c_int

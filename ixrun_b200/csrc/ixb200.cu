@@ -1355,13 +1355,19 @@ extern "C" size_t ixb_attn_scratch_bytes(int64_t hq, int64_t head_dim, int64_t s
 template <int D>
 static cudaError_t launch_attn(int64_t hq, int64_t hkv, int64_t splits, cudaStream_t st, const void *q, const void *k_cache,
                                const void *v_cache, const int32_t *pos, void *scratch, float scale, int64_t batch,
-                               int64_t q_stride, int64_t batch_stride)
+                               int64_t q_stride, int64_t batch_stride, int64_t max_seq, const AttnJoin &join)
 {
     const int64_t rep = hq / hkv;
+    // CTAs per group: about two per SM over all groups and sequences, what runs at once (40 sequences: 1.85 ms a step of the
+    // 1B decoder with two or four per SM, 1.94 with eight), never more than there are parts
+    auto ctas = [&](int64_t groups) {
+        return (unsigned)std::max<int64_t>(1, std::min<int64_t>(splits, (2 * num_sms() + groups * batch - 1) / (groups * batch)));
+    };
 #define IXB_ATTN(G)                                                                                                        \
-    return launch_glue(k_attn_decode<D, G>, dim3((unsigned)(hq / G), (unsigned)splits, (unsigned)batch), dim3(256), st,   \
+    return launch_glue(k_attn_decode<D, G>, dim3((unsigned)(hq / G), ctas(hq / G), (unsigned)batch), dim3(256), st,       \
                        (const __nv_bfloat16 *)q, (const __nv_bfloat16 *)k_cache, (const __nv_bfloat16 *)v_cache, pos,      \
-                       (float *)scratch, (uint32_t)hq, (uint32_t)hkv, scale, (uint32_t)q_stride, (size_t)batch_stride)
+                       (float *)scratch, (uint32_t)hq, (uint32_t)hkv, scale, (uint32_t)q_stride, (size_t)batch_stride,     \
+                       (uint32_t)splits, (uint32_t)max_seq, join)
     switch (rep) {                      // all query heads of a KV head in one CTA where that is a supported group size
     case 2: IXB_ATTN(2);
     case 3: IXB_ATTN(3);
@@ -1373,10 +1379,10 @@ static cudaError_t launch_attn(int64_t hq, int64_t hkv, int64_t splits, cudaStre
 #undef IXB_ATTN
 }
 
-extern "C" int ixb_attn_decode(const void *q, const void *k_cache, const void *v_cache, const int32_t *pos, const void *gate,
-                               int64_t gate_stride, void *out, void *scratch, size_t scratch_bytes, int64_t hq, int64_t hkv,
-                               int64_t head_dim, int64_t splits, float scale, int64_t batch, int64_t q_stride,
-                               int64_t batch_stride, int64_t gate_row_stride, ixb_stream_t stream)
+static int attn_decode_impl(const void *q, const void *k_cache, const void *v_cache, const int32_t *pos, const void *gate,
+                            int64_t gate_stride, void *out, void *scratch, size_t scratch_bytes, int64_t hq, int64_t hkv,
+                            int64_t head_dim, int64_t splits, float scale, int64_t batch, int64_t q_stride,
+                            int64_t batch_stride, int64_t gate_row_stride, int64_t max_seq, void *tickets, ixb_stream_t stream)
 {
     if (!q || !k_cache || !v_cache || !pos || !out || !scratch) return fail(IXB_E_ARG, "NULL pointer argument");
     if (hq <= 0 || hkv <= 0 || hq % hkv || splits <= 0 || splits > kAttnMaxSplits) return fail(IXB_E_ARG, "bad shape");
@@ -1384,19 +1390,39 @@ extern "C" int ixb_attn_decode(const void *q, const void *k_cache, const void *v
     if (head_dim != 64 && head_dim != 128 && head_dim != 256) return fail(IXB_E_UNSUPPORTED, "head_dim=%lld: 64, 128 or 256", (long long)head_dim);
     if (scratch_bytes < (size_t)batch * ixb_attn_scratch_bytes(hq, head_dim, splits)) return fail(IXB_E_SCRATCH, "attention scratch too small");
     if (((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache) & 15u) return fail(IXB_E_ARG, "q / caches are not 16-byte aligned");
-    if ((uintptr_t)scratch & 7u) return fail(IXB_E_ARG, "attention scratch is misaligned");
+    if ((uintptr_t)scratch & (tickets ? 15u : 7u)) return fail(IXB_E_ARG, "attention scratch is misaligned");
     cudaStream_t st = (cudaStream_t)stream;
+    const AttnJoin join = {(uint32_t *)tickets, (__nv_bfloat16 *)out, (const __nv_bfloat16 *)gate, (uint32_t)gate_stride, (uint32_t)gate_row_stride};
     cudaError_t e;
-    if (head_dim == 64) e = launch_attn<64>(hq, hkv, splits, st, q, k_cache, v_cache, pos, scratch, scale, batch, q_stride, batch_stride);
-    else if (head_dim == 128) e = launch_attn<128>(hq, hkv, splits, st, q, k_cache, v_cache, pos, scratch, scale, batch, q_stride, batch_stride);
-    else e = launch_attn<256>(hq, hkv, splits, st, q, k_cache, v_cache, pos, scratch, scale, batch, q_stride, batch_stride);
+    if (head_dim == 64) e = launch_attn<64>(hq, hkv, splits, st, q, k_cache, v_cache, pos, scratch, scale, batch, q_stride, batch_stride, max_seq, join);
+    else if (head_dim == 128) e = launch_attn<128>(hq, hkv, splits, st, q, k_cache, v_cache, pos, scratch, scale, batch, q_stride, batch_stride, max_seq, join);
+    else e = launch_attn<256>(hq, hkv, splits, st, q, k_cache, v_cache, pos, scratch, scale, batch, q_stride, batch_stride, max_seq, join);
     if (e != cudaSuccess) return fail(IXB_E_CUDA, "k_attn_decode launch: %s", cudaGetErrorString(e));
     int rc = launch_check("k_attn_decode");
-    if (rc) return rc;
+    if (rc || tickets) return rc;
     const unsigned threads = (unsigned)std::max<int64_t>(head_dim, (splits + 31) / 32 * 32);
     IXB_GLUE("k_attn_combine", launch_glue(k_attn_combine, dim3((unsigned)hq, (unsigned)batch), dim3(threads), st, (const float *)scratch,
                                            (__nv_bfloat16 *)out, (const __nv_bfloat16 *)gate, pos, (uint32_t)splits, (uint32_t)head_dim,
                                            (uint32_t)gate_stride, (uint32_t)gate_row_stride));
+}
+
+extern "C" int ixb_attn_decode(const void *q, const void *k_cache, const void *v_cache, const int32_t *pos, const void *gate,
+                               int64_t gate_stride, void *out, void *scratch, size_t scratch_bytes, int64_t hq, int64_t hkv,
+                               int64_t head_dim, int64_t splits, float scale, int64_t batch, int64_t q_stride,
+                               int64_t batch_stride, int64_t gate_row_stride, ixb_stream_t stream)
+{
+    return attn_decode_impl(q, k_cache, v_cache, pos, gate, gate_stride, out, scratch, scratch_bytes, hq, hkv, head_dim, splits, scale,
+                            batch, q_stride, batch_stride, gate_row_stride, 0, nullptr, stream);
+}
+
+extern "C" int ixb_attn_decode_join(const void *q, const void *k_cache, const void *v_cache, const int32_t *pos, const void *gate,
+                                    int64_t gate_stride, void *out, void *scratch, size_t scratch_bytes, void *tickets, int64_t hq,
+                                    int64_t hkv, int64_t head_dim, int64_t splits, float scale, int64_t batch, int64_t q_stride,
+                                    int64_t batch_stride, int64_t gate_row_stride, int64_t max_seq, ixb_stream_t stream)
+{
+    if (!tickets || max_seq <= 0 || max_seq > 0x7fffffffLL) return fail(IXB_E_ARG, "tickets and the caches' rows are needed");
+    return attn_decode_impl(q, k_cache, v_cache, pos, gate, gate_stride, out, scratch, scratch_bytes, hq, hkv, head_dim, splits, scale,
+                            batch, q_stride, batch_stride, gate_row_stride, max_seq, tickets, stream);
 }
 
 template <int D>

@@ -325,168 +325,275 @@ k_rope_kv8(__nv_bfloat16 *q, const __nv_bfloat16 *__restrict__ k, const __nv_bfl
 }
 
 // ---------------------------------------------------------------- single-query attention over the static cache
-// grid (groups, splits), 256 threads (8 warps).  A group is G consecutive query heads that share one KV head
-// (G = query heads per KV head, or 1): the K and V rows of a position are loaded once and used for all G heads.
-// The context [0, n_ctx) (n_ctx = pos[0] + 1) is cut into contiguous ranges, one per CTA: at most `splits` of them, and
-// none shorter than kAttnMinRange positions (attn_ranges; the CTAs beyond have nothing to do).  A short range is all
-// fixed cost -- joining the CTA's partial states -- so forty sequences of 150 to 300 positions cut 18 ways took 84 us a
-// layer; the number of ranges depends on the sequence alone, so it gets the same bits alone or in a batch.  A warp walks its share of a range
-// PPW positions at a time: D / 8 lanes hold 8 elements each of a position's K and V rows (one 16-byte load each, the
-// next iteration's rows requested before this one's arithmetic), a shuffle tree gives the G scores, and every
-// lane keeps a running maximum, denominator and weighted V sum per head (online softmax).  The CTA's warps are joined
-// in shared memory; the split's (maximum, denominator, sum[D]) per head goes to `part`; k_attn_combine joins the splits.
-constexpr uint32_t kAttnMinRange = 64;                 // positions: what the 8 warps of a CTA have in flight for D = 128
-__device__ __forceinline__ uint32_t attn_ranges(uint32_t n_ctx, uint32_t splits)
+// grid (groups, CTAs per group, sequences), 256 threads.  A group is G consecutive query heads that share one KV head (G =
+// query heads per KV head, or 1): the K and V rows of a position are loaded once and used for all G heads.
+// The context [0, n_ctx) (n_ctx = pos[0] + 1) is dealt out in chunks of kAttnChunk positions: part s of at most `splits`
+// takes the chunks s, s + splits, ...  A part of a few positions is all fixed cost, so forty sequences of 150 to 300
+// positions cut 18 ways took 84 us a layer; which chunks make a part depends on the sequence alone, so it gets the same
+// bits alone or in a batch, and a CTA walks as many parts as the grid leaves it.
+// Bound by latency at batch 1 (4 MB of cache are 0.7 us of HBM), so a chunk is one short chain: all its K and V rows are
+// requested at once (a position's K row by four threads, its V row by D / 8), the scores of all heads take two shuffles,
+// a warp per head turns them into weights, every thread sums its positions' V, and the threads' sums are joined once per
+// part.  With a running softmax per lane group and joins of eight such states per head instead, a CTA took 10700 cycles
+// for 64 positions (12.5 us a launch for 1025 positions of 16 / 8 heads of 128 under the profiler; 29 us for 4097 of
+// 6 / 2 heads of 256; 34 us for forty sequences of 225); now 9.4, 16.5 and 25 us.
+// With max_seq (rows of the cache) the first loads do not wait for the position: they read whatever rows the part would
+// take at full length, and what lies beyond the position is dropped.  With tickets (one word per sequence and group, zero
+// between launches) the last CTA of a group joins the parts itself; otherwise k_attn_combine does.
+constexpr uint32_t kAttnChunk = 64;                    // positions: what the 8 warps of a CTA have in flight for D = 128
+constexpr int kAttnMaxSplits = 256;
+__device__ __forceinline__ uint32_t attn_parts(uint32_t n_ctx, uint32_t splits)
 {
-    return min(splits, (n_ctx + kAttnMinRange - 1u) / kAttnMinRange);
+    return min(splits, (n_ctx + kAttnChunk - 1u) / kAttnChunk);
 }
+struct AttnJoin {
+    uint32_t *tickets;
+    __nv_bfloat16 *out;
+    const __nv_bfloat16 *gate;
+    uint32_t gate_stride, gate_row_stride;
+};
 
 template <int D, int G>
 __global__ void __launch_bounds__(256)
 k_attn_decode(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat16 *__restrict__ k_cache,
               const __nv_bfloat16 *__restrict__ v_cache, const int32_t *pos, float *part, uint32_t hq, uint32_t hkv,
-              float scale, uint32_t q_stride, size_t batch_stride)
+              float scale, uint32_t q_stride, size_t batch_stride, uint32_t splits, uint32_t max_seq, AttnJoin join)
 {
     // blockIdx.z: the sequence (its query row, its caches batch_stride elements after the previous one's, its position)
     q += (size_t)blockIdx.z * q_stride;
     k_cache += (size_t)blockIdx.z * batch_stride;
     v_cache += (size_t)blockIdx.z * batch_stride;
     pos += blockIdx.z;
-    part += (size_t)blockIdx.z * hq * gridDim.y * (D + 2);
-    constexpr int LPP = D / 8;                         // lanes per position
-    constexpr int PPW = 32 / LPP;                      // positions per warp iteration
-    constexpr int NS = 8;                              // partial states per head in the CTA: one per warp
-    __shared__ float sm_m[G][NS], sm_l[G][NS];
-    __shared__ float sm_acc[NS][D];                    // one head at a time
+    // scratch: sums [sequences][hq][splits][D], then (maximum, denominator) [sequences][hq][splits]
+    float2 *part_ml = (float2 *)(part + (size_t)gridDim.z * hq * splits * D) + (size_t)blockIdx.z * hq * splits;
+    part += (size_t)blockIdx.z * hq * splits * D;
+    constexpr int NW = 8;                              // warps
+    constexpr int C = (int)kAttnChunk;
+    constexpr int KC = D / 32;                         // 16-byte pieces of a K row per thread (four threads per position)
+    constexpr int VT = D / 8;                          // threads per V row
+    constexpr int VG = 256 / VT, VP = C / VG;          // groups of threads, positions of a chunk per group
+    constexpr int HG = G * D * NW * 4 <= 16384 ? G : 16384 / (D * NW * 4);        // heads joined at a time
+    __shared__ __align__(16) float sm_q[G][D];         // scaled queries
+    __shared__ float sm_s[G][C], sm_c[G];              // a chunk's scores, then weights; the sums' rescaling
+    __shared__ __align__(16) float sm_acc[NW][HG][D];
+    __shared__ float sm_w[G][kAttnMaxSplits], sm_sum[G];
+    __shared__ uint32_t sm_prev;
     asm volatile("griddepcontrol.launch_dependents;");
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    const uint32_t head0 = blockIdx.x * G, split = blockIdx.y, splits = gridDim.y;
+    const uint32_t head0 = blockIdx.x * G;
     const uint32_t kvh = head0 / (hq / hkv);
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int sub = lane / LPP, li = lane % LPP;       // which of the warp's positions, which 8 elements
-    const uint32_t n_ctx = (uint32_t)pos[0] + 1u, used = attn_ranges(n_ctx, splits);
-    if (split >= used) return;
-    const uint32_t per = (n_ctx + used - 1) / used, p0 = split * per, p1 = min(p0 + per, n_ctx);
-    float qv[G][8];
-#pragma unroll
-    for (int h = 0; h < G; ++h) {
-        unpack8(*(const uint4 *)(q + (size_t)(head0 + h) * D + li * 8), qv[h]);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) qv[h][j] *= scale;
-    }
-    float m[G], l[G], acc[G][8];
-#pragma unroll
-    for (int h = 0; h < G; ++h) {
-        m[h] = -INFINITY;
-        l[h] = 0.f;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[h][j] = 0.f;
-    }
-    // the trip count is the same for all lanes of a warp (the shuffles below need every lane); a lane whose position
-    // lies beyond the range reads position p1 - 1 and drops the result
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int kp = tid >> 2, kt = tid & 3;             // K: position of the chunk, which pieces (kt, kt + 4, ...)
+    const int vg = tid / VT, vd = (tid % VT) * 8;      // V: positions vg, vg + VG, ..., eight dimensions
     const size_t row_stride = (size_t)hkv * D;
-    const __nv_bfloat16 *kb = k_cache + (size_t)kvh * D + li * 8, *vb = v_cache + (size_t)kvh * D + li * 8;
-    // a ring of PF iterations' rows in registers: the loads of iteration i + PF are requested before the arithmetic
-    // of iteration i, so a warp has PF round trips to memory in flight
-    constexpr int PF = 4;
-    constexpr uint32_t STR = 8 * PPW;                  // positions the CTA covers per iteration
-    uint32_t pb = p0 + (uint32_t)(wid * PPW);
-    uint4 kq[PF], vq[PF];
+    const __nv_bfloat16 *kb = k_cache + (size_t)kvh * D + kt * 8, *vb = v_cache + (size_t)kvh * D + vd;
+    const uint32_t last = (uint32_t)pos[0];
+    uint4 kr[KC], vr[VP];
+    auto fetch_k = [&](uint32_t c, uint32_t limit) {
+        const __nv_bfloat16 *src = kb + min(c * kAttnChunk + kp, limit) * row_stride;
 #pragma unroll
-    for (int st = 0; st < PF; ++st) {
-        kq[st] = make_uint4(0, 0, 0, 0);
-        vq[st] = kq[st];
-        const uint32_t cur = pb + st * STR;
-        if (cur < p1) {                                // warp uniform
-            const uint32_t p = min(cur + (uint32_t)sub, p1 - 1u);
-            kq[st] = *(const uint4 *)(kb + p * row_stride);
-            vq[st] = *(const uint4 *)(vb + p * row_stride);
-        }
+        for (int j = 0; j < KC; ++j) kr[j] = *(const uint4 *)(src + j * 32);
+    };
+    auto fetch_v = [&](uint32_t c, uint32_t limit) {
+#pragma unroll
+        for (int j = 0; j < VP; ++j) vr[j] = *(const uint4 *)(vb + min(c * kAttnChunk + vg + j * VG, limit) * row_stride);
+    };
+    if (max_seq) {
+        fetch_k(blockIdx.y, max_seq - 1u);
+        fetch_v(blockIdx.y, max_seq - 1u);
     }
-    for (; pb < p1; pb += PF * STR) {
+    for (int i = tid; i < G * D; i += 256) sm_q[i / D][i % D] = bf2f(q[(size_t)head0 * D + i]) * scale;
+    const uint32_t n_ctx = (max_seq ? min(last, max_seq - 1u) : last) + 1u, used = attn_parts(n_ctx, splits);
+    if (blockIdx.y >= used) return;
+    __syncthreads();
+    if (!max_seq) {
+        fetch_k(blockIdx.y, n_ctx - 1u);
+        fetch_v(blockIdx.y, n_ctx - 1u);
+    }
+    for (uint32_t s = blockIdx.y; s < used; s += gridDim.y) {
+        float acc[G][8];
 #pragma unroll
-        for (int st = 0; st < PF; ++st) {
-            const uint32_t cur = pb + st * STR;
-            if (cur >= p1) break;                      // warp uniform
-            const bool live = cur + (uint32_t)sub < p1;
-            float kf[8], vf[8];
-            unpack8(kq[st], kf);
-            unpack8(vq[st], vf);
-            const uint32_t nxt = cur + PF * STR;
-            if (nxt < p1) {                            // warp uniform
-                const uint32_t p = min(nxt + (uint32_t)sub, p1 - 1u);
-                kq[st] = *(const uint4 *)(kb + p * row_stride);
-                vq[st] = *(const uint4 *)(vb + p * row_stride);
-            }
+        for (int h = 0; h < G; ++h)
 #pragma unroll
-            for (int h = 0; h < G; ++h) {
-                float s = 0.f;
+            for (int j = 0; j < 8; ++j) acc[h][j] = 0.f;
+        float M = -INFINITY, L = 0.f;                  // of head wid, in warp wid
+        for (uint32_t c = s; c * kAttnChunk < n_ctx; c += splits) {
+            const bool more = (c + splits) * kAttnChunk < n_ctx;
+            const uint32_t nxt = more ? c + splits : s + gridDim.y;       // the part's next chunk, or the next part's first
+            const bool ahead = more || nxt < used;
+            float sc[G];
 #pragma unroll
-                for (int j = 0; j < 8; ++j) s = fmaf(qv[h][j], kf[j], s);
+            for (int h = 0; h < G; ++h) sc[h] = 0.f;
 #pragma unroll
-                for (int d = LPP / 2; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
-                if (live) {
-                    const float mn = fmaxf(m[h], s), c = __expf(m[h] - mn), e = __expf(s - mn);
-                    l[h] = l[h] * c + e;
+            for (int j = 0; j < KC; ++j) {
+                float kf[8];
+                unpack8(kr[j], kf);
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) acc[h][j] = fmaf(acc[h][j], c, e * vf[j]);
-                    m[h] = mn;
+                for (int h = 0; h < G; ++h) {
+                    const float4 q0 = *(const float4 *)&sm_q[h][kt * 8 + j * 32], q1 = *(const float4 *)&sm_q[h][kt * 8 + j * 32 + 4];
+                    sc[h] = fmaf(kf[3], q0.w, fmaf(kf[2], q0.z, fmaf(kf[1], q0.y, fmaf(kf[0], q0.x, sc[h]))));
+                    sc[h] = fmaf(kf[7], q1.w, fmaf(kf[6], q1.z, fmaf(kf[5], q1.y, fmaf(kf[4], q1.x, sc[h]))));
                 }
             }
+            if (ahead) fetch_k(nxt, n_ctx - 1u);
+            const bool live = c * kAttnChunk + kp < n_ctx;
+#pragma unroll
+            for (int h = 0; h < G; ++h) {
+                sc[h] += __shfl_xor_sync(0xffffffffu, sc[h], 1);
+                sc[h] += __shfl_xor_sync(0xffffffffu, sc[h], 2);
+                if (kt == (h & 3)) sm_s[h][kp] = live ? sc[h] : -INFINITY;
+            }
+            __syncthreads();
+            if (wid < G) {                             // a warp per head (a chunk has at least one live position)
+                const float s0 = sm_s[wid][lane], s1 = sm_s[wid][lane + 32];
+                float mx = fmaxf(s0, s1);
+#pragma unroll
+                for (int d = 16; d > 0; d >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, d));
+                mx = fmaxf(mx, M);
+                const float base = mx == -INFINITY ? 0.f : mx;     // nothing but -inf so far: weights 0
+                const float p0 = __expf(s0 - base), p1 = __expf(s1 - base), cr = __expf(M - base);
+                sm_s[wid][lane] = p0;
+                sm_s[wid][lane + 32] = p1;
+                if (lane == 0) sm_c[wid] = cr;
+                L = L * cr + warp_sum(p0 + p1);
+                M = mx;
+            }
+            __syncthreads();
+            if (c != s) {
+#pragma unroll
+                for (int h = 0; h < G; ++h)
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) acc[h][j] *= sm_c[h];
+            }
+#pragma unroll
+            for (int j = 0; j < VP; ++j) {
+                float vf[8];
+                unpack8(vr[j], vf);
+                if (c * kAttnChunk + vg + j * VG >= n_ctx) continue;       // (not read, or rows beyond the position)
+#pragma unroll
+                for (int h = 0; h < G; ++h) {
+                    const float p = sm_s[h][vg + j * VG];
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) acc[h][k] = fmaf(p, vf[k], acc[h][k]);
+                }
+            }
+            if (ahead) fetch_v(nxt, n_ctx - 1u);
+            if (more) __syncthreads();                 // the weights are read: the next chunk's scores may follow
         }
+        // join: the warp's groups of threads by shuffles, the warps in shared memory, HG heads at a time
+        float *dst = part + ((size_t)head0 * splits + s) * D;
+#pragma unroll
+        for (int h0 = 0; h0 < G; h0 += HG) {
+            if (h0 || s != blockIdx.y) __syncthreads();            // sm_acc is free
+#pragma unroll
+            for (int hh = 0; hh < HG; ++hh) {
+                if (h0 + hh >= G) break;
+                float (&v)[8] = acc[h0 + hh < G ? h0 + hh : 0];
+#pragma unroll
+                for (int d = VT; d < 32; d <<= 1)
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) v[k] += __shfl_xor_sync(0xffffffffu, v[k], d);
+                if (lane < VT) {
+                    *(float4 *)&sm_acc[wid][hh][vd] = make_float4(v[0], v[1], v[2], v[3]);
+                    *(float4 *)&sm_acc[wid][hh][vd + 4] = make_float4(v[4], v[5], v[6], v[7]);
+                }
+            }
+            __syncthreads();
+            for (int i = tid; i < HG * D && h0 + i / D < G; i += 256) {
+                float a = 0.f;
+#pragma unroll
+                for (int w = 0; w < NW; ++w) a += sm_acc[w][i / D][i % D];
+                dst[(size_t)(h0 + i / D) * splits * D + i % D] = a;
+            }
+        }
+        if (wid < G && lane == 0) part_ml[(size_t)(head0 + wid) * splits + s] = make_float2(M, L);
     }
-    // join the warp's PPW partial states in registers, then the NS states of the CTA, head by head
-#pragma unroll
-    for (int h = 0; h < G; ++h) {
-#pragma unroll
-        for (int d = LPP; d < 32; d <<= 1) {
-            const float mo = __shfl_xor_sync(0xffffffffu, m[h], d), mn = fmaxf(m[h], mo);
-            const float c = m[h] == -INFINITY ? 0.f : __expf(m[h] - mn), co = mo == -INFINITY ? 0.f : __expf(mo - mn);
-            l[h] = l[h] * c + __shfl_xor_sync(0xffffffffu, l[h], d) * co;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) acc[h][j] = acc[h][j] * c + __shfl_xor_sync(0xffffffffu, acc[h][j], d) * co;
-            m[h] = mn;
-        }
-    }
-    if (lane == 0) {
-#pragma unroll
-        for (int h = 0; h < G; ++h) {
-            sm_m[h][wid] = m[h];
-            sm_l[h][wid] = l[h];
-        }
-    }
-#pragma unroll
-    for (int h = 0; h < G; ++h) {
-        __syncthreads();                               // sm_acc is free (and, first time, sm_m / sm_l are written)
-        if (sub == 0) {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) sm_acc[wid][li * 8 + j] = acc[h][j];
-        }
+    if (!join.tickets) return;
+    // ---- the last CTA of the group joins the parts
+    const uint32_t ctas = min(gridDim.y, used);
+    uint32_t *ticket = join.tickets + (size_t)blockIdx.z * gridDim.x + blockIdx.x;
+    __threadfence();                                   // this thread's share of the parts, before the ticket
+    __syncthreads();
+    if (ctas > 1u) {
+        if (threadIdx.x == 0) sm_prev = atomicAdd(ticket, 1u);
         __syncthreads();
-        float M = -INFINITY;
+        if (sm_prev != ctas - 1u) return;
+        __threadfence();
+        if (threadIdx.x == 0) *ticket = 0u;            // zero again for the next launch
+    }
+    // all of the group's sums are requested at once, as far as registers go: a thread takes four dimensions of a head and
+    // every PG-th part (rounds of eight dependent loads of one value: 29 us a launch at a 4097-token context, not 16.5)
+    constexpr int QD = G * D / 4, PG = QD >= 256 ? 1 : 256 / QD, MAXQ = (QD + 255) / 256;      // quads, part groups, quads per thread
+    constexpr int UN = 16;
+    const int pg = QD >= 256 ? 0 : tid / QD, q0 = QD >= 256 ? tid : tid % QD;
+    float4 first[UN];
+    auto sums = [&](int qd, uint32_t s) { return (const float4 *)(part + ((size_t)(head0 + qd * 4 / D) * splits + s) * D + qd * 4 % D); };
 #pragma unroll
-        for (int s2 = 0; s2 < NS; ++s2) M = fmaxf(M, sm_m[h][s2]);
-        float *out = part + ((size_t)(head0 + h) * splits + split) * (D + 2);
-        if (threadIdx.x < D) {
-            float a = 0.f;
+    for (int k = 0; k < UN; ++k) {
+        const uint32_t s = pg + k * PG;
+        first[k] = q0 < QD && pg < PG && s < used ? __ldcg(sums(q0, s)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    if (wid < G) {                                     // a warp per head: the parts' weights and their sum
+        const float2 *p = part_ml + (size_t)(head0 + wid) * splits;
+        float mx = -INFINITY, sum = 0.f;
+        for (uint32_t s = lane; s < used; s += 32) mx = fmaxf(mx, __ldcg(p + s).x);
 #pragma unroll
-            for (int s2 = 0; s2 < NS; ++s2)
-                if (sm_m[h][s2] != -INFINITY) a += sm_acc[s2][threadIdx.x] * __expf(sm_m[h][s2] - M);
-            out[2 + threadIdx.x] = a;
+        for (int d = 16; d > 0; d >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, d));
+        for (uint32_t s = lane; s < used; s += 32) {
+            const float2 ml = __ldcg(p + s);
+            const float c = ml.x == -INFINITY ? 0.f : __expf(ml.x - mx);
+            sm_w[wid][s] = c;
+            sum += ml.y * c;
         }
-        if (threadIdx.x == 0) {
-            float L = 0.f;
-            for (int s2 = 0; s2 < NS; ++s2)
-                if (sm_m[h][s2] != -INFINITY) L += sm_l[h][s2] * __expf(sm_m[h][s2] - M);
-            out[0] = M;
-            out[1] = L;
+        sum = warp_sum(sum);
+        if (lane == 0) sm_sum[wid] = sum;
+    }
+    __syncthreads();
+    float *sm_p = &sm_acc[0][0][0];                    // [PG][G * D]: fits, PG * G * D <= 1024 or PG == 1
+#pragma unroll
+    for (int i = 0; i < MAXQ; ++i) {
+        const int qd = q0 + i * 256;
+        if (qd >= QD || pg >= PG) continue;
+        const int h = qd * 4 / D;
+        float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+        auto add = [&](const float4 &v, float w) {
+            a.x = fmaf(v.x, w, a.x); a.y = fmaf(v.y, w, a.y); a.z = fmaf(v.z, w, a.z); a.w = fmaf(v.w, w, a.w);
+        };
+#pragma unroll
+        for (int k = 0; k < UN; ++k) {
+            const uint32_t s = pg + k * PG;
+            if (s < used) add(i ? __ldcg(sums(qd, s)) : first[k], sm_w[h][s]);
         }
+        for (uint32_t s0 = pg + UN * PG; s0 < used; s0 += UN * PG) {
+            float4 v[UN];
+#pragma unroll
+            for (int k = 0; k < UN; ++k) {
+                const uint32_t s = s0 + k * PG;
+                v[k] = s < used ? __ldcg(sums(qd, s)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+#pragma unroll
+            for (int k = 0; k < UN; ++k)
+                if (s0 + k * PG < used) add(v[k], sm_w[h][s0 + k * PG]);
+        }
+        *(float4 *)(sm_p + (size_t)pg * G * D + qd * 4) = a;
+    }
+    __syncthreads();
+    for (int i = tid; i < G * D; i += 256) {
+        const int h = i / D, d = i % D;
+        float a = sm_p[i];
+#pragma unroll
+        for (int g = 1; g < PG; ++g) a += sm_p[g * G * D + i];
+        float o = bfround(a / sm_sum[h]);
+        if (join.gate) {
+            const float gv = bf2f(join.gate[(size_t)blockIdx.z * join.gate_row_stride + (size_t)(head0 + h) * join.gate_stride + d]);
+            o = o * bfround(sigmoid_f(gv));
+        }
+        join.out[((size_t)blockIdx.z * hq + head0 + h) * D + d] = __float2bfloat16_rn(o);
     }
 }
 
 // grid q heads, D threads: out[head][d] = sum over the splits, optional sigmoid gate (gate[head][d], bf16).
 // The splits' maxima and denominators are fetched by one thread each, the weighted sums with independent loads.
-constexpr int kAttnMaxSplits = 256;
 __global__ void __launch_bounds__(256)
 k_attn_combine(const float *__restrict__ part, __nv_bfloat16 *out, const __nv_bfloat16 *__restrict__ gate, const int32_t *pos,
                uint32_t max_splits, uint32_t D, uint32_t gate_stride, uint32_t gate_row_stride)
@@ -495,17 +602,19 @@ k_attn_combine(const float *__restrict__ part, __nv_bfloat16 *out, const __nv_bf
     asm volatile("griddepcontrol.launch_dependents;");
     const uint32_t head = blockIdx.x, t = threadIdx.x;
     // blockIdx.y: the sequence
-    part += (size_t)blockIdx.y * gridDim.x * max_splits * (D + 2);
+    const float2 *part_ml = (const float2 *)(part + (size_t)gridDim.y * gridDim.x * max_splits * D) +
+                            ((size_t)blockIdx.y * gridDim.x + head) * max_splits;
+    part += (size_t)blockIdx.y * gridDim.x * max_splits * D;
     out += (size_t)blockIdx.y * gridDim.x * D;
     if (gate) gate += (size_t)blockIdx.y * gate_row_stride;
     float gv = 0.f;
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (gate && t < D) gv = bf2f(gate[(size_t)head * gate_stride + t]);
-    const uint32_t splits = attn_ranges((uint32_t)pos[blockIdx.y] + 1u, max_splits);
-    const float *p = part + (size_t)head * max_splits * (D + 2);
+    const uint32_t splits = attn_parts((uint32_t)pos[blockIdx.y] + 1u, max_splits);
+    const float *p = part + (size_t)head * max_splits * D;
     float ms = -INFINITY, ls = 0.f;
     if (t < splits) {
-        const float2 ml = *(const float2 *)(p + (size_t)t * (D + 2));
+        const float2 ml = part_ml[t];
         ms = ml.x;
         ls = ml.y;
     }
@@ -522,12 +631,12 @@ k_attn_combine(const float *__restrict__ part, __nv_bfloat16 *out, const __nv_bf
     const float L = cta_sum(ls * c, red);              // (its barriers also publish wgt)
     if (t >= D) return;
     float a0 = 0.f, a1 = 0.f;
-    const float *pt = p + 2 + t;
+    const float *pt = p + t;
     uint32_t s2 = 0;
     for (; s2 + 16 <= splits; s2 += 16) {              // sixteen independent loads in flight
         float v[16];
 #pragma unroll
-        for (int k = 0; k < 16; ++k) v[k] = pt[(size_t)(s2 + k) * (D + 2)];
+        for (int k = 0; k < 16; ++k) v[k] = pt[(size_t)(s2 + k) * D];
 #pragma unroll
         for (int k = 0; k < 16; k += 2) {
             a0 = fmaf(v[k], wgt[s2 + k], a0);
@@ -537,7 +646,7 @@ k_attn_combine(const float *__restrict__ part, __nv_bfloat16 *out, const __nv_bf
     {
         float v[16];
 #pragma unroll
-        for (int k = 0; k < 16; ++k) v[k] = s2 + k < splits ? pt[(size_t)(s2 + k) * (D + 2)] : 0.f;
+        for (int k = 0; k < 16; ++k) v[k] = s2 + k < splits ? pt[(size_t)(s2 + k) * D] : 0.f;
 #pragma unroll
         for (int k = 0; k < 16; ++k) a0 = fmaf(v[k], s2 + k < splits ? wgt[s2 + k] : 0.f, a0);
     }

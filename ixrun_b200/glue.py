@@ -125,6 +125,7 @@ class AttnDecode:
             groups = hq // rep if rep in (2, 3, 4, 6, 8) else hq
             splits = max(1, min(256, sms // (groups * self.batch)))
         self.splits = int(splits)
+        self.tickets = torch.zeros(self.batch * hq, dtype=torch.int32, device=device)     # zero between launches
         self.scratch = torch.empty(self.batch * _lib.lib().ixb_attn_scratch_bytes(hq, head_dim, self.splits), dtype=torch.uint8,
                                    device=device)
 
@@ -147,12 +148,13 @@ class AttnDecode:
         if out is None:
             out = torch.empty((b, self.hq * self.d) if b > 1 else (self.hq * self.d,), dtype=torch.bfloat16, device=q.device)
         with torch.cuda.device(q.device):
-            _lib.check(_lib.lib().ixb_attn_decode(q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), pos.data_ptr(),
-                                                  None if gate is None else gate.data_ptr(),
-                                                  gate_stride if gate_stride is not None else self.d, out.data_ptr(),
-                                                  self.scratch.data_ptr(), self.scratch.numel(), self.hq, self.hkv, self.d,
-                                                  self.splits, float(scale if scale is not None else self.d ** -0.5), b,
-                                                  q_stride or 0, batch_stride, gate_row_stride, _st(q)))
+            _lib.check(_lib.lib().ixb_attn_decode_join(q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), pos.data_ptr(),
+                                                       None if gate is None else gate.data_ptr(),
+                                                       gate_stride if gate_stride is not None else self.d, out.data_ptr(),
+                                                       self.scratch.data_ptr(), self.scratch.numel(), self.tickets.data_ptr(),
+                                                       self.hq, self.hkv, self.d, self.splits,
+                                                       float(scale if scale is not None else self.d ** -0.5), b,
+                                                       q_stride or 0, batch_stride, gate_row_stride, k_cache.shape[-3], _st(q)))
         return out
 
 

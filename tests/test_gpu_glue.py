@@ -97,6 +97,46 @@ def test_rope_kv_and_attention(hq, hkv, d, rot, norm):
     close(out, vc[0].float().repeat_interleave(rep, dim=0).reshape(-1), BF16_ULP)
 
 
+@pytest.mark.parametrize("ctx", [1, 63, 64, 65, 193, 700])
+@pytest.mark.parametrize("hq,hkv,d,splits", [(4, 2, 64, 3), (16, 8, 128, 18), (6, 2, 256, 5), (5, 1, 128, 1), (8, 1, 64, 256)])
+def test_attn_decode_parts(hq, hkv, d, splits, ctx):
+    """Chunks of 64 positions: one position, one short of a chunk, a whole one, one more, more chunks than parts; one part
+    and the most.  What lies in the cache beyond the position (NaN here) is read ahead and must not count; a sequence gets
+    the same bits alone (many CTAs) and among 24 (few, which take several parts each); the two-launch form of the C
+    interface agrees to the rounding of its joining sums (bf16 outputs: one unit in the last place, 2^-7 of a value)."""
+    from ixrun_b200 import _lib
+    from ixrun_b200.glue import AttnDecode
+
+    dev, max_seq, b = "cuda", 760, 24
+    gen = torch.Generator(device=dev).manual_seed(ctx)
+    kc = torch.randn(b, max_seq, hkv, d, generator=gen, device=dev).bfloat16()
+    vc = torch.randn(b, max_seq, hkv, d, generator=gen, device=dev).bfloat16()
+    q = torch.randn(b, hq * d, generator=gen, device=dev).bfloat16()
+    gate = torch.randn(b, hq * d, generator=gen, device=dev).bfloat16()
+    pos = (torch.arange(b, device=dev, dtype=torch.int32) * 13 + ctx - 1).clamp_(max=max_seq - 1)
+    for r in range(b):
+        kc[r, int(pos[r]) + 1:] = float("nan")
+        vc[r, int(pos[r]) + 1:] = float("nan")
+    many = AttnDecode(hq, hkv, d, dev, splits=splits, batch=b)
+    out = many(q, kc, vc, pos, gate=gate, gate_row_stride=hq * d)
+    assert not bool(many.tickets.any())
+    one = AttnDecode(hq, hkv, d, dev, splits=splits)
+    for r in (0, 1, 7, 23):
+        alone = one(q[r], kc[r], vc[r], pos[r:r + 1], gate=gate[r])
+        assert torch.equal(alone, out[r])
+        n = int(pos[r]) + 1
+        s = torch.einsum("ghd,sgd->ghs", q[r].double().view(hkv, hq // hkv, d), kc[r, :n].double()) * d ** -0.5
+        ref = torch.einsum("ghs,sgd->ghd", s.softmax(-1), vc[r, :n].double()).reshape(-1)
+        ref = ref.bfloat16() * torch.sigmoid(gate[r].float()).bfloat16()
+        close(alone, ref, 2 * BF16_ULP)
+        two = torch.empty_like(alone)
+        _lib.check(_lib.lib().ixb_attn_decode(q[r].data_ptr(), kc[r].data_ptr(), vc[r].data_ptr(), pos[r:].data_ptr(),
+                                              gate[r].data_ptr(), d, two.data_ptr(), one.scratch.data_ptr(), one.scratch.numel(),
+                                              hq, hkv, d, splits, d ** -0.5, 1, 0, 0, 0, _lib.stream_ptr(q.device)))
+        assert ((two.float() - alone.float()).abs() <= 2.0 ** -7 * alone.float().abs() + 2.0 ** -16).all()
+    assert not bool(one.tickets.any())
+
+
 @pytest.mark.parametrize("rows,pos0", [(1, 0), (1, 90), (63, 0), (64, 64), (65, 0), (200, 37)])
 @pytest.mark.parametrize("hq,hkv,d", [(4, 2, 64), (3, 3, 128), (6, 1, 128)])
 def test_attn_prefill(hq, hkv, d, rows, pos0):
