@@ -1015,12 +1015,12 @@ static std::atomic<int> g_p6_pdl{0};
 
 extern "C" int ixb_set_pdl(int on) { return g_p6_pdl.exchange(on ? 1 : 0); }
 
-template <int XS, bool MULTI>
+template <int XS, int MR>
 static cudaError_t launch_p6(const P6 &p, const void *x, uint32_t m_rows, const void *bias, void *y, int y_f32,
                              float4 *slots, uint32_t *tickets, const P6Plan &pl, const P6Push &push, cudaStream_t st)
 {
     static bool attr_set[64] = {false};
-    cudaError_t oe = opt_in_smem(k_p6_mma<XS, MULTI>, attr_set, 227 * 1024);
+    cudaError_t oe = opt_in_smem(k_p6_mma<XS, MR>, attr_set, 227 * 1024);
     if (oe != cudaSuccess) return oe;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(pl.grid);
@@ -1032,7 +1032,7 @@ static cudaError_t launch_p6(const P6 &p, const void *x, uint32_t m_rows, const 
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = g_p6_pdl.load() ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, k_p6_mma<XS, MULTI>, p, (const __nv_bfloat16 *)x, m_rows, (const __nv_bfloat16 *)bias, y, y_f32,
+    return cudaLaunchKernelEx(&cfg, k_p6_mma<XS, MR>, p, (const __nv_bfloat16 *)x, m_rows, (const __nv_bfloat16 *)bias, y, y_f32,
                               slots, tickets, pl.nb, pl.xstride, pl.cq, pl.cr, pl.unit, push);
 }
 
@@ -1059,7 +1059,10 @@ static int p6_gemv_impl(const ixb_p6 *t, const void *x, int64_t m_rows, const vo
     if (pu.fin && ((p.out_f & 1u) || pl.grid * (uint32_t)kP6Threads * 2u < (uint32_t)m_rows * p.out_f))
         return fail(IXB_E_UNSUPPORTED, "a finishing GEMV needs an even out_f and at most %u outputs", pl.grid * (uint32_t)kP6Threads * 2u);
     cudaStream_t st = (cudaStream_t)stream;
-    auto launch = m_rows > 1 ? (pl.xs ? launch_p6<1, true> : launch_p6<0, true>) : (pl.xs ? launch_p6<1, false> : launch_p6<0, false>);
+    auto launch = m_rows == 1  ? (pl.xs ? launch_p6<1, 1> : launch_p6<0, 1>)
+                  : m_rows == 2 ? (pl.xs ? launch_p6<1, 2> : launch_p6<0, 2>)
+                  : m_rows <= 4 ? (pl.xs ? launch_p6<1, 4> : launch_p6<0, 4>)
+                                : (pl.xs ? launch_p6<1, 8> : launch_p6<0, 8>);
     cudaError_t e = launch(p, x, (uint32_t)m_rows, bias, y, y_is_f32, slots, tickets, pl, pu, st);
     if (e != cudaSuccess) return fail(IXB_E_CUDA, "k_p6_mma launch: %s", cudaGetErrorString(e));
     return launch_check("k_p6_mma");

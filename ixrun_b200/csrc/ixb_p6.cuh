@@ -500,13 +500,14 @@ __global__ void __launch_bounds__(256) k_p6_decode_bf16(P6 p, __nv_bfloat16 *out
 // last arriver sums the slots in CTA order and clears them.  tickets[] (gridDim.x + 1 words) and cta_slots must be
 // zero before the first launch and are left zero, so one scratch buffer serves launches of any shape in turn.  XS = 1: activations staged in shared memory (bf16, padded rows); XS = 0: read from
 // global memory.
-template <int XS, bool MULTI>
+template <int XS, int MR>
 __global__ void __launch_bounds__(kP6Threads, 1)
 k_p6_mma(P6 p, const __nv_bfloat16 *__restrict__ x, uint32_t m_rows, const __nv_bfloat16 *__restrict__ bias, void *y,
          int y_f32, float4 *cta_slots, uint32_t *tickets, uint32_t nb, uint32_t xstride, uint32_t cq, uint32_t cr, uint32_t unit,
          P6Push push)
 {
     extern __shared__ __align__(128) unsigned char p6_smem[];
+    constexpr bool MULTI = MR > 1;
     using SM = P6Smem<MULTI>;
     __nv_bfloat16 *xs = (__nv_bfloat16 *)(p6_smem + SM::kFixed);                         // [m_rows][xstride]
 
@@ -632,17 +633,26 @@ k_p6_mma(P6 p, const __nv_bfloat16 *__restrict__ x, uint32_t m_rows, const __nv_
     auto finish_tile = [&](uint32_t R, uint32_t wlo, uint32_t whi, bool inside, uint32_t clo, uint32_t span) {
         const uint32_t t0 = R * KB;
         float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (uint32_t w = wlo; w <= whi; ++w) {
-            const uint32_t wb = p6_begin(w, wq, wr);
-            if (wb == p6_begin(w + 1, wq, wr)) continue;                // a warp without blocks
-            // the run of warp w meets tile R: R is its first tile unless the run began in the tile before
-            const unsigned char *part = p6_smem + w * SM::kWarp + SM::kParts + (cb0 + wb >= t0 ? 0 : SM::kPart);
-            if (MULTI) {
-                const float4 v = ((const float4 *)part)[lane];
-                s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
-            } else {                                                    // only activation row 0 counts: lanes t == 0, c[0] and c[2]
-                s.x += ((const float *)part)[g];
-                s.z += ((const float *)part)[g + 8];
+        // (eight warps' parts requested together: one after the other, 24 of them were 0.5 us of a small layer's 5.4)
+        for (uint32_t w0 = wlo; w0 <= whi; w0 += 8u) {
+            float4 v[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                const uint32_t w = w0 + k, wb = p6_begin(w, wq, wr);
+                v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (w > whi || wb == p6_begin(w + 1, wq, wr)) continue;  // not of this tile; a warp without blocks
+                // the run of warp w meets tile R: R is its first tile unless the run began in the tile before
+                const unsigned char *part = p6_smem + w * SM::kWarp + SM::kParts + (cb0 + wb >= t0 ? 0 : SM::kPart);
+                if (MULTI) {
+                    v[k] = ((const float4 *)part)[lane];
+                } else {                                                // only activation row 0 counts: lanes t == 0, c[0] and c[2]
+                    v[k].x = ((const float *)part)[g];
+                    v[k].z = ((const float *)part)[g + 8];
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                s.x += v[k].x; s.y += v[k].y; s.z += v[k].z; s.w += v[k].w;
             }
         }
         if (inside) {
@@ -780,7 +790,6 @@ k_p6_mma(P6 p, const __nv_bfloat16 *__restrict__ x, uint32_t m_rows, const __nv_
         const uint32_t my_a = tiles + (lane >> 4) * 512u + ((lane >> 3) & 1) * 256u + (lane & 7) * 2u;              // + row * 16
         const uint32_t my_b = tiles + 1024u + (lane >> 4) * 256u + ((lane >> 3) & 1) * 128u + (lane & 7) * 2u;      // + m * 16
         const uint32_t es = (uint32_t)__cvta_generic_to_shared(estage), pitch = XS ? xstride : p.in_f;
-        constexpr int MR = MULTI ? 8 : 1;
         uint32_t at = my_a;                                               // where this lane's weight lies
         auto outlier_steps = [&](uint32_t s64, const __nv_bfloat16 *xm, int32_t jlo, int32_t jhi, auto check) {
             constexpr bool kCheck = decltype(check)::value;
@@ -793,8 +802,7 @@ k_p6_mma(P6 p, const __nv_bfloat16 *__restrict__ x, uint32_t m_rows, const __nv_
                 }
                 const __nv_bfloat16 *xe = xm + (((e & 0xFFFu) - s64) & 0xFFFu);
 #pragma unroll
-                for (int m = 0; m < MR; ++m)
-                    if (!MULTI || (uint32_t)m < m_rows) xv[m] = __bfloat16_as_ushort(xe[(size_t)m * pitch]);
+                for (int m = 0; m < MR; ++m) xv[m] = __bfloat16_as_ushort(xe[min((uint32_t)m, m_rows - 1u) * pitch]);
                 return e;
             };
             uint32_t e = fetch(jlo + lane);
@@ -805,7 +813,6 @@ k_p6_mma(P6 p, const __nv_bfloat16 *__restrict__ x, uint32_t m_rows, const __nv_
                 bool bad = false;
 #pragma unroll
                 for (int m = 0; m < MR; ++m) {
-                    if (MULTI && (uint32_t)m >= m_rows) break;
                     if (kCheck && (xv[m] & 0x7F80u) == 0x7F80u) {
                         bad = true;
                         xv[m] = 0;
