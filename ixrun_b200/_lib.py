@@ -22,10 +22,10 @@ SYMBOLS = (
     "ixb_decode", "ixb_gemv_scratch_bytes", "ixb_gemv", "ixb_gemv_static",
     "ixb_gemm_scratch_bytes", "ixb_gemm",
     "ixb_pack_workspace_bytes", "ixb_quantize_codes", "ixb_count_codes", "ixb_pack_codes", "ixb_group_scale", "ixb_tpab_decode", "ixb_tpab_gemv_scratch_bytes", "ixb_tpab_gemv",
-    "ixb_p6_blocks", "ixb_p6_build", "ixb_p6_decode", "ixb_p6_gemv_scratch_bytes", "ixb_p6_gemv", "ixb_set_pdl",
-    "ixb_p6_gemm_scratch_bytes", "ixb_p6_gemm",
+    "ixb_p6_blocks", "ixb_p6_build", "ixb_p6_plane", "ixb_p6_entries", "ixb_p6_decode", "ixb_p6_gemv_scratch_bytes", "ixb_p6_gemv", "ixb_set_pdl",
+    "ixb_p6_gemm_scratch_bytes", "ixb_p6_gemm", "ixb_p6_rows",
     "ixb_allreduce_bytes", "ixb_allreduce", "ixb_p6_gemv_push", "ixb_allreduce_finish", "ixb_p6_gemv_allreduce", "ixb_allreduce_spin_limit",
-    "ixb_add_rmsnorm", "ixb_allreduce_finish_add_rmsnorm", "ixb_swiglu", "ixb_rope_kv", "ixb_attn_scratch_bytes", "ixb_attn_decode", "ixb_conv_update", "ixb_gdn_step", "ixb_gdn_conv_step",
+    "ixb_add_rmsnorm", "ixb_allreduce_finish_add_rmsnorm", "ixb_swiglu", "ixb_rope_kv", "ixb_attn_scratch_bytes", "ixb_attn_decode", "ixb_attn_decode_join", "ixb_attn_prefill", "ixb_conv_update", "ixb_gdn_step", "ixb_gdn_conv_step",
 )
 
 
