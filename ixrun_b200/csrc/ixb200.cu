@@ -256,8 +256,13 @@ __global__ void __launch_bounds__(256) k_decode(Streams s, const int32_t *q1, co
     for (int i = 0; i < 32 / kPer; ++i) r[i] = 0;
     decode_word_fast(src, w, c, tab_addr, [](int) {}, [&](int i, uint32_t v) { r[i / kPer] |= v << (kBits * (i % kPer)); });
     uint4 *o = (uint4 *)((char *)out + (size_t)e0 * (OUT == 0 ? 1 : 2));
+    if (((uintptr_t)out & 31u) == 0) {
 #pragma unroll
-    for (int j = 0; j < 8 / kPer; ++j) o[j] = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+        for (int j = 0; j < 4 / kPer; ++j) st_sector(o + 2 * j, r + 8 * j);
+    } else {
+#pragma unroll
+        for (int j = 0; j < 8 / kPer; ++j) o[j] = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+    }
 }
 
 // --------------------------------------------------------------- gemv -------

@@ -528,4 +528,11 @@ __device__ __forceinline__ SlotSrc stage_block(const Streams &s, const StageRole
     return src;
 }
 
+// 32 bytes in one store: a whole sector (two 16-byte stores send it to L2 twice); p 32-byte aligned
+__device__ __forceinline__ void st_sector(void *p, const uint32_t *r)
+{
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]),
+                 "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
+}
+
 }  // namespace ixb

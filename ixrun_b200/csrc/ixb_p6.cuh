@@ -429,50 +429,67 @@ __device__ __forceinline__ uint32_t p6_part_of(uint32_t pos, uint32_t q, uint32_
     return pos < big ? pos / (q + 1u) : r + (pos - big) / q;      // q > 0 whenever pos >= big
 }
 
-// layout -> bf16 weights in one pass, with the GEMV's own conversion: the
-// block's outliers are dropped into a zeroed image of the lanes' registers in shared memory first and OR-ed over the
-// placeholders (+0.0), so every weight is stored once, in 16-byte pieces; needs in_f % 8 == 0 and a 16-byte aligned
-// output.  One warp per block.
+// One outlier of a block over its placeholder, in the register of the lane that holds the element: row r, column c of the
+// block sit in lane 4 (r & 7) + (c >> 4), pair 4 ((c >> 2) & 3) + 2 ((c >> 1) & 1) + (r >> 3), half c & 1 (the inverse of
+// p6_elem).  e is the same in all lanes.
+__device__ __forceinline__ void p6_or_entry(uint32_t (&f)[16], uint32_t e, int lane)
+{
+    const uint32_t r = (e >> 12) & 15u, c = e & 63u;
+    const uint32_t v = (uint32_t)lane == 4u * (r & 7u) + (c >> 4) ? ((c & 1u) ? e & 0xFFFF0000u : e >> 16) : 0u;
+    const uint32_t at = 4u * ((c >> 2) & 3u) + 2u * ((c >> 1) & 1u) + (r >> 3);
+#pragma unroll
+    for (int q = 0; q < 16; ++q)
+        if (at == (uint32_t)q) f[q] |= v;
+}
+// ... and its place in an image [4 mma][32 lanes][4 registers] of those registers, for the blocks with many
+__device__ __forceinline__ uint32_t p6_image_at(uint32_t e)
+{
+    const uint32_t r = (e >> 12) & 15u, c = e & 63u;
+    return ((((c >> 2) & 3u) * 32u + 4u * (r & 7u) + (c >> 4)) * 4u + 2u * ((c >> 1) & 1u) + (r >> 3)) * 4u + 2u * (c & 1u);
+}
+
+// layout -> bf16 weights in one pass, with the GEMV's own conversion.  Bound by memory (2.76 bytes per weight): the
+// plane is requested before the offsets, one or two outliers go straight into their lane's register, more through an
+// image of the lanes' registers in shared memory, and every weight is stored once, a 32-byte sector per lane and row where
+// the alignment allows.  Needs in_f % 8 == 0 and a 16-byte aligned output.  One warp per block.
 __global__ void __launch_bounds__(256) k_p6_decode_bf16(P6 p, __nv_bfloat16 *out)
 {
-    __shared__ uint4 images[8 * 128];                // per warp: [4 mma][32 lanes] the lane's four A registers
+    __shared__ uint4 images[8 * 128];
     uint32_t b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     int lane = threadIdx.x & 31;
     if (b >= p.rt * p.kb) return;                    // whole warps leave together
-    // the plane first: the chain of offsets, entries and image below hides its way from memory
     const unsigned char *blk = p.plane + (size_t)b * kP6BlockBytes;
     const uint4 a = __ldg((const uint4 *)blk + lane);
     const uint2 a2 = __ldg((const uint2 *)(blk + 512) + lane);
-    uint4 *img = images + (threadIdx.x >> 5) * 128;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) img[q * 32 + lane] = make_uint4(0, 0, 0, 0);
-    __syncwarp();
-    {
-        const uint32_t img_s = (uint32_t)__cvta_generic_to_shared(img);
-        const int32_t lo = __ldg(p.blk_off + b), hi = __ldg(p.blk_off + b + 1);
-        for (int32_t j = lo + lane; j < hi; j += 32) {
-            const uint32_t e = __ldg(p.esc + j);
-            // element (row r, column c) of the block sits in lane 4 (r & 7) + (c >> 4), pair 4 ((c >> 2) & 3) +
-            // 2 ((c >> 1) & 1) + (r >> 3), half c & 1 (the inverse of p6_elem)
-            const uint32_t r = (e >> 12) & 15u, c = e & 63u;
-            const uint32_t ln = 4u * (r & 7u) + (c >> 4), j4 = (c >> 2) & 3u, q = 2u * ((c >> 1) & 1u) + (r >> 3);
-            const uint32_t off = ((j4 * 32u + ln) * 4u + q) * 4u + 2u * (c & 1u);
-            asm volatile("st.shared.u16 [%0], %1;" ::"r"(img_s + off), "h"((unsigned short)(e >> 16)) : "memory");
-        }
-    }
-    __syncwarp();
+    const int32_t lo = __ldg(p.blk_off + b), hi = __ldg(p.blk_off + b + 1);
     uint32_t R = b / p.kb, kbi = b - R * p.kb;
     const uint32_t w[6] = {a.x, a.y, a.z, a.w, a2.x, a2.y};
     uint32_t f[16];
     p6_unpack(w, 0x42804280u, p6_scale2(p.scale[R * p.scale_stride]), f);
+    // placeholders are +0.0, so OR-ing the outlier weights in is exact
+    if (hi - lo <= 2) {
+        for (int32_t j = lo; j < hi; ++j) p6_or_entry(f, __ldg(p.esc + j), lane);
+    } else {
+        uint4 *img = images + (threadIdx.x >> 5) * 128;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {                    // placeholders are +0.0, so OR-ing the outlier weights in is exact
-        const uint4 v = img[q * 32 + lane];
-        f[4 * q] |= v.x;
-        f[4 * q + 1] |= v.y;
-        f[4 * q + 2] |= v.z;
-        f[4 * q + 3] |= v.w;
+        for (int q = 0; q < 4; ++q) img[q * 32 + lane] = make_uint4(0, 0, 0, 0);
+        __syncwarp();
+        const uint32_t img_s = (uint32_t)__cvta_generic_to_shared(img);
+        for (int32_t j = lo + lane; j < hi; j += 32) {
+            const uint32_t e = __ldg(p.esc + j);
+            asm volatile("st.shared.u16 [%0], %1;" ::"r"(img_s + p6_image_at(e)), "h"((unsigned short)(e >> 16)) : "memory");
+        }
+        __syncwarp();
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const uint4 v = img[q * 32 + lane];
+            f[4 * q] |= v.x;
+            f[4 * q + 1] |= v.y;
+            f[4 * q + 2] |= v.z;
+            f[4 * q + 3] |= v.w;
+        }
     }
+    const bool wide = (p.in_f & 15u) == 0 && ((uintptr_t)out & 31u) == 0;       // a lane's 32 bytes of a row are one sector
     // pair 4 j + q: row g + 8 (q & 1), columns 4 j + 2 (q >> 1) + {0, 1} of the lane's 16
     const uint32_t col0 = kbi * kTileCols + 16 * (lane & 3);
 #pragma unroll
@@ -481,11 +498,15 @@ __global__ void __launch_bounds__(256) k_p6_decode_bf16(P6 p, __nv_bfloat16 *out
         if (row >= p.out_f || col0 >= p.in_f) continue;
         __nv_bfloat16 *dst = out + (size_t)row * p.in_f + col0;
         const uint32_t r[8] = {f[0 + s], f[2 + s], f[4 + s], f[6 + s], f[8 + s], f[10 + s], f[12 + s], f[14 + s]};
-        if (col0 + 16u <= p.in_f) {
+        if (wide) {
+            st_sector(dst, r);
+        } else if (col0 + 16u <= p.in_f) {
             ((uint4 *)dst)[0] = make_uint4(r[0], r[1], r[2], r[3]);
             ((uint4 *)dst)[1] = make_uint4(r[4], r[5], r[6], r[7]);
         } else {
-            for (uint32_t c = 0; col0 + c < p.in_f; ++c) ((uint16_t *)dst)[c] = (uint16_t)(r[c >> 1] >> (16 * (c & 1)));
+#pragma unroll
+            for (uint32_t c = 0; c < 16u; ++c)
+                if (col0 + c < p.in_f) ((uint16_t *)dst)[c] = (uint16_t)(r[c >> 1] >> (16 * (c & 1)));
         }
     }
 }

@@ -310,3 +310,27 @@ def test_p6_gemv_infinite_activation_reaches_only_its_rows():
                 assert bool(torch.isnan(got[r]))
             else:
                 assert bool(torch.isinf(got[r])) and bool(got[r] > 0) == bool(codes[r, col] > 0), r
+
+
+@pytest.mark.parametrize("out_f,in_f", [(48, 64), (33, 72), (50, 2176), (16, 8)])
+@pytest.mark.parametrize("shift,scale", [(0, 0.0071), (8, 0.0071), (0, 2.0 ** -131), (0, 2.0 ** 120)])
+def test_p6_decode_stores(out_f, in_f, shift, scale):
+    """Sector stores and 16-byte ones (rows or an output that is only 16-byte aligned), blocks with none, one, two and many
+    outliers; subnormal and huge weights; the streams' decoder on the same codes.  Bit for bit, and nothing beside the output is written."""
+    from ixrun_b200.p6 import P6Packed
+    from ixrun_b200.gpu_pack import pack_codes_gpu
+
+    gen = torch.Generator(device="cuda").manual_seed(in_f)
+    codes = torch.randint(-32, 32, (out_f, in_f), generator=gen, device="cuda").to(torch.int8)
+    n_kb = (in_f + 63) // 64
+    for kb, n in zip(range(n_kb), (0, 1, 2, 3, 40) * n_kb):
+        for k in range(n):
+            codes[(5 * k) % min(out_f, 16), min(64 * kb + (7 * k) % 64, in_f - 1)] = 100 - k
+    scale = torch.tensor(scale, dtype=torch.bfloat16)
+    want = (codes.float() * scale.float().cuda()).bfloat16()
+    buf = torch.full((out_f * in_f + 64,), 7.0, dtype=torch.bfloat16, device="cuda")
+    for src in (P6Packed(codes.reshape(-1), scale, out_f, in_f), pack_codes_gpu(codes, scale, out_f, in_f)):
+        buf.fill_(7.0)
+        got = src.decode(out=buf[16 + shift:16 + shift + out_f * in_f], kind="bf16")
+        assert torch.equal(got.view(torch.int16), want.view(torch.int16))
+        assert bool((buf[:16 + shift] == 7).all()) and bool((buf[16 + shift + out_f * in_f:] == 7).all())
