@@ -14,10 +14,6 @@ from . import _lib
 __all__ = ["gdn_conv_step", "add_rmsnorm", "finish_add_rmsnorm", "swiglu", "rope_kv", "AttnDecode", "attn_prefill", "conv_update", "gdn_step", "rope_tables"]
 
 
-def _st(t):
-    return _lib.stream_ptr(t.device)
-
-
 def _bf16(*ts):
     for t in ts:
         if t is not None and (t.dtype != torch.bfloat16 or not t.is_contiguous() or not t.is_cuda):
@@ -30,9 +26,9 @@ def add_rmsnorm(h: torch.Tensor, delta: torch.Tensor | None, w: torch.Tensor, ep
     rows, hidden = h.reshape(-1, h.shape[-1]).shape
     if out is None:
         out = torch.empty_like(h)
-    with torch.cuda.device(h.device):
+    with _lib.on_device(h.get_device()) as st:
         _lib.check(_lib.lib().ixb_add_rmsnorm(h.data_ptr(), None if delta is None else delta.data_ptr(), w.data_ptr(),
-                                              float(eps), out.data_ptr(), rows, hidden, _st(h)))
+                                              float(eps), out.data_ptr(), rows, hidden, st))
     return out
 
 
@@ -44,9 +40,9 @@ def finish_add_rmsnorm(ar, h: torch.Tensor, w: torch.Tensor, eps: float, out: to
     rows, hidden = h.reshape(-1, h.shape[-1]).shape
     if out is None:
         out = torch.empty_like(h)
-    with torch.cuda.device(h.device):
+    with _lib.on_device(h.get_device()) as st:
         _lib.check(_lib.lib().ixb_allreduce_finish_add_rmsnorm(ar._ptrs, ar.rank, ar.world, ar.n_max, h.data_ptr(), w.data_ptr(),
-                                                               float(eps), out.data_ptr(), rows, hidden, _st(h)))
+                                                               float(eps), out.data_ptr(), rows, hidden, st))
     return out
 
 
@@ -71,8 +67,8 @@ def swiglu(g: torch.Tensor, u: torch.Tensor, out: torch.Tensor | None = None):
     if out is None:
         out = torch.empty(g.shape, dtype=torch.bfloat16, device=g.device)
     _bf16(out)
-    with torch.cuda.device(g.device):
-        _lib.check(_lib.lib().ixb_swiglu(g.data_ptr(), u.data_ptr(), out.data_ptr(), rows, cols, pitch, _st(g)))
+    with _lib.on_device(g.get_device()) as st:
+        _lib.check(_lib.lib().ixb_swiglu(g.data_ptr(), u.data_ptr(), out.data_ptr(), rows, cols, pitch, st))
     return out
 
 
@@ -102,12 +98,12 @@ def rope_kv(q, k, v, pos, k_cache, v_cache, cos, sin, hq: int, hkv: int, head_di
     batch_stride = max_seq * hkv * head_dim if batched else 0
     if batched and (k_cache.dim() != 4 or k_cache.shape[0] < rows or pos.numel() < rows):
         raise ValueError("batched caches are [rows, max_seq, hkv, head_dim] with one position per row")
-    with torch.cuda.device(q.device):
+    with _lib.on_device(q.get_device()) as st:
         _lib.check(_lib.lib().ixb_rope_kv(q.data_ptr(), k.data_ptr(), v.data_ptr(), pos.data_ptr(), k_cache.data_ptr(),
                                           v_cache.data_ptr(), None if q_norm is None else q_norm.data_ptr(),
                                           None if k_norm is None else k_norm.data_ptr(), cos.data_ptr(), sin.data_ptr(),
                                           rows, hq, hkv, head_dim, rot_dim or head_dim, float(eps), q_stride, max_seq,
-                                          kv_pitch, batch_stride, _st(q)))
+                                          kv_pitch, batch_stride, st))
     return q
 
 
@@ -147,14 +143,14 @@ class AttnDecode:
         batch_stride = k_cache.shape[-3] * self.hkv * self.d if b > 1 and not shared_cache else 0
         if out is None:
             out = torch.empty((b, self.hq * self.d) if b > 1 else (self.hq * self.d,), dtype=torch.bfloat16, device=q.device)
-        with torch.cuda.device(q.device):
+        with _lib.on_device(q.get_device()) as st:
             _lib.check(_lib.lib().ixb_attn_decode_join(q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), pos.data_ptr(),
                                                        None if gate is None else gate.data_ptr(),
                                                        gate_stride if gate_stride is not None else self.d, out.data_ptr(),
                                                        self.scratch.data_ptr(), self.scratch.numel(), self.tickets.data_ptr(),
                                                        self.hq, self.hkv, self.d, self.splits,
                                                        float(scale if scale is not None else self.d ** -0.5), b,
-                                                       q_stride or 0, batch_stride, gate_row_stride, k_cache.shape[-3], _st(q)))
+                                                       q_stride or 0, batch_stride, gate_row_stride, k_cache.shape[-3], st))
         return out
 
 
@@ -171,11 +167,11 @@ def attn_prefill(q, k_cache, v_cache, pos0: int, hq: int, hkv: int, head_dim: in
     elif out.numel() != rows * hq * head_dim:
         raise ValueError("out must be [rows, hq*head_dim]")
     _bf16(out)
-    with torch.cuda.device(q.device):
+    with _lib.on_device(q.get_device()) as st:
         _lib.check(_lib.lib().ixb_attn_prefill(q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(), rows,
                                                int(pos0), hq, hkv, head_dim,
                                                float(scale if scale is not None else head_dim ** -0.5), pitch,
-                                               k_cache.shape[-3], _st(q)))
+                                               k_cache.shape[-3], st))
     return out
 
 
@@ -184,10 +180,10 @@ def conv_update(x, state, w, bias=None, out=None):
     _bf16(x, state, w, bias)
     if out is None:
         out = torch.empty_like(x)
-    with torch.cuda.device(x.device):
+    with _lib.on_device(x.get_device()) as st:
         _lib.check(_lib.lib().ixb_conv_update(x.data_ptr(), state.data_ptr(), w.data_ptr(),
                                               None if bias is None else bias.data_ptr(), out.data_ptr(), x.numel(),
-                                              w.shape[-1], _st(x)))
+                                              w.shape[-1], st))
     return out
 
 
@@ -198,10 +194,10 @@ def gdn_step(qkv, z, a, b, A_log, dt_bias, norm_w, state, hk: int, hv: int, eps:
         raise ValueError("state, A_log and dt_bias are fp32")
     if out is None:
         out = torch.empty(hv * 128, dtype=torch.bfloat16, device=qkv.device)
-    with torch.cuda.device(qkv.device):
+    with _lib.on_device(qkv.get_device()) as st:
         _lib.check(_lib.lib().ixb_gdn_step(qkv.data_ptr(), z.data_ptr(), a.data_ptr(), b.data_ptr(), A_log.data_ptr(),
                                            dt_bias.data_ptr(), norm_w.data_ptr(), state.data_ptr(), out.data_ptr(), hk, hv,
-                                           float(eps), _st(qkv)))
+                                           float(eps), st))
     return out
 
 
@@ -217,9 +213,9 @@ def gdn_conv_step(qkv_raw, conv_state, conv_w, pos, z, a, b, A_log, dt_bias, nor
         raise ValueError("state, A_log and dt_bias are fp32, pos int32")
     if out is None:
         out = torch.empty(hv * 128, dtype=torch.bfloat16, device=qkv_raw.device)
-    with torch.cuda.device(qkv_raw.device):
+    with _lib.on_device(qkv_raw.get_device()) as st:
         _lib.check(_lib.lib().ixb_gdn_conv_step(qkv_raw.data_ptr(), conv_state.data_ptr(), conv_w.data_ptr(), pos.data_ptr(),
                                                 z.data_ptr(), a.data_ptr(), b.data_ptr(), A_log.data_ptr(), dt_bias.data_ptr(),
                                                 norm_w.data_ptr(), state.data_ptr(), out.data_ptr(), hk, hv, float(eps),
-                                                _st(qkv_raw)))
+                                                st))
     return out
