@@ -403,7 +403,11 @@ k_attn_decode(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat16 *__restri
         fetch_v(blockIdx.y, max_seq - 1u);
     }
     for (int i = tid; i < G * D; i += 256) sm_q[i / D][i % D] = bf2f(q[(size_t)head0 * D + i]) * scale;
-    const uint32_t n_ctx = (max_seq ? min(last, max_seq - 1u) : last) + 1u, used = attn_parts(n_ctx, splits);
+    const uint32_t n_ctx = max_seq ? min(last + 1u, max_seq) : last + 1u, used = attn_parts(n_ctx, splits);
+    if (used == 0u && join.tickets && blockIdx.y == 0) {               // position -1: the mean over nothing
+        for (int i = tid; i < G * D; i += 256)
+            join.out[((size_t)blockIdx.z * hq + head0 + i / D) * D + i % D] = __float2bfloat16_rn(__int_as_float(0x7FFFFFFF));
+    }
     if (blockIdx.y >= used) return;
     __syncthreads();
     if (!max_seq) {

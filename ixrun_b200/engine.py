@@ -16,6 +16,7 @@ import os
 import torch
 import torch.nn as nn
 import torch.nn.functional as F
+from torch.autograd import forward_ad
 
 from .fused import _pick_split
 from .linear import _set_parent_child, iter_quantizable_linears
@@ -28,6 +29,14 @@ FUSED_MAX_ROWS = 8        # rows served by the CUDA-core fused kernel
 TC_MAX_ROWS = 64          # rows served by the tensor-core fused kernel (when enabled)
 # Rows served in passes of the same kernel, without a bias (decode + dense matmul adds it before the one rounding).
 PASSES_MAX_ROWS = 128
+
+
+def _plain(x) -> bool:
+    """True if nothing but the values of x is asked of an operation on it: no gradient, tangent, batching transform or
+    trace that a dense matmul would carry and a kernel on raw pointers would drop."""
+    return type(x) is torch.Tensor and not (x.requires_grad and torch.is_grad_enabled()) and forward_ad._current_level < 0 \
+        and torch._C._functorch.peek_interpreter_stack() is None and not torch.jit.is_tracing() \
+        and not torch.compiler.is_compiling()
 
 
 class StreamingLinear(nn.Module):
@@ -143,7 +152,8 @@ class StreamingLinear(nn.Module):
                 y = res.gemv(x, bias=self._bias_bf16)
             elif self._use_p6_gemm and rows <= TC_MAX_ROWS and self.in_features % 64 == 0:
                 y = res.gemm(x, bias=self._bias_bf16)
-            elif self._use_p6_gemm and rows > FUSED_MAX_ROWS and self._bias is None and self.in_features % 8 == 0:
+            elif self._use_p6_gemm and rows > FUSED_MAX_ROWS and self._bias is None and self.in_features % 8 == 0 \
+                    and self._w_buf is not None and _plain(x):
                 y = res.rows(x)
             if y is not None:
                 return y if x.dim() == 2 else y.view(x.shape[:-1] + (self.out_features,))

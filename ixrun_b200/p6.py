@@ -210,6 +210,8 @@ class P6Packed:
         """y[M, out_f] = x[M, in_f] @ W.T in bf16 for any M >= 1 and in_f a multiple of 8, up to 64 rows per pass over the
         resident layout."""
         x2 = self._rows(x)
+        if x2.data_ptr() % 16:
+            x2 = x2.clone()
         m = x2.shape[0]
         out = self._out(m, None, torch.bfloat16, None, "gemm")
         passes = -(-m // self.GEMM_MAX_ROWS)

@@ -252,3 +252,34 @@ def test_graphed_call_with_host_buffers_is_one_launch_per_call():
         assert torch.equal(y, lay(x.cuda()).cpu())
     with pytest.raises(RuntimeError):
         GraphedCall(lay, torch.zeros(1, 1024).bfloat16().cuda()).run_host(x)
+
+
+@pytest.mark.parametrize("in_f,rows", [(512, 65), (512, 128), (512, 129), (1056, 24), (1056, 100)])
+def test_streaming_linear_passes_keep_what_a_dense_matmul_gives(in_f, rows):
+    """9..128 rows without a bias in passes of the resident kernel: values against float64 (one bf16 rounding, 2^-8), an
+    unaligned input, gradients, vmap and forward-mode tangents as from the matmul that took these calls before."""
+    from ixrun_b200.engine import StreamingLinear
+
+    out_f = 200
+    gen = torch.Generator(device="cuda").manual_seed(rows)
+    w = (torch.randn(out_f, in_f, generator=gen, device="cuda") * 0.05).bfloat16()
+    lin = StreamingLinear.from_weight(w)
+    x = torch.randn(rows, in_f, generator=gen, device="cuda").bfloat16()
+    if rows > 64 or in_f % 64:
+        with pytest.raises(RuntimeError):
+            lin(x)                                             # no decode buffer: refused, as always
+    lin._set_shared_buf(torch.empty(out_f * in_f, dtype=torch.bfloat16, device="cuda"))
+    wd = lin._res.decode(kind="bf16").double()
+    ref = x.double() @ wd.t()
+    ok = lambda y, r: bool(((y.double() - r).abs() <= r.abs() * 2.0 ** -8 + 1e-5 * r.abs().max()).all())
+    assert ok(lin(x), ref) and lin(x).shape == (rows, out_f)
+    odd = torch.empty(rows * in_f + 1, dtype=torch.bfloat16, device="cuda")[1:].view(rows, in_f)
+    odd.copy_(x)
+    assert ok(lin(odd), ref)
+    xg = x.clone().requires_grad_()
+    lin(xg).sum().backward()
+    assert ok(xg.grad, wd.sum(0).expand(rows, in_f))
+    t = torch.ones_like(x)
+    _, tangent = torch.func.jvp(lin, (x,), (t,))
+    assert ok(tangent, t.double() @ wd.t())
+    assert ok(torch.func.vmap(lin)(x.view(1, rows, in_f))[0], ref)
