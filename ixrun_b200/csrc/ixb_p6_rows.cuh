@@ -11,8 +11,8 @@
 // as the GEMV; on top of that one mma per 16 x 16 weights and eight rows, 64 rows being where the mma rate takes over.
 // Feeding the converted weights to tcgen05 through shared memory instead (the form this kernel replaced) moves four
 // bytes of shared memory per weight and hands every 64 columns over twice between converters, copies and tensor core:
-// 17408 x 5120 took 44 us at 16 rows and 60 us at 64, of which 27 us were hand-over with no work in it.  Here nothing
-// is handed over between warps but the activations.
+// 17408 x 5120 took 40 us at 16 rows and 57 us at 64, of which 27 us were hand-over with no work in it.  Here nothing
+// is handed over between warps but the activations: 26 and 47 us.
 //
 // CTA  = 8 row tiles (128 weight rows) x a contiguous range of column blocks; K is split over the CTAs of a cluster as
 //        far as it takes to fill the chip, and the splits' sums are added in rank order through distributed shared memory.

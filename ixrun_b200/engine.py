@@ -92,8 +92,8 @@ class StreamingLinear(nn.Module):
                 self.register_buffer("_q2", q2, persistent=False)
         self.register_buffer("_scale", dp.scale, persistent=False)
         self._y32 = None
-        # 9..64 rows on the resident layout: one pass over the packed bytes on the tcgen05 tensor cores
-        # (ixb_p6_gemm, in_f % 64 == 0); set _use_p6_gemm = False to take decode + dense matmul instead.
+        # 9..64 rows on the resident layout: one pass over the packed bytes on the tensor cores
+        # (ixb_p6_gemm, in_f % 64 == 0; without a bias also two passes up to PASSES_MAX_ROWS); set _use_p6_gemm = False to take decode + dense matmul instead.
         # _use_tc: the older tensor-core kernel that reads the streams (needs them kept, in_f % 1024 == 0); off.
         self._use_p6_gemm = True
         self._use_tc = False

@@ -103,7 +103,7 @@ def main():
             torch.cuda.synchronize()
             ms = e0.elapsed_time(e1) / steps
             batched.append({"sequences": b, "ms_per_step": round(ms, 4), "tokens_per_s": round(b / ms * 1e3, 1),
-                            "linears": "fused GEMV" if b <= 8 else "tcgen05 GEMM"})
+                            "linears": "fused GEMV" if b <= 8 else "fused GEMM"})
             del dec
             torch.cuda.empty_cache()
     print(json.dumps({

@@ -1,8 +1,8 @@
 """Per-token glue kernels of a decode step (see ``csrc/ixb_glue.cuh``): thin wrappers over the C ABI.
 
 The reference leaves this work to HuggingFace eager code and to fla's Triton
-kernels (ixrun/fla_patch.py:23-72).  Every function is one launch (attention:
-two) on the current stream, allocates nothing when its outputs are passed in,
+kernels (ixrun/fla_patch.py:23-72).  Every function is one launch
+on the current stream, allocates nothing when its outputs are passed in,
 and can be captured in a CUDA graph: positions are device tensors.
 """
 from __future__ import annotations

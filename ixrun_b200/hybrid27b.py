@@ -328,7 +328,7 @@ def launches_per_token(cfg: HybridConfig, world: int) -> int:
     """Kernels of this library in one token step (packed GEMVs, glue, exchange)."""
     n = 0
     for li in range(cfg.n_layers):
-        n += (6 if cfg.is_attn(li) else 4) + 4 + (2 if world > 1 else 0)      # a finishing kernel per exchange
+        n += (5 if cfg.is_attn(li) else 4) + 4 + (2 if world > 1 else 0)      # a finishing kernel per exchange
     return n + 1 + (1 if world > 1 else 0)
 
 

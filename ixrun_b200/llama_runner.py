@@ -10,9 +10,10 @@ attention over the static cache -> o_proj GEMV -> RMSNorm -> gate/up GEMVs ->
 SwiGLU -> down GEMV.  The packed linears run the fused decode+GEMV kernel; with
 `glue="kernels"` the work between them is this library's glue kernels (residual
 add + RMSNorm, RoPE + cache write, split-context attention, SwiGLU) and q|k|v
-and gate|up are one fused packed tensor each: 10 launches per layer, all taking
+and gate|up are one fused packed tensor each: 9 launches per layer, all taking
 part in programmatic dependent launch; with
-`glue="eager"` it is plain torch.  Prefill (many rows) always takes the torch path.
+`glue="eager"` it is plain torch.  A prompt (many rows) runs on the glue kernels too, with the
+weights decoded and dense matmuls; eager torch with `glue="eager"` or a head_dim of 256.
 
 `weights="packed"` uses StreamingLinear (fused kernels); `weights="decoded"`
 builds the same model with the packed weights decoded to bf16 and dense

@@ -11,7 +11,7 @@ launches sit back to back in a CUDA graph that rotates over enough copies of the
 layer to keep the weights out of L2, and the graph is replayed until the timed
 region is long (the number a model step sees).
 Kernels: p6 / p6gemm / p6decode (resident layout: fused GEMV for 1..8 rows,
-tcgen05 GEMM for up to 64 rows, decode to bf16; p6decode+dense = decode then a
+GEMM for up to 64 rows, decode to bf16; p6decode+dense = decode then a
 dense matmul, what the GEMM replaces), gemv / gemm / decode (the reference's streams read directly), dense (bf16
 matmul on decoded weights, the "cached mode" of the reference).
 """

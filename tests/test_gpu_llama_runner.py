@@ -91,7 +91,7 @@ def test_batched_decoder_gives_every_sequence_its_own_tokens():
 
 
 def test_batched_decoder_on_the_tensor_core_gemm():
-    """Twelve sequences: the linears run on the tcgen05 GEMM (another summation order than the GEMV), so a sequence's
+    """Twelve sequences: the linears run on the small-M GEMM (another summation order than the GEMV), so a sequence's
     logits agree with its batch-1 decode to bf16 noise instead of bit for bit."""
     from ixrun_b200.llama_runner import BatchedGreedyDecoder
 
