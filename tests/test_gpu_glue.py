@@ -98,8 +98,7 @@ def test_rope_kv_and_attention(hq, hkv, d, rot, norm):
 
 
 @pytest.mark.parametrize("ctx", [1, 63, 64, 65, 193, 700])
-@pytest.mark.parametrize("hq,hkv,d,splits", [(4, 2, 64, 3), (16, 8, 128, 18), (6, 2, 256, 5), (5, 1, 128, 1), (8, 1, 64, 256),
-                                             (4, 4, 64, 5), (5, 1, 64, 1), (14, 2, 64, 18)])
+@pytest.mark.parametrize("hq,hkv,d,splits", [(4, 2, 64, 3), (16, 8, 128, 18), (6, 2, 256, 5), (5, 1, 128, 1), (8, 1, 64, 256)])
 def test_attn_decode_parts(hq, hkv, d, splits, ctx):
     """Chunks of 64 positions: one position, one short of a chunk, a whole one, one more, more chunks than parts; one part
     and the most.  What lies in the cache beyond the position (NaN here) is read ahead and must not count; a sequence gets
@@ -136,35 +135,6 @@ def test_attn_decode_parts(hq, hkv, d, splits, ctx):
                                               hq, hkv, d, splits, d ** -0.5, 1, 0, 0, 0, _lib.stream_ptr(q.device)))
         assert ((two.float() - alone.float()).abs() <= 2.0 ** -7 * alone.float().abs() + 2.0 ** -16).all()
     assert not bool(one.tickets.any())
-
-
-class _NoLaunch:
-    """stands in for the C library: a call that gets as far as a launch fails the test instead of handing a host pointer on"""
-
-    def __getattr__(self, name):
-        return lambda *a: pytest.fail(f"{name} was called")
-
-
-@pytest.mark.parametrize("host", ["q", "pos", "gate", "out"])
-def test_attn_decode_and_rope_refuse_host_tensors(monkeypatch, host):
-    from ixrun_b200 import _lib
-    from ixrun_b200.glue import AttnDecode, rope_kv, rope_tables
-
-    bf = dict(dtype=torch.bfloat16, device="cuda")
-    t = {"q": torch.zeros(256, **bf), "gate": torch.zeros(256, **bf), "out": torch.zeros(256, **bf),
-         "pos": torch.zeros(1, dtype=torch.int32, device="cuda")}
-    kc, vc = torch.zeros(32, 2, 64, **bf), torch.zeros(32, 2, 64, **bf)
-    kv = torch.zeros(1, 128, **bf)
-    cos, sin = rope_tables(32, 64, 10000.0, "cuda")
-    ad = AttnDecode(4, 2, 64, "cuda")
-    ad(t["q"], kc, vc, t["pos"], out=t["out"], gate=t["gate"])
-    t[host] = t[host].cpu()
-    monkeypatch.setattr(_lib, "lib", lambda: _NoLaunch())
-    with pytest.raises(ValueError):
-        ad(t["q"], kc, vc, t["pos"], out=t["out"], gate=t["gate"])
-    if host in ("q", "pos"):
-        with pytest.raises(ValueError):
-            rope_kv(t["q"], kv, kv, t["pos"], kc, vc, cos, sin, 4, 2, 64, q_stride=256)
 
 
 @pytest.mark.parametrize("rows,pos0", [(1, 0), (1, 90), (63, 0), (64, 64), (65, 0), (200, 37)])
