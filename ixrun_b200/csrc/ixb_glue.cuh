@@ -373,9 +373,14 @@ k_attn_decode(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat16 *__restri
     constexpr int VT = D / 8;                          // threads per V row
     constexpr int VG = 256 / VT, VP = C / VG;          // groups of threads, positions of a chunk per group
     constexpr int HG = G * D * NW * 4 <= 16384 ? G : 16384 / (D * NW * 4);        // heads joined at a time
+    // the last CTA's join: quads of dimensions, and the groups of threads that share out the parts; their sums take the place
+    // of the warps' ([PG][G * D] floats: more than [NW][HG][D] for one head of 64)
+    constexpr int QD = G * D / 4, PG = QD >= 256 ? 1 : 256 / QD;
+    constexpr int NR = PG * G > NW * HG ? (PG * G + HG - 1) / HG : NW;
+    static_assert(PG * G * D <= NR * HG * D && NW <= NR, "sums of the join fit");
     __shared__ __align__(16) float sm_q[G][D];         // scaled queries
     __shared__ float sm_s[G][C], sm_c[G];              // a chunk's scores, then weights; the sums' rescaling
-    __shared__ __align__(16) float sm_acc[NW][HG][D];
+    __shared__ __align__(16) float sm_acc[NR][HG][D];
     __shared__ float sm_w[G][kAttnMaxSplits], sm_sum[G];
     __shared__ uint32_t sm_prev;
     asm volatile("griddepcontrol.launch_dependents;");
@@ -527,7 +532,7 @@ k_attn_decode(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat16 *__restri
     }
     // all of the group's sums are requested at once, as far as registers go: a thread takes four dimensions of a head and
     // every PG-th part (rounds of eight dependent loads of one value: 29 us a launch at a 4097-token context, not 16.5)
-    constexpr int QD = G * D / 4, PG = QD >= 256 ? 1 : 256 / QD, MAXQ = (QD + 255) / 256;      // quads, part groups, quads per thread
+    constexpr int MAXQ = (QD + 255) / 256;             // quads per thread
     constexpr int UN = 16;
     const int pg = QD >= 256 ? 0 : tid / QD, q0 = QD >= 256 ? tid : tid % QD;
     float4 first[UN];
@@ -553,7 +558,7 @@ k_attn_decode(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat16 *__restri
         if (lane == 0) sm_sum[wid] = sum;
     }
     __syncthreads();
-    float *sm_p = &sm_acc[0][0][0];                    // [PG][G * D]: fits, PG * G * D <= 1024 or PG == 1
+    float *sm_p = &sm_acc[0][0][0];                    // [PG][G * D]
 #pragma unroll
     for (int i = 0; i < MAXQ; ++i) {
         const int qd = q0 + i * 256;

@@ -98,7 +98,8 @@ def test_rope_kv_and_attention(hq, hkv, d, rot, norm):
 
 
 @pytest.mark.parametrize("ctx", [1, 63, 64, 65, 193, 700])
-@pytest.mark.parametrize("hq,hkv,d,splits", [(4, 2, 64, 3), (16, 8, 128, 18), (6, 2, 256, 5), (5, 1, 128, 1), (8, 1, 64, 256)])
+@pytest.mark.parametrize("hq,hkv,d,splits", [(4, 2, 64, 3), (16, 8, 128, 18), (6, 2, 256, 5), (5, 1, 128, 1), (8, 1, 64, 256),
+                                             (4, 4, 64, 5), (5, 1, 64, 1), (14, 2, 64, 18)])
 def test_attn_decode_parts(hq, hkv, d, splits, ctx):
     """Chunks of 64 positions: one position, one short of a chunk, a whole one, one more, more chunks than parts; one part
     and the most.  What lies in the cache beyond the position (NaN here) is read ahead and must not count; a sequence gets

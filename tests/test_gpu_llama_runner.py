@@ -44,6 +44,27 @@ def test_graph_step_equals_eager_and_matches_decoded_weights():
     assert agree == 8
 
 
+def test_steps_with_as_many_kv_heads_as_heads():
+    """Plain multi-head attention with heads of 64: one head per CTA in the decode attention.  Steps, three sequences in
+    lock-step and a verification of three tokens against the decoded weights."""
+    from ixrun_b200.llama_runner import BatchedGreedyDecoder, LlamaConfig, PackedLlama, Verifier, synthetic_llama
+
+    cfg = LlamaConfig(n_layers=2, hidden=256, intermediate=512, n_heads=4, n_kv_heads=4, head_dim=64, vocab=1000, max_seq=160)
+    layers, embed, head = synthetic_llama(cfg, seed=7)
+    packed, dense = (PackedLlama(cfg, layers, embed, head, weights=w) for w in ("packed", "decoded"))
+    prompt = torch.randint(0, cfg.vocab, (130,), generator=torch.Generator().manual_seed(8))
+    near = lambda a, b: bool((a - b).abs().max() <= 0.05 * b.abs().max())      # bf16 noise, as above
+    assert near(packed.prefill(prompt), dense.prefill(prompt))
+    toks = prompt[:3].cuda()
+    ref = torch.cat([dense.step(toks[i], 130 + i) for i in range(3)])
+    steps = torch.cat([packed.step(toks[i], 130 + i) for i in range(3)])
+    assert near(steps, ref)
+    assert torch.equal(Verifier(packed, 3)(toks, 130), steps)
+    dec = BatchedGreedyDecoder(packed, 3)
+    dec.prefill([prompt] * 3)
+    assert near(dec.step(toks[:1].expand(3)), ref[:1].expand(3, -1))
+
+
 def test_prefill_in_several_passes_keeps_the_same_cache_and_logits(monkeypatch):
     """A prompt longer than one pass: the later passes attend to the cache of the earlier ones.  Same arithmetic per row up
     to the order of the matmuls' sums, so the results agree to bf16 noise."""
