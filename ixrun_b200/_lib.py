@@ -186,11 +186,14 @@ def stream_ptr(device=None) -> int:
 class on_device:
     """``with on_device(index) as stream``: makes the device current (only if it is not) and gives its current stream as an
     integer.  What torch.cuda.device and torch.cuda.current_stream do, without their objects: the two take about 5 us of
-    a call whose kernel takes as long."""
+    a call whose kernel takes as long.  A tensor that is on no GPU (get_device() gives -1) is refused: torch.cuda.device(-1)
+    would do nothing, and the kernel would get a host pointer."""
 
     __slots__ = ("idx", "guard")
 
     def __init__(self, index: int):
+        if index < 0:
+            raise ValueError("expected a CUDA tensor")
         self.idx = index
 
     def __enter__(self) -> int:

@@ -94,6 +94,8 @@ def rope_kv(q, k, v, pos, k_cache, v_cache, cos, sin, hq: int, hkv: int, head_di
         raise ValueError("k and v must be [rows, hkv*head_dim] with the same row pitch")
     if q_stride is None:
         q_stride = _rows_view(q, "q")[2]
+    elif q.dtype != torch.bfloat16 or not q.is_cuda:
+        raise ValueError("q: bf16 CUDA tensor expected")
     max_seq = k_cache.shape[-3]
     batch_stride = max_seq * hkv * head_dim if batched else 0
     if batched and (k_cache.dim() != 4 or k_cache.shape[0] < rows or pos.numel() < rows):
@@ -134,7 +136,12 @@ class AttnDecode:
         are B positions of ONE sequence (caches [max_seq, hkv, head_dim], pos[r] = index of the newest key query r may
         see): causal attention of a short run of new tokens, as in the verification step of speculative decoding."""
         _bf16(k_cache, v_cache)
-        b = self.batch
+        b, n = self.batch, self.batch * self.hq * self.d
+        for t in (q, gate, out):
+            if t is not None and (t.dtype != torch.bfloat16 or not t.is_cuda):
+                raise ValueError("bf16 CUDA tensors expected")
+        if not pos.is_cuda or q.numel() < n or (out is not None and out.numel() < n):
+            raise ValueError("pos must be a CUDA tensor, q and out hold batch * hq * head_dim numbers")
         if b > 1:
             if q_stride is None:
                 q_stride = _rows_view(q, "q")[2]

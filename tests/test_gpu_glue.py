@@ -138,6 +138,35 @@ def test_attn_decode_parts(hq, hkv, d, splits, ctx):
     assert not bool(one.tickets.any())
 
 
+class _NoLaunch:
+    """stands in for the C library: a call that gets as far as a launch fails the test instead of handing a host pointer on"""
+
+    def __getattr__(self, name):
+        return lambda *a: pytest.fail(f"{name} was called")
+
+
+@pytest.mark.parametrize("host", ["q", "pos", "gate", "out"])
+def test_attn_decode_and_rope_refuse_host_tensors(monkeypatch, host):
+    from ixrun_b200 import _lib
+    from ixrun_b200.glue import AttnDecode, rope_kv, rope_tables
+
+    bf = dict(dtype=torch.bfloat16, device="cuda")
+    t = {"q": torch.zeros(256, **bf), "gate": torch.zeros(256, **bf), "out": torch.zeros(256, **bf),
+         "pos": torch.zeros(1, dtype=torch.int32, device="cuda")}
+    kc, vc = torch.zeros(32, 2, 64, **bf), torch.zeros(32, 2, 64, **bf)
+    kv = torch.zeros(1, 128, **bf)
+    cos, sin = rope_tables(32, 64, 10000.0, "cuda")
+    ad = AttnDecode(4, 2, 64, "cuda")
+    ad(t["q"], kc, vc, t["pos"], out=t["out"], gate=t["gate"])
+    t[host] = t[host].cpu()
+    monkeypatch.setattr(_lib, "lib", lambda: _NoLaunch())
+    with pytest.raises(ValueError):
+        ad(t["q"], kc, vc, t["pos"], out=t["out"], gate=t["gate"])
+    if host in ("q", "pos"):
+        with pytest.raises(ValueError):
+            rope_kv(t["q"], kv, kv, t["pos"], kc, vc, cos, sin, 4, 2, 64, q_stride=256)
+
+
 @pytest.mark.parametrize("rows,pos0", [(1, 0), (1, 90), (63, 0), (64, 64), (65, 0), (200, 37)])
 @pytest.mark.parametrize("hq,hkv,d", [(4, 2, 64), (3, 3, 128), (6, 1, 128)])
 def test_attn_prefill(hq, hkv, d, rows, pos0):

@@ -129,3 +129,11 @@ def test_ctypes_prototypes_match_the_header():
         body = re.search(r"typedef struct " + struct + r"\s*\{(.*?)\}\s*" + struct + r"\s*;", hdr_nc, flags=re.S).group(1)
         fields = [f for f in body.split(";") if f.strip()]
         assert len(fields) == len(mirror._fields_), f"{struct}: header has {len(fields)} fields, the mirror {len(mirror._fields_)}"
+
+
+def test_on_device_refuses_a_tensor_that_is_on_no_gpu():
+    """A host tensor's device index is -1, which torch.cuda.device takes as 'leave the device as it is'."""
+    from ixrun_b200 import _lib
+
+    with pytest.raises(ValueError):
+        _lib.on_device(torch.zeros(1).get_device())
