@@ -9,8 +9,8 @@
 //   plane   every element of code -32 .. 31 owns a 6-bit field F = 32 + code; put at bits 6..1 of the low byte it makes
 //           a bf16 number of the binade [64, 128):
 //             (F << 1) | 0x4280 = 64 + F = 96 + code
-//           so a packed subtraction of 96 gives the code exactly, and the packed multiplication by the scale rounds the
-//           exact product once: the reference's dequantised weight bf16(f32(code) * f32(scale))
+//           so a packed subtraction of 96 gives the code exactly, and the packed multiplication by the scale (plus 0, so
+//           that code 0 gives +0.0 whatever the scale's sign) rounds the exact product once: the reference's dequantised weight bf16(f32(code) * f32(scale))
 //           (ixrun/quantize.py:182, ixrun/fused.py:169-170), bit for bit, for any scale.
 //           Other codes ("outliers") leave the placeholder F = 32 (weight 0).  (Before, F was part of 1 + code / 32 over
 //           two binades, one fused multiply-add per pair instead of two operations, but it held -16 .. 31 only: 1.2 % of
@@ -323,11 +323,13 @@ __device__ __forceinline__ void p6_ldmatrix(uint32_t (&r)[4], uint32_t addr)
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
 }
-// two bf16 numbers 96 + code -> the two weights; s2: the scale in both halves
+// two bf16 numbers 96 + code -> the two weights; s2: the scale in both halves.  The product is a fused multiply-add of +0:
+// the same value, rounded once, but +0.0 for code 0 and a scale of either sign, so that a placeholder is all zero bits.
 __device__ __forceinline__ uint32_t p6_weights(uint32_t v, uint32_t s2)
 {
     uint32_t w;
-    asm("{\n\t.reg .b32 c;\n\tadd.rn.bf16x2 c, %1, %2;\n\tmul.rn.bf16x2 %0, c, %3;\n\t}" : "=r"(w) : "r"(v), "r"(0xC2C0C2C0u), "r"(s2));
+    asm("{\n\t.reg .b32 c;\n\tadd.rn.bf16x2 c, %1, %2;\n\tfma.rn.bf16x2 %0, c, %3, %4;\n\t}"
+        : "=r"(w) : "r"(v), "r"(0xC2C0C2C0u), "r"(s2), "r"(0u));
     return w;
 }
 // a lane's six plane words -> its 16 pairs of weights; e2 = 0x42804280 (kept in a register by the caller)

@@ -334,3 +334,31 @@ def test_p6_decode_stores(out_f, in_f, shift, scale):
         got = src.decode(out=buf[16 + shift:16 + shift + out_f * in_f], kind="bf16")
         assert torch.equal(got.view(torch.int16), want.view(torch.int16))
         assert bool((buf[:16 + shift] == 7).all()) and bool((buf[16 + shift + out_f * in_f:] == 7).all())
+
+
+@pytest.mark.parametrize("in_f", [192, 200])
+def test_p6_negative_scale(in_f):
+    """A scale below zero: code 0 becomes +0.0 (the product would be -0.0, which has the same value), outliers of either
+    sign keep theirs, in the decoder and at every row count of the kernels (fp32 sums against float64: the bound of the
+    tests above)."""
+    from ixrun_b200.p6 import P6Packed
+
+    gen = torch.Generator(device="cuda").manual_seed(in_f)
+    out_f = 50
+    codes = torch.randint(-127, 128, (out_f, in_f), generator=gen, device="cuda").to(torch.int8)
+    codes[:16] = torch.randint(-32, 32, (16, in_f), generator=gen, device="cuda").to(torch.int8)
+    codes[3, 5], codes[4, 6], codes[5, 80] = -100, 90, -33         # blocks with one, two outliers
+    scale = torch.tensor(-0.0071, dtype=torch.bfloat16, device="cuda")
+    want = (codes.float() * scale.float()).bfloat16()
+    p6 = P6Packed(codes.reshape(-1), scale, out_f, in_f)
+    got = p6.decode(kind="bf16")
+    assert torch.equal(got, want)
+    assert torch.equal(got.view(torch.int16), torch.where(codes == 0, 0.0, want).bfloat16().view(torch.int16))
+    x = torch.randn(50, in_f, generator=gen, device="cuda").bfloat16()
+    ref = x.double() @ want.double().t()
+    near = lambda y, m: float((y.double() - ref[:m]).abs().max() / ref.abs().max()) < 2e-5
+    assert near(p6.gemv(x[:8], out_dtype=torch.float32), 8)
+    if in_f % 64 == 0:
+        assert near(p6.gemm(x[:23], out_dtype=torch.float32), 23)
+    y = p6.rows(x)
+    assert bool(((y.double() - ref).abs() <= ref.abs() * 2.0 ** -8 + 1e-5 * ref.abs().max()).all())
