@@ -148,6 +148,10 @@ class AttnDecode:
             if pos.numel() < b or (not shared_cache and (k_cache.dim() != 4 or k_cache.shape[0] < b)):
                 raise ValueError("batched caches are [B, max_seq, hkv, head_dim] with one position per sequence")
         batch_stride = k_cache.shape[-3] * self.hkv * self.d if b > 1 and not shared_cache else 0
+        # rows of a sequence that both caches hold, whatever their shapes: the kernel reads ahead of the position
+        max_seq = (min(k_cache.numel(), v_cache.numel()) - (b - 1) * batch_stride) // (self.hkv * self.d)
+        if batch_stride:
+            max_seq = min(max_seq, k_cache.shape[-3])
         if out is None:
             out = torch.empty((b, self.hq * self.d) if b > 1 else (self.hq * self.d,), dtype=torch.bfloat16, device=q.device)
         with _lib.on_device(q.get_device()) as st:
@@ -157,7 +161,7 @@ class AttnDecode:
                                                        self.scratch.data_ptr(), self.scratch.numel(), self.tickets.data_ptr(),
                                                        self.hq, self.hkv, self.d, self.splits,
                                                        float(scale if scale is not None else self.d ** -0.5), b,
-                                                       q_stride or 0, batch_stride, gate_row_stride, k_cache.shape[-3], st))
+                                                       q_stride or 0, batch_stride, gate_row_stride, max_seq, st))
         return out
 
 

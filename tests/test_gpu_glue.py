@@ -167,6 +167,41 @@ def test_attn_decode_and_rope_refuse_host_tensors(monkeypatch, host):
             rope_kv(t["q"], kv, kv, t["pos"], kc, vc, cos, sin, 4, 2, 64, q_stride=256)
 
 
+@pytest.mark.parametrize("view", [lambda c: c.view(96, 128), lambda c: c.view(-1), lambda c: c.view(1, 96, 128), lambda c: c.view(1, 96, 2, 64)])
+def test_attn_decode_takes_a_cache_of_any_shape(view):
+    """One sequence's cache is max_seq * hkv * head_dim numbers; the same bits in every shape."""
+    from ixrun_b200.glue import AttnDecode
+
+    bf = dict(dtype=torch.bfloat16, device="cuda")
+    kc, vc, q = torch.randn(96, 2, 64, **bf), torch.randn(96, 2, 64, **bf), torch.randn(256, **bf)
+    pos = torch.tensor([80], dtype=torch.int32, device="cuda")
+    ad = AttnDecode(4, 2, 64, "cuda", splits=3)
+    assert torch.equal(ad(q, view(kc), view(vc), pos), ad(q, kc, vc, pos))
+
+
+def test_attn_decode_reads_ahead_in_what_both_caches_hold(monkeypatch):
+    """The rows that the kernel may touch before it knows the position, as the library is told: those of the shorter cache."""
+    from ixrun_b200 import _lib
+    from ixrun_b200.glue import AttnDecode
+
+    seen = []
+
+    class Record:
+        def ixb_attn_decode_join(self, *a):
+            seen.append(a[-2])
+            return 0
+
+    bf = dict(dtype=torch.bfloat16, device="cuda")
+    pos = torch.zeros(2, dtype=torch.int32, device="cuda")
+    one, two = AttnDecode(4, 2, 64, "cuda", splits=3), AttnDecode(4, 2, 64, "cuda", splits=3, batch=2)
+    monkeypatch.setattr(_lib, "lib", lambda: Record())
+    for k, v, want in ((96, 96, 96), (96, 70, 70), (70, 96, 70)):
+        one(torch.zeros(256, **bf), torch.zeros(k, 2, 64, **bf), torch.zeros(v, 2, 64, **bf), pos)
+        assert seen.pop() == want
+    two(torch.zeros(2, 256, **bf), torch.zeros(3, 96, 2, 64, **bf), torch.zeros(3, 96, 2, 64, **bf), pos)
+    assert seen.pop() == 96
+
+
 @pytest.mark.parametrize("rows,pos0", [(1, 0), (1, 90), (63, 0), (64, 64), (65, 0), (200, 37)])
 @pytest.mark.parametrize("hq,hkv,d", [(4, 2, 64), (3, 3, 128), (6, 1, 128)])
 def test_attn_prefill(hq, hkv, d, rows, pos0):
