@@ -288,16 +288,19 @@ class PackedLlama(torch.nn.Module):
         return F.linear(xn[-1:], self.lm_head).float()
 
     @torch.no_grad()
-    def prefill(self, ids: torch.Tensor, chunk: int = 256) -> torch.Tensor:
+    def prefill(self, ids: torch.Tensor, chunk: int | None = None) -> torch.Tensor:
         """Run the prompt through the model (many rows per linear: decode +
-        dense matmul path); returns the logits of the last prompt token."""
+        dense matmul path); returns the logits of the last prompt token.
+        chunk: the most rows that go through the model together, which bounds the memory of a pass's activations.  None:
+        PREFILL_ROWS on the glue kernels, 256 on the eager path (whose score matrices take rows * max_seq)."""
         logits = None
         if self.weights == "packed" and self.glue == "kernels" and self.cfg.head_dim in (64, 128):
-            rows, n = max(chunk, self.PREFILL_ROWS), ids.numel()
+            rows, n = self.PREFILL_ROWS if chunk is None else chunk, ids.numel()
             ids = ids.to(self.tok.device)
             for s in range(0, n, rows):
                 logits = self._prefill_kernels(ids[s:s + rows], s, s + rows >= n)
             return logits
+        chunk = 256 if chunk is None else chunk
         for s in range(0, ids.numel(), chunk):
             part = ids[s:s + chunk].to(self.tok.device)
             pos = torch.arange(s, s + part.numel(), device=part.device)

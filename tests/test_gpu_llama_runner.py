@@ -67,13 +67,15 @@ def test_steps_with_as_many_kv_heads_as_heads():
 
 def test_prefill_in_several_passes_keeps_the_same_cache_and_logits(monkeypatch):
     """A prompt longer than one pass: the later passes attend to the cache of the earlier ones.  Same arithmetic per row up
-    to the order of the matmuls' sums, so the results agree to bf16 noise."""
+    to the order of the matmuls' sums, so the results agree to bf16 noise.  No pass takes more rows than asked for."""
     cfg, packed, dense = tiny()
     prompt = torch.randint(0, cfg.vocab, (83,), generator=torch.Generator().manual_seed(4))
     one = packed.prefill(prompt)
     k1, v1 = packed.k_cache[:, :83].clone(), packed.v_cache[:, :83].clone()
-    monkeypatch.setattr(type(packed), "PREFILL_ROWS", 20)
+    rows, inner = [], packed._prefill_kernels
+    monkeypatch.setattr(packed, "_prefill_kernels", lambda ids, *a: (rows.append(ids.numel()), inner(ids, *a))[1])
     several = packed.prefill(prompt, chunk=20)
+    assert rows == [20, 20, 20, 20, 3]
     ref = dense.prefill(prompt)
     for a, b in ((one, ref), (several, ref), (packed.k_cache[:, :83], k1), (packed.v_cache[:, :83], v1), (k1, dense.k_cache[:, :83])):
         assert (a.float() - b.float()).abs().max() <= 0.05 * b.float().abs().max()
