@@ -111,7 +111,8 @@ def rope_kv(q, k, v, pos, k_cache, v_cache, cos, sin, hq: int, hkv: int, head_di
 
 class AttnDecode:
     """Single-query grouped-query attention over static KV caches, for one sequence or a batch of them; owns the scratch
-    of the context splits."""
+    of the context splits and the tickets by which the last CTA knows itself: launches that may overlap (different
+    streams without ordering) need separate objects."""
 
     def __init__(self, hq: int, hkv: int, head_dim: int, device, splits: int | None = None, batch: int = 1):
         self.hq, self.hkv, self.d, self.batch = hq, hkv, head_dim, int(batch)

@@ -202,6 +202,28 @@ def test_attn_decode_reads_ahead_in_what_both_caches_hold(monkeypatch):
     assert seen.pop() == 96
 
 
+def test_attn_decode_recovers_from_overlapping_launches():
+    """Launches of one object on two streams at once, with different numbers of parts, spoil each other's results but not
+    those of later calls: the tickets are zero again."""
+    from ixrun_b200.glue import AttnDecode
+
+    bf = dict(dtype=torch.bfloat16, device="cuda")
+    kc, vc, q = torch.randn(1200, 2, 128, **bf), torch.randn(1200, 2, 128, **bf), torch.randn(512, **bf)
+    pos = [torch.tensor([n], dtype=torch.int32, device="cuda") for n in (1100, 170, 20, -1)]
+    ad = AttnDecode(4, 2, 128, "cuda", splits=18)
+    want = [ad(q, kc, vc, p) for p in pos[:3]]
+    streams = [torch.cuda.Stream() for _ in pos]
+    torch.cuda.synchronize()
+    for _ in range(100):
+        for s, p in zip(streams, pos):
+            with torch.cuda.stream(s):
+                ad(q, kc, vc, p)
+    torch.cuda.synchronize()
+    assert not bool(ad.tickets.any())
+    for p, w in zip(pos, want):
+        assert torch.equal(ad(q, kc, vc, p), w)
+
+
 @pytest.mark.parametrize("rows,pos0", [(1, 0), (1, 90), (63, 0), (64, 64), (65, 0), (200, 37)])
 @pytest.mark.parametrize("hq,hkv,d", [(4, 2, 64), (3, 3, 128), (6, 1, 128)])
 def test_attn_prefill(hq, hkv, d, rows, pos0):
