@@ -27,8 +27,6 @@ __all__ = ["Int8XEngine", "StreamingLinear", "GraphLinear", "ResourceScheduler",
 
 FUSED_MAX_ROWS = 8        # rows served by the CUDA-core fused kernel
 TC_MAX_ROWS = 64          # rows served by the tensor-core fused kernel (when enabled)
-# Rows served in passes of the same kernel, without a bias (decode + dense matmul adds it before the one rounding).
-PASSES_MAX_ROWS = 128
 
 
 def _plain(x) -> bool:
@@ -93,7 +91,8 @@ class StreamingLinear(nn.Module):
         self.register_buffer("_scale", dp.scale, persistent=False)
         self._y32 = None
         # 9..64 rows on the resident layout: one pass over the packed bytes on the tensor cores
-        # (ixb_p6_gemm, in_f % 64 == 0; without a bias also two passes up to PASSES_MAX_ROWS); set _use_p6_gemm = False to take decode + dense matmul instead.
+        # (ixb_p6_gemm, in_f % 64 == 0; without a bias also in_f % 8 == 0); set _use_p6_gemm = False to take decode + dense
+        # matmul instead.
         # _use_tc: the older tensor-core kernel that reads the streams (needs them kept, in_f % 1024 == 0); off.
         self._use_p6_gemm = True
         self._use_tc = False
@@ -146,14 +145,19 @@ class StreamingLinear(nn.Module):
     def forward(self, x):
         rows = x.numel() // self.in_features
         res = self._res
-        if res is not None and x.dtype == torch.bfloat16 and x.shape[-1] == self.in_features and rows <= PASSES_MAX_ROWS:
+        if res is not None and x.dtype == torch.bfloat16 and x.shape[-1] == self.in_features and rows <= TC_MAX_ROWS:
             y = None
             if 1 <= rows <= FUSED_MAX_ROWS:
                 y = res.gemv(x, bias=self._bias_bf16)
-            elif self._use_p6_gemm and rows <= TC_MAX_ROWS and self.in_features % 64 == 0:
+            elif self._use_p6_gemm and self.in_features % 64 == 0:
                 y = res.gemm(x, bias=self._bias_bf16)
             elif self._use_p6_gemm and rows > FUSED_MAX_ROWS and self._bias is None and self.in_features % 8 == 0 \
                     and self._w_buf is not None and _plain(x):
+                # Without a bias, which decode + dense matmul adds before the one rounding.  A call outside a graph, this
+                # kernel and that route: 2048 x 2080 10.4 and 21.4 us with 24 rows, 12.5 and 21.4 with 64; 8192 x 8224 32
+                # and 56, 48 and 60.  (Above 48 rows layers of 25 to 40 million weights lose up to 7 us: 6144 x 6176 25.5
+                # and 32, 40 and 33.)  Two passes for more rows lose nearly everywhere: 6144 x 6144 with 65 rows 55 and
+                # 38 us, 17408 x 5120 with 128 rows 105 and 80.
                 y = res.rows(x)
             if y is not None:
                 return y if x.dim() == 2 else y.view(x.shape[:-1] + (self.out_features,))

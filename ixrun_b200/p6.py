@@ -207,22 +207,17 @@ class P6Packed:
         return out
 
     def rows(self, x: torch.Tensor) -> torch.Tensor:
-        """y[M, out_f] = x[M, in_f] @ W.T in bf16 for any M >= 1 and in_f a multiple of 8, up to 64 rows per pass over the
-        resident layout."""
+        """y[M, out_f] = x[M, in_f] @ W.T in bf16 for 1 <= M <= 64 and in_f a multiple of 8, in one pass over the resident
+        layout; x of any alignment."""
         x2 = self._rows(x)
         if x2.data_ptr() % 16:
             x2 = x2.clone()
         m = x2.shape[0]
         out = self._out(m, None, torch.bfloat16, None, "gemm")
-        passes = -(-m // self.GEMM_MAX_ROWS)
-        step = -(-(-(-m // passes)) // 8) * 8            # even passes of whole groups of eight rows
-        L = _lib.lib()
         with _lib.on_device(self._index) as stream:
-            for r in range(0, m, step):
-                rc = L.ixb_p6_rows(self._ref, x2.data_ptr() + 2 * r * self.in_f, min(step, m - r), None,
-                                   out.data_ptr() + 2 * r * self.out_f, 0, stream)
-                if rc:
-                    _lib.check(rc)
+            rc = _lib.lib().ixb_p6_rows(self._ref, x2.data_ptr(), m, None, out.data_ptr(), 0, stream)
+        if rc:
+            _lib.check(rc)
         return out
 
     def gemv_push(self, x: torch.Tensor, ar) -> int:
