@@ -152,7 +152,7 @@ class StreamingLinear(nn.Module):
             elif self._use_p6_gemm and self.in_features % 64 == 0:
                 y = res.gemm(x, bias=self._bias_bf16)
             elif self._use_p6_gemm and rows > FUSED_MAX_ROWS and self._bias is None and self.in_features % 8 == 0 \
-                    and self._w_buf is not None and _plain(x):
+                    and self._w_buf is not None and x.get_device() == res._index and _plain(x):
                 # Without a bias, which decode + dense matmul adds before the one rounding.  A call outside a graph, this
                 # kernel and that route: 2048 x 2080 10.4 and 21.4 us with 24 rows, 12.5 and 21.4 with 64; 8192 x 8224 32
                 # and 56, 48 and 60.  (Above 48 rows layers of 25 to 40 million weights lose up to 7 us: 6144 x 6176 25.5

@@ -153,8 +153,8 @@ class P6Packed:
 
     def _rows(self, x: torch.Tensor) -> torch.Tensor:
         """x as contiguous bf16 rows [M, in_f]"""
-        if x.dtype != torch.bfloat16:
-            raise ValueError("activations must be bf16")
+        if x.dtype != torch.bfloat16 or not x.is_cuda:
+            raise ValueError("activations must be bf16 on a GPU")
         if x.dim() != 2 or x.shape[1] != self.in_f:
             x = x.reshape(-1, self.in_f)
         return x if x.is_contiguous() else x.contiguous()

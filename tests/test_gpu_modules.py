@@ -289,3 +289,27 @@ def test_streaming_linear_passes_keep_what_a_dense_matmul_gives(in_f, rows):
     with fwAD.dual_level():
         y, tangent = fwAD.unpack_dual(lin(fwAD.make_dual(x, t)))
         assert ok(y, ref) and ok(tangent, t.double() @ wd.t())
+
+
+@pytest.mark.parametrize("in_f", [1024, 1056])
+def test_streaming_linear_refuses_host_activations(monkeypatch, in_f):
+    """No host pointer reaches a kernel: refused by the wrapper, or by the dense matmul where that took the call before.  (The
+    library is replaced by one that fails the test when a kernel on the activations is asked for.)"""
+    from ixrun_b200 import _lib
+    from ixrun_b200.engine import StreamingLinear
+
+    w = (torch.randn(64, in_f, device="cuda") * 0.05).bfloat16()
+    lin = StreamingLinear.from_weight(w)
+    lin._set_shared_buf(torch.empty(64 * in_f, dtype=torch.bfloat16, device="cuda"))
+    real = _lib.lib()
+
+    class NoLaunch:
+        def __getattr__(self, name):
+            if name in ("ixb_p6_gemv", "ixb_p6_gemm", "ixb_p6_rows"):
+                return lambda *a: pytest.fail(f"{name} was called")
+            return getattr(real, name)
+
+    monkeypatch.setattr(_lib, "lib", lambda: NoLaunch())
+    for rows in (1, 8, 9, 64, 65):
+        with pytest.raises((ValueError, RuntimeError)):
+            lin(torch.zeros(rows, in_f).bfloat16())
