@@ -30,11 +30,14 @@ TC_MAX_ROWS = 64          # rows served by the tensor-core fused kernel (when en
 
 
 def _plain(x) -> bool:
-    """True if nothing but the values of x is asked of an operation on it: no gradient, tangent, batching transform or
-    trace that a dense matmul would carry and a kernel on raw pointers would drop."""
+    """True if nothing but the values of x is asked of an operation on it: no gradient, tangent, batching transform,
+    trace, autocast or mode that a dense matmul would carry and a kernel on raw pointers would drop, and x's memory holds
+    its values (a strided tensor without a pending negation)."""
     return type(x) is torch.Tensor and not (x.requires_grad and torch.is_grad_enabled()) and forward_ad._current_level < 0 \
         and torch._C._functorch.peek_interpreter_stack() is None and not torch.jit.is_tracing() \
-        and not torch.compiler.is_compiling()
+        and not torch.compiler.is_compiling() and not torch.is_autocast_enabled("cuda") \
+        and not torch._C._is_torch_function_mode_enabled() and torch._C._len_torch_dispatch_stack() == 0 \
+        and x.layout == torch.strided and not x.is_neg()
 
 
 class StreamingLinear(nn.Module):

@@ -313,3 +313,40 @@ def test_streaming_linear_refuses_host_activations(monkeypatch, in_f):
     for rows in (1, 8, 9, 64, 65):
         with pytest.raises((ValueError, RuntimeError)):
             lin(torch.zeros(rows, in_f).bfloat16())
+
+
+def test_streaming_linear_leaves_autocast_and_modes_to_the_dense_matmul():
+    """9..64 rows with in_f not a multiple of 64: the result's type under autocast, what dispatch and function modes see, and
+    an input with a pending negation, as with decode + dense matmul."""
+    from torch.overrides import TorchFunctionMode
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    from ixrun_b200.engine import StreamingLinear
+
+    lin = StreamingLinear.from_weight((torch.randn(64, 1056, device="cuda") * 0.05).bfloat16())
+    lin._set_shared_buf(torch.empty(64 * 1056, dtype=torch.bfloat16, device="cuda"))
+    x = torch.randn(24, 1056, device="cuda").bfloat16()
+    with torch.no_grad():
+        y = lin(x)
+        with torch.autocast("cuda", dtype=torch.float16):
+            assert lin(x).dtype == torch.float16
+        seen = []
+
+        class Dispatch(TorchDispatchMode):
+            def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+                seen.append(str(func))
+                return func(*args, **(kwargs or {}))
+
+        class Function(TorchFunctionMode):
+            def __torch_function__(self, func, types, args=(), kwargs=None):
+                seen.append(func.__name__)
+                return func(*args, **(kwargs or {}))
+
+        with Dispatch():
+            lin(x)
+        assert any("mm" in s for s in seen)
+        seen.clear()
+        with Function():
+            lin(x)
+        assert "linear" in seen
+        assert (lin(torch._neg_view(x)).float() + y.float()).abs().max() <= 2.0 ** -7 * y.float().abs().max()
