@@ -2,15 +2,20 @@
 // new rows sits at position pos0 + r, its key and value are in the cache already, and it attends to positions
 // 0 .. pos0 + r.  The eager path runs this as fp32 matmuls around a masked softmax over the whole static cache.
 //
-// Bound: the tensor core (4 MMA steps of 16 x 8 x 16 per 16 x 8 scores and head dimension 16: one for Q K^T, two for
-// P V): a 1000-row prompt's 16 x 136 pairs of 64-row and 64-key tiles of 16 heads are 12.6 us at mma.sync's rate.  What it
+// Bound: the tensor core (8 MMA steps of 16 x 8 x 16 per 16 x 16 scores and head dimension 16: two for Q K^T, six for
+// P V): a 1000-row prompt's 16 x 136 pairs of 64-row and 64-key tiles of 16 heads are 17 us at mma.sync's rate.  What it
 // has to fight is the chain of key tiles of the last rows and the uneven lengths: CTA = 64 rows of one query head, two
 // groups of four warps (16 rows a warp) take the even and the odd key tiles, each through its own two cp.async stages, and
 // join at the end; the row tiles with the longest contexts of all heads start first.  Q K^T: bf16 operands, fp32 sums.  The
-// probabilities stay fp32-like: p = hi + lo with two bf16 numbers (17 significant bits) and two MMAs, so nothing is lost
-// against the fp32 path; the denominator is summed from the fp32 values.
-// Measured (1000 rows, 16 query / 8 KV heads of 128, under the profiler): 34 us; 50 with one group per CTA and the heads
-// one after the other.
+// probabilities are held in fp32, and so are they multiplied: p = three bf16 numbers of 8 significant bits each, three MMAs.
+// The tensor core cuts the low bits of what it adds to a large sum, so a key tile's P V starts from zero and joins the
+// running sums by fp32 fused multiply-adds; the denominator is summed from the fp32 values.
+// (An infinite value in the cache gives NaN: the parts of a probability may be zero or negative.)
+// Against 64 bits (16 / 8 heads of 128, 4 / 4 and 8 / 1 of 64; 65 to 1000 rows, and 200 behind 1500; scores and values of
+// three sizes): the share of outputs that are not the correctly rounded bf16 number is 0.5 to 50 in 100,000, that of fp32
+// matmuls around a softmax 1 to 130; 5 to 260 with two bf16 numbers and running sums in the tensor core.
+// Measured (16 query / 8 KV heads of 128, graph): 65 / 300 / 1000 / 2048 rows 6.9 / 13.5 / 37 / 128 us, with two bf16
+// numbers 6.4 / 12.5 / 34 / 115; with one group per CTA and the heads one after the other 50 for 1000 rows.
 #pragma once
 #include "ixb_p6.cuh"
 
@@ -126,28 +131,40 @@ k_attn_prefill(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat16 *__restr
                 s[n][i] = exp2f(s[n][i] - base[i >> 1]);
                 l[i >> 1] += s[n][i];
             }
+        // probabilities as three bf16 numbers whose sum they are (8 significant bits each; the differences are exact):
+        // [part][keys 16 kk][a0: row g, keys 2 t; a1: row g + 8; a2, a3: keys 8 further]
+        uint32_t pa[3][kApKeys / 16][4];
 #pragma unroll
-        for (int n = 0; n < D / 8; ++n) {
-            o[n][0] *= corr[0]; o[n][1] *= corr[0];
-            o[n][2] *= corr[1]; o[n][3] *= corr[1];
-        }
-#pragma unroll
-        for (int kk = 0; kk < kApKeys / 16; ++kk) {
-            uint32_t hi[4], lo[4];                      // a0: row g, keys 2 t; a1: row g + 8; a2, a3: keys 8 further
+        for (int kk = 0; kk < kApKeys / 16; ++kk)
 #pragma unroll
             for (int a = 0; a < 4; ++a) {
-                const float x0 = s[2 * kk + (a >> 1)][2 * (a & 1)], x1 = s[2 * kk + (a >> 1)][2 * (a & 1) + 1];
-                hi[a] = ap_pack(x0, x1);
-                lo[a] = ap_pack(x0 - __uint_as_float(hi[a] << 16), x1 - __uint_as_float(hi[a] & 0xFFFF0000u));
+                float x0 = s[2 * kk + (a >> 1)][2 * (a & 1)], x1 = s[2 * kk + (a >> 1)][2 * (a & 1) + 1];
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    pa[c][kk][a] = ap_pack(x0, x1);
+                    x0 -= __uint_as_float(pa[c][kk][a] << 16);
+                    x1 -= __uint_as_float(pa[c][kk][a] & 0xFFFF0000u);
+                }
             }
 #pragma unroll
-            for (int d2 = 0; d2 < D / 16; ++d2) {
+        for (int d2 = 0; d2 < D / 16; ++d2) {
+            float w[2][4];                              // the tile's own sums: the tensor core cuts what it adds to a large one
+#pragma unroll
+            for (int i = 0; i < 4; ++i) w[0][i] = w[1][i] = 0.f;
+#pragma unroll
+            for (int kk = 0; kk < kApKeys / 16; ++kk) {
                 uint32_t b[4];                          // keys 16 kk .. + 15, dimensions 16 d2 .. + 15
                 ap_ldmatrix_t(b, sv + st + ((kk * 16 + (lane & 15)) * PITCH + d2 * 16 + (lane >> 4) * 8) * 2u);
-                p6_mma(o[2 * d2], hi[0], hi[1], hi[2], hi[3], b[0], b[1]);
-                p6_mma(o[2 * d2 + 1], hi[0], hi[1], hi[2], hi[3], b[2], b[3]);
-                p6_mma(o[2 * d2], lo[0], lo[1], lo[2], lo[3], b[0], b[1]);
-                p6_mma(o[2 * d2 + 1], lo[0], lo[1], lo[2], lo[3], b[2], b[3]);
+#pragma unroll
+                for (int c = 2; c >= 0; --c) {
+                    p6_mma(w[0], pa[c][kk][0], pa[c][kk][1], pa[c][kk][2], pa[c][kk][3], b[0], b[1]);
+                    p6_mma(w[1], pa[c][kk][0], pa[c][kk][1], pa[c][kk][2], pa[c][kk][3], b[2], b[3]);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                o[2 * d2][i] = fmaf(o[2 * d2][i], corr[i >> 1], w[0][i]);
+                o[2 * d2 + 1][i] = fmaf(o[2 * d2 + 1][i], corr[i >> 1], w[1][i]);
             }
         }
         cp_async_wait<0>();

@@ -229,8 +229,7 @@ def test_attn_decode_recovers_from_overlapping_launches():
 def test_attn_prefill(hq, hkv, d, rows, pos0):
     """Row and key tiles of 64: one row, one short of a tile, a whole one, one more; from the start and behind a context.
     Bound: the bf16 output is off by at most half a unit in the last place, 2^-8 of the value (8 significant bits; the
-    value may sit at the bottom of its binade); probabilities of 17 bits that sum to 1 add 2^-17 of the largest value, the
-    fp32 exponentials and sums less than 2^-17 of it."""
+    value may sit at the bottom of its binade); the fp32 exponentials and sums add less than 2^-16 of the largest value."""
     from ixrun_b200.glue import attn_prefill
 
     max_seq, dev = pos0 + rows + 30, "cuda"
