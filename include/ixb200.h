@@ -221,11 +221,13 @@ size_t ixb_p6_gemv_scratch_bytes(int64_t out_f, int64_t in_f, int64_t m_rows);
 int ixb_p6_gemv(const ixb_p6 *t, const void *x_device, int64_t m_rows, const void *bias_device,
                 void *y_device, int y_is_f32, void *scratch_device, size_t scratch_bytes, ixb_stream_t stream);
 /* Small-M GEMM on the resident layout: 1..64 activation rows, y[m][n] as ixb_p6_gemv defines it, in one pass over
- * the tensor's bytes; the bf16 weights exist only in registers, and the sums of K splits are joined inside a cluster of
- * CTAs in a fixed order (reproducible).  Takes the place of the reference's decode + dense matmul for 9..64 rows
+ * the tensor's bytes; the bf16 weights exist only in registers or shared memory, and the sums of K splits are added in a
+ * fixed order (reproducible).  Takes the place of the reference's decode + dense matmul for 9..64 rows
  * (ixrun/engine.py:171-173; precedent for a fused kernel: ixrun/tpab_gemm.py:34-94).
- * ixb_p6_gemm: in_f a multiple of 64; scratch: ixb_p6_gemm_scratch_bytes bytes, 256-byte aligned, any contents (a few
- *   bytes today).  ixb_p6_rows: the same without scratch, in_f a multiple of 8. */
+ * ixb_p6_rows: in_f a multiple of 8, no scratch (splits are joined inside a cluster of CTAs).
+ * ixb_p6_gemm: in_f a multiple of 64; scratch of at least 256 bytes, 256-byte aligned, any contents.  With
+ *   ixb_p6_gemm_scratch_bytes bytes it may take a tcgen05 kernel whose partial sums lie there, for more than 32 rows of the
+ *   layers where that is faster; with fewer it is ixb_p6_rows. */
 int ixb_p6_rows(const ixb_p6 *t, const void *x_device, int64_t m_rows, const void *bias_device, void *y_device, int y_is_f32,
                 ixb_stream_t stream);
 size_t ixb_p6_gemm_scratch_bytes(int64_t out_f, int64_t in_f, int64_t m_rows);

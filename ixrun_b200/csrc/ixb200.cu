@@ -6,6 +6,7 @@
 #include "ixb_common.cuh"
 #include "ixb_gemm_tc.cuh"
 #include "ixb_attn_prefill.cuh"
+#include "ixb_p6_gemm.cuh"
 #include "ixb_p6_rows.cuh"
 #include "ixb_pack.cuh"
 #include "ixb_p6.cuh"
@@ -1607,39 +1608,128 @@ static int pr_resident(int v, int s, int *out)
 }
 
 // K splits (CTAs of a cluster) for a row count: the fewest rounds of steps over the whole grid.  A step is one column block
-// per part, about 0.6 us; joining the splits' sums through distributed shared memory costs about two of them.
-static int pr_splits(const P6 &p, int v, uint32_t *splits)
+// per part; what a round costs beside its steps is about four of them, and joining the splits' sums through distributed
+// shared memory two.  (Eleven layers of 1024 x 3072 to 17408 x 5120, 16 to 64 rows, 1 to 8 splits each: the choice is within
+// 0.3 us of the best.)
+struct PrPlan {
+    uint32_t splits, rounds, steps;
+};
+static int pr_plan(uint32_t rt, uint32_t kb, int v, PrPlan *plan)
 {
-    const uint32_t groups = (p.rt + kPrTiles - 1) / kPrTiles, parts = kPrVariants[v].parts;
+    const uint32_t groups = (rt + kPrTiles - 1) / kPrTiles, parts = kPrVariants[v].parts;
     uint32_t best = 0;
-    for (uint32_t s = 1; s <= (uint32_t)kPrMaxSplits && s <= p.kb; ++s) {
+    for (uint32_t s = 1; s <= (uint32_t)kPrMaxSplits && s <= kb; ++s) {
         int resident = 0, rc = pr_resident(v, (int)s, &resident);
         if (rc) return rc;
         const uint32_t rounds = (groups * s + (uint32_t)resident - 1) / (uint32_t)resident;
-        const uint32_t steps = ((p.kb + s - 1) / s + parts - 1) / parts;
+        const uint32_t steps = ((kb + s - 1) / s + parts - 1) / parts;
         const uint32_t cost = rounds * (steps + 4u + (s > 1u ? 2u : 0u));
         if (!best || cost < best) {
             best = cost;
-            *splits = s;
+            *plan = {s, rounds, steps};
         }
     }
     return IXB_OK;
+}
+static int pr_variant_of(uint32_t m_rows)
+{
+    int v = 0;
+    while (kPrVariants[v].nt * 8u < m_rows) ++v;
+    return v;
+}
+
+static PgPlan make_pg_plan(uint32_t out_f, uint32_t in_f)
+{
+    PgPlan p;
+    const uint32_t rt = (out_f + kTileRows - 1) / kTileRows, kb = (in_f + kTileCols - 1) / kTileCols;
+    p.groups = (rt + kPgConv - 1) / kPgConv;
+    // K is split only as far as it takes to give about every SM one CTA; a split keeps at least eight column blocks
+    uint32_t splits = std::max<uint32_t>(1u, (uint32_t)num_sms() / p.groups);
+    splits = std::min<uint32_t>(splits, std::max<uint32_t>(1u, kb / 8u));
+    p.splits = std::min<uint32_t>(splits, 16u);
+    p.grid = p.groups * p.splits;
+    return p;
+}
+
+// Whether k_p6_gemm (and its finalizing kernel) takes less time than k_p6_rows, in us, from lines through the measured times
+// of eleven layers at 33, 40, 48, 56 and 64 rows (within 6 % for this kernel, 8 % for the other): up to 32 rows k_p6_rows is
+// the faster one everywhere (but by 0.4 us at 300 x 16384).
+static bool pg_is_faster(uint32_t out_f, uint32_t in_f, uint32_t m_rows, const PrPlan &pr)
+{
+    if (m_rows <= 32u || in_f % kTileCols) return false;
+    const uint32_t nt = kPrVariants[pr_variant_of(m_rows)].nt;
+    const float per_step = nt <= 5u ? 1.31f : nt <= 6u ? 1.43f : 1.66f, fixed = (nt <= 5u ? 5.2f : nt <= 6u ? 5.4f : 6.0f) - (pr.splits == 1u ? 2.5f : 0.f);
+    const float t_rows = (float)pr.rounds * (fixed + per_step * (float)pr.steps);
+    const PgPlan pg = make_pg_plan(out_f, in_f);
+    const float stages = (float)((in_f / kTileCols + pg.splits - 1) / pg.splits);
+    const float per_stage = 0.405f + (m_rows > 48u ? 0.0055f * (float)(m_rows - 48u) : 0.f);
+    const float t_gemm = 8.6f + 4e-6f * (float)m_rows * (float)out_f + per_stage * stages;
+    return t_gemm < 0.96f * t_rows;
+}
+static size_t pg_scratch_bytes(const PgPlan &plan, uint32_t out_f, uint32_t m_rows)
+{
+    return 256 + (size_t)plan.splits * m_rows * out_f * sizeof(float);
 }
 
 extern "C" size_t ixb_p6_gemm_scratch_bytes(int64_t out_f, int64_t in_f, int64_t m_rows)
 {
     if (out_f <= 0 || in_f <= 0 || m_rows < 1 || m_rows > kPrMaxRows || out_f * in_f > 800000000LL) return 0;
-    return 256;                                          // (sums of K splits stay in shared memory)
+    const uint32_t o = (uint32_t)out_f, i = (uint32_t)in_f, m = (uint32_t)m_rows;
+    PrPlan pr = {1, 1, 1};
+    if (m <= 32u || pr_plan((o + kTileRows - 1) / kTileRows, (i + kTileCols - 1) / kTileCols, pr_variant_of(m), &pr)) return 256;
+    return pg_is_faster(o, i, m, pr) ? pg_scratch_bytes(make_pg_plan(o, i), o, m) : 256;
+}
+
+static int p6_rows_run(const P6 &p, const void *x, uint32_t m_rows, const void *bias, void *y, int y_is_f32, const PrPlan &plan,
+                       ixb_stream_t stream);
+static int p6_rows_args(const P6 &p, const void *x, int64_t m_rows, const void *y)
+{
+    if (!x || !y) return fail(IXB_E_ARG, "NULL pointer argument");
+    if (m_rows < 1 || m_rows > kPrMaxRows) return fail(IXB_E_UNSUPPORTED, "m_rows=%lld outside 1..%d", (long long)m_rows, kPrMaxRows);
+    if (p.in_f % 8u) return fail(IXB_E_UNSUPPORTED, "in_f=%u is not a multiple of 8", p.in_f);
+    if ((uintptr_t)x & 15u) return fail(IXB_E_ARG, "x is not 16-byte aligned");
+    return IXB_OK;
 }
 
 extern "C" int ixb_p6_gemm(const ixb_p6 *t, const void *x, int64_t m_rows, const void *bias, void *y, int y_is_f32,
                            void *scratch, size_t scratch_bytes, ixb_stream_t stream)
 {
-    if (!t || !x || !y || !scratch) return fail(IXB_E_ARG, "NULL pointer argument");
-    if (t->in_f % kTileCols) return fail(IXB_E_UNSUPPORTED, "in_f=%lld is not a multiple of %d", (long long)t->in_f, kTileCols);
+    P6 p;
+    int rc = to_p6(t, &p);
+    if (rc) return rc;
+    if (!scratch) return fail(IXB_E_ARG, "NULL pointer argument");
+    if (p.in_f % (uint32_t)kTileCols) return fail(IXB_E_UNSUPPORTED, "in_f=%u is not a multiple of %d", p.in_f, kTileCols);
     if ((uintptr_t)scratch & 255u) return fail(IXB_E_ARG, "scratch is not 256-byte aligned");
     if (scratch_bytes < 256u) return fail(IXB_E_SCRATCH, "gemm scratch too small");
-    return ixb_p6_rows(t, x, m_rows, bias, y, y_is_f32, stream);
+    if ((rc = p6_rows_args(p, x, m_rows, y))) return rc;
+    PrPlan pr = {1, 1, 1};
+    if ((rc = pr_plan(p.rt, p.kb, pr_variant_of((uint32_t)m_rows), &pr))) return rc;
+    const PgPlan plan = make_pg_plan(p.out_f, p.in_f);
+    // a scratch of 256 bytes is enough for every call: k_p6_rows needs none
+    if (!pg_is_faster(p.out_f, p.in_f, (uint32_t)m_rows, pr) || scratch_bytes < pg_scratch_bytes(plan, p.out_f, (uint32_t)m_rows))
+        return p6_rows_run(p, x, (uint32_t)m_rows, bias, y, y_is_f32, pr, stream);
+    cudaStream_t st = (cudaStream_t)stream;
+    static bool attr_set[64] = {false};
+    IXB_CUDA(opt_in_smem(k_p6_gemm, attr_set, (int)kPgSmemBytes));
+    uint32_t *err = (uint32_t *)scratch;
+    float *part = (float *)((char *)scratch + 256);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(plan.grid);
+    cfg.blockDim = dim3(kPgThreads);
+    cfg.dynamicSmemBytes = kPgSmemBytes;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = g_p6_pdl.load() ? 1 : 0;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, k_p6_gemm, p, (const __nv_bfloat16 *)x, (uint32_t)m_rows, part, err, plan);
+    if (e != cudaSuccess) return fail(IXB_E_CUDA, "k_p6_gemm launch: %s", cudaGetErrorString(e));
+    if ((rc = launch_check("k_p6_gemm"))) return rc;
+    const uint32_t total = (uint32_t)m_rows * p.out_f;
+    IXB_GLUE("k_gemm_finalize", launch_glue(k_gemm_finalize, dim3((total + 255) / 256), dim3(256), st, (const float *)part,
+                                            plan.splits, (uint32_t)m_rows, p.out_f, (const __nv_bfloat16 *)bias, y, y_is_f32,
+                                            (const uint32_t *)err));
 }
 
 extern "C" int ixb_p6_rows(const ixb_p6 *t, const void *x, int64_t m_rows, const void *bias, void *y, int y_is_f32,
@@ -1647,15 +1737,17 @@ extern "C" int ixb_p6_rows(const ixb_p6 *t, const void *x, int64_t m_rows, const
 {
     P6 p;
     int rc = to_p6(t, &p);
-    if (rc) return rc;
-    if (!x || !y) return fail(IXB_E_ARG, "NULL pointer argument");
-    if (m_rows < 1 || m_rows > kPrMaxRows) return fail(IXB_E_UNSUPPORTED, "m_rows=%lld outside 1..%d", (long long)m_rows, kPrMaxRows);
-    if (p.in_f % 8u) return fail(IXB_E_UNSUPPORTED, "in_f=%u is not a multiple of 8", p.in_f);
-    if ((uintptr_t)x & 15u) return fail(IXB_E_ARG, "x is not 16-byte aligned");
-    int v = 0;
-    while (kPrVariants[v].nt * 8u < (uint32_t)m_rows) ++v;
-    uint32_t splits = 1;
-    if ((rc = pr_splits(p, v, &splits))) return rc;
+    if (rc || (rc = p6_rows_args(p, x, m_rows, y))) return rc;
+    PrPlan plan = {1, 1, 1};
+    if ((rc = pr_plan(p.rt, p.kb, pr_variant_of((uint32_t)m_rows), &plan))) return rc;
+    return p6_rows_run(p, x, (uint32_t)m_rows, bias, y, y_is_f32, plan, stream);
+}
+
+static int p6_rows_run(const P6 &p, const void *x, uint32_t m_rows, const void *bias, void *y, int y_is_f32, const PrPlan &plan,
+                       ixb_stream_t stream)
+{
+    const int v = pr_variant_of(m_rows);
+    const uint32_t splits = plan.splits;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((p.rt + kPrTiles - 1) / kPrTiles * splits);
     cfg.blockDim = dim3(kPrVariants[v].parts * 128u);
@@ -1669,7 +1761,7 @@ extern "C" int ixb_p6_rows(const ixb_p6 *t, const void *x, int64_t m_rows, const
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = g_p6_pdl.load() ? 2 : 1;
-    IXB_GLUE("k_p6_rows", cudaLaunchKernelEx(&cfg, kPrVariants[v].kernel, p, (const __nv_bfloat16 *)x, (uint32_t)m_rows,
+    IXB_GLUE("k_p6_rows", cudaLaunchKernelEx(&cfg, kPrVariants[v].kernel, p, (const __nv_bfloat16 *)x, m_rows,
                                              (const __nv_bfloat16 *)bias, y, y_is_f32, splits));
 }
 

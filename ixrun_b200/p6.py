@@ -95,7 +95,7 @@ class P6Packed:
                                     self.scale.data_ptr(), self.out_f, self.in_f, stride)
         self._ref = C.byref(self.struct)             # (keeps the struct alive)
         self._index = dev.index
-        self._gemv_need = None
+        self._gemv_need, self._gemm_need = None, {}      # scratch bytes; the latter by row count
         self.resident_bytes = nb * BLOCK_BYTES + 4 * (nb + 1 + n_esc) + 2
         self.scratch = scratch if scratch is not None else GemvScratch.shared(dev)
 
@@ -199,7 +199,11 @@ class P6Packed:
             raise ValueError(f"unsupported GEMM shape: {m} rows")
         L = _lib.lib()
         with _lib.on_device(self._index) as stream:
-            s = self.scratch.reserve(256)                # (checked, not used: the splits' sums stay in shared memory)
+            need = self._gemm_need.get(m)
+            if need is None:
+                need = self._gemm_need[m] = int(L.ixb_p6_gemm_scratch_bytes(self.out_f, self.in_f, m))
+            # partial sums of the tcgen05 form: a buffer of the call's own, so calls on several streams do not share it
+            s = self.scratch.reserve(256) if need <= 256 else torch.empty(need, dtype=torch.uint8, device=self.device)
             rc = L.ixb_p6_gemm(self._ref, x2.data_ptr(), m, None if bias is None else bias.data_ptr(), out.data_ptr(),
                                1 if out.dtype == torch.float32 else 0, s.data_ptr(), s.numel(), stream)
         if rc:
