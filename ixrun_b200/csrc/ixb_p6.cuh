@@ -10,8 +10,9 @@
 //           a bf16 number of the binade [64, 128):
 //             (F << 1) | 0x4280 = 64 + F = 96 + code
 //           so a packed subtraction of 96 gives the code exactly, and the packed multiplication by the scale (plus 0, so
-//           that code 0 gives +0.0 whatever the scale's sign) rounds the exact product once: the reference's dequantised weight bf16(f32(code) * f32(scale))
-//           (ixrun/quantize.py:182, ixrun/fused.py:169-170), bit for bit, for any scale.
+//           that code 0 gives +0.0 whatever the scale's sign) rounds the exact product once: the reference's dequantised
+//           weight bf16(f32(code) * f32(scale)) (ixrun/quantize.py:182, ixrun/fused.py:169-170), bit for bit, for any
+//           scale (but for the sign of that zero).
 //           Other codes ("outliers") leave the placeholder F = 32 (weight 0).  (Before, F was part of 1 + code / 32 over
 //           two binades, one fused multiply-add per pair instead of two operations, but it held -16 .. 31 only: 1.2 % of
 //           the benchmark distribution were outliers, 4 bytes and an extra step each, against 0.07 % now.)

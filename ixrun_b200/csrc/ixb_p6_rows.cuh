@@ -7,12 +7,13 @@
 // precedent for a fused kernel: ixrun/tpab_gemm.py:34-94).  Here the weights become the A operands of mma.sync in
 // registers, as in the GEMV (k_p6_mma).
 //
-// What bounds it: 6.4 bits of HBM per weight and about six instructions per pair of weights for the conversion, the same
-// as the GEMV; on top of that one mma per 16 x 16 weights and eight rows, 64 rows being where the mma rate takes over.
-// Feeding the converted weights to tcgen05 through shared memory instead (the form this kernel replaced) moves four
-// bytes of shared memory per weight and hands every 64 columns over twice between converters, copies and tensor core:
-// 17408 x 5120 took 40 us at 16 rows and 57 us at 64, of which 27 us were hand-over with no work in it.  Here nothing
-// is handed over between warps but the activations: 26 and 47 us.
+// What bounds it: 6.05 bits of HBM per weight and four instructions per pair of weights for the conversion (six where the
+// field is split), the same as the GEMV; on top of that one mma per 16 x 16 weights and eight rows, 64 rows being where the
+// mma rate takes over.  Feeding the converted weights to tcgen05 through shared memory instead (k_p6_gemm) moves four bytes of
+// shared memory per weight and hands every 64 columns over twice between converters, copies and tensor core: 17408 x 5120
+// takes 40 us there at 16 rows and 57 us at 64, of which 27 us are hand-over with no work in it.  Here nothing is handed over
+// between warps but the activations: 26 and 49 us.  (Where the row groups do not fill the chip, k_p6_gemm is the faster one
+// above 32 rows: pg_is_faster.)
 //
 // CTA  = 8 row tiles (128 weight rows) x a contiguous range of column blocks; K is split over the CTAs of a cluster as
 //        far as it takes to fill the chip, and the splits' sums are added in rank order through distributed shared memory.
@@ -166,22 +167,18 @@ k_p6_rows(P6 p, const __nv_bfloat16 *__restrict__ x, uint32_t m_rows, const __nv
             const int32_t lo = __shfl_sync(0xffffffffu, off_l[i], (int)(s - win)), hi = __shfl_sync(0xffffffffu, off_l[i], (int)(s + 1u - win));
             if (!have[i] || lo == hi) continue;        // (warp uniform) no outliers in the block
             // the block's outliers into the image
-            auto at = [&](uint32_t e) {                // where the entry's element lies among the lanes' A registers (inverse of p6_elem)
-                const uint32_t r = (e >> 12) & 15u, c = e & 63u;
-                return img_s + ((((c >> 2) & 3u) * 32u + 4u * (r & 7u) + (c >> 4)) * 4u + 2u * ((c >> 1) & 1u) + (r >> 3)) * 4u + 2u * (c & 1u);
-            };
             auto patch = [&](uint32_t where, uint32_t v) {
                 asm volatile("st.shared.u16 [%0], %1;" ::"r"(where), "h"((unsigned short)v) : "memory");
             };
             uint32_t where = 0;
             if (lo + lane < hi) {
                 const uint32_t e = p6_lds32(d + kP6BlockBytes + lane * 4);
-                where = at(e);
+                where = img_s + p6_image_at(e);
                 patch(where, e >> 16);
             }
             for (int32_t j = lo + 32 + lane; j < hi; j += 32) {        // rare: more than 32 in a block
                 const uint32_t e = __ldg(p.esc + j);
-                patch(at(e), e >> 16);
+                patch(img_s + p6_image_at(e), e >> 16);
             }
             __syncwarp();
 #pragma unroll
@@ -194,7 +191,7 @@ k_p6_rows(P6 p, const __nv_bfloat16 *__restrict__ x, uint32_t m_rows, const __nv
             }
             __syncwarp();
             if (lo + lane < hi) patch(where, 0);
-            for (int32_t j = lo + 32 + lane; j < hi; j += 32) patch(at(__ldg(p.esc + j)), 0);
+            for (int32_t j = lo + 32 + lane; j < hi; j += 32) patch(img_s + p6_image_at(__ldg(p.esc + j)), 0);
             __syncwarp();
         }
         const uint32_t xb = xpart + slot_of(s) * (PARTS * SM::kX) + xl;
