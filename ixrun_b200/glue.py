@@ -125,6 +125,8 @@ class AttnDecode:
             splits = max(1, min(256, sms // (groups * self.batch)))
         self.splits = int(splits)
         self.tickets = torch.zeros(self.batch * hq, dtype=torch.int32, device=device)     # zero between launches
+        if self.tickets.is_cuda and not torch.cuda.is_current_stream_capturing():
+            torch.cuda.current_stream(self.tickets.device).synchronize()       # zero for a first call on any stream
         self.scratch = torch.empty(self.batch * _lib.lib().ixb_attn_scratch_bytes(hq, head_dim, self.splits), dtype=torch.uint8,
                                    device=device)
 

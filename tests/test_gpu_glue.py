@@ -224,6 +224,24 @@ def test_attn_decode_recovers_from_overlapping_launches():
         assert torch.equal(ad(q, kc, vc, p), w)
 
 
+def test_attn_decode_is_ready_for_any_stream():
+    """An object made on a busy stream, in memory that held something else, and first called on another stream."""
+    from ixrun_b200.glue import AttnDecode
+
+    bf = dict(dtype=torch.bfloat16, device="cuda")
+    kc, vc, q = torch.randn(1200, 2, 128, **bf), torch.randn(1200, 2, 128, **bf), torch.randn(512, **bf)
+    pos = torch.tensor([1100], dtype=torch.int32, device="cuda")
+    want = AttnDecode(4, 2, 128, "cuda", splits=18)(q, kc, vc, pos)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(torch.cuda.Stream()):
+        held = torch.full((4,), 7, dtype=torch.int32, device="cuda")
+        torch.cuda.synchronize()
+        del held                                                   # its block is the next one of this size on this stream
+        torch.cuda._sleep(20_000_000)
+        ad = AttnDecode(4, 2, 128, "cuda", splits=18)
+    assert torch.equal(ad(q, kc, vc, pos), want)
+
+
 @pytest.mark.parametrize("rows,pos0", [(1, 0), (1, 90), (63, 0), (64, 64), (65, 0), (200, 37)])
 @pytest.mark.parametrize("hq,hkv,d", [(4, 2, 64), (3, 3, 128), (6, 1, 128)])
 def test_attn_prefill(hq, hkv, d, rows, pos0):
