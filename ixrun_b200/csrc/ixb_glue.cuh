@@ -527,8 +527,10 @@ k_attn_decode(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat16 *__restri
     __syncthreads();
     if (ctas > 1u) {
         if (threadIdx.x == 0) {
-            const uint32_t mine = blockIdx.y ? 1u : gridDim.y - ctas + 1u, before = atomicAdd(ticket, mine);
-            sm_last = before % gridDim.y + mine >= gridDim.y;
+            const uint32_t mine = blockIdx.y ? 1u : gridDim.y - ctas + 1u;
+            uint32_t before = atomicAdd(ticket, mine);
+            if (before >= gridDim.y) before %= gridDim.y;              // (launches that overlap)
+            sm_last = before + mine >= gridDim.y;
         }
         __syncthreads();
         if (!sm_last) return;
