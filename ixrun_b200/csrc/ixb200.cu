@@ -1652,7 +1652,8 @@ static PgPlan make_pg_plan(uint32_t out_f, uint32_t in_f)
 }
 
 // Whether k_p6_gemm (and its finalizing kernel) takes less time than k_p6_rows, in us, from lines through the measured times
-// of eleven layers at 33, 40, 48, 56 and 64 rows (within 6 % for this kernel, 8 % for the other): up to 32 rows k_p6_rows is
+// of eleven layers at 33, 40, 48, 56 and 64 rows (most within 6 %).  It is taken where it is the faster one by more than 4 %,
+// and was then on all of them; at most 3 % are left (8192 x 8192 with 64 rows, 41.8 and 42.8 us).  Up to 32 rows k_p6_rows is
 // the faster one everywhere (but by 0.4 us at 300 x 16384).
 static bool pg_is_faster(uint32_t out_f, uint32_t in_f, uint32_t m_rows, const PrPlan &pr)
 {

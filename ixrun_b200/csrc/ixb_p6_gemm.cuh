@@ -8,8 +8,8 @@
 // 0.5 at 64, and 8.6 us around it; k_p6_rows has no such hand-over, but its time per step grows with the rows (1.3 us per
 // three column blocks at 40 rows, 1.7 at 64), and its K splits are at most a cluster.  So this kernel is the faster one where
 // a CTA has many column blocks or the row groups are few.  Here and there, graph with dependent launch, 40 / 56 / 64 rows:
-// 6144 x 5120 21.3 / 24.0 / 25.5 and 23.1 / 28.6 / 29.2 us, 300 x 16384 14.5 / 15.5 / 15.9 and 18.4 / 23.0 / 23.3,
-// 5120 x 17408 47.2 / 50.5 / 54.5 and 45.7 / 57.0 / 57.8; 17408 x 5120 45.9 / 55.5 / 57.0 and 38.4 / 48.2 / 48.6.
+// 6144 x 5120 21.0 / 24.2 / 24.8 and 23.1 / 28.6 / 29.2 us, 300 x 16384 14.3 / 15.2 / 15.8 and 18.4 / 23.0 / 23.3,
+// 5120 x 17408 44.6 / 49.4 / 52.0 and 45.7 / 57.0 / 57.8; 17408 x 5120 47.3 / 54.4 / 59.7 and 38.4 / 48.2 / 48.6.
 //
 //   CTA      = 128 weight rows (8 row tiles) x a contiguous range of column blocks (split-K over at most a few CTAs,
 //              so that about one CTA per SM is busy); the fp32 partial results of the splits are summed in a fixed
@@ -19,13 +19,13 @@
 //              matrices without swizzle; the core-matrix columns of both operands are 16 bytes further apart than their size, which makes
 //              the 16-byte stores of the converter warps and of the activation copies conflict free.  Six stages.
 //   warps    0,2,3  activation loaders, every third stage each: cp.async of the rows as soon as the slot is free
-//            1      one thread issues four tcgen05.mma (M = 128 rows, N = tokens, K = 16) per stage into a
-//                   128 x N fp32 accumulator and commits the slot back to its producers
+//            1      one thread issues four tcgen05.mma (M = 128 rows, N = tokens, K = 16) per stage into one of four
+//                   128 x N fp32 accumulators and commits the slot back to its producers
 //            4..27  converters, three per row tile, every third block each: P6 blocks through a private cp.async
 //                   ring (as in the GEMV), the GEMV's shift / mask / fma conversion, four 16-byte stores into the
 //                   B operand, then the block's outliers (requested two blocks ahead) written over their
 //                   placeholders.  The chain per block is latency bound, hence many converter warps.
-//            0..3   epilogue: tcgen05.ld of the accumulator, partial results to global memory
+//            0..3   epilogue: tcgen05.ld of the accumulators, their sums to global memory
 // Every wait on an mbarrier is bounded; a wait that gives up sets the error word (the finalizing kernel then poisons
 // the output) and the kernel carries on to its end, so TMEM is always released.
 #pragma once
@@ -56,7 +56,10 @@ constexpr int kPgGroups = kPgStages / kPgGroup;
 constexpr int kPgBars = 2 * kPgGroups + 1;
 static_assert(kPgStages % kPgGroup == 0, "whole groups of stages");
 constexpr uint32_t kPgSmemBytes = kPgBarOff + kPgBars * 8 + 16;
-constexpr uint32_t kPgTmemCols = 64;
+// Stage i adds into accumulator i % kPgAcc: the tensor core cuts the low bits of what it adds to a large sum, so four short
+// chains lose less than one long one.  Relative error of fp32 results against 64 bits, one chain / four / k_p6_rows:
+// 5120 x 17408 6.0e-6 / 1.3e-6 / 1.8e-6, 300 x 16384 8.5e-7 / 2.0e-7 / 5.4e-7, 6144 x 5120 1.5e-6 / 3.2e-7 / 6.9e-7; no slower.
+constexpr uint32_t kPgAcc = 4, kPgTmemCols = kPgAcc * kPgTok;
 static_assert(kPgABytes % 16 == 0 && kPgBBytes % 16 == 0 && kPgBarOff % 8 == 0, "operand stages and barriers keep their alignment");
 static_assert(kPgSmemBytes <= 227 * 1024, "fits the shared memory of one SM");
 
@@ -189,10 +192,10 @@ k_p6_gemm(P6 p, const __nv_bfloat16 *__restrict__ x, uint32_t m_tok, float *__re
                     uint64_t dx = umma_desc(a_stage(st), kPgALbo, 128u);   // activations: the N side
 #pragma unroll
                     for (uint32_t k = 0; k < kTileCols / 16; ++k) {
-                        const uint32_t acc = (i | k) ? 1u : 0u;
+                        const uint32_t acc = i >= kPgAcc || k ? 1u : 0u;
                         asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
                                      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-                                     :: "r"(tmem_base), "l"(dw), "l"(dx), "r"(idesc), "r"(acc), "r"(0u) : "memory");
+                                     :: "r"(tmem_base + i % kPgAcc * kPgTok), "l"(dw), "l"(dx), "r"(idesc), "r"(acc), "r"(0u) : "memory");
                         dw += (2u * kPgBLbo) >> 4;                        // two core matrices further along K
                         dx += (2u * kPgALbo) >> 4;
                     }
@@ -315,17 +318,25 @@ k_p6_gemm(P6 p, const __nv_bfloat16 *__restrict__ x, uint32_t m_tok, float *__re
         float *dst = part + (size_t)split * m_tok * p.out_f + row;
 #pragma unroll 1
         for (uint32_t c0 = 0; c0 < m_tok; c0 += 16) {
-            uint32_t r[16];
-            const uint32_t taddr = tmem_base + ((uint32_t)(warp * 32) << 16) + c0;
-            asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-                         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                           "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-                         : "r"(taddr) : "memory");
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            float v[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) v[j] = 0.f;
+#pragma unroll 1
+            for (uint32_t q = 0; q < min(nk, kPgAcc); ++q) {        // (warp uniform) an accumulator without a stage was never written
+                uint32_t r[16];
+                const uint32_t taddr = tmem_base + ((uint32_t)(warp * 32) << 16) + q * kPgTok + c0;
+                asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                             : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                               "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                             : "r"(taddr) : "memory");
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                for (int j = 0; j < 16; ++j) v[j] += __uint_as_float(r[j]);
+            }
             if (row < p.out_f) {
 #pragma unroll
                 for (uint32_t j = 0; j < 16u; ++j)                   // the warp's 32 rows of one token: 128 contiguous bytes
-                    if (c0 + j < m_tok) dst[(size_t)(c0 + j) * p.out_f] = __uint_as_float(r[j]);
+                    if (c0 + j < m_tok) dst[(size_t)(c0 + j) * p.out_f] = v[j];
             }
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
