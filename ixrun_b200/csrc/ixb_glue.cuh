@@ -518,24 +518,26 @@ k_attn_decode(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat16 *__restri
         if (wid < G && lane == 0) part_ml[(size_t)(head0 + wid) * splits + s] = make_float2(M, L);
     }
     if (!join.tickets) return;
-    // ---- the last CTA of the group joins the parts.  A launch adds as many tickets as the group has CTAs (the first one adds
-    // those of the CTAs without a part), and whoever passes that number takes it off again: the count is zero after any
-    // number of whole launches, also of launches that overlapped, whose own results are lost.
+    // ---- the last CTA of the group joins the parts.  A launch takes as many tickets as the group has CTAs (the first one
+    // takes those of the CTAs without a part) and the count wraps to zero there: it is zero after any number of whole
+    // launches, also of launches that overlapped, whose own results are lost.
     const uint32_t ctas = min(gridDim.y, used);
     uint32_t *ticket = join.tickets + (size_t)blockIdx.z * gridDim.x + blockIdx.x;
     __threadfence();                                   // this thread's share of the parts, before the ticket
     __syncthreads();
     if (ctas > 1u) {
-        if (threadIdx.x == 0) {
-            const uint32_t mine = blockIdx.y ? 1u : gridDim.y - ctas + 1u;
-            uint32_t before = atomicAdd(ticket, mine);
-            if (before >= gridDim.y) before %= gridDim.y;              // (launches that overlap)
-            sm_last = before + mine >= gridDim.y;
+        const uint32_t end = gridDim.y - 1u;
+        if (blockIdx.y || ctas == gridDim.y) {
+            if (threadIdx.x == 0) sm_last = atomicInc(ticket, end) == end;
+        } else if (wid == 0) {
+            bool mine = false;
+            for (uint32_t k = lane; k <= gridDim.y - ctas; k += 32) mine |= atomicInc(ticket, end) == end;
+            mine = __any_sync(0xffffffffu, mine);
+            if (lane == 0) sm_last = mine;
         }
         __syncthreads();
         if (!sm_last) return;
         __threadfence();
-        if (threadIdx.x == 0) atomicSub(ticket, gridDim.y);
     }
     // all of the group's sums are requested at once, as far as registers go: a thread takes four dimensions of a head and
     // every PG-th part (rounds of eight dependent loads of one value: 29 us a launch at a 4097-token context, not 16.5)
