@@ -192,13 +192,13 @@ class on_device:
     __slots__ = ("idx", "guard")
 
     def __init__(self, index: int):
-        if index < 0:
-            raise ValueError("expected a CUDA tensor")
         self.idx = index
 
     def __enter__(self) -> int:
         if torch._C._cuda_getDevice() == self.idx:
             self.guard = None
+        elif self.idx < 0:
+            raise ValueError("expected a CUDA tensor")
         else:
             self.guard = torch.cuda.device(self.idx)
             self.guard.__enter__()

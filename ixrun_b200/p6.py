@@ -199,7 +199,7 @@ class P6Packed:
             raise ValueError(f"unsupported GEMM shape: {m} rows")
         L = _lib.lib()
         with _lib.on_device(self._index) as stream:
-            need = self._gemm_need.get(m)
+            need = 256 if m <= 32 else self._gemm_need.get(m)        # (k_p6_rows up to 32 rows)
             if need is None:
                 need = self._gemm_need[m] = int(L.ixb_p6_gemm_scratch_bytes(self.out_f, self.in_f, m))
             # partial sums of the tcgen05 form: a buffer of the call's own, so calls on several streams do not share it

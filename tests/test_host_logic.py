@@ -131,9 +131,11 @@ def test_ctypes_prototypes_match_the_header():
         assert len(fields) == len(mirror._fields_), f"{struct}: header has {len(fields)} fields, the mirror {len(mirror._fields_)}"
 
 
-def test_on_device_refuses_a_tensor_that_is_on_no_gpu():
+def test_on_device_refuses_a_tensor_that_is_on_no_gpu(monkeypatch):
     """A host tensor's device index is -1, which torch.cuda.device takes as 'leave the device as it is'."""
     from ixrun_b200 import _lib
 
+    monkeypatch.setattr(torch._C, "_cuda_getDevice", lambda: 0)
     with pytest.raises(ValueError):
-        _lib.on_device(torch.zeros(1).get_device())
+        with _lib.on_device(torch.zeros(1).get_device()):
+            pass
