@@ -123,7 +123,7 @@ __global__ void k_count_l1(Streams s, uint32_t nb, int32_t *cnt1)
 
 // Exclusive scans of n int32 values (in place allowed), one CTA of 1024 threads each: CTA 0 scans in -> out, CTA 1 (if the
 // grid has one) in2 -> out2; totals[CTA] (may be null) takes the sum.  8192 values per round: a warp scans eight rows of 32
-// (25600 values: 8.4 us, 19 with 1024 per round).
+// (25600 values: 10 us, 19 with 1024 per round).
 __global__ void __launch_bounds__(1024) k_excl_scan(const int32_t *in, int32_t *out, uint32_t n, const int32_t *in2 = nullptr,
                                                     int32_t *out2 = nullptr, int32_t *totals = nullptr)
 {

@@ -285,7 +285,7 @@ k_rope_kv(__nv_bfloat16 *q, const __nv_bfloat16 *__restrict__ k, const __nv_bflo
 
 // The same without norms and with the whole head rotated, 16-byte aligned rows: a thread takes eight pairs (elements 8 part
 // .. + 7 and those D / 2 further), so a head is D / 16 threads and many rows fill their CTAs (1000 rows of 24 heads of 128:
-// 4.8 us, against 26 with a CTA of 64 threads per row and head, under the profiler).
+// 5.7 us, against 26 with a CTA of 64 threads per row and head, under the profiler).
 __global__ void __launch_bounds__(128)
 k_rope_kv8(__nv_bfloat16 *q, const __nv_bfloat16 *__restrict__ k, const __nv_bfloat16 *__restrict__ v, const int32_t *pos,
            __nv_bfloat16 *k_cache, __nv_bfloat16 *v_cache, const float *__restrict__ cos_tab, const float *__restrict__ sin_tab,
@@ -336,7 +336,7 @@ k_rope_kv8(__nv_bfloat16 *q, const __nv_bfloat16 *__restrict__ k, const __nv_bfl
 // a warp per head turns them into weights, every thread sums its positions' V, and the threads' sums are joined once per
 // part.  With a running softmax per lane group and joins of eight such states per head instead, a CTA took 10700 cycles
 // for 64 positions (12.5 us a launch for 1025 positions of 16 / 8 heads of 128 under the profiler; 29 us for 4097 of
-// 6 / 2 heads of 256; 34 us for forty sequences of 225); now 9.4, 16.5 and 25 us.
+// 6 / 2 heads of 256; 34 us for forty sequences of 225); now 8.2, 16 and 23 us.
 // With max_seq (rows of the cache) the first loads do not wait for the position: they read whatever rows the part would
 // take at full length, and what lies beyond the position is dropped.  With tickets (one word per sequence and group, zero
 // between launches) the last CTA of a group joins the parts itself; otherwise k_attn_combine does.

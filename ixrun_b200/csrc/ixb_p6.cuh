@@ -144,7 +144,7 @@ __device__ __forceinline__ int p6_code_of(const uint32_t (&cw)[8], int p, int h)
 }
 
 // codes [out_f, in_f] -> plane blocks and the number of outliers of every block (one warp per block).  Bound by memory:
-// 12 us for 5120 x 5120, 33 with one byte per load.
+// 13 us for 5120 x 5120, 33 with one byte per load.
 __global__ void __launch_bounds__(256)
 k_p6_plane(const int8_t *__restrict__ codes, uint32_t out_f, uint32_t in_f, uint32_t rt, uint32_t kb,
            unsigned char *plane, int32_t *blk_cnt)

@@ -7,7 +7,7 @@
 namespace ixb {
 
 // max |w| over the tensor as bf16 bits (non-negative floats order like their bit patterns); NaN payloads are ignored.
-// Bound by memory: eight numbers per load, all of a thread's loads independent (5120 x 5120: 17 us, 50 with one number per
+// Bound by memory: eight numbers per load, all of a thread's loads independent (5120 x 5120: 15 us, 50 with one number per
 // load).
 __global__ void __launch_bounds__(256) k_absmax(const uint16_t *__restrict__ w, uint32_t n, uint32_t *out_bits)
 {
@@ -62,7 +62,7 @@ __device__ __forceinline__ int quantise_code(uint32_t bf16_bits, float sc, float
 // One warp per 1024-element block.  MODE 0: quantise from bf16 weights and write codes; MODE 1: read existing codes.
 // Both write the B1 words and the block's level-1 / level-2 counts.  Whole blocks of aligned tensors: a lane takes
 // eight consecutive elements four times, so that loads (16 / 8 bytes), codes and B1 bytes are contiguous across the warp
-// (5120 x 5120 in mode 0: 24 us, 154 when a lane walked its 32 elements one by one and divided each).
+// (5120 x 5120 in mode 0: 26 us, 154 when a lane walked its 32 elements one by one and divided each).
 template <int MODE>
 __global__ void __launch_bounds__(256)
 k_codes_and_counts(const uint16_t *__restrict__ w, const uint32_t *absmax_bits, int8_t *codes, uint32_t n,
@@ -166,7 +166,7 @@ __device__ __forceinline__ void write_image(uint32_t *stream, const uint32_t *im
 // Streams must be zero on entry.  One warp per block, lane = word of 32 elements.  Bound by instructions: a lane runs its
 // elements backwards and shifts every field in at the low end of its own bits (3 words of level 1, 5 of level 2, one of
 // the second bitmap), with predicates and no branches but for the rare level 3; the lanes' bits meet in an image of the
-// block's words in shared memory, which is written in whole words.  5120 x 5120: 54 us; 91 with a branch per
+// block's words in shared memory, which is written in whole words.  5120 x 5120: 57 us; 91 with a branch per
 // element, 104 with one global atomic per field.
 constexpr int kPackB2 = 0, kPackL1 = 36, kPackL2 = 140, kPackWords = 308;    // 33, 97 and 161 words at most
 __global__ void __launch_bounds__(256)
