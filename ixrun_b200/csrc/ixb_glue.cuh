@@ -518,23 +518,16 @@ k_attn_decode(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat16 *__restri
         if (wid < G && lane == 0) part_ml[(size_t)(head0 + wid) * splits + s] = make_float2(M, L);
     }
     if (!join.tickets) return;
-    // ---- the last CTA of the group joins the parts.  A launch takes as many tickets as the group has CTAs (the first one
-    // takes those of the CTAs without a part) and the count wraps to zero there: it is zero after any number of whole
-    // launches, also of launches that overlapped, whose own results are lost.
+    // ---- the last CTA of the group joins the parts.  The CTAs with work add numbers whose sum is zero to the ticket, the first
+    // one 1 - ctas and the others 1: it is zero again exactly when all of them have come.  So nobody resets it, and it is zero
+    // after launches that overlapped too (whose own results are lost).
     const uint32_t ctas = min(gridDim.y, used);
     uint32_t *ticket = join.tickets + (size_t)blockIdx.z * gridDim.x + blockIdx.x;
     __threadfence();                                   // this thread's share of the parts, before the ticket
     __syncthreads();
     if (ctas > 1u) {
-        const uint32_t end = gridDim.y - 1u;
-        if (blockIdx.y || ctas == gridDim.y) {
-            if (threadIdx.x == 0) sm_last = atomicInc(ticket, end) == end;
-        } else if (wid == 0) {
-            bool mine = false;
-            for (uint32_t k = lane; k <= gridDim.y - ctas; k += 32) mine |= atomicInc(ticket, end) == end;
-            mine = __any_sync(0xffffffffu, mine);
-            if (lane == 0) sm_last = mine;
-        }
+        const uint32_t mine = blockIdx.y ? 1u : 1u - ctas;
+        if (threadIdx.x == 0) sm_last = atomicAdd(ticket, mine) + mine == 0u;
         __syncthreads();
         if (!sm_last) return;
         __threadfence();
