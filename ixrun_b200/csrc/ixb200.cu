@@ -2,12 +2,14 @@
 // Built for sm_100a only.  See include/ixb200.h for the contract of each call.
 #include "../../include/ixb200.h"
 #include <cstdlib>
+#include <cuda.h>
+#include <cudaTypedefs.h>
 #include <cuda_fp16.h>
 #include "ixb_common.cuh"
 #include "ixb_gemm_tc.cuh"
 #include "ixb_attn_prefill.cuh"
-#include "ixb_p6_gemm.cuh"
 #include "ixb_p6_rows.cuh"
+#include "ixb_p6_umma.cuh"
 #include "ixb_pack.cuh"
 #include "ixb_p6.cuh"
 #include "ixb_allreduce.cuh"
@@ -18,6 +20,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 
 namespace ixb {
 
@@ -998,7 +1001,7 @@ static P6Plan make_p6_plan(uint32_t out_f, uint32_t in_f, uint32_t m_rows)
     const uint32_t units = p.nb / p.unit;
     p.cq = units / p.grid;
     p.cr = units % p.grid;
-    p.xstride = kb * kTileCols + 8u;
+    p.xstride = kb * kTileCols + 16u;                        // rows 32 bytes apart in the banks: 8-byte reads of eight rows without conflicts
     uint32_t xbytes = m_rows * p.xstride * 2u;
     const uint32_t fixed = (uint32_t)(m_rows > 1u ? P6Smem<true>::kFixed : P6Smem<false>::kFixed);
     p.xs = fixed + xbytes <= 227u * 1024u;
@@ -1564,16 +1567,15 @@ extern "C" int ixb_gemm(const ixb_packed *w, const int32_t *blk_q1, const int32_
 }
 
 // ------------------------------------------------ small-M GEMM on the resident P6 layout
-// The kernel's variants: n-tiles of eight activation rows, parts of K and stages per CTA (ixb_p6_rows.cuh).  Up to 32 rows
-// four parts (16 warps) fit the registers, more rows need the accumulators of three parts' worth.
+// ---- on mma.sync (ixb_p6_rows.cuh): up to 24 rows of layers with several outliers per block.
+// The kernel's variants: n-tiles of eight activation rows, parts of K and stages per CTA.
 struct PrVariant {
     void (*kernel)(P6, const __nv_bfloat16 *, uint32_t, const __nv_bfloat16 *, void *, int, uint32_t);
     uint32_t nt, parts, smem;
 };
 template <int NT, int PARTS, int STAGES>
 static constexpr PrVariant pr_variant() { return {k_p6_rows<NT, PARTS, STAGES>, NT, PARTS, PrSmem<NT, PARTS, STAGES>::kBytes}; }
-static const PrVariant kPrVariants[] = {pr_variant<2, 4, 4>(), pr_variant<3, 4, 4>(), pr_variant<4, 4, 4>(),
-                                        pr_variant<5, 3, 4>(), pr_variant<6, 3, 4>(), pr_variant<8, 3, 4>()};
+static const PrVariant kPrVariants[] = {pr_variant<2, 4, 4>(), pr_variant<3, 4, 4>()};
 constexpr int kPrVariantCount = sizeof(kPrVariants) / sizeof(kPrVariants[0]);
 constexpr int kPrMaxSplits = 8;                          // CTAs of a portable cluster
 
@@ -1638,58 +1640,147 @@ static int pr_variant_of(uint32_t m_rows)
     return v;
 }
 
-static PgPlan make_pg_plan(uint32_t out_f, uint32_t in_f)
+// ---- the same on tcgen05 (ixb_p6_umma.cuh)
+// cuTensorMapEncodeTiled, a function of the driver; null if there is none
+static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder()
 {
-    PgPlan p;
-    const uint32_t rt = (out_f + kTileRows - 1) / kTileRows, kb = (in_f + kTileCols - 1) / kTileCols;
-    p.groups = (rt + kPgConv - 1) / kPgConv;
-    // K is split only as far as it takes to give about every SM one CTA; a split keeps at least eight column blocks
-    uint32_t splits = std::max<uint32_t>(1u, (uint32_t)num_sms() / p.groups);
-    splits = std::min<uint32_t>(splits, std::max<uint32_t>(1u, kb / 8u));
-    p.splits = std::min<uint32_t>(splits, 16u);
-    p.grid = p.groups * p.splits;
-    return p;
+    static const PFN_cuTensorMapEncodeTiled_v12000 fn = []() -> PFN_cuTensorMapEncodeTiled_v12000 {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &f, 12000, cudaEnableDefault, &found) != cudaSuccess ||
+            found != cudaDriverEntryPointSuccess)
+            return nullptr;
+        return (PFN_cuTensorMapEncodeTiled_v12000)f;
+    }();
+    return fn;
 }
 
-// Whether k_p6_gemm (and its finalizing kernel) takes less time than k_p6_rows, in us, from lines through the measured times
-// of eleven layers at 33, 40, 48, 56 and 64 rows (most within 6 %).  It is taken where it is the faster one by more than 4 %,
-// and was then on all of them; at most 3 % are left (8192 x 8192 with 64 rows, 41.8 and 42.8 us).  Up to 32 rows k_p6_rows is
-// the faster one everywhere (but by 0.4 us at 300 x 16384).
-static bool pg_is_faster(uint32_t out_f, uint32_t in_f, uint32_t m_rows, const PrPlan &pr)
+constexpr int kPuMaxSplits = 16;                         // CTAs of a cluster (above 8 by opt-in)
+// clusters of 1 .. kPuMaxSplits CTAs that run at once on the current device (0: none of that size), and the kernel made ready
+static int pu_rooms(const int **rooms)
 {
-    if (m_rows <= 32u || in_f % kTileCols) return false;
-    const uint32_t nt = kPrVariants[pr_variant_of(m_rows)].nt;
-    const float per_step = nt <= 5u ? 1.31f : nt <= 6u ? 1.43f : 1.66f, fixed = (nt <= 5u ? 5.2f : nt <= 6u ? 5.4f : 6.0f) - (pr.splits == 1u ? 2.5f : 0.f);
-    const float t_rows = (float)pr.rounds * (fixed + per_step * (float)pr.steps);
-    const PgPlan pg = make_pg_plan(out_f, in_f);
-    const float stages = (float)((in_f / kTileCols + pg.splits - 1) / pg.splits);
-    const float per_stage = 0.405f + (m_rows > 48u ? 0.0055f * (float)(m_rows - 48u) : 0.f);
-    const float t_gemm = 8.6f + 4e-6f * (float)m_rows * (float)out_f + per_stage * stages;
-    return t_gemm < 0.96f * t_rows;
+    struct Rooms { int n[kPuMaxSplits + 1]; cudaError_t err; };
+    static Rooms table[64];
+    static std::once_flag once[64];
+    int dev = 0;
+    IXB_CUDA(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64) return fail(IXB_E_UNSUPPORTED, "device ordinal %d outside 0..63", dev);
+    std::call_once(once[dev], [dev]() {
+        Rooms &t = table[dev];
+        t.err = cudaFuncSetAttribute(k_p6_umma<kPuMaxRows>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PuCfg<kPuMaxRows>::kSmem);
+        if (t.err == cudaSuccess) t.err = cudaFuncSetAttribute(k_p6_umma<kPuMaxRows>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        for (int s = 1; s <= kPuMaxSplits && t.err == cudaSuccess; ++s) {
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3((unsigned)(s * 148));
+            cfg.blockDim = dim3(kPuThreads);
+            cfg.dynamicSmemBytes = PuCfg<kPuMaxRows>::kSmem;
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = (unsigned)s;
+            attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+            cfg.attrs = attr;
+            cfg.numAttrs = 1;
+            t.err = cudaOccupancyMaxActiveClusters(&t.n[s], k_p6_umma<kPuMaxRows>, &cfg);
+        }
+    });
+    if (table[dev].err != cudaSuccess) return fail(IXB_E_CUDA, "k_p6_umma: %s", cudaGetErrorString(table[dev].err));
+    *rooms = table[dev].n;
+    return IXB_OK;
 }
-static size_t pg_scratch_bytes(const PgPlan &plan, uint32_t out_f, uint32_t m_rows)
+// K splits (CTAs of a cluster): the least time, counted in column blocks (0.255 us each).  Beside its blocks a launch takes 2, or
+// 4 + splits where sums are joined; and where it fills more than 0.43 of the places for its clusters, up to 18 more, because the
+// launch behind it then finds no room to begin in (dependent launches in a graph).  Fitted to fourteen layers of 320 x 512 to
+// 17408 x 17408, 1 to 16 splits each: the choice is within 0.2 us of the best everywhere.  Without dependent launches a launch
+// takes about 20 blocks longer whatever it fills (5000 x 2176, 23 rows: 2 splits 10.9 us, 3 10.1; dependent 8.1 and 8.3).
+static int pu_plan(uint32_t rt, uint32_t kb, uint32_t *splits)
 {
-    return 256 + (size_t)plan.splits * m_rows * out_f * sizeof(float);
+    const bool dependent = g_p6_pdl.load() != 0;
+    const uint32_t groups = (rt + kPuTiles - 1) / kPuTiles;
+    const int *rooms;
+    const int rc = pu_rooms(&rooms);
+    if (rc) return rc;
+    float best = 0.f;
+    for (uint32_t s = 1; s <= (uint32_t)kPuMaxSplits && s <= kb; ++s) {
+        if (rooms[s] <= 0) continue;
+        const uint32_t room = (uint32_t)rooms[s], rounds = (groups + room - 1) / room;
+        const float used = (float)groups / (float)room;
+        const float blocks = (float)(rounds * ((kb + s - 1) / s));
+        const float cost = dependent ? blocks + (s == 1u ? 2.f : 4.f + (float)s) + (rounds > 1u ? 10.f * (float)rounds : used > 0.43f ? 31.f * (used - 0.43f) : 0.f)
+                                     : blocks + (s == 1u ? 0.f : 5.f) + 20.f * (float)(rounds - 1u);
+        if (best == 0.f || cost < best) {
+            best = cost;
+            *splits = s;
+        }
+    }
+    return best > 0.f ? IXB_OK : fail(IXB_E_CUDA, "k_p6_umma does not fit this device");
 }
-
-extern "C" size_t ixb_p6_gemm_scratch_bytes(int64_t out_f, int64_t in_f, int64_t m_rows)
+static int p6_umma_run(const P6 &p, const void *x, uint32_t m_rows, const void *bias, void *y, int y_is_f32, uint32_t splits,
+                       ixb_stream_t stream)
 {
-    if (out_f <= 0 || in_f <= 0 || m_rows < 1 || m_rows > kPrMaxRows || out_f * in_f > 800000000LL) return 0;
-    const uint32_t o = (uint32_t)out_f, i = (uint32_t)in_f, m = (uint32_t)m_rows;
-    PrPlan pr = {1, 1, 1};
-    if (m <= 32u || pr_plan((o + kTileRows - 1) / kTileRows, (i + kTileCols - 1) / kTileCols, pr_variant_of(m), &pr)) return 256;
-    return pg_is_faster(o, i, m, pr) ? pg_scratch_bytes(make_pg_plan(o, i), o, m) : 256;
+    const PFN_cuTensorMapEncodeTiled_v12000 encode = tensor_map_encoder();
+    if (!encode) return fail(IXB_E_UNSUPPORTED, "the driver has no cuTensorMapEncodeTiled");
+    CUtensorMap wmap, xmap;
+    const cuuint32_t one[3] = {1, 1, 1};
+    {
+        const cuuint64_t dims[3] = {kP6BlockBytes / 4, p.kb, p.rt}, strides[2] = {kP6BlockBytes, (cuuint64_t)p.kb * kP6BlockBytes};
+        const cuuint32_t box[3] = {kP6BlockBytes / 4, 2, kPuTiles};
+        const CUresult r = encode(&wmap, CU_TENSOR_MAP_DATA_TYPE_UINT32, 3, const_cast<unsigned char *>(p.plane), dims, strides, box, one,
+                                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (r != CUDA_SUCCESS) return fail(IXB_E_CUDA, "tensor map of the plane: error %d", (int)r);
+    }
+    {
+        const cuuint64_t dims[2] = {p.in_f, m_rows}, strides[1] = {(cuuint64_t)p.in_f * 2};
+        const cuuint32_t box[2] = {kTileCols, (m_rows + 15u) & ~15u};
+        const CUresult r = encode(&xmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(x), dims, strides, box, one,
+                                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (r != CUDA_SUCCESS) return fail(IXB_E_CUDA, "tensor map of the activations: error %d", (int)r);
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((p.rt + kPuTiles - 1) / kPuTiles * splits);
+    cfg.blockDim = dim3(kPuThreads);
+    cfg.dynamicSmemBytes = PuCfg<kPuMaxRows>::kSmem;
+    cfg.stream = (cudaStream_t)stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = splits;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = g_p6_pdl.load() ? 2 : 1;
+    IXB_GLUE("k_p6_umma", cudaLaunchKernelEx(&cfg, k_p6_umma<kPuMaxRows>, p, wmap, xmap, m_rows, (const __nv_bfloat16 *)bias, y, y_is_f32, splits));
 }
 
 static int p6_rows_run(const P6 &p, const void *x, uint32_t m_rows, const void *bias, void *y, int y_is_f32, const PrPlan &plan,
                        ixb_stream_t stream);
-static int p6_rows_args(const P6 &p, const void *x, int64_t m_rows, const void *y)
+// 1..64 rows, in_f a multiple of 8
+static int p6_rows_any(const P6 &p, int64_t n_esc, const void *x, int64_t m_rows, const void *bias, void *y, int y_is_f32, ixb_stream_t stream)
 {
     if (!x || !y) return fail(IXB_E_ARG, "NULL pointer argument");
-    if (m_rows < 1 || m_rows > kPrMaxRows) return fail(IXB_E_UNSUPPORTED, "m_rows=%lld outside 1..%d", (long long)m_rows, kPrMaxRows);
+    if (m_rows < 1 || m_rows > kPuMaxRows) return fail(IXB_E_UNSUPPORTED, "m_rows=%lld outside 1..%d", (long long)m_rows, kPuMaxRows);
     if (p.in_f % 8u) return fail(IXB_E_UNSUPPORTED, "in_f=%u is not a multiple of 8", p.in_f);
     if ((uintptr_t)x & 15u) return fail(IXB_E_ARG, "x is not 16-byte aligned");
-    return IXB_OK;
+    int rc;
+    // Blocks with several outliers cost k_p6_umma more: its converters are what a stage waits for.  17408 x 5120 at 16 rows with
+    // 1.4 / 3.8 / 7.9 / 23 / 47 / 112 outliers per block, k_p6_rows and k_p6_umma: 28.1 and 26.9 us / 29.3, 29.9 / 29.5, 32.3 / 30.8, 36.2 /
+    // 45.2, 46.4 / 72.3, 63.7; at 32 rows and more k_p6_umma is the faster one of all.
+    const float density = (float)n_esc / ((float)p.rt * (float)p.kb);
+    if (m_rows <= kPrMaxRows && density > 3.f && density < 50.f) {
+        PrPlan plan = {1, 1, 1};
+        if ((rc = pr_plan(p.rt, p.kb, pr_variant_of((uint32_t)m_rows), &plan))) return rc;
+        return p6_rows_run(p, x, (uint32_t)m_rows, bias, y, y_is_f32, plan, stream);
+    }
+    uint32_t splits = 1;
+    if ((rc = pu_plan(p.rt, p.kb, &splits))) return rc;
+    return p6_umma_run(p, x, (uint32_t)m_rows, bias, y, y_is_f32, splits, stream);
+}
+
+extern "C" size_t ixb_p6_gemm_scratch_bytes(int64_t out_f, int64_t in_f, int64_t m_rows)
+{
+    if (out_f <= 0 || in_f <= 0 || m_rows < 1 || m_rows > kPuMaxRows || out_f * in_f > 800000000LL) return 0;
+    return m_rows <= 32 ? 256 : 512;      // no kernel uses it; more than 32 rows have always been told to bring more than the 256 that are enough
 }
 
 extern "C" int ixb_p6_gemm(const ixb_p6 *t, const void *x, int64_t m_rows, const void *bias, void *y, int y_is_f32,
@@ -1702,35 +1793,7 @@ extern "C" int ixb_p6_gemm(const ixb_p6 *t, const void *x, int64_t m_rows, const
     if (p.in_f % (uint32_t)kTileCols) return fail(IXB_E_UNSUPPORTED, "in_f=%u is not a multiple of %d", p.in_f, kTileCols);
     if ((uintptr_t)scratch & 255u) return fail(IXB_E_ARG, "scratch is not 256-byte aligned");
     if (scratch_bytes < 256u) return fail(IXB_E_SCRATCH, "gemm scratch too small");
-    if ((rc = p6_rows_args(p, x, m_rows, y))) return rc;
-    PrPlan pr = {1, 1, 1};
-    if ((rc = pr_plan(p.rt, p.kb, pr_variant_of((uint32_t)m_rows), &pr))) return rc;
-    const PgPlan plan = make_pg_plan(p.out_f, p.in_f);
-    // a scratch of 256 bytes is enough for every call: k_p6_rows needs none
-    if (!pg_is_faster(p.out_f, p.in_f, (uint32_t)m_rows, pr) || scratch_bytes < pg_scratch_bytes(plan, p.out_f, (uint32_t)m_rows))
-        return p6_rows_run(p, x, (uint32_t)m_rows, bias, y, y_is_f32, pr, stream);
-    cudaStream_t st = (cudaStream_t)stream;
-    static bool attr_set[64] = {false};
-    IXB_CUDA(opt_in_smem(k_p6_gemm, attr_set, (int)kPgSmemBytes));
-    uint32_t *err = (uint32_t *)scratch;
-    float *part = (float *)((char *)scratch + 256);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(plan.grid);
-    cfg.blockDim = dim3(kPgThreads);
-    cfg.dynamicSmemBytes = kPgSmemBytes;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = g_p6_pdl.load() ? 1 : 0;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, k_p6_gemm, p, (const __nv_bfloat16 *)x, (uint32_t)m_rows, part, err, plan);
-    if (e != cudaSuccess) return fail(IXB_E_CUDA, "k_p6_gemm launch: %s", cudaGetErrorString(e));
-    if ((rc = launch_check("k_p6_gemm"))) return rc;
-    const uint32_t total = (uint32_t)m_rows * p.out_f;
-    IXB_GLUE("k_gemm_finalize", launch_glue(k_gemm_finalize, dim3((total + 255) / 256), dim3(256), st, (const float *)part,
-                                            plan.splits, (uint32_t)m_rows, p.out_f, (const __nv_bfloat16 *)bias, y, y_is_f32,
-                                            (const uint32_t *)err));
+    return p6_rows_any(p, t->n_esc, x, m_rows, bias, y, y_is_f32, stream);
 }
 
 extern "C" int ixb_p6_rows(const ixb_p6 *t, const void *x, int64_t m_rows, const void *bias, void *y, int y_is_f32,
@@ -1738,10 +1801,7 @@ extern "C" int ixb_p6_rows(const ixb_p6 *t, const void *x, int64_t m_rows, const
 {
     P6 p;
     int rc = to_p6(t, &p);
-    if (rc || (rc = p6_rows_args(p, x, m_rows, y))) return rc;
-    PrPlan plan = {1, 1, 1};
-    if ((rc = pr_plan(p.rt, p.kb, pr_variant_of((uint32_t)m_rows), &plan))) return rc;
-    return p6_rows_run(p, x, (uint32_t)m_rows, bias, y, y_is_f32, plan, stream);
+    return rc ? rc : p6_rows_any(p, t->n_esc, x, m_rows, bias, y, y_is_f32, stream);
 }
 
 static int p6_rows_run(const P6 &p, const void *x, uint32_t m_rows, const void *bias, void *y, int y_is_f32, const PrPlan &plan,

@@ -6,14 +6,15 @@
 // block (16 rows x 64 columns, one warp) sits at a fixed address, and turning it
 // into tensor-core operands costs four instructions per PAIR of weights:
 //
-//   plane   every element of code -32 .. 31 owns a 6-bit field F = 32 + code; put at bits 6..1 of the low byte it makes
-//           a bf16 number of the binade [64, 128):
-//             (F << 1) | 0x4280 = 64 + F = 96 + code
-//           so a packed subtraction of 96 gives the code exactly, and the packed multiplication by the scale (plus 0, so
+//   plane   every element of code -32 .. 31 owns a 6-bit field F = 32 + code; put at the low end of the mantissa it makes
+//           a bf16 number of the binade [128, 256):
+//             F | 0x4300 = 128 + F = 160 + code
+//           so a packed subtraction of 160 gives the code exactly, and the packed multiplication by the scale (plus 0, so
 //           that code 0 gives +0.0 whatever the scale's sign) rounds the exact product once: the reference's dequantised
 //           weight bf16(f32(code) * f32(scale)) (ixrun/quantize.py:182, ixrun/fused.py:169-170), bit for bit, for any
 //           scale (but for the sign of that zero).
-//           Other codes ("outliers") leave the placeholder F = 32 (weight 0).  (Before, F was part of 1 + code / 32 over
+//           Other codes ("outliers") leave the placeholder F = 32 (weight 0).  (F used to be bits 6..1 of a number of
+//           [64, 128): a shift more for every second pair.  Before that it was part of 1 + code / 32 over
 //           two binades, one fused multiply-add per pair instead of two operations, but it held -16 .. 31 only: 1.2 % of
 //           the benchmark distribution were outliers, 4 bytes and an extra step each, against 0.07 % now.)
 //           Blocks of 16 rows x 64 columns, ragged edges padded with
@@ -49,13 +50,16 @@ constexpr int kTileCols = 64;
 
 // Lane l of a block: g = l >> 2, t = l & 3.  Its 16 pairs p = 4 j + q (j = 0..3 the mma, q = 0..3 the A register):
 //   row    = 16 R + g + 8 (q & 1)
-//   column = 64 kb + 16 t + 4 j + 2 (q >> 1) + h          (h = 0 low half, 1 high half of the register)
-// i.e. the k index of mma j is permuted so that a lane needs the 16 consecutive activations 16 t .. 16 t + 15.
+//   column = 64 kb + 16 j + 4 t + 2 (q >> 1) + h          (h = 0 low half, 1 high half of the register)
+// i.e. the k index of mma j is permuted inside its 16 columns so that a lane needs four consecutive activations, and a block's
+// registers are the words 8 j + 2 t + (q >> 1) of its rows in column order: what tcgen05.st.16x256b makes of them in tensor
+// memory, so that k_p6_umma can take the activations as they lie in memory.  (The GEMV alone would rather have 16 consecutive
+// activations per lane, 16 t + 4 j: two 16-byte reads per block instead of four 8-byte ones.)
 __device__ __forceinline__ void p6_elem(int lane, int p, int h, uint32_t &row_in_tile, uint32_t &col_in_tile)
 {
     int g = lane >> 2, t = lane & 3, j = p >> 2, q = p & 3;
     row_in_tile = (uint32_t)(g + 8 * (q & 1));
-    col_in_tile = (uint32_t)(16 * t + 4 * j + 2 * (q >> 1) + h);
+    col_in_tile = (uint32_t)(16 * j + 4 * t + 2 * (q >> 1) + h);
 }
 // (SRC & MASK) | ACC
 __device__ __forceinline__ uint32_t p6_and_or(uint32_t src, uint32_t mask, uint32_t acc)
@@ -110,34 +114,53 @@ __device__ __forceinline__ uint32_t p6_get(const uint32_t (&w)[6], int p, int h)
 }
 
 // ------------------------------------------------------------------ build ---
-// the lane's 32 codes of block (R, kbi): out[0..3] row g, out[4..7] row g + 8, 16 consecutive columns each, as bytes;
-// elements beyond the tensor are 0.  Two 16-byte loads where rows and tensor allow.
+// word j of lane t of a quad <-> word t of lane j
+__device__ __forceinline__ void p6_quad_transpose(uint32_t (&a)[4], int lane)
+{
+#pragma unroll
+    for (int d = 1; d <= 2; d <<= 1) {
+        const bool up = lane & d;
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const int lo = d == 1 ? 2 * k : k, hi = lo + d;
+            const uint32_t got = __shfl_xor_sync(0xffffffffu, up ? a[lo] : a[hi], d);
+            if (up) a[lo] = got;
+            else a[hi] = got;
+        }
+    }
+}
+// the lane's 32 codes of block (R, kbi): out[0..3] row g, out[4..7] row g + 8, the four columns 16 j + 4 t .. + 3 as the bytes
+// of word j; elements beyond the tensor are 0.  Two 16-byte loads, dealt out over the quad, where rows and tensor allow.
 __device__ __forceinline__ void p6_load_codes(const int8_t *__restrict__ codes, uint32_t out_f, uint32_t in_f, uint32_t R,
                                               uint32_t kbi, int lane, uint32_t (&out)[8])
 {
-    const uint32_t col0 = kbi * kTileCols + 16 * (lane & 3);
     const bool vec = ((in_f & 15u) | ((uintptr_t)codes & 15u)) == 0;
 #pragma unroll
     for (int s = 0; s < 2; ++s) {
         const uint32_t row = R * kTileRows + (lane >> 2) + 8 * s;
-        uint4 v = make_uint4(0, 0, 0, 0);
-        const int8_t *src = codes + (size_t)row * in_f + col0;
-        if (row < out_f && vec) {
-            if (col0 < in_f) v = __ldg((const uint4 *)src);             // in_f % 16 == 0: all 16 columns or none
-            out[4 * s] = v.x; out[4 * s + 1] = v.y; out[4 * s + 2] = v.z; out[4 * s + 3] = v.w;
+        const int8_t *src = codes + (size_t)row * in_f + kbi * kTileCols;
+        uint32_t w[4] = {0, 0, 0, 0};
+        if (vec) {
+            const uint32_t c0 = 16 * (lane & 3);
+            if (row < out_f && kbi * kTileCols + c0 < in_f) {                   // in_f % 16 == 0: all 16 columns or none
+                const uint4 v = __ldg((const uint4 *)(src + c0));
+                w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
+            }
+            p6_quad_transpose(w, lane);
         } else {
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                uint32_t u = 0;
+            for (int j = 0; j < 4; ++j)
 #pragma unroll
-                for (int c = 0; c < 4; ++c)
-                    if (row < out_f && col0 + 4 * k + c < in_f) u |= (uint32_t)(uint8_t)src[4 * k + c] << (8 * c);
-                out[4 * s + k] = u;
-            }
+                for (int c = 0; c < 4; ++c) {
+                    const uint32_t at = 16 * j + 4 * (lane & 3) + c;
+                    if (row < out_f && kbi * kTileCols + at < in_f) w[j] |= (uint32_t)(uint8_t)src[at] << (8 * c);
+                }
         }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) out[4 * s + j] = w[j];
     }
 }
-// element h of pair p out of them (column 4 (p >> 2) + 2 ((p & 3) >> 1) + h of row g + 8 (p & 1), see p6_elem)
+// element h of pair p out of them (byte 2 ((p & 3) >> 1) + h of word p >> 2 of row g + 8 (p & 1), see p6_elem)
 __device__ __forceinline__ int p6_code_of(const uint32_t (&cw)[8], int p, int h)
 {
     return (int)(int8_t)(cw[4 * (p & 1) + (p >> 2)] >> (8 * (2 * ((p & 3) >> 1) + h)));
@@ -208,7 +231,7 @@ k_p6_esc(const int8_t *__restrict__ codes, uint32_t out_f, uint32_t in_f, uint32
 
 // ---------------------------------------------------------------- decode ----
 // plane -> int8 codes (OUT 0) or bf16 weights (OUT 1), row major [out_f, in_f]; outliers come out as 0 here.
-// A lane holds 16 consecutive columns of two rows: one or two 16-byte stores per row.
+// A lane holds four times four consecutive columns of two rows: 4 or 8 bytes per store.
 template <int OUT>
 __global__ void __launch_bounds__(256) k_p6_decode_plane(P6 p, void *out)
 {
@@ -221,29 +244,30 @@ __global__ void __launch_bounds__(256) k_p6_decode_plane(P6 p, void *out)
     const uint4 a = ((const uint4 *)blk)[lane];
     const uint2 a2 = ((const uint2 *)(blk + 512))[lane];
     uint32_t w[6] = {a.x, a.y, a.z, a.w, a2.x, a2.y};
-    const bool vec = (OUT == 0 ? (p.in_f & 15u) == 0 : (p.in_f & 7u) == 0) && ((uintptr_t)out & 15u) == 0;
+    const bool vec = (p.in_f & 3u) == 0 && ((uintptr_t)out & (OUT == 0 ? 3u : 7u)) == 0;
 #pragma unroll
     for (int s = 0; s < 2; ++s) {                    // row g, row g + 8
-        uint32_t row = R * kTileRows + (lane >> 2) + 8 * s, col0 = kbi * kTileCols + 16 * (lane & 3);
-        if (row >= p.out_f || col0 >= p.in_f) continue;
-        uint32_t r[OUT == 0 ? 4 : 8];
+        const uint32_t row = R * kTileRows + (lane >> 2) + 8 * s;
+        if (row >= p.out_f) continue;
 #pragma unroll
-        for (int i = 0; i < (OUT == 0 ? 4 : 8); ++i) r[i] = 0;
+        for (int j = 0; j < 4; ++j) {                // columns col0 + c = pair 4 j + 2 (c >> 1) + s, half c & 1
+            const uint32_t col0 = kbi * kTileCols + 16 * j + 4 * (lane & 3);
+            uint32_t r[2] = {0u, 0u};
 #pragma unroll
-        for (int c = 0; c < 16; ++c) {               // column col0 + c = pair 4 (c >> 2) + 2 ((c >> 1) & 1) + s, half c & 1
-            int code = p6_code(p6_get(w, 4 * (c >> 2) + 2 * ((c >> 1) & 1) + s, c & 1));
-            if (OUT == 0) r[c >> 2] |= (uint32_t)(code & 0xff) << (8 * (c & 3));
-            else r[c >> 1] |= (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn((float)code * sc)) << (16 * (c & 1));
-        }
-        size_t o = (size_t)row * p.in_f + col0;
-        if (vec && col0 + 16u <= p.in_f) {
-            uint4 *dst = (uint4 *)((char *)out + o * (OUT == 0 ? 1 : 2));
-            dst[0] = make_uint4(r[0], r[1], r[2], r[3]);
-            if (OUT == 1) dst[1] = make_uint4(r[4], r[5], r[6], r[7]);
-        } else {
-            for (uint32_t c = 0; c < 16u && col0 + c < p.in_f; ++c) {
-                if (OUT == 0) ((int8_t *)out)[o + c] = (int8_t)((r[c >> 2] >> (8 * (c & 3))) & 0xff);
-                else ((uint16_t *)out)[o + c] = (uint16_t)((r[c >> 1] >> (16 * (c & 1))) & 0xffff);
+            for (int c = 0; c < 4; ++c) {
+                const int code = p6_code(p6_get(w, 4 * j + 2 * (c >> 1) + s, c & 1));
+                if (OUT == 0) r[0] |= (uint32_t)(code & 0xff) << (8 * c);
+                else r[c >> 1] |= (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn((float)code * sc)) << (16 * (c & 1));
+            }
+            const size_t o = (size_t)row * p.in_f + col0;
+            if (vec && col0 < p.in_f) {
+                if (OUT == 0) *(uint32_t *)((char *)out + o) = r[0];
+                else *(uint2 *)((char *)out + 2 * o) = make_uint2(r[0], r[1]);
+            } else {
+                for (uint32_t c = 0; c < 4u && col0 + c < p.in_f; ++c) {
+                    if (OUT == 0) ((int8_t *)out)[o + c] = (int8_t)((r[0] >> (8 * c)) & 0xff);
+                    else ((uint16_t *)out)[o + c] = (uint16_t)((r[c >> 1] >> (16 * (c & 1))) & 0xffff);
+                }
             }
         }
     }
@@ -324,27 +348,27 @@ __device__ __forceinline__ void p6_ldmatrix(uint32_t (&r)[4], uint32_t addr)
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
 }
-// two bf16 numbers 96 + code -> the two weights; s2: the scale in both halves.  The product is a fused multiply-add of +0:
+// two bf16 numbers 160 + code -> the two weights; s2: the scale in both halves.  The product is a fused multiply-add of +0:
 // the same value, rounded once, but +0.0 for code 0 and a scale of either sign, so that a placeholder is all zero bits.
 __device__ __forceinline__ uint32_t p6_weights(uint32_t v, uint32_t s2)
 {
     uint32_t w;
     asm("{\n\t.reg .b32 c;\n\tadd.rn.bf16x2 c, %1, %2;\n\tfma.rn.bf16x2 %0, c, %3, %4;\n\t}"
-        : "=r"(w) : "r"(v), "r"(0xC2C0C2C0u), "r"(s2), "r"(0u));
+        : "=r"(w) : "r"(v), "r"(0xC320C320u), "r"(s2), "r"(0u));
     return w;
 }
-// a lane's six plane words -> its 16 pairs of weights; e2 = 0x42804280 (kept in a register by the caller)
+// a lane's six plane words -> its 16 pairs of weights; e2 = 0x43004300 (kept in a register by the caller)
 __device__ __forceinline__ void p6_unpack(const uint32_t (&w)[6], uint32_t e2, uint32_t s2, uint32_t (&f)[16])
 {
 #pragma unroll
     for (int k = 0; k < 6; ++k) {
-        f[2 * k] = p6_weights(p6_and_or(w[k] << 1, 0x007E007Eu, e2), s2);
-        f[2 * k + 1] = p6_weights(p6_and_or(w[k] >> 5, 0x007E007Eu, e2), s2);
+        f[2 * k] = p6_weights(p6_and_or(w[k], 0x003F003Fu, e2), s2);
+        f[2 * k + 1] = p6_weights(p6_and_or(w[k] >> 6, 0x003F003Fu, e2), s2);
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        uint32_t v = p6_and_or(w[i] >> 11, 0x001E001Eu, e2);
-        v = p6_and_or(w[4 + (i >> 1)] >> (7 + 2 * (i & 1)), 0x00600060u, v);
+        uint32_t v = p6_and_or(w[i] >> 12, 0x000F000Fu, e2);
+        v = p6_and_or(w[4 + (i >> 1)] >> (8 + 2 * (i & 1)), 0x00300030u, v);
         f[12 + i] = p6_weights(v, s2);
     }
 }
@@ -432,84 +456,62 @@ __device__ __forceinline__ uint32_t p6_part_of(uint32_t pos, uint32_t q, uint32_
     return pos < big ? pos / (q + 1u) : r + (pos - big) / q;      // q > 0 whenever pos >= big
 }
 
-// One outlier of a block over its placeholder, in the register of the lane that holds the element: row r, column c of the
-// block sit in lane 4 (r & 7) + (c >> 4), pair 4 ((c >> 2) & 3) + 2 ((c >> 1) & 1) + (r >> 3), half c & 1 (the inverse of
-// p6_elem).  e is the same in all lanes.
-__device__ __forceinline__ void p6_or_entry(uint32_t (&f)[16], uint32_t e, int lane)
-{
-    const uint32_t r = (e >> 12) & 15u, c = e & 63u;
-    const uint32_t v = (uint32_t)lane == 4u * (r & 7u) + (c >> 4) ? ((c & 1u) ? e & 0xFFFF0000u : e >> 16) : 0u;
-    const uint32_t at = 4u * ((c >> 2) & 3u) + 2u * ((c >> 1) & 1u) + (r >> 3);
-#pragma unroll
-    for (int q = 0; q < 16; ++q)
-        if (at == (uint32_t)q) f[q] |= v;
-}
-// ... and its place in an image [4 mma][32 lanes][4 registers] of those registers, for the blocks with many
+// An outlier's place in an image [4 mma][32 lanes][4 registers] of a block's registers (the inverse of p6_elem): row r, column c of
+// the block sit in lane 4 (r & 7) + ((c >> 2) & 3), pair 4 (c >> 4) + 2 ((c >> 1) & 1) + (r >> 3), half c & 1.
 __device__ __forceinline__ uint32_t p6_image_at(uint32_t e)
 {
     const uint32_t r = (e >> 12) & 15u, c = e & 63u;
-    return ((((c >> 2) & 3u) * 32u + 4u * (r & 7u) + (c >> 4)) * 4u + 2u * ((c >> 1) & 1u) + (r >> 3)) * 4u + 2u * (c & 1u);
+    return (((c >> 4) * 32u + 4u * (r & 7u) + ((c >> 2) & 3u)) * 4u + 2u * ((c >> 1) & 1u) + (r >> 3)) * 4u + 2u * (c & 1u);
 }
 
 // layout -> bf16 weights in one pass, with the GEMV's own conversion.  Bound by memory (2.76 bytes per weight): the
-// plane is requested before the offsets, one or two outliers go straight into their lane's register, more through an
-// image of the lanes' registers in shared memory, and every weight is stored once, a 32-byte sector per lane and row where
-// the alignment allows.  Needs in_f % 8 == 0 and a 16-byte aligned output.  One warp per block.
-__global__ void __launch_bounds__(256) k_p6_decode_bf16(P6 p, __nv_bfloat16 *out)
+// plane is requested before the offsets, the block's weights go through a tile in shared memory (16-byte pieces swizzled) where
+// its outliers overwrite their placeholders, and every weight is stored once, a 32-byte sector per lane where the alignment
+// allows; eight CTAs per SM are in flight.  17408 x 5120 40.2 us (38.0 at the copy rate), 12288 x 2048 10.9, 2048 x 6144 6.0;
+// with the words dealt out over the quads by shuffles 40.5, 11.1 and 6.3, stored in 8-byte pieces 40.4, 11.5 and 7.3.
+// Needs in_f % 8 == 0 and a 16-byte aligned output.  One warp per block.
+__global__ void __launch_bounds__(256, 8) k_p6_decode_bf16(P6 p, __nv_bfloat16 *out)
 {
-    __shared__ uint4 images[8 * 128];
-    uint32_t b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    int lane = threadIdx.x & 31;
+    __shared__ uint4 tiles[8 * 128];
+    const uint32_t b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
     if (b >= p.rt * p.kb) return;                    // whole warps leave together
     const unsigned char *blk = p.plane + (size_t)b * kP6BlockBytes;
     const uint4 a = __ldg((const uint4 *)blk + lane);
     const uint2 a2 = __ldg((const uint2 *)(blk + 512) + lane);
     const int32_t lo = __ldg(p.blk_off + b), hi = __ldg(p.blk_off + b + 1);
-    uint32_t R = b / p.kb, kbi = b - R * p.kb;
+    const uint32_t R = b / p.kb, kbi = b - R * p.kb;
     const uint32_t w[6] = {a.x, a.y, a.z, a.w, a2.x, a2.y};
     uint32_t f[16];
-    p6_unpack(w, 0x42804280u, p6_scale2(p.scale[R * p.scale_stride]), f);
-    // placeholders are +0.0, so OR-ing the outlier weights in is exact
-    if (hi - lo <= 2) {
-        for (int32_t j = lo; j < hi; ++j) p6_or_entry(f, __ldg(p.esc + j), lane);
-    } else {
-        uint4 *img = images + (threadIdx.x >> 5) * 128;
+    p6_unpack(w, 0x43004300u, p6_scale2(p.scale[R * p.scale_stride]), f);
+    const uint32_t tile = (uint32_t)__cvta_generic_to_shared(tiles + (threadIdx.x >> 5) * 128);
+    auto piece = [&](uint32_t r, uint32_t c) { return tile + r * 128u + (c ^ (r & 7u)) * 16u; };     // columns 8 c .. 8 c + 7 of row r
+    const uint32_t g = (uint32_t)lane >> 2, t = (uint32_t)lane & 3u;
+    // pair 4 j + q: row g + 8 (q & 1), columns 16 j + 4 t + 2 (q >> 1) + {0, 1} of the block
 #pragma unroll
-        for (int q = 0; q < 4; ++q) img[q * 32 + lane] = make_uint4(0, 0, 0, 0);
-        __syncwarp();
-        const uint32_t img_s = (uint32_t)__cvta_generic_to_shared(img);
-        for (int32_t j = lo + lane; j < hi; j += 32) {
-            const uint32_t e = __ldg(p.esc + j);
-            asm volatile("st.shared.u16 [%0], %1;" ::"r"(img_s + p6_image_at(e)), "h"((unsigned short)(e >> 16)) : "memory");
-        }
-        __syncwarp();
+    for (int s = 0; s < 2; ++s)
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const uint4 v = img[q * 32 + lane];
-            f[4 * q] |= v.x;
-            f[4 * q + 1] |= v.y;
-            f[4 * q + 2] |= v.z;
-            f[4 * q + 3] |= v.w;
-        }
+        for (int j = 0; j < 4; ++j)
+            asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(piece(g + 8u * s, 2u * j + (t >> 1)) + (t & 1u) * 8u), "r"(f[4 * j + s]), "r"(f[4 * j + 2 + s]) : "memory");
+    __syncwarp();
+    for (int32_t j = lo + lane; j < hi; j += 32) {
+        const uint32_t e = __ldg(p.esc + j), r = (e >> 12) & 15u, c = e & 63u;
+        asm volatile("st.shared.u16 [%0], %1;" ::"r"(piece(r, c >> 3) + (c & 7u) * 2u), "h"((unsigned short)(e >> 16)) : "memory");
     }
+    __syncwarp();
     const bool wide = (p.in_f & 15u) == 0 && ((uintptr_t)out & 31u) == 0;       // a lane's 32 bytes of a row are one sector
-    // pair 4 j + q: row g + 8 (q & 1), columns 4 j + 2 (q >> 1) + {0, 1} of the lane's 16
-    const uint32_t col0 = kbi * kTileCols + 16 * (lane & 3);
 #pragma unroll
-    for (int s = 0; s < 2; ++s) {
-        uint32_t row = R * kTileRows + (lane >> 2) + 8 * s;
-        if (row >= p.out_f || col0 >= p.in_f) continue;
-        __nv_bfloat16 *dst = out + (size_t)row * p.in_f + col0;
-        const uint32_t r[8] = {f[0 + s], f[2 + s], f[4 + s], f[6 + s], f[8 + s], f[10 + s], f[12 + s], f[14 + s]};
+    for (int k = 0; k < 2; ++k) {
+        const uint32_t r = 8u * k + g, c = 2u * t, row = R * kTileRows + r, col = kbi * kTileCols + 8u * c;
+        const uint4 v0 = p6_lds128(piece(r, c)), v1 = p6_lds128(piece(r, c + 1u));
+        if (row >= p.out_f || col >= p.in_f) continue;
+        __nv_bfloat16 *dst = out + (size_t)row * p.in_f + col;
         if (wide) {
-            st_sector(dst, r);
-        } else if (col0 + 16u <= p.in_f) {
-            ((uint4 *)dst)[0] = make_uint4(r[0], r[1], r[2], r[3]);
-            ((uint4 *)dst)[1] = make_uint4(r[4], r[5], r[6], r[7]);
-        } else {
-#pragma unroll
-            for (uint32_t c = 0; c < 16u; ++c)
-                if (col0 + c < p.in_f) ((uint16_t *)dst)[c] = (uint16_t)(r[c >> 1] >> (16 * (c & 1)));
+            const uint32_t v[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+            st_sector(dst, v);
+        } else {                                     // in_f % 8 == 0: eight columns or none
+            ((uint4 *)dst)[0] = v0;
+            if (col + 16u <= p.in_f) ((uint4 *)dst)[1] = v1;
         }
     }
 }
@@ -606,7 +608,7 @@ k_p6_mma(P6 p, const __nv_bfloat16 *__restrict__ x, uint32_t m_rows, const __nv_
         } else {
             sc_cur = (uint32_t)__bfloat16_as_ushort(p.scale[0]);
         }
-        asm volatile("mov.b32 %0, 0x42804280;" : "=r"(e2));            // opaque, so that it stays a register operand
+        asm volatile("mov.b32 %0, 0x43004300;" : "=r"(e2));            // opaque, so that it stays a register operand
     }
     auto set_scale = [&](uint32_t bits) { s2 = bits | bits << 16; };
     set_scale(sc_cur);
@@ -758,8 +760,8 @@ k_p6_mma(P6 p, const __nv_bfloat16 *__restrict__ x, uint32_t m_rows, const __nv_
         const uint32_t R_first = R;
         // this lane's activations: row min(g, m_rows - 1) (rows beyond m_rows only feed unused C columns)
         const uint32_t xrow = min((uint32_t)g, m_rows - 1u);
-        const __nv_bfloat16 *xg = x + (size_t)xrow * p.in_f + 16 * t;                                  // XS = 0
-        const uint32_t xs_l = (uint32_t)__cvta_generic_to_shared(xs) + (xrow * xstride + 16 * t) * 2u;   // XS = 1
+        const __nv_bfloat16 *xg = x + (size_t)xrow * p.in_f + 4 * t;                                   // XS = 0
+        const uint32_t xs_l = (uint32_t)__cvta_generic_to_shared(xs) + (xrow * xstride + 4 * t) * 2u;    // XS = 1
         uint32_t cs = 0, is = 3 * kP6BlockBytes;     // byte offsets of the ring slot to consume next / to refill next
         const uint32_t d8 = ring_s + 512 + lane * 8;
         const bool lo16 = lane < 16;
@@ -775,26 +777,26 @@ k_p6_mma(P6 p, const __nv_bfloat16 *__restrict__ x, uint32_t m_rows, const __nv_
                 cp_async_commit();
                 n16 += kP6BlockBytes;
                 pf_left -= more ? 1u : 0u;
-                uint4 x0, x1;
+                uint2 xv[4];
                 if (!XS) {                                        // requested ahead of the wait for the block
-                    x0 = *(const uint4 *)((const char *)xg + xo);
-                    x1 = *(const uint4 *)((const char *)xg + xo + 16);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) xv[j] = *(const uint2 *)((const char *)xg + xo + 32 * j);
                 }
                 cp_async_wait<3>();                               // this lane's chunks of the block have landed ...
                 __syncwarp();                                     // ... and so have the other lanes'
                 const uint4 a = p6_lds128(d16 + cs);
                 const uint2 a2 = p6_lds64(d8 + cs);
                 if (XS) {
-                    x0 = p6_lds128(xs_l + xo);
-                    x1 = p6_lds128(xs_l + xo + 16u);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) xv[j] = p6_lds64(xs_l + xo + 32u * j);
                 }
                 const uint32_t w[6] = {a.x, a.y, a.z, a.w, a2.x, a2.y};
                 uint32_t f[16];
                 p6_unpack(w, e2, s2, f);
-                p6_mma(c, f[0], f[1], f[2], f[3], x0.x, x0.y);
-                p6_mma(c1, f[4], f[5], f[6], f[7], x0.z, x0.w);
-                p6_mma(c, f[8], f[9], f[10], f[11], x1.x, x1.y);
-                p6_mma(c1, f[12], f[13], f[14], f[15], x1.z, x1.w);
+                p6_mma(c, f[0], f[1], f[2], f[3], xv[0].x, xv[0].y);
+                p6_mma(c1, f[4], f[5], f[6], f[7], xv[1].x, xv[1].y);
+                p6_mma(c, f[8], f[9], f[10], f[11], xv[2].x, xv[2].y);
+                p6_mma(c1, f[12], f[13], f[14], f[15], xv[3].x, xv[3].y);
                 is = cs;
                 cs = cs == (uint32_t)(3 * kP6BlockBytes) ? 0u : cs + (uint32_t)kP6BlockBytes;
                 xo += kTileCols * 2u;

@@ -1,19 +1,16 @@
-// Small-M GEMM on the resident P6 layout: 9..64 activation rows (batched serving, speculative verification) against a
-// packed tensor in one pass over its bytes.
+// Small-M GEMM on the resident P6 layout on mma.sync, for 9..24 activation rows of layers with several outliers per block (the
+// other calls of 9..64 rows are k_p6_umma's, ixb_p6_umma.cuh).
 //
-//   Y[m][n] = sum_k X[m][k] * bf16(code[n][k] * scale)        m < m_rows <= 64
+//   Y[m][n] = sum_k X[m][k] * bf16(code[n][k] * scale)        m < m_rows <= 24
 //
 // The reference runs this case as decode -> bf16 weight in HBM -> dense matmul (ixrun/engine.py:171-173; structural
 // precedent for a fused kernel: ixrun/tpab_gemm.py:34-94).  Here the weights become the A operands of mma.sync in
 // registers, as in the GEMV (k_p6_mma).
 //
 // What bounds it: 6.05 bits of HBM per weight and four instructions per pair of weights for the conversion (six where the
-// field is split), the same as the GEMV; on top of that one mma per 16 x 16 weights and eight rows, 64 rows being where the
-// mma rate takes over.  Feeding the converted weights to tcgen05 through shared memory instead (k_p6_gemm) moves four bytes of
-// shared memory per weight and hands every 64 columns over twice between converters, copies and tensor core: 17408 x 5120
-// takes 40 us there at 16 rows and 57 us at 64, of which 27 us are hand-over with no work in it.  Here nothing is handed over
-// between warps but the activations: 26 and 49 us.  (Where the row groups do not fill the chip, k_p6_gemm is the faster one
-// above 32 rows: pg_is_faster.)
+// field is split), the same as the GEMV; on top of that one mma per 16 x 16 weights and eight rows, and a barrier of four warps
+// per block: 17408 x 5120 with 16 rows 26.2 us.  Its steps have slack for a block's outliers, which k_p6_umma's converters lack
+// (8 per block: 29.5 and 32.3 us).
 //
 // CTA  = 8 row tiles (128 weight rows) x a contiguous range of column blocks; K is split over the CTAs of a cluster as
 //        far as it takes to fill the chip, and the splits' sums are added in rank order through distributed shared memory.
@@ -28,10 +25,10 @@
 
 namespace ixb {
 
-constexpr int kPrMaxRows = 64;
+constexpr int kPrMaxRows = 24;
 constexpr int kPrTiles = 8;                              // row tiles per CTA
 constexpr int kPrRows = kPrTiles * kTileRows;            // 128
-constexpr uint32_t kPrXPitch = kTileCols * 2 + 16;       // bytes of one activation row in a stage: 16-byte reads without conflicts
+constexpr uint32_t kPrXPitch = kTileCols * 2 + 32;       // bytes of one activation row in a stage: 8-byte reads without conflicts
 constexpr int kPrRedPitch = kPrRows + 4;                 // floats of one token in the sums: conflict free from the C fragments
 
 template <int NT, int PARTS, int STAGES>
@@ -130,7 +127,7 @@ k_p6_rows(P6 p, const __nv_bfloat16 *__restrict__ x, uint32_t m_rows, const __nv
     for (int q = 0; q < 4; ++q) ((uint4 *)img)[q * 32 + lane] = make_uint4(0, 0, 0, 0);
     const uint32_t img_s = (uint32_t)__cvta_generic_to_shared(img);
     uint32_t s2[2], e2;
-    asm volatile("mov.b32 %0, 0x42804280;" : "=r"(e2));
+    asm volatile("mov.b32 %0, 0x43004300;" : "=r"(e2));
 #pragma unroll
     for (int i = 0; i < 2; ++i) s2[i] = p6_scale2(p.scale[(have[i] ? tile0 + i : 0u) * p.scale_stride]);
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -144,7 +141,7 @@ k_p6_rows(P6 p, const __nv_bfloat16 *__restrict__ x, uint32_t m_rows, const __nv
     for (int i = 0; i < 2; ++i)
 #pragma unroll
         for (int n = 0; n < NT; ++n) acc[i][n][0] = acc[i][n][1] = acc[i][n][2] = acc[i][n][3] = 0.f;
-    const uint32_t xl = (uint32_t)g * kPrXPitch + 32u * t;             // this lane's 16 activations of row g: + 8 n rows
+    const uint32_t xl = (uint32_t)g * kPrXPitch + 8u * t;              // this lane's activations of row g, 4 of every 16: + 8 n rows
     for (uint32_t s = 0; s < steps; ++s) {
         cp_async_wait<STAGES - 2>();                   // step s has landed for this thread ...
         asm volatile("bar.sync %0, 128;" ::"r"(part + 1u) : "memory");   // ... and for the part, which is done with step s - 1
@@ -195,24 +192,24 @@ k_p6_rows(P6 p, const __nv_bfloat16 *__restrict__ x, uint32_t m_rows, const __nv
             __syncwarp();
         }
         const uint32_t xb = xpart + slot_of(s) * (PARTS * SM::kX) + xl;
-        uint4 x0 = p6_lds128(xb), x1 = p6_lds128(xb + 16);
+        uint2 xv[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) xv[j] = p6_lds64(xb + 32u * j);
 #pragma unroll
         for (int n = 0; n < NT; ++n) {
-            uint4 y0, y1;
+            uint2 yv[4];
             if (n + 1 < NT) {
-                y0 = p6_lds128(xb + (n + 1) * 8 * kPrXPitch);
-                y1 = p6_lds128(xb + (n + 1) * 8 * kPrXPitch + 16);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) yv[j] = p6_lds64(xb + (n + 1) * 8 * kPrXPitch + 32u * j);
             }
 #pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                p6_mma(acc[i][n], f[i][0], f[i][1], f[i][2], f[i][3], x0.x, x0.y);
-                p6_mma(acc[i][n], f[i][4], f[i][5], f[i][6], f[i][7], x0.z, x0.w);
-                p6_mma(acc[i][n], f[i][8], f[i][9], f[i][10], f[i][11], x1.x, x1.y);
-                p6_mma(acc[i][n], f[i][12], f[i][13], f[i][14], f[i][15], x1.z, x1.w);
-            }
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    p6_mma(acc[i][n], f[i][4 * j], f[i][4 * j + 1], f[i][4 * j + 2], f[i][4 * j + 3], xv[j].x, xv[j].y);
             if (n + 1 < NT) {
-                x0 = y0;
-                x1 = y1;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) xv[j] = yv[j];
             }
         }
     }

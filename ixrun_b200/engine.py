@@ -157,10 +157,9 @@ class StreamingLinear(nn.Module):
             elif self._use_p6_gemm and rows > FUSED_MAX_ROWS and self._bias is None and self.in_features % 8 == 0 \
                     and self._w_buf is not None and x.get_device() == res._index and _plain(x):
                 # Without a bias, which decode + dense matmul adds before the one rounding.  A call outside a graph, this
-                # kernel and that route: 2048 x 2080 10.4 and 21.4 us with 24 rows, 12.5 and 21.4 with 64; 8192 x 8224 32
-                # and 56, 48 and 60.  (Above 48 rows layers of 25 to 40 million weights lose up to 7 us: 6144 x 6176 25.5
-                # and 32, 40 and 33.)  Two passes for more rows lose nearly everywhere: 6144 x 6144 with 65 rows 55 and
-                # 38 us, 17408 x 5120 with 128 rows 105 and 80.
+                # kernel and that route: 2048 x 2080 12.5 and 32.5 us with 24 rows, 12.8 and 21.8 with 64; 8192 x 8224 27 and 55,
+                # 29 and 61; 6144 x 6176 22 and 33, 23 and 33.  (Two passes for more rows lost nearly everywhere to decode + dense
+                # matmul when a pass took twice as long.)
                 y = res.rows(x)
             if y is not None:
                 return y if x.dim() == 2 else y.view(x.shape[:-1] + (self.out_features,))

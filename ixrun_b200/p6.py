@@ -2,7 +2,7 @@
 
 The (3,5,8) streams remain the interchange format; ``P6Packed.from_packed``
 transcodes them on the GPU, keeping every int8 code.  P6 spends 6 plane bits per weight on a field that *is* part of the
-bf16 number ``96 + code`` (codes -32..31), so a subtraction and a multiplication
+bf16 number ``160 + code`` (codes -32..31), so a subtraction and a multiplication
 per pair of weights yield the reference's ``bf16(code * scale)``; every other code goes
 to a short list.
 """
@@ -95,7 +95,7 @@ class P6Packed:
                                     self.scale.data_ptr(), self.out_f, self.in_f, stride)
         self._ref = C.byref(self.struct)             # (keeps the struct alive)
         self._index = dev.index
-        self._gemv_need, self._gemm_need = None, {}      # scratch bytes; the latter by row count
+        self._gemv_need = None                           # scratch bytes
         self.resident_bytes = nb * BLOCK_BYTES + 4 * (nb + 1 + n_esc) + 2
         self.scratch = scratch if scratch is not None else GemvScratch.shared(dev)
 
@@ -197,15 +197,13 @@ class P6Packed:
         out = self._out(m, out, out_dtype, bias, "gemm")
         if not 1 <= m <= self.GEMM_MAX_ROWS:
             raise ValueError(f"unsupported GEMM shape: {m} rows")
+        if self.in_f % 64:
+            raise _lib.IxbError(f"in_f={self.in_f} is not a multiple of 64")
         L = _lib.lib()
         with _lib.on_device(self._index) as stream:
-            need = 256 if m <= 32 else self._gemm_need.get(m)        # (k_p6_rows up to 32 rows)
-            if need is None:
-                need = self._gemm_need[m] = int(L.ixb_p6_gemm_scratch_bytes(self.out_f, self.in_f, m))
-            # partial sums of the tcgen05 form: a buffer of the call's own, so calls on several streams do not share it
-            s = self.scratch.reserve(256) if need <= 256 else torch.empty(need, dtype=torch.uint8, device=self.device)
-            rc = L.ixb_p6_gemm(self._ref, x2.data_ptr(), m, None if bias is None else bias.data_ptr(), out.data_ptr(),
-                               1 if out.dtype == torch.float32 else 0, s.data_ptr(), s.numel(), stream)
+            # (ixb_p6_gemm is the same launch for callers with a scratch)
+            rc = L.ixb_p6_rows(self._ref, x2.data_ptr(), m, None if bias is None else bias.data_ptr(), out.data_ptr(),
+                               1 if out.dtype == torch.float32 else 0, stream)
         if rc:
             _lib.check(rc)
         return out

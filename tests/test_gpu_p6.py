@@ -391,3 +391,33 @@ def test_p6_negative_scale(in_f):
         assert near(p6.gemm(x[:23], out_dtype=torch.float32), 23)
     y = p6.rows(x)
     assert bool(((y.double() - ref).abs() <= ref.abs() * 2.0 ** -8 + 1e-5 * ref.abs().max()).all())
+
+
+@pytest.mark.parametrize("m", [9, 16, 17, 33, 64])
+@pytest.mark.parametrize("out_f,in_f,per_block", [(16, 64, 0), (16, 64, 2), (144, 1000, 4), (2064, 128, 2), (300, 4160, 49),
+                                                  (300, 4160, 51), (129, 17408, 1)])
+def test_p6_rows_edges(out_f, in_f, per_block, m):
+    """9..64 rows where their kernels can go wrong: one column block, an odd number of them, a ragged last one, a last row group
+    of one tile, both sides of the rule on outliers per block (3 and 50), an activation of infinity.  Bound: fp32 sums of at most
+    17408 exact products in chains, 2e-5 of the largest result as above."""
+    from ixrun_b200.p6 import P6Packed
+
+    gen = torch.Generator(device="cuda").manual_seed(out_f + in_f + m)
+    codes = (torch.randn(out_f, in_f, generator=gen, device="cuda") * 8).round().clamp(-31, 31)
+    rt, kb = (out_f + 15) // 16, (in_f + 63) // 64
+    at = torch.randperm(out_f * in_f, generator=gen, device="cuda")[:per_block * rt * kb]
+    codes.view(-1)[at] = torch.where(codes.view(-1)[at] < 0, -127.0, 100.0)
+    p6 = P6Packed(codes.to(torch.int8), torch.tensor(0.007, dtype=torch.bfloat16), out_f, in_f)
+    w = (codes * p6.scale.float()).bfloat16().double()
+    x = torch.randn(m, in_f, generator=gen, device="cuda").bfloat16()
+    call = p6.gemm if in_f % 64 == 0 else p6.rows
+    ref = x.double() @ w.t()
+    assert float((call(x).double() - ref).abs().max() / ref.abs().max()) < 2e-5 + 2.0 ** -8
+    if in_f % 64 == 0:
+        y = p6.gemm(x, out_dtype=torch.float32)
+        assert float((y.double() - ref).abs().max() / ref.abs().max()) < 2e-5
+    # infinity times a weight is infinity of its sign, or NaN for a weight of 0; it reaches only its own row of activations
+    x[3, in_f // 2] = float("inf")
+    y, ref = call(x), (x.double() @ w.t()).bfloat16()
+    assert torch.equal(y[3].nan_to_num(nan=7.0, posinf=1.0, neginf=-1.0), ref[3].nan_to_num(nan=7.0, posinf=1.0, neginf=-1.0))
+    assert torch.isfinite(y[torch.arange(m, device="cuda") != 3]).all()
