@@ -10,6 +10,7 @@
 #include "ixb_attn_prefill.cuh"
 #include "ixb_p6_rows.cuh"
 #include "ixb_p6_umma.cuh"
+#include "ixb_p6_short.cuh"
 #include "ixb_pack.cuh"
 #include "ixb_p6.cuh"
 #include "ixb_allreduce.cuh"
@@ -1045,6 +1046,49 @@ static cudaError_t launch_p6(const P6 &p, const void *x, uint32_t m_rows, const 
                               slots, tickets, pl.nb, pl.xstride, pl.cq, pl.cr, pl.unit, push);
 }
 
+#define IXB_GLUE(what, call)                                                                    \
+    do {                                                                                      \
+        cudaError_t e_ = (call);                                                              \
+        if (e_ != cudaSuccess) return fail(IXB_E_CUDA, "%s launch: %s", what, cudaGetErrorString(e_)); \
+        return launch_check(what);                                                            \
+    } while (0)
+
+// The form for few blocks per warp (ixb_p6_short.cuh); 0 CTAs: not for this layer.  The rule does not look at m_rows, so that a row
+// gets the same bits alone or beside others.
+static PsPlan make_ps_plan(const P6 &p, uint32_t m_rows)
+{
+    PsPlan pl = {0, 0, 0, 0, 0};
+    const uint32_t sms = (uint32_t)num_sms(), tiles = (p.rt + sms - 1) / sms, slice = (p.kb + kPsWarps - 1) / kPsWarps;
+    if (p.in_f % 8u || tiles > kPsMaxBlocks || slice > kPsMaxBlocks || tiles * slice > kPsMaxBlocks) return pl;
+    pl.tiles = tiles;
+    pl.slice = slice;
+    pl.xpitch = ps_xpitch(slice);
+    pl.smem = kPsWarps * 2048u + kPsWarps * m_rows * pl.xpitch + tiles * kPsWarps * ps_part(m_rows > 1u) * 4u;
+    // (the largest: one tile, 8 column blocks, 8 rows: 32 + 132 + 8 KB; 8 tiles, 1 block: 32 + 20 + 64)
+    static_assert(kPsWarps * 2048u + kPsWarps * 8u * ps_xpitch(kPsMaxBlocks) + kPsWarps * ps_part(true) * 4u <= 227u * 1024u, "fits");
+    pl.grid = (p.rt + tiles - 1) / tiles;                // as few CTAs as finish in the same number of tiles
+    return pl;
+}
+
+template <bool MULTI>
+static cudaError_t launch_ps(const P6 &p, const void *x, uint32_t m_rows, const void *bias, void *y, int y_f32, const PsPlan &pl, const P6Push &push, cudaStream_t st)
+{
+    static bool attr_set[64] = {false};
+    cudaError_t oe = opt_in_smem(k_p6_short<MULTI>, attr_set, 227 * 1024);
+    if (oe != cudaSuccess) return oe;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(pl.grid);
+    cfg.blockDim = dim3(kPsThreads);
+    cfg.dynamicSmemBytes = pl.smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = g_p6_pdl.load() ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, k_p6_short<MULTI>, p, (const __nv_bfloat16 *)x, m_rows, (const __nv_bfloat16 *)bias, y, y_f32, pl, push);
+}
+
 static int p6_gemv_impl(const ixb_p6 *t, const void *x, int64_t m_rows, const void *bias, void *y, int y_is_f32,
                         void *scratch, size_t scratch_bytes, const P6Push &push, ixb_stream_t stream)
 {
@@ -1065,8 +1109,14 @@ static int p6_gemv_impl(const ixb_p6 *t, const void *x, int64_t m_rows, const vo
     float4 *slots = (float4 *)((char *)scratch + 1024);
     P6Push pu = push;
     pu.done = tickets + 255;                                   // ... and, in the last word, the count of finished warps
-    if (pu.fin && ((p.out_f & 1u) || pl.grid * (uint32_t)kP6Threads * 2u < (uint32_t)m_rows * p.out_f))
-        return fail(IXB_E_UNSUPPORTED, "a finishing GEMV needs an even out_f and at most %u outputs", pl.grid * (uint32_t)kP6Threads * 2u);
+    const PsPlan ps = make_ps_plan(p, (uint32_t)m_rows);
+    const uint32_t threads = ps.grid ? ps.grid * (uint32_t)kPsThreads : pl.grid * (uint32_t)kP6Threads;
+    if (pu.fin && ((p.out_f & 1u) || threads * 2u < (uint32_t)m_rows * p.out_f))
+        return fail(IXB_E_UNSUPPORTED, "a finishing GEMV needs an even out_f and at most %u outputs", threads * 2u);
+    if (ps.grid) {
+        auto launch = m_rows == 1 ? launch_ps<false> : launch_ps<true>;
+        IXB_GLUE("k_p6_short", launch(p, x, (uint32_t)m_rows, bias, y, y_is_f32, ps, pu, (cudaStream_t)stream));
+    }
     cudaStream_t st = (cudaStream_t)stream;
     auto launch = m_rows == 1  ? (pl.xs ? launch_p6<1, 1> : launch_p6<0, 1>)
                   : m_rows == 2 ? (pl.xs ? launch_p6<1, 2> : launch_p6<0, 2>)
@@ -1250,12 +1300,6 @@ static cudaError_t launch_glue(void (*kernel)(KArgs...), dim3 grid, dim3 block, 
     cfg.numAttrs = g_p6_pdl.load() ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
-#define IXB_GLUE(what, call)                                                                    \
-    do {                                                                                      \
-        cudaError_t e_ = (call);                                                              \
-        if (e_ != cudaSuccess) return fail(IXB_E_CUDA, "%s launch: %s", what, cudaGetErrorString(e_)); \
-        return launch_check(what);                                                            \
-    } while (0)
 
 static bool norm_vector_ok(const void *h, const void *delta, const void *w, const void *xn, int64_t hidden, int64_t limit)
 {

@@ -447,6 +447,59 @@ __device__ __forceinline__ void p6_store_pair(const P6Push &push, uint32_t e, ui
     }
 }
 
+// The exchange's second half, by the same kernel: every thread of the grid looks after one pair of outputs (the first n / 2
+// threads have one).  The words of this rank come from this very launch -- from CTAs that are all resident, one per SM -- and the
+// other ranks' from their launches of the same call.
+template <int THREADS>
+__device__ __forceinline__ void p6_finish_exchange(const P6Push &push, uint32_t push_e, uint32_t out_f, uint32_t m_rows,
+                                                   const __nv_bfloat16 *__restrict__ bias, void *y, int y_f32)
+{
+    const uint32_t n = m_rows * out_f, i = (blockIdx.x * THREADS + threadIdx.x) * 2u, W = push.world;
+    if (i < n) {
+        const uint32_t limit = *(volatile uint32_t *)push.err ? 64u : push.spin_limit;
+        const uint2 *mine = push.mine;
+        float o0 = 0.f, o1 = 0.f;
+        for (uint32_t s = 0; s < W; ++s) {
+            const uint2 *src = mine + ((size_t)((push_e & 1u) * W + s)) * push.n_max + i;
+            uint32_t v0, m0, v1, m1, polls = 0;
+            for (;;) {
+                asm volatile("ld.volatile.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v0), "=r"(m0), "=r"(v1), "=r"(m1) : "l"(src) : "memory");
+                if (m0 == push_e && m1 == push_e) break;
+                __nanosleep(20);
+                if (++polls > limit) {
+                    *push.err = 1u + s;                // sender s never arrived: the result is wrong, not a hang
+                    break;
+                }
+            }
+            o0 += __uint_as_float(v0);
+            o1 += __uint_as_float(v1);
+        }
+        const uint32_t r0 = i % out_f;               // n is even and so is out_f: both values belong to one activation row
+        if (y_f32) {
+            float2 r;
+            r.x = bias ? o0 + __bfloat162float(bias[r0]) : o0;
+            r.y = bias ? o1 + __bfloat162float(bias[r0 + 1]) : o1;
+            *(float2 *)((float *)y + i) = r;
+        } else {
+            __nv_bfloat16 h0 = __float2bfloat16_rn(o0), h1 = __float2bfloat16_rn(o1);
+            if (bias) {
+                h0 = __hadd(h0, bias[r0]);
+                h1 = __hadd(h1, bias[r0 + 1]);
+            }
+            *(__nv_bfloat162 *)((__nv_bfloat16 *)y + i) = __halves2bfloat162(h0, h1);
+        }
+    }
+    // the last warp of the grid to get here advances the call counters: by now every CTA has read them
+    __syncwarp();
+    if ((threadIdx.x & 31u) == 0) {
+        __threadfence();
+        if (atomicAdd(push.done, 1u) == gridDim.x * (THREADS / 32u) - 1u) {
+            for (uint32_t k = 0; k < push.counters; ++k) push.epoch[k] = push_e;
+            *push.done = 0;
+        }
+    }
+}
+
 // n elements cut into `parts` contiguous parts, the first r = n % parts of them one longer than q = n / parts:
 // first element of part i, and the part that holds element pos (no 64-bit arithmetic, no division on the way in)
 __device__ __forceinline__ uint32_t p6_begin(uint32_t i, uint32_t q, uint32_t r) { return i * q + min(i, r); }
@@ -967,57 +1020,7 @@ k_p6_mma(P6 p, const __nv_bfloat16 *__restrict__ x, uint32_t m_rows, const __nv_
             finish_tile(R, wlo, whi, inside, clo, span);
         }
     }
-    if (!push.fin) return;
-
-    // ---- the exchange's second half, by the same kernel: every thread of the grid looks after one pair of outputs
-    // (the first n / 2 threads have one).  The words of this rank come from this very launch -- from CTAs that are
-    // all resident, one per SM -- and the other ranks' from their launches of the same call.
-    {
-        const uint32_t n = m_rows * p.out_f, i = (blockIdx.x * kP6Threads + threadIdx.x) * 2u, W = push.world;
-        if (i < n) {
-            const uint32_t limit = *(volatile uint32_t *)push.err ? 64u : push.spin_limit;
-            const uint2 *mine = push.mine;
-            float o0 = 0.f, o1 = 0.f;
-            for (uint32_t s = 0; s < W; ++s) {
-                const uint2 *src = mine + ((size_t)((push_e & 1u) * W + s)) * push.n_max + i;
-                uint32_t v0, m0, v1, m1, polls = 0;
-                for (;;) {
-                    asm volatile("ld.volatile.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v0), "=r"(m0), "=r"(v1), "=r"(m1) : "l"(src) : "memory");
-                    if (m0 == push_e && m1 == push_e) break;
-                    __nanosleep(20);
-                    if (++polls > limit) {
-                        *push.err = 1u + s;                // sender s never arrived: the result is wrong, not a hang
-                        break;
-                    }
-                }
-                o0 += __uint_as_float(v0);
-                o1 += __uint_as_float(v1);
-            }
-            const uint32_t r0 = i % p.out_f;               // n is even and so is out_f: both values belong to one activation row
-            if (y_f32) {
-                float2 r;
-                r.x = bias ? o0 + __bfloat162float(bias[r0]) : o0;
-                r.y = bias ? o1 + __bfloat162float(bias[r0 + 1]) : o1;
-                *(float2 *)((float *)y + i) = r;
-            } else {
-                __nv_bfloat16 h0 = __float2bfloat16_rn(o0), h1 = __float2bfloat16_rn(o1);
-                if (bias) {
-                    h0 = __hadd(h0, bias[r0]);
-                    h1 = __hadd(h1, bias[r0 + 1]);
-                }
-                *(__nv_bfloat162 *)((__nv_bfloat16 *)y + i) = __halves2bfloat162(h0, h1);
-            }
-        }
-        // the last warp of the grid to get here advances the call counters: by now every CTA has read them
-        __syncwarp();
-        if (lane == 0) {
-            __threadfence();
-            if (atomicAdd(push.done, 1u) == gridDim.x * kP6Warps - 1u) {
-                for (uint32_t k = 0; k < push.counters; ++k) push.epoch[k] = push_e;
-                *push.done = 0;
-            }
-        }
-    }
+    if (push.fin) p6_finish_exchange<kP6Threads>(push, push_e, p.out_f, m_rows, bias, y, y_f32);
 }
 
 }  // namespace ixb

@@ -421,3 +421,33 @@ def test_p6_rows_edges(out_f, in_f, per_block, m):
     y, ref = call(x), (x.double() @ w.t()).bfloat16()
     assert torch.equal(y[3].nan_to_num(nan=7.0, posinf=1.0, neginf=-1.0), ref[3].nan_to_num(nan=7.0, posinf=1.0, neginf=-1.0))
     assert torch.isfinite(y[torch.arange(m, device="cuda") != 3]).all()
+
+
+@pytest.mark.parametrize("dense", [False, True])
+@pytest.mark.parametrize("out_f,in_f", [(16, 8), (40, 1000), (2384, 128), (300, 2176), (2048, 8192), (2048, 8256), (18944, 512),
+                                        (19000, 512)])
+def test_p6_gemv_few_blocks(out_f, in_f, dense):
+    """1..8 rows on layers of few blocks per warp, and both sides of the rule (8 blocks): fewer column blocks than warps, slices
+    of unequal length, a ragged last block, CTAs with fewer tiles than others, more outliers than lanes, an infinite activation.
+    Bound: fp32 sums of at most 8256 exact products, 2e-5 of the largest result as above."""
+    from ixrun_b200.p6 import P6Packed
+
+    gen = torch.Generator(device="cuda").manual_seed(out_f + in_f)
+    codes = torch.randn(out_f, in_f, generator=gen, device="cuda") * (60 if dense else 10)
+    codes = codes.round().clamp(-127, 127).to(torch.int8)
+    p6 = P6Packed(codes, torch.tensor(-0.007, dtype=torch.bfloat16), out_f, in_f)
+    w = (codes.float() * p6.scale.float()).bfloat16().double()
+    x = torch.randn(8, in_f, generator=gen, device="cuda").bfloat16()
+    ref = x.double() @ w.t()
+    bias = torch.randn(out_f, generator=gen, device="cuda").bfloat16()
+    y8 = p6.gemv(x, out_dtype=torch.float32)
+    assert float((y8.double() - ref).abs().max() / ref.abs().max()) < 2e-5
+    for m in (1, 2, 5):
+        assert torch.equal(p6.gemv(x[:m], out_dtype=torch.float32), y8[:m])
+    assert torch.equal(p6.gemv(x[:3], bias=bias), y8[:3].bfloat16() + bias)
+    if (out_f, in_f) in ((2048, 8256), (19000, 512)):
+        return                                       # the other kernel: an infinity that meets an outlier is NaN there
+    x[1, in_f // 2] = float("-inf")
+    y, ref = p6.gemv(x), (x.double() @ w.t()).bfloat16()
+    assert torch.equal(y[1].nan_to_num(nan=7.0, posinf=1.0, neginf=-1.0), ref[1].nan_to_num(nan=7.0, posinf=1.0, neginf=-1.0))
+    assert torch.equal(y[[0, 2, 3, 4, 5, 6, 7]], y8[[0, 2, 3, 4, 5, 6, 7]].bfloat16())
