@@ -48,6 +48,24 @@ __device__ __forceinline__ int code_level(int c)
     return a <= 3 ? 0 : (a <= 15 ? 1 : 2);
 }
 
+// ---- four codes at a time, as the bytes of a word (two's complement)
+// 0xff where a byte's top bit is set, 0 elsewhere
+__device__ __forceinline__ uint32_t byte_signs(uint32_t w)
+{
+    uint32_t v;
+    asm("prmt.b32 %0, %1, %1, 0xBA98;" : "=r"(v) : "r"(w));
+    return v;
+}
+// the top bits of the bytes: |code| > 3, |code| > 15
+__device__ __forceinline__ void code_levels4(uint32_t w, uint32_t &over3, uint32_t &over15)
+{
+    const uint32_t neg = byte_signs(w), a = (w ^ neg) + (neg & 0x01010101u);       // |code|, at most 128: no byte carries
+    over3 = (a + 0x7C7C7C7Cu) & 0x80808080u;
+    over15 = (a + 0x70707070u) & 0x80808080u;
+}
+// the top bits of the four bytes as a number (bits 7, 15, 23, 31 meet at 28 .. 31, the other products below without a carry)
+__device__ __forceinline__ uint32_t top_bits(uint32_t y) { return (y * 0x00204081u) >> 28; }
+
 // code = clamp(rint(w / sc)), the division rounded to fp32 as the reference does.  w * (1 / sc) is within 2^-22 of the
 // quotient, which for |code| < 128 is 3e-5: away from the halves between two codes both round to the same code, and only
 // near them (or beyond 128, infinite, NaN, a scale without a reciprocal) the division itself is taken.
@@ -61,8 +79,10 @@ __device__ __forceinline__ int quantise_code(uint32_t bf16_bits, float sc, float
 
 // One warp per 1024-element block.  MODE 0: quantise from bf16 weights and write codes; MODE 1: read existing codes.
 // Both write the B1 words and the block's level-1 / level-2 counts.  Whole blocks of aligned tensors: a lane takes
-// eight consecutive elements four times, so that loads (16 / 8 bytes), codes and B1 bytes are contiguous across the warp
-// (5120 x 5120 in mode 0: 26 us, 154 when a lane walked its 32 elements one by one and divided each).
+// eight consecutive elements four times, so that loads (16 / 8 bytes), codes and B1 bytes are contiguous across the warp.  The
+// fast path rounds by an addition of 1.5 * 2^23, whose low byte is the code, and finds the levels of four codes at a time
+// (5120 x 5120 in mode 0: 18.6 us, 27 with a rounding instruction and a comparison per element, 154 when a lane walked its 32
+// elements one by one and divided each).
 template <int MODE>
 __global__ void __launch_bounds__(256)
 k_codes_and_counts(const uint16_t *__restrict__ w, const uint32_t *absmax_bits, int8_t *codes, uint32_t n,
@@ -94,19 +114,31 @@ k_codes_and_counts(const uint16_t *__restrict__ w, const uint32_t *absmax_bits, 
         for (int it = 0; it < 4; ++it) {
             const uint32_t e = b * kBlk + it * 256u + lane * 8u;
             const uint32_t wr[4] = {wv[it].x, wv[it].y, wv[it].z, wv[it].w}, cr[2] = {cv[it].x, cv[it].y};
-            uint32_t co[2] = {0, 0}, m1 = 0, e2 = 0;
+            uint32_t co[2] = {cr[0], cr[1]};
+            if (MODE == 0) {
+                uint32_t r[8];
+                bool plain = true;                       // no quotient near a half, none beyond the range
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                int c;
-                if (MODE == 0) {
-                    c = quantise_code((wr[i >> 1] >> (16 * (i & 1))) & 0xffffu, sc, inv);
-                    co[i >> 2] |= (uint32_t)(c & 0xff) << (8 * (i & 3));
-                } else {
-                    c = (int)(int8_t)(cr[i >> 2] >> (8 * (i & 3)));
+                for (int i = 0; i < 8; ++i) {
+                    const float v = __uint_as_float(i & 1 ? wr[i >> 1] & 0xffff0000u : wr[i >> 1] << 16), q = v * inv, t = q + 12582912.f;
+                    plain = plain && fabsf(q - (t - 12582912.f)) < 0.499f && fabsf(q) < 127.4f;
+                    r[i] = __float_as_uint(t);
                 }
-                const int lv = code_level(c);
-                m1 |= (uint32_t)(lv == 0) << i;
-                e2 |= (uint32_t)(lv == 1) << i;
+                if (!plain) {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) r[i] = (uint32_t)quantise_code((wr[i >> 1] >> (16 * (i & 1))) & 0xffffu, sc, inv);
+                }
+#pragma unroll
+                for (int k = 0; k < 2; ++k)
+                    co[k] = __byte_perm(__byte_perm(r[4 * k], r[4 * k + 1], 0x0040), __byte_perm(r[4 * k + 2], r[4 * k + 3], 0x0040), 0x5410);
+            }
+            uint32_t m1 = 0, e2 = 0;
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                uint32_t over3, over15;
+                code_levels4(co[k], over3, over15);
+                m1 |= (top_bits(over3) ^ 15u) << (4 * k);
+                e2 |= top_bits(over3 & ~over15) << (4 * k);
             }
             if (MODE == 0) *(uint2 *)(codes + e) = make_uint2(co[0], co[1]);
             ((uint8_t *)b1)[e >> 3] = (uint8_t)m1;
@@ -163,11 +195,13 @@ __device__ __forceinline__ void write_image(uint32_t *stream, const uint32_t *im
     }
 }
 
-// Streams must be zero on entry.  One warp per block, lane = word of 32 elements.  Bound by instructions: a lane runs its
-// elements backwards and shifts every field in at the low end of its own bits (3 words of level 1, 5 of level 2, one of
-// the second bitmap), with predicates and no branches but for the rare level 3; the lanes' bits meet in an image of the
-// block's words in shared memory, which is written in whole words.  5120 x 5120: 57 us; 91 with a branch per
-// element, 104 with one global atomic per field.
+// Streams must be zero on entry.  One warp per block, lane = word of 32 elements.  Bound by instructions: levels and fields
+// are made four at a time; a lane runs its elements backwards, eight at a time, and brings every field in at the low end of a
+// group's bits (a multiplication and an addition: logic and shifts have half their rate), with predicates and no branches but
+// for the rare level 3; a group then goes in at the low end of the lane's bits (3 words of level 1, 5 of level 2, one of the
+// second bitmap).  The lanes' bits meet in an image of the block's words in shared memory, which is written in whole words.
+// 5120 x 5120: 35 us; 58 with every field shifted into the lane's bits by itself, 91 with a branch per element, 104 with one
+// global atomic per field.
 constexpr int kPackB2 = 0, kPackL1 = 36, kPackL2 = 140, kPackWords = 308;    // 33, 97 and 161 words at most
 __global__ void __launch_bounds__(256)
 k_pack(const int8_t *__restrict__ codes, uint32_t n, const int32_t *__restrict__ a_blk, const int32_t *__restrict__ c_blk,
@@ -194,13 +228,19 @@ k_pack(const int8_t *__restrict__ codes, uint32_t n, const int32_t *__restrict__
         for (int i = 0; i < 32; ++i)
             if ((uint32_t)i < valid) cw[i >> 2] |= (uint32_t)(uint8_t)codes[e0 + i] << (8 * (i & 3));
     }
-    uint32_t m1 = 0, e2 = 0;
+    uint32_t m1 = 0, e2 = 0, fld[8];                     // levels 1 and 2; the fields of either, four per word
 #pragma unroll
-    for (int i = 0; i < 32; ++i) {
-        const int lv = (uint32_t)i < valid ? code_level((int)(int8_t)(cw[i >> 2] >> (8 * (i & 3)))) : 3;
-        m1 |= (uint32_t)(lv == 0) << i;
-        e2 |= (uint32_t)(lv == 1) << i;
+    for (int k = 0; k < 8; ++k) {
+        uint32_t over3, over15;
+        code_levels4(cw[k], over3, over15);
+        m1 |= (top_bits(over3) ^ 15u) << (4 * k);
+        e2 |= top_bits(over3 & ~over15) << (4 * k);
+        const uint32_t f1 = ((cw[k] & 0x07070707u) + 0x03030303u) & 0x07070707u;       // code + 3
+        const uint32_t f2 = ((cw[k] & 0x1F1F1F1Fu) + 0x0F0F0F0Fu) & 0x1F1F1F1Fu;       // code + 15
+        const uint32_t big = byte_signs(over3);
+        fld[k] = (f1 & ~big) | (f2 & big);
     }
+    m1 &= lowmask(valid);                                // (elements beyond the tensor are no level 1; codes of 0 are no level 2)
     const uint32_t nl = ~m1 & (valid == 32u ? 0xffffffffu : (1u << valid) - 1u);     // not level 1
     const uint32_t a0 = (uint32_t)a_blk[b], c0 = (uint32_t)c_blk[b], r0 = b * kBlk - a0;    // the block's first ranks
     const uint32_t i1 = warp_incl_scan(__popc(m1), lane), i2 = warp_incl_scan(__popc(e2), lane);
@@ -212,21 +252,30 @@ k_pack(const int8_t *__restrict__ codes, uint32_t n, const int32_t *__restrict__
     // levels 1 and 2 and the second bitmap, from the last element to the first
     uint32_t v1[3] = {0, 0, 0}, v2[5] = {0, 0, 0, 0, 0}, vb[1] = {0};
 #pragma unroll
-    for (int i = 31; i >= 0; --i) {
-        const uint32_t c = (cw[i >> 2] >> (8 * (i & 3))) & 0xffu;       // the code modulo 256
-        if ((m1 >> i) & 1u) {
-            v1[2] = __funnelshift_l(v1[1], v1[2], 3);
-            v1[1] = __funnelshift_l(v1[0], v1[1], 3);
-            v1[0] = v1[0] << 3 | ((c + 3u) & 7u);
+    for (int q = 3; q >= 0; --q) {
+        uint32_t g1 = 0, gb = 0;
+#pragma unroll
+        for (int h = 1; h >= 0; --h) {
+            uint32_t g2 = 0;
+#pragma unroll
+            for (int i = 3; i >= 0; --i) {
+                const int at = 8 * q + 4 * h + i;
+                const uint32_t f = __byte_perm(fld[2 * q + h], 0, 0x4440 + i);
+                const bool is1 = m1 & (1u << at), is2 = e2 & (1u << at), isn = nl & (1u << at);
+                if (is1) g1 = g1 * 8u + f;
+                if (is2) g2 = g2 * 32u + f;
+                if (isn) gb = gb * 2u + (is2 ? 1u : 0u);
+            }
+            const uint32_t sh = 5u * __popc(e2 & (15u << (8 * q + 4 * h)));
+#pragma unroll
+            for (int k = 4; k > 0; --k) v2[k] = __funnelshift_l(v2[k - 1], v2[k], sh);
+            v2[0] = v2[0] << sh | g2;
         }
-        if ((nl >> i) & 1u) vb[0] = vb[0] << 1 | ((e2 >> i) & 1u);
-        if ((e2 >> i) & 1u) {
-            v2[4] = __funnelshift_l(v2[3], v2[4], 5);
-            v2[3] = __funnelshift_l(v2[2], v2[3], 5);
-            v2[2] = __funnelshift_l(v2[1], v2[2], 5);
-            v2[1] = __funnelshift_l(v2[0], v2[1], 5);
-            v2[0] = v2[0] << 5 | ((c + 15u) & 31u);
-        }
+        const uint32_t c1q = __popc(m1 & (255u << (8 * q))), cnq = __popc(nl & (255u << (8 * q))), sh = 3u * c1q;
+        v1[2] = __funnelshift_l(v1[1], v1[2], sh);
+        v1[1] = __funnelshift_l(v1[0], v1[1], sh);
+        v1[0] = v1[0] << sh | g1;
+        vb[0] = vb[0] << cnq | gb;
     }
     __syncwarp();                                        // the image is zero
     or_bits(img + kPackL1, 3u * a - (3u * a0 & ~31u), v1);

@@ -58,3 +58,25 @@ def test_gpu_pack_matches_host_packer(out_f, in_f):
         from ixrun_b200.packed import DevicePacked
 
         assert torch.equal(d2.gemv(x), DevicePacked(h2).gemv(x))
+
+
+@pytest.mark.parametrize("n_rows,in_f,shift", [(3, 1024, 0), (5, 1056, 0), (7, 992, 1)])
+def test_quantise_near_halves_and_beyond_the_range(n_rows, in_f, shift):
+    """Quotients next to every half between two codes (from both sides, by one bf16 step and less) and the largest
+    ones, in whole blocks and ragged ones, aligned and not: the codes of the reference's rounding in fp32, and the packed
+    streams decode back to them."""
+    from ixrun_b200.gpu_pack import quantize_pack_gpu
+
+    n = n_rows * in_f
+    half = (torch.arange(n) % 255 - 127).float() + 0.5
+    v = half * torch.tensor([1.0, 1.0 - 2.0 ** -8, 1.0 + 2.0 ** -8, 0.998])[torch.arange(n) // 255 % 4]
+    w = (v * 0.0123).bfloat16()
+    w[3] = 127.9 * 0.0123
+    buf = torch.zeros(n + 8, dtype=torch.bfloat16, device="cuda")
+    buf[shift:shift + n] = w.cuda()
+    wd = buf[shift:shift + n].view(n_rows, in_f)
+    dp, codes = quantize_pack_gpu(wd, return_codes=True)
+    scale = (wd.abs().max().clamp_min(1e-8) / 127.0).bfloat16()
+    assert torch.equal(dp.scale, scale)
+    assert torch.equal(codes, (wd.float() / scale.float()).round().clamp(-127, 127).to(torch.int8))
+    assert torch.equal(dp.decode(kind="codes"), codes)
