@@ -174,6 +174,26 @@ def lib():
     return L
 
 
+_host = None
+
+
+def host():
+    """The extension for the host side of a call (csrc/ixb_host.cpp), built first if it is missing or stale."""
+    global _host
+    if _host is None:
+        if _build.host_is_stale():
+            try:
+                _build.build_host()
+            except Exception as e:
+                raise IxbError(f"_ixbhost.so is missing or older than its source and cannot be built here: {e}") from e
+        from . import _ixbhost
+
+        L = lib()
+        _ixbhost.bind(C.cast(L.ixb_p6_gemv, C.c_void_p).value, C.cast(L.ixb_p6_rows, C.c_void_p).value, check)
+        _host = _ixbhost
+    return _host
+
+
 def check(rc: int):
     if rc != 0:
         raise IxbError(f"ixb200 error {rc}: {lib().ixb_last_error().decode()}")

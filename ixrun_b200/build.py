@@ -1,9 +1,10 @@
-"""Build the CUDA shared library in-tree (``ixrun_b200/libixb200.so``).
+"""Build the CUDA shared library (``ixrun_b200/libixb200.so``) and the Python extension for the host side of a call
+(``ixrun_b200/_ixbhost.so``) in-tree.
 
     python -m ixrun_b200.build [--force] [--verbose]
 
 nvcc cross-compiles for sm_100a without a GPU.  The library has no Python or
-torch dependency; the package binds it with ctypes.
+torch dependency; the package binds it with ctypes.  The extension is built against the torch and Python that run this.
 """
 from __future__ import annotations
 
@@ -89,5 +90,63 @@ def build(force: bool = False, verbose: bool = False) -> str:
             fcntl.flock(lock, fcntl.LOCK_UN)
 
 
+HOST_SO = os.path.join(HERE, "_ixbhost.so")
+HOST_SRC = os.path.join(CSRC, "ixb_host.cpp")
+
+
+def _torch_dir() -> str:
+    import importlib.util
+
+    return list(importlib.util.find_spec("torch").submodule_search_locations)[0]
+
+
+def host_hash() -> str:
+    """Hash of the extension's source, of this file and of the versions it is built against."""
+    import hashlib
+
+    h = hashlib.sha256(sys.version.encode())
+    for f in (HOST_SRC, os.path.abspath(__file__), os.path.join(_torch_dir(), "version.py")):
+        with open(f, "rb") as fh:
+            h.update(fh.read())
+    return h.hexdigest()
+
+
+def host_is_stale() -> bool:
+    if not os.path.exists(HOST_SO) or not os.path.exists(HOST_SO + ".srchash"):
+        return True
+    with open(HOST_SO + ".srchash") as f:
+        return f.read().strip() != host_hash()
+
+
+def build_host(force: bool = False) -> str:
+    """Compile the extension, as `build` does the library: a temporary file, moved into place under a lock."""
+    import fcntl
+    import sysconfig
+
+    with open(HOST_SO + ".lock", "w") as lock:
+        fcntl.flock(lock, fcntl.LOCK_EX)
+        try:
+            if not force and not host_is_stale():
+                return HOST_SO
+            tmp, t = f"{HOST_SO}.tmp{os.getpid()}", _torch_dir()
+            cuda = os.path.dirname(os.path.dirname(os.path.realpath(nvcc_path())))
+            r = subprocess.run(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-I{sysconfig.get_paths()['include']}",
+                                f"-I{t}/include", f"-I{t}/include/torch/csrc/api/include", f"-I{cuda}/include", HOST_SRC,
+                                "-o", tmp, f"-L{t}/lib", "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"],
+                               capture_output=True, text=True)
+            if r.returncode != 0:
+                sys.stderr.write(r.stdout + r.stderr)
+                if os.path.exists(tmp):
+                    os.remove(tmp)
+                raise RuntimeError("g++ failed building _ixbhost.so")
+            os.replace(tmp, HOST_SO)
+            with open(HOST_SO + ".srchash", "w") as f:
+                f.write(host_hash())
+            return HOST_SO
+        finally:
+            fcntl.flock(lock, fcntl.LOCK_UN)
+
+
 if __name__ == "__main__":
     print(build(force="--force" in sys.argv, verbose="--verbose" in sys.argv))
+    print(build_host(force="--force" in sys.argv))

@@ -67,17 +67,19 @@ class StreamingLinear(nn.Module):
         if resident == "streams" and not keep_streams:
             raise ValueError("resident='streams' needs the streams")
         dp = packed if isinstance(packed, DevicePacked) else DevicePacked(packed)
-        self.out_features = dp.out_f
-        self.in_features = dp.in_f
-        self.N = dp.N
-        self.level_bits = (3, 5, 8)
-        self.counts = dp.counts
-        self.total_bytes = dp.total_bytes
-        self._dp = dp
-        self._use_triton = True
-        # the fused kernel on the streams handles any in_f that is a multiple of 32
-        self._use_fused = keep_streams and self.in_features % 32 == 0
-        self._split_chunk = 0
+        # (none of these is a parameter, module or buffer: past nn.Module.__setattr__, which takes 1.3 us each)
+        self.__dict__.update(
+            out_features=dp.out_f, in_features=dp.in_f, N=dp.N, level_bits=(3, 5, 8), counts=dp.counts, total_bytes=dp.total_bytes,
+            _dp=dp, _use_triton=True,
+            # the fused kernel on the streams handles any in_f that is a multiple of 32
+            _use_fused=keep_streams and dp.in_f % 32 == 0, _split_chunk=0,
+            _y32=None,
+            # 9..64 rows on the resident layout: one pass over the packed bytes on the tensor cores
+            # (ixb_p6_gemm, in_f % 64 == 0; without a bias also in_f % 8 == 0); set _use_p6_gemm = False to take decode + dense
+            # matmul instead.
+            # _use_tc: the older tensor-core kernel that reads the streams (needs them kept, in_f % 1024 == 0); off.
+            _use_p6_gemm=True, _use_tc=False, _w_buf=None,
+            _res=None)                           # the resident re-layout
         if keep_streams:
             for key, val in (("_b1", dp.b1), ("_b2", dp.b2), ("_l1", dp.l1), ("_l2", dp.l2), ("_l3", dp.l3),
                              ("_b1_blk", dp.blk_q1), ("_b2_blk", dp.blk_q2)):
@@ -92,27 +94,17 @@ class StreamingLinear(nn.Module):
                 self.register_buffer("_q1", q1, persistent=False)
                 self.register_buffer("_q2", q2, persistent=False)
         self.register_buffer("_scale", dp.scale, persistent=False)
-        self._y32 = None
-        # 9..64 rows on the resident layout: one pass over the packed bytes on the tensor cores
-        # (ixb_p6_gemm, in_f % 64 == 0; without a bias also in_f % 8 == 0); set _use_p6_gemm = False to take decode + dense
-        # matmul instead.
-        # _use_tc: the older tensor-core kernel that reads the streams (needs them kept, in_f % 1024 == 0); off.
-        self._use_p6_gemm = True
-        self._use_tc = False
         if bias is not None:
             self.register_buffer("_bias", bias.detach().clone().to(dp.device), persistent=False)
             self._bias_bf16 = self._bias.to(torch.bfloat16)
         else:
-            self._bias = None
-            self._bias_bf16 = None
-        self._w_buf = None
-        self._res = None                         # the resident re-layout
+            self.__dict__.update(_bias=None, _bias_bf16=None)
         if resident == "p6":
             from .p6 import P6Packed
 
-            self._res = P6Packed.from_packed(dp)
+            self.__dict__["_res"] = P6Packed.from_packed(dp)
             if not keep_streams:
-                self._dp = None                  # the streams (and their rank tables) are released with it
+                self.__dict__["_dp"] = None                  # the streams (and their rank tables) are released with it
 
     @classmethod
     def from_weight(cls, weight: torch.Tensor, bias=None, **kw):
@@ -146,8 +138,12 @@ class StreamingLinear(nn.Module):
         return src.decode(out=self._w_buf[: self.N], kind="bf16")
 
     def forward(self, x):
-        rows = x.numel() // self.in_features
         res = self._res
+        if res is not None:
+            y = (res._call or res.make_call())(x, self._bias_bf16, self._use_p6_gemm)
+            if y is not None:
+                return y
+        rows = x.numel() // self.in_features
         if res is not None and x.dtype == torch.bfloat16 and x.shape[-1] == self.in_features and rows <= TC_MAX_ROWS:
             y = None
             if 1 <= rows <= FUSED_MAX_ROWS:

@@ -19,30 +19,25 @@ __all__ = ["quantize_pack_gpu", "pack_codes_gpu", "int8x_quantize_gpu"]
 
 
 def _pack(codes: torch.Tensor, scale: torch.Tensor, b1, q1, q2, counts, out_f: int, in_f: int) -> DevicePacked:
-    dev = codes.device
+    index = codes.get_device()
     n1, n2, n3 = counts
-    b2 = torch.empty((n2 + n3 + 31) // 32, dtype=torch.int32, device=dev)
-    l1 = torch.empty((3 * n1 + 31) // 32, dtype=torch.int32, device=dev)
-    l2 = torch.empty((5 * n2 + 31) // 32, dtype=torch.int32, device=dev)
-    l3 = torch.empty(n3, dtype=torch.uint8, device=dev)
+    # (the kernel that follows waits for nothing but the host: as little as possible happens here)
+    b2, l1, l2, l3 = _lib.host().empty(index, ((n2 + n3 + 31) // 32, "i"), ((3 * n1 + 31) // 32, "i"),
+                                       ((5 * n2 + 31) // 32, "i"), (n3, "B"))
     st = _lib.packed_struct(b1, b2, l1, l2, l3, scale, out_f, in_f)
-    with torch.cuda.device(dev):
-        _lib.check(_lib.lib().ixb_pack_codes(codes.data_ptr(), C.byref(st), q1.data_ptr(), q2.data_ptr(),
-                                             _lib.stream_ptr(dev)))
-    dp = DevicePacked.from_device_streams(b1, b2, l1, l2, l3, scale, out_f, in_f, blk_q1=q1, blk_q2=q2)
+    with _lib.on_device(index) as stream:
+        _lib.check(_lib.lib().ixb_pack_codes(codes.data_ptr(), C.byref(st), q1.data_ptr(), q2.data_ptr(), stream))
+    dp = DevicePacked.from_device_streams(b1, b2, l1, l2, l3, scale, out_f, in_f, blk_q1=q1, blk_q2=q2, struct=st)
     dp.counts = [n1, n2, n3]
     dp.total_bytes = 2 + 4 * (b1.numel() + b2.numel() + l1.numel() + l2.numel()) + n3
     return dp
 
 
-def _tables(n: int, dev):
+def _tables(n: int, index: int, *more):
+    """Library, workspace, B1, the two rank tables, and what else is asked for as (n, type)"""
     nb = (n + 1023) // 1024
     L = _lib.lib()
-    ws = torch.empty(L.ixb_pack_workspace_bytes(n), dtype=torch.uint8, device=dev)
-    b1 = torch.empty((n + 31) // 32, dtype=torch.int32, device=dev)
-    q1 = torch.empty(nb, dtype=torch.int32, device=dev)
-    q2 = torch.empty(nb, dtype=torch.int32, device=dev)
-    return L, ws, b1, q1, q2
+    return L, *_lib.host().empty(index, (L.ixb_pack_workspace_bytes(n), "B"), ((n + 31) // 32, "i"), (nb, "i"), (nb, "i"), *more)
 
 
 @torch.no_grad()
@@ -52,15 +47,12 @@ def quantize_pack_gpu(weight: torch.Tensor, return_codes: bool = False):
         raise ValueError("quantize_pack_gpu needs a 2-D bf16 CUDA tensor")
     w = weight.contiguous()
     out_f, in_f = w.shape
-    n, dev = w.numel(), w.device
-    L, ws, b1, q1, q2 = _tables(n, dev)
-    codes = torch.empty(n, dtype=torch.int8, device=dev)
-    scale = torch.empty((), dtype=torch.bfloat16, device=dev)
+    n, index = w.numel(), w.get_device()
+    L, ws, b1, q1, q2, codes, scale = _tables(n, index, (n, "b"), (-1, "h"))
     counts = (C.c_int64 * 3)()
-    with torch.cuda.device(dev):
+    with _lib.on_device(index) as stream:
         _lib.check(L.ixb_quantize_codes(w.data_ptr(), n, scale.data_ptr(), codes.data_ptr(), b1.data_ptr(),
-                                        q1.data_ptr(), q2.data_ptr(), counts, ws.data_ptr(), ws.numel(),
-                                        _lib.stream_ptr(dev)))
+                                        q1.data_ptr(), q2.data_ptr(), counts, ws.data_ptr(), ws.numel(), stream))
     dp = _pack(codes, scale, b1, q1, q2, [int(c) for c in counts], out_f, in_f)
     return (dp, codes.view(out_f, in_f)) if return_codes else dp
 
@@ -72,7 +64,7 @@ def pack_codes_gpu(codes: torch.Tensor, scale: torch.Tensor, out_f: int, in_f: i
         raise ValueError("pack_codes_gpu needs out_f*in_f int8 codes on a CUDA device")
     c = codes.contiguous().reshape(-1)
     dev = c.device
-    L, ws, b1, q1, q2 = _tables(c.numel(), dev)
+    L, ws, b1, q1, q2 = _tables(c.numel(), c.get_device())
     counts = (C.c_int64 * 3)()
     with torch.cuda.device(dev):
         _lib.check(L.ixb_count_codes(c.data_ptr(), c.numel(), b1.data_ptr(), q1.data_ptr(), q2.data_ptr(), counts,

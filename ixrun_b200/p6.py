@@ -74,28 +74,27 @@ class P6Packed:
         L = _lib.lib()
         nb = int(L.ixb_p6_blocks(self.out_f, self.in_f))
         # sizes include the slack that the GEMV's prefetch may read
-        self.plane = torch.empty((nb + SLACK_BLOCKS) * BLOCK_BYTES // 4, dtype=torch.int32, device=dev)
-        self.blk_off = torch.empty(nb + 1, dtype=torch.int32, device=dev)
+        index, host = c.get_device(), _lib.host()
+        self.plane, self.blk_off, ws = host.empty(index, ((nb + SLACK_BLOCKS) * BLOCK_BYTES // 4, "i"), (nb + 1, "i"), ((nb + 1) * 4, "B"))
         self.scale = scale.detach().to(dev, torch.bfloat16).reshape(-1).contiguous()
         if self.scale.numel() not in (1, (self.out_f + 15) // 16):
             raise ValueError("scale must hold one value, or one per 16-row tile")
         stride = 0 if self.scale.numel() == 1 else 1
         self.sections = [(0, self.out_f)]            # (first row, rows) of every fused part
-        ws = torch.empty((nb + 1) * 4, dtype=torch.uint8, device=dev)
         count = C.c_int64()
-        with torch.cuda.device(dev):
-            st = _lib.stream_ptr(dev)
+        with _lib.on_device(index) as st:
             _lib.check(L.ixb_p6_plane(c.data_ptr(), self.out_f, self.in_f, self.plane.data_ptr(), self.blk_off.data_ptr(),
                                       C.byref(count), ws.data_ptr(), ws.numel(), st))
             self.n_esc = n_esc = int(count.value)
-            self.esc = torch.empty(n_esc + SLACK_ENTRIES, dtype=torch.int32, device=dev)
+            self.esc, = host.empty(index, (n_esc + SLACK_ENTRIES, "i"))
             _lib.check(L.ixb_p6_entries(c.data_ptr(), self.scale.data_ptr(), stride, self.out_f, self.in_f,
                                         self.blk_off.data_ptr(), self.esc.data_ptr(), n_esc, st))
         self.struct = _lib.P6Struct(self.plane.data_ptr(), self.blk_off.data_ptr(), self.esc.data_ptr(), n_esc,
                                     self.scale.data_ptr(), self.out_f, self.in_f, stride)
         self._ref = C.byref(self.struct)             # (keeps the struct alive)
-        self._index = dev.index
+        self._index = index
         self._gemv_need = None                           # scratch bytes
+        self._call = None                                # the extension's object for this tensor
         self.resident_bytes = nb * BLOCK_BYTES + 4 * (nb + 1 + n_esc) + 2
         self.scratch = scratch if scratch is not None else GemvScratch.shared(dev)
 
@@ -132,6 +131,13 @@ class P6Packed:
                    total_bytes=sum(d.total_bytes for d in dps), **kw)
         self.sections = sections
         return self
+
+    def make_call(self):
+        """The extension's call (x, bias, many) -> y, or None for what it leaves to `gemv`, `gemm` and the dense matmul."""
+        L = _lib.lib()
+        s = self.scratch.reserve(int(L.ixb_p6_gemv_scratch_bytes(self.out_f, self.in_f, 1)))
+        self._call = _lib.host().p6(C.addressof(self.struct), self.out_f, self.in_f, self._index, s)
+        return self._call
 
     def split(self, y: torch.Tensor):
         """Views of a one-row output [1, out_f] (or [out_f]) per fused part."""

@@ -51,23 +51,23 @@ class DevicePacked:
         self._init_tables()
 
     @classmethod
-    def from_device_streams(cls, b1, b2, l1, l2, l3, scale, out_f: int, in_f: int, blk_q1=None, blk_q2=None):
+    def from_device_streams(cls, b1, b2, l1, l2, l3, scale, out_f: int, in_f: int, blk_q1=None, blk_q2=None, struct=None):
         """Wrap streams that already live on the device (no copies); the gran=1024 rank tables are
-        computed unless given."""
+        computed unless given.  struct: the streams' C structure, if the caller has it."""
         self = cls.__new__(cls)
         self.device = b1.device
         self.out_f, self.in_f, self.N = int(out_f), int(in_f), int(out_f) * int(in_f)
         self.counts = None
         self.total_bytes = 0
         self.b1, self.b2, self.l1, self.l2, self.l3 = b1, b2, l1, l2, l3
-        self.scale = scale.reshape(()).to(torch.bfloat16)
-        self._init_tables(blk_q1, blk_q2)
+        self.scale = scale if scale.dim() == 0 and scale.dtype == torch.bfloat16 else scale.reshape(()).to(torch.bfloat16)
+        self._init_tables(blk_q1, blk_q2, struct if self.scale is scale else None)
         return self
 
     # ------------------------------------------------------------ plumbing --
-    def _init_tables(self, blk_q1=None, blk_q2=None):
-        self.struct = _lib.packed_struct(self.b1, self.b2, self.l1, self.l2, self.l3, self.scale,
-                                         self.out_f, self.in_f)
+    def _init_tables(self, blk_q1=None, blk_q2=None, struct=None):
+        self.struct = struct if struct is not None else _lib.packed_struct(self.b1, self.b2, self.l1, self.l2, self.l3, self.scale,
+                                                                           self.out_f, self.in_f)
         self.n_blocks = (self.N + BLOCK - 1) // BLOCK
         if blk_q1 is None or blk_q2 is None:
             blk_q1, blk_q2 = self.prefix_tables(BLOCK, self.n_blocks)
@@ -98,10 +98,9 @@ class DevicePacked:
         flat = out.reshape(-1)
         if flat.dtype != dtype or flat.numel() < self.N or not flat.is_contiguous():
             raise ValueError("decode output must be a contiguous tensor of the right dtype and size")
-        with torch.cuda.device(self.device):
+        with _lib.on_device(self.b1.get_device()) as stream:
             _lib.check(_lib.lib().ixb_decode(C.byref(self.struct), self.blk_q1.data_ptr(), self.blk_q2.data_ptr(),
-                                             flat.data_ptr(), 0 if kind == "codes" else 1,
-                                             _lib.stream_ptr(self.device)))
+                                             flat.data_ptr(), 0 if kind == "codes" else 1, stream))
         return flat[: self.N].view(self.out_f, self.in_f)
 
     def scratch(self, m_rows: int) -> torch.Tensor:

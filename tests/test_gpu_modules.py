@@ -350,3 +350,41 @@ def test_streaming_linear_leaves_autocast_and_modes_to_the_dense_matmul():
             lin(x)
         assert "linear" in seen
         assert (lin(torch._neg_view(x)).float() + y.float()).abs().max() <= 2.0 ** -7 * y.float().abs().max()
+
+
+@pytest.mark.parametrize("in_f,bias", [(128, False), (128, True), (200, False)])
+def test_call_through_the_extension_is_the_python_path(in_f, bias):
+    """The extension's call takes ordinary activations and leaves the rest: every form gives what the Python path gives."""
+    from ixrun_b200.engine import StreamingLinear
+
+    class Sub(torch.Tensor):
+        pass
+
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    w = (torch.randn(96, in_f, generator=gen, device="cuda") * 0.02).bfloat16()
+    b = torch.randn(96, generator=gen, device="cuda").bfloat16() if bias else None
+    lin = StreamingLinear.from_weight(w, bias=b)
+    lin._set_shared_buf(torch.empty(96 * in_f, dtype=torch.bfloat16, device="cuda"))
+    big = torch.randn(4, 64, 2 * in_f + 8, generator=gen, device="cuda").bfloat16()
+    forms = [big[0, 0, :in_f].clone(), big[:1, 0, :in_f], big[0, :8, :in_f].contiguous(), big[0, :9, :in_f].contiguous(),
+             big[0, :64, :in_f].contiguous(), big[0, :64, :in_f], big[:, :2, :in_f].contiguous(), big[:, :3, :in_f].contiguous(),
+             big[:2, :, :in_f].contiguous(), big[0, ::2, 8:8 + in_f],
+             big[0, :2, :in_f].contiguous().requires_grad_(), big[0, :2, :in_f].contiguous().as_subclass(Sub),
+             big[0, :in_f, :3].t().contiguous() if in_f <= 64 else big[0, :3, :in_f].t().contiguous().t()]
+    stream = torch.cuda.Stream()
+    for many in (True, False):
+        lin._use_p6_gemm = many
+        for x in forms:
+            lin._res._call = None
+            torch.cuda.synchronize()
+            with torch.cuda.stream(stream):
+                y = lin(x)
+            lin._res._call = lambda *a: None
+            ref = lin(x)
+            torch.cuda.synchronize()
+            assert type(y) is type(ref) and y.shape == ref.shape and y.dtype == ref.dtype and torch.equal(y, ref)
+    lin._res._call = None
+    for bad in (torch.randn(2, in_f).bfloat16(), torch.randn(2, in_f + 8, device="cuda").bfloat16()):
+        with pytest.raises(Exception):
+            lin(bad)
+    assert lin(torch.randn(2, in_f, device="cuda")).dtype == torch.float32          # another type: the dense matmul
