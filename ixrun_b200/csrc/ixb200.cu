@@ -1311,11 +1311,12 @@ extern "C" int ixb_allreduce_finish(void *const *peer_buffers, int rank, int wor
 // ------------------------------------------------------- per-token glue kernels
 // one launch with the programmatic-stream-serialization attribute when ixb_set_pdl is on
 template <class... KArgs, class... Args>
-static cudaError_t launch_glue(void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStream_t st, Args... args)
+static cudaError_t launch_glue_smem(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -1323,6 +1324,11 @@ static cudaError_t launch_glue(void (*kernel)(KArgs...), dim3 grid, dim3 block, 
     cfg.attrs = attr;
     cfg.numAttrs = g_p6_pdl.load() ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+template <class... KArgs, class... Args>
+static cudaError_t launch_glue(void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStream_t st, Args... args)
+{
+    return launch_glue_smem(kernel, grid, block, 0, st, args...);
 }
 
 static bool norm_vector_ok(const void *h, const void *delta, const void *w, const void *xn, int64_t hidden, int64_t limit)
@@ -1443,11 +1449,28 @@ static cudaError_t launch_attn(int64_t hq, int64_t hkv, int64_t splits, cudaStre
     auto ctas = [&](int64_t groups) {
         return (unsigned)std::max<int64_t>(1, std::min<int64_t>(splits, (2 * num_sms() + groups * batch - 1) / (groups * batch)));
     };
-#define IXB_ATTN(G)                                                                                                        \
-    return launch_glue(k_attn_decode<D, G>, dim3((unsigned)(hq / G), ctas(hq / G), (unsigned)batch), dim3(256), st,       \
-                       (const __nv_bfloat16 *)q, (const __nv_bfloat16 *)k_cache, (const __nv_bfloat16 *)v_cache, pos,      \
-                       (float *)scratch, (uint32_t)hq, (uint32_t)hkv, scale, (uint32_t)q_stride, (size_t)batch_stride,     \
-                       (uint32_t)splits, (uint32_t)max_seq, join)
+    // One CTA for all parts of a group and sequence from where there are 240 of them: 16 / 8 heads of 128, sequences of 150 to
+    // 300 and of 500 to 1000 positions, many CTAs against one, us: 192 of them (24 sequences) 19.0 / 15.8 and 37.6 / 43.9, 240
+    // 22.6 / 17.2 and 47.6 / 47.9, 320 26.8 / 18.9 and 65 / 52, 1024 69 / 40 and 163 / 115; of 3000 positions 115 / 115 for 240
+    // and 161 / 123 for 320.  Not eight heads to a group: too many registers for two CTAs of 64 (240 of 3000 positions:
+    // 173 / 185).
+    auto local = [&](int64_t groups, int64_t g) { return join.tickets && g < 8 && groups * batch >= 240; };
+#define IXB_ATTN(G)                                                                                                            \
+    do {                                                                                                                       \
+        const bool one = local(hq / G, G);                                                                                     \
+        constexpr bool LOCAL = G < 8;                                                                                          \
+        const size_t ring = one && D <= 128 ? 2u * (D / 32 + (size_t)kAttnChunk * D / 2048) * 4096u : 0u;                      \
+        if (ring) {                                                                                                            \
+            static bool attr_set[64] = {false};                                                                                \
+            const cudaError_t oe = opt_in_smem(k_attn_decode<D, G, LOCAL>, attr_set, (int)ring);                               \
+            if (oe != cudaSuccess) return oe;                                                                                  \
+        }                                                                                                                      \
+        return launch_glue_smem(one ? k_attn_decode<D, G, LOCAL> : k_attn_decode<D, G, false>,                                 \
+                                dim3((unsigned)(hq / G), one ? 1u : ctas(hq / G), (unsigned)batch), dim3(256), ring, st,       \
+                                (const __nv_bfloat16 *)q, (const __nv_bfloat16 *)k_cache, (const __nv_bfloat16 *)v_cache, pos, \
+                                (float *)scratch, (uint32_t)hq, (uint32_t)hkv, scale, (uint32_t)q_stride, (size_t)batch_stride,\
+                                (uint32_t)splits, (uint32_t)max_seq, join);                                                    \
+    } while (0)
     switch (rep) {                      // all query heads of a KV head in one CTA where that is a supported group size
     case 2: IXB_ATTN(2);
     case 3: IXB_ATTN(3);

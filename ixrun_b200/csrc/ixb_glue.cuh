@@ -346,6 +346,16 @@ __device__ __forceinline__ uint32_t attn_parts(uint32_t n_ctx, uint32_t splits)
 {
     return min(splits, (n_ctx + kAttnChunk - 1u) / kAttnChunk);
 }
+// LOCAL: one CTA per group and sequence takes all of its parts.  Their sums stay in shared memory (as many as six kilobytes
+// hold; the rest go through the scratch) and nothing is published: the same sums in the same order as by many CTAs, so the same
+// bits.  Bound by the chain of a chunk, not by its bytes (a fifth to a half of the copy rate), so three CTAs of an SM run it
+// side by side.  Heads of 64 and 128 have two chunks in flight through shared memory, a thread's own pieces (nobody else reads
+// them, so no barrier waits for them); the warps' sums take the place of the chunk that was taken last, without which only two
+// CTAs fit.  Forty sequences of 150 to 300 positions, 16 / 8 heads of 128: 26.8 us by many CTAs, 17.9 with the next chunk in
+// registers, 18.9 with two in shared memory; of 500 to 1000 positions 65, 49 and 52, and thirty of them 48, 49 and 48.  (One
+// running softmax over all chunks instead of parts: 14.7 and 38, but other bits than the sequence's own.)
+__host__ __device__ constexpr int attn_keep(int d, int g) { return 1536 / (g * d) > 0 ? 1536 / (g * d) : 1; }
+__host__ __device__ constexpr int attn_local_ctas(int d, int g) { return g * d <= 256 ? 3 : g * d <= 512 ? 2 : 1; }       // per SM: registers
 struct AttnJoin {
     uint32_t *tickets;
     __nv_bfloat16 *out;
@@ -353,8 +363,8 @@ struct AttnJoin {
     uint32_t gate_stride, gate_row_stride;
 };
 
-template <int D, int G>
-__global__ void __launch_bounds__(256)
+template <int D, int G, bool LOCAL>
+__global__ void __launch_bounds__(256, LOCAL ? attn_local_ctas(D, G) : 1)
 k_attn_decode(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat16 *__restrict__ k_cache,
               const __nv_bfloat16 *__restrict__ v_cache, const int32_t *pos, float *part, uint32_t hq, uint32_t hkv,
               float scale, uint32_t q_stride, size_t batch_stride, uint32_t splits, uint32_t max_seq, AttnJoin join)
@@ -380,9 +390,18 @@ k_attn_decode(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat16 *__restri
     static_assert(PG * G * D <= NR * HG * D && NW <= NR, "sums of the join fit");
     __shared__ __align__(16) float sm_q[G][D];         // scaled queries
     __shared__ float sm_s[G][C], sm_c[G];              // a chunk's scores, then weights; the sums' rescaling
-    __shared__ __align__(16) float sm_acc[NR][HG][D];
+    constexpr bool RING = LOCAL && D <= 128;
+    __shared__ __align__(16) float sm_acc_own[RING ? 1 : NR * HG * D];
     __shared__ float sm_w[G][kAttnMaxSplits], sm_sum[G];
     __shared__ uint32_t sm_last;
+    constexpr int KEEP = LOCAL ? attn_keep(D, G) : 1;
+    __shared__ __align__(16) float sm_part[LOCAL ? KEEP : 1][LOCAL ? G * D : 4];
+    __shared__ float2 sm_ml[LOCAL ? G : 1][KEEP];
+    extern __shared__ __align__(16) uint4 sm_ring[];   // [2][KC + VP][256 threads]
+    // the warps' sums: [NR][HG][D], with a ring in the half of the chunk that was taken last
+    static_assert(!RING || NR * HG * D * 4 <= (KC + VP) * 4096, "fits");
+    float *sm_acc = sm_acc_own;
+    auto acc_at = [&](int w, int h, int d) -> float & { return sm_acc[(w * HG + h) * D + d]; };
     asm volatile("griddepcontrol.launch_dependents;");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const uint32_t head0 = blockIdx.x * G;
@@ -394,6 +413,24 @@ k_attn_decode(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat16 *__restri
     const __nv_bfloat16 *kb = k_cache + (size_t)kvh * D + kt * 8, *vb = v_cache + (size_t)kvh * D + vd;
     const uint32_t last = (uint32_t)pos[0];
     uint4 kr[KC], vr[VP];
+    const uint32_t ring = RING ? (uint32_t)__cvta_generic_to_shared(sm_ring) + tid * 16u : 0u;
+    uint32_t visit = 0;                                // chunks taken so far; even ones lie in the first half of the ring
+    auto piece = [&](uint32_t i, int j) { return ring + ((i & 1u) * (KC + VP) + j) * 4096u; };
+    auto request = [&](uint32_t c, uint32_t i, uint32_t limit) {       // chunk c as the i-th to be taken
+        const __nv_bfloat16 *src = kb + min(c * kAttnChunk + kp, limit) * row_stride;
+#pragma unroll
+        for (int j = 0; j < KC; ++j)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(piece(i, j)), "l"(src + j * 32) : "memory");
+#pragma unroll
+        for (int j = 0; j < VP; ++j)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(piece(i, KC + j)), "l"(vb + min(c * kAttnChunk + vg + j * VG, limit) * row_stride) : "memory");
+        cp_async_commit();
+    };
+    auto taken = [&](uint32_t addr) {
+        uint4 v;
+        asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+        return v;
+    };
     auto fetch_k = [&](uint32_t c, uint32_t limit) {
         const __nv_bfloat16 *src = kb + min(c * kAttnChunk + kp, limit) * row_stride;
 #pragma unroll
@@ -403,7 +440,17 @@ k_attn_decode(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat16 *__restri
 #pragma unroll
         for (int j = 0; j < VP; ++j) vr[j] = *(const uint4 *)(vb + min(c * kAttnChunk + vg + j * VG, limit) * row_stride);
     };
-    if (max_seq) {
+    auto write_out = [&](int h, int d, float v) {      // head h of the group, dimension d
+        float o = bfround(v);
+        if (join.gate) {
+            const float gv = bf2f(join.gate[(size_t)blockIdx.z * join.gate_row_stride + (size_t)(head0 + h) * join.gate_stride + d]);
+            o = o * bfround(sigmoid_f(gv));
+        }
+        join.out[((size_t)blockIdx.z * hq + head0 + h) * D + d] = __float2bfloat16_rn(o);
+    };
+    if (RING) {
+        request(0u, 0u, max_seq - 1u);                 // (LOCAL has max_seq)
+    } else if (max_seq) {
         fetch_k(blockIdx.y, max_seq - 1u);
         fetch_v(blockIdx.y, max_seq - 1u);
     }
@@ -413,7 +460,17 @@ k_attn_decode(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat16 *__restri
         for (int i = tid; i < G * D; i += 256)
             join.out[((size_t)blockIdx.z * hq + head0 + i / D) * D + i % D] = __float2bfloat16_rn(__int_as_float(0x7FFFFFFF));
     }
-    if (blockIdx.y >= used) return;
+    if (blockIdx.y >= used) {
+        if (RING) cp_async_wait<0>();
+        return;
+    }
+    uint32_t ps = 0, pc = 0;                           // part and chunk requested last
+    auto request_next = [&](uint32_t i) {
+        pc = (pc + splits) * kAttnChunk < n_ctx ? pc + splits : ++ps;
+        if (ps < used) request(pc, i, n_ctx - 1u);
+        else cp_async_commit();
+    };
+    if (RING) request_next(1u);
     __syncthreads();
     if (!max_seq) {
         fetch_k(blockIdx.y, n_ctx - 1u);
@@ -433,6 +490,11 @@ k_attn_decode(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat16 *__restri
             float sc[G];
 #pragma unroll
             for (int h = 0; h < G; ++h) sc[h] = 0.f;
+            if (RING) {
+                cp_async_wait<1>();                    // the chunk is there, the next one may be on its way
+#pragma unroll
+                for (int j = 0; j < KC; ++j) kr[j] = taken(piece(visit, j));
+            }
 #pragma unroll
             for (int j = 0; j < KC; ++j) {
                 float kf[8];
@@ -444,7 +506,7 @@ k_attn_decode(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat16 *__restri
                     sc[h] = fmaf(kf[7], q1.w, fmaf(kf[6], q1.z, fmaf(kf[5], q1.y, fmaf(kf[4], q1.x, sc[h]))));
                 }
             }
-            if (ahead) fetch_k(nxt, n_ctx - 1u);
+            if (!RING && ahead) fetch_k(nxt, n_ctx - 1u);
             const bool live = c * kAttnChunk + kp < n_ctx;
 #pragma unroll
             for (int h = 0; h < G; ++h) {
@@ -477,6 +539,7 @@ k_attn_decode(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat16 *__restri
 #pragma unroll
             for (int j = 0; j < VP; ++j) {
                 float vf[8];
+                if (RING) vr[j] = taken(piece(visit, KC + j));
                 unpack8(vr[j], vf);
                 if (c * kAttnChunk + vg + j * VG >= n_ctx) continue;       // (not read, or rows beyond the position)
 #pragma unroll
@@ -486,14 +549,22 @@ k_attn_decode(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat16 *__restri
                     for (int k = 0; k < 8; ++k) acc[h][k] = fmaf(p, vf[k], acc[h][k]);
                 }
             }
-            if (ahead) fetch_v(nxt, n_ctx - 1u);
+            if (!RING && ahead) fetch_v(nxt, n_ctx - 1u);
+            if (RING && more) {
+                request_next(visit + 2u);              // into the pieces that this thread has just taken
+                ++visit;
+            }
             if (more) __syncthreads();                 // the weights are read: the next chunk's scores may follow
         }
         // join: the warp's groups of threads by shuffles, the warps in shared memory, HG heads at a time
+        if (RING) {
+            sm_acc = (float *)(sm_ring + (visit & 1u) * (KC + VP) * 256u);
+            __syncthreads();                           // nobody takes pieces of it any more
+        }
         float *dst = part + ((size_t)head0 * splits + s) * D;
 #pragma unroll
         for (int h0 = 0; h0 < G; h0 += HG) {
-            if (h0 || s != blockIdx.y) __syncthreads();            // sm_acc is free
+            if (h0 || (!RING && s != blockIdx.y)) __syncthreads();  // sm_acc is free
 #pragma unroll
             for (int hh = 0; hh < HG; ++hh) {
                 if (h0 + hh >= G) break;
@@ -503,29 +574,38 @@ k_attn_decode(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat16 *__restri
 #pragma unroll
                     for (int k = 0; k < 8; ++k) v[k] += __shfl_xor_sync(0xffffffffu, v[k], d);
                 if (lane < VT) {
-                    *(float4 *)&sm_acc[wid][hh][vd] = make_float4(v[0], v[1], v[2], v[3]);
-                    *(float4 *)&sm_acc[wid][hh][vd + 4] = make_float4(v[4], v[5], v[6], v[7]);
+                    *(float4 *)&acc_at(wid, hh, vd) = make_float4(v[0], v[1], v[2], v[3]);
+                    *(float4 *)&acc_at(wid, hh, vd + 4) = make_float4(v[4], v[5], v[6], v[7]);
                 }
             }
             __syncthreads();
             for (int i = tid; i < HG * D && h0 + i / D < G; i += 256) {
                 float a = 0.f;
 #pragma unroll
-                for (int w = 0; w < NW; ++w) a += sm_acc[w][i / D][i % D];
-                dst[(size_t)(h0 + i / D) * splits * D + i % D] = a;
+                for (int w = 0; w < NW; ++w) a += acc_at(w, i / D, i % D);
+                if (LOCAL && s < (uint32_t)KEEP) sm_part[s][h0 * D + i] = a;
+                else dst[(size_t)(h0 + i / D) * splits * D + i % D] = a;
             }
         }
-        if (wid < G && lane == 0) part_ml[(size_t)(head0 + wid) * splits + s] = make_float2(M, L);
+        if (RING && s + 1u < used) {
+            __syncthreads();                           // the sums are read
+            request_next(visit + 2u);
+            ++visit;
+        }
+        if (wid < G && lane == 0) {
+            if (LOCAL && s < (uint32_t)KEEP) sm_ml[wid][s] = make_float2(M, L);
+            else part_ml[(size_t)(head0 + wid) * splits + s] = make_float2(M, L);
+        }
     }
-    if (!join.tickets) return;
+    if (!LOCAL && !join.tickets) return;
     // ---- the last CTA of the group joins the parts.  The CTAs with work add numbers whose sum is zero to the ticket, the first
     // one 1 - ctas and the others 1: it is zero again exactly when all of them have come.  So nobody resets it, and it is zero
     // after launches that overlapped too (whose own results are lost).
     const uint32_t ctas = min(gridDim.y, used);
     uint32_t *ticket = join.tickets + (size_t)blockIdx.z * gridDim.x + blockIdx.x;
-    __threadfence();                                   // this thread's share of the parts, before the ticket
+    if (!LOCAL) __threadfence();                       // this thread's share of the parts, before the ticket
     __syncthreads();
-    if (ctas > 1u) {
+    if (!LOCAL && ctas > 1u) {
         const uint32_t mine = blockIdx.y ? 1u : 1u - ctas;
         if (threadIdx.x == 0) sm_last = atomicAdd(ticket, mine) + mine == 0u;
         __syncthreads();
@@ -535,23 +615,27 @@ k_attn_decode(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat16 *__restri
     // all of the group's sums are requested at once, as far as registers go: a thread takes four dimensions of a head and
     // every PG-th part (rounds of eight dependent loads of one value: 29 us a launch at a 4097-token context, not 16.5)
     constexpr int MAXQ = (QD + 255) / 256;             // quads per thread
-    constexpr int UN = 16;
+    constexpr int UN = LOCAL ? 1 : 16;
     const int pg = QD >= 256 ? 0 : tid / QD, q0 = QD >= 256 ? tid : tid % QD;
     float4 first[UN];
-    auto sums = [&](int qd, uint32_t s) { return (const float4 *)(part + ((size_t)(head0 + qd * 4 / D) * splits + s) * D + qd * 4 % D); };
+    auto sums = [&](int qd, uint32_t s) -> float4 {
+        if (LOCAL && s < (uint32_t)KEEP) return *(const float4 *)&sm_part[s][qd * 4];
+        return __ldcg((const float4 *)(part + ((size_t)(head0 + qd * 4 / D) * splits + s) * D + qd * 4 % D));
+    };
 #pragma unroll
     for (int k = 0; k < UN; ++k) {
         const uint32_t s = pg + k * PG;
-        first[k] = q0 < QD && pg < PG && s < used ? __ldcg(sums(q0, s)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        first[k] = q0 < QD && pg < PG && s < used ? sums(q0, s) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
     if (wid < G) {                                     // a warp per head: the parts' weights and their sum
         const float2 *p = part_ml + (size_t)(head0 + wid) * splits;
+        auto max_sum = [&](uint32_t s) { return LOCAL && s < (uint32_t)KEEP ? sm_ml[wid][s] : __ldcg(p + s); };
         float mx = -INFINITY, sum = 0.f;
-        for (uint32_t s = lane; s < used; s += 32) mx = fmaxf(mx, __ldcg(p + s).x);
+        for (uint32_t s = lane; s < used; s += 32) mx = fmaxf(mx, max_sum(s).x);
 #pragma unroll
         for (int d = 16; d > 0; d >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, d));
         for (uint32_t s = lane; s < used; s += 32) {
-            const float2 ml = __ldcg(p + s);
+            const float2 ml = max_sum(s);
             const float c = ml.x == -INFINITY ? 0.f : __expf(ml.x - mx);
             sm_w[wid][s] = c;
             sum += ml.y * c;
@@ -560,7 +644,7 @@ k_attn_decode(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat16 *__restri
         if (lane == 0) sm_sum[wid] = sum;
     }
     __syncthreads();
-    float *sm_p = &sm_acc[0][0][0];                    // [PG][G * D]
+    float *sm_p = sm_acc;                              // [PG][G * D]
 #pragma unroll
     for (int i = 0; i < MAXQ; ++i) {
         const int qd = q0 + i * 256;
@@ -573,14 +657,14 @@ k_attn_decode(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat16 *__restri
 #pragma unroll
         for (int k = 0; k < UN; ++k) {
             const uint32_t s = pg + k * PG;
-            if (s < used) add(i ? __ldcg(sums(qd, s)) : first[k], sm_w[h][s]);
+            if (s < used) add(i ? sums(qd, s) : first[k], sm_w[h][s]);
         }
         for (uint32_t s0 = pg + UN * PG; s0 < used; s0 += UN * PG) {
             float4 v[UN];
 #pragma unroll
             for (int k = 0; k < UN; ++k) {
                 const uint32_t s = s0 + k * PG;
-                v[k] = s < used ? __ldcg(sums(qd, s)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                v[k] = s < used ? sums(qd, s) : make_float4(0.f, 0.f, 0.f, 0.f);
             }
 #pragma unroll
             for (int k = 0; k < UN; ++k)
@@ -594,12 +678,7 @@ k_attn_decode(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat16 *__restri
         float a = sm_p[i];
 #pragma unroll
         for (int g = 1; g < PG; ++g) a += sm_p[g * G * D + i];
-        float o = bfround(a / sm_sum[h]);
-        if (join.gate) {
-            const float gv = bf2f(join.gate[(size_t)blockIdx.z * join.gate_row_stride + (size_t)(head0 + h) * join.gate_stride + d]);
-            o = o * bfround(sigmoid_f(gv));
-        }
-        join.out[((size_t)blockIdx.z * hq + head0 + h) * D + d] = __float2bfloat16_rn(o);
+        write_out(h, d, a / sm_sum[h]);
     }
 }
 

@@ -138,6 +138,34 @@ def test_attn_decode_parts(hq, hkv, d, splits, ctx):
     assert not bool(one.tickets.any())
 
 
+@pytest.mark.parametrize("hq,hkv,d,splits", [(2, 1, 64, 18), (16, 8, 128, 18), (16, 8, 128, 3), (12, 4, 128, 65), (16, 4, 128, 9),
+                                             (12, 2, 64, 18), (3, 3, 128, 1), (6, 2, 256, 9), (8, 2, 256, 2)])
+def test_attn_decode_one_cta_per_group(hq, hkv, d, splits):
+    """So many sequences that one CTA takes all parts of a group: no position (NaN), one, the edges of a chunk and of a part,
+    more parts than are kept in shared memory, the whole cache.  Each sequence has the bits that it has alone."""
+    from ixrun_b200.glue import AttnDecode
+
+    dev, max_seq, b = "cuda", 1300, -(-240 // hkv)
+    gen = torch.Generator(device=dev).manual_seed(hq)
+    kc = torch.randn(b, max_seq, hkv, d, generator=gen, device=dev).bfloat16()
+    vc = torch.randn(b, max_seq, hkv, d, generator=gen, device=dev).bfloat16()
+    q = torch.randn(b, hq * d, generator=gen, device=dev).bfloat16()
+    gate = torch.randn(b, hq * d, generator=gen, device=dev).bfloat16()
+    edges = [-1, 0, 62, 63, 64, 127, 128, 64 * splits - 1, 64 * splits, 64 * splits + 64, 700, max_seq - 1]
+    pos = torch.tensor([edges[i % len(edges)] for i in range(b)], dtype=torch.int32, device=dev).clamp_(max=max_seq - 1)
+    beyond = torch.arange(max_seq, device=dev)[None, :] > pos[:, None]
+    kc[beyond] = float("nan")
+    vc[beyond] = float("nan")
+    many = AttnDecode(hq, hkv, d, dev, splits=splits, batch=b)
+    one = AttnDecode(hq, hkv, d, dev, splits=splits)
+    for g in (None, gate):
+        out = many(q, kc, vc, pos, gate=g, gate_row_stride=hq * d if g is not None else 0)
+        assert not bool(many.tickets.any())
+        for r in list(range(len(edges))) + [b - 1]:
+            alone = one(q[r], kc[r], vc[r], pos[r:r + 1], gate=None if g is None else g[r])
+            assert torch.equal(alone.view(torch.int16), out[r].view(torch.int16))
+
+
 class _NoLaunch:
     """stands in for the C library: a call that gets as far as a launch fails the test instead of handing a host pointer on"""
 
