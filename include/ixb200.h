@@ -226,7 +226,9 @@ int ixb_p6_gemv(const ixb_p6 *t, const void *x_device, int64_t m_rows, const voi
  * (ixrun/engine.py:171-173; precedent for a fused kernel: ixrun/tpab_gemm.py:34-94).
  * ixb_p6_rows: in_f a multiple of 8, no scratch (splits are joined inside a cluster of CTAs).
  * ixb_p6_gemm: the same for in_f a multiple of 64; a scratch of at least 256 bytes, 256-byte aligned, is asked for (its
- *   kernels once kept partial sums there) and left alone. */
+ *   kernels once kept partial sums there) and left alone.
+ * Waits inside the kernels are bounded and count their own work only, not a kernel ahead that they wait for; a launch in which
+ * one runs out leaves NaN in its outputs. */
 int ixb_p6_rows(const ixb_p6 *t, const void *x_device, int64_t m_rows, const void *bias_device, void *y_device, int y_is_f32,
                 ixb_stream_t stream);
 size_t ixb_p6_gemm_scratch_bytes(int64_t out_f, int64_t in_f, int64_t m_rows);

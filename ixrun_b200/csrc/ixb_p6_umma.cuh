@@ -27,8 +27,11 @@
 // by TMA 30.3; packed weights by TMA instead of registers, so that the loads of outliers and weights wait for nobody, 25.4 (by
 // eight one-dimensional bulk copies a stage 27.5).
 //
-// Every wait on an mbarrier is bounded; a thread whose wait gave up does not wait again, the CTA's sums become NaN and the kernel
-// carries on to its end, so tensor memory is always released.
+// Every wait on an mbarrier is bounded, and no thread begins one that depends on the activations before the kernel ahead is
+// complete: such a wait counts this CTA's own copies, conversions and MMAs only, however long that kernel takes.  A thread whose
+// wait gave up asks for nothing more; the loaders then wait (bounded too) for the copies that they did ask for and every thread for
+// the MMAs that were issued, so that nothing lands in memory that has got another use; the CTA's outputs become NaN, and the
+// kernel carries on to its end, so tensor memory is always released.
 #pragma once
 #include <cuda.h>
 #include "ixb_gemm_tc.cuh"
@@ -47,7 +50,7 @@ constexpr int kPuLoadWarp = kPuMmaWarp + 1;              // 25
 constexpr int kPuWLoadWarp = kPuLoadWarp + 1;            // 26
 constexpr int kPuWarps = kPuWLoadWarp + 1;
 constexpr int kPuThreads = kPuWarps * 32;                // 864
-constexpr uint32_t kPuWaitLimit = 1u << 18;
+constexpr uint32_t kPuWaitLimit = 1u << 20;               // polls
 constexpr uint32_t kPuTmemCols = 512;                    // all of it: 256 columns of accumulators, 256 of weights
 constexpr uint32_t kPuStages = 4;                        // of two column blocks: 64 columns of tensor memory each, and their activations
 constexpr uint32_t kPuWStages = 2 * kPuStages;           // ... of packed weights in shared memory
@@ -201,7 +204,8 @@ k_p6_umma(P6 p, const __grid_constant__ CUtensorMap wmap, const __grid_constant_
         // ---- the activations of a stage (rows and columns beyond x arrive as zeros; rows of 128 bytes, their 16-byte pieces
         // swizzled) as soon as the stage four before it is done
         asm volatile("griddepcontrol.wait;" ::: "memory");
-        for (uint32_t i = 0; i < ns; ++i) {
+        uint32_t i = 0;
+        for (; i < ns; ++i) {
             const uint32_t s = i & (kPuStages - 1u), bar = xfull0 + 8u * s, n = min(2u, nk - 2u * i);
             ok = ok && pu_wait(empty0 + 8u * s, (i / kPuStages & 1u) ^ 1u);
             if (__any_sync(0xffffffffu, !ok)) break;
@@ -213,14 +217,26 @@ k_p6_umma(P6 p, const __grid_constant__ CUtensorMap wmap, const __grid_constant_
             }
             __syncwarp();
         }
+        // the copies that may still be in flight (the tensor core's warp waits for them too, unless it gave up)
+        bool landed = true;
+        for (uint32_t j = i > kPuStages ? i - kPuStages : 0u; j < i; ++j)
+            landed = pu_wait(xfull0 + 8u * (j & (kPuStages - 1u)), j / kPuStages & 1u) && landed;
+        ok = ok && landed;
     } else if (warp == kPuWLoadWarp) {
         // ---- the packed weights of a stage as soon as those of the stage eight before it are converted (the barriers of converted
         // weights are as many as the slots of packed ones: a warp that runs behind by a whole round is never waited past)
-        for (uint32_t i = 0; i + kPuWStages < ns; ++i) {
+        uint32_t i = 0;
+        for (; i + kPuWStages < ns; ++i) {
+            // (from the fifth stage on the converters wait for the tensor core, and that for activations)
+            if (i == kPuStages) asm volatile("griddepcontrol.wait;" ::: "memory");
             ok = ok && pu_wait(full0 + 8u * (i & (kPuWStages - 1u)), i / kPuWStages & 1u);
             if (__any_sync(0xffffffffu, !ok)) break;
             load_w(i + kPuWStages);
         }
+        bool landed = true;                                            // as above
+        for (uint32_t j = i, end = min(ns, i + kPuWStages); j < end; ++j)
+            landed = pu_wait(wfull0 + 8u * (j & (kPuWStages - 1u)), j / kPuWStages & 1u) && landed;
+        ok = ok && landed;
     } else if (warp == kPuMmaWarp) {
         // ---- the warp that feeds the tensor core; its addresses and descriptors are uniform, slots unrolled, because a stage
         // takes as long as this warp's chain of instructions if that is long.  (Tokens m_tok .. n_pad - 1 of a stage are whatever
@@ -228,7 +244,8 @@ k_p6_umma(P6 p, const __grid_constant__ CUtensorMap wmap, const __grid_constant_
         const uint32_t idesc = pu_idesc(n_pad), el = pu_elect(), accs = pu_accs(n_pad);
         uint32_t d = tmem;                                              // the accumulator of the next block
         const uint64_t dx0 = umma_desc(smem0, 16u, 1024u) | 2ull << 61;     // eight rows of 128 bytes, 128-byte swizzle
-        for (uint32_t i0 = 0; i0 < ns; i0 += kPuWStages) {
+        asm volatile("griddepcontrol.wait;" ::: "memory");             // (a wait for activations is not one for the kernel ahead)
+        for (uint32_t i0 = 0; i0 < ns && ok; i0 += kPuWStages) {
             const uint32_t par = i0 / kPuWStages & 1u;
 #pragma unroll
             for (uint32_t ws = 0; ws < kPuWStages; ++ws) {
@@ -236,7 +253,8 @@ k_p6_umma(P6 p, const __grid_constant__ CUtensorMap wmap, const __grid_constant_
                 if (i0 + ws >= ns) break;
                 ok = ok && pu_wait(xfull0 + 8u * st, ws / kPuStages & 1u);            // (two rounds of these to one of the weights')
                 ok = ok && pu_wait(full0 + 8u * ws, par);
-                __syncwarp();                                           // (no lane falls a phase behind the one that issues)
+                ok = __all_sync(0xffffffffu, ok);                       // (also: no lane falls a phase behind the one that issues)
+                if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
                 for (uint32_t h = 0; h < 2u; ++h) {
@@ -321,6 +339,8 @@ k_p6_umma(P6 p, const __grid_constant__ CUtensorMap wmap, const __grid_constant_
                     for (int32_t j = at + 32; j < hi; j += 32) put(img_s + p6_image_at(__ldg(p.esc + j)), 0);
                 }
             }
+            // (the first wait for the tensor core, and so for activations)
+            if (i >= 2u * kPuStages && i < 2u * kPuStages + kPuPhases) asm volatile("griddepcontrol.wait;" ::: "memory");
             ok = ok && pu_wait(empty0 + 8u * slot, (i / (2u * kPuStages) & 1u) ^ 1u);  // the slot's last reader (the tensor core) is done
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             __syncwarp();
@@ -335,12 +355,12 @@ k_p6_umma(P6 p, const __grid_constant__ CUtensorMap wmap, const __grid_constant_
         }
     }
     __syncwarp();
-    ok = ok && pu_wait(done_bar, 0u);
+    // (also: the kernels ahead may still read what y held)
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    ok = pu_wait(done_bar, 0u) && ok;                                   // (the MMAs that were issued are done, whoever gave up)
     if (!ok) *failed = 1u;
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     __syncthreads();                                                    // nobody uses the stages and the rings any more
-    // the kernels ahead may still read what y held
-    asm volatile("griddepcontrol.wait;" ::: "memory");
     const bool bad = *failed != 0u;
     float *red = (float *)pu_smem;                                      // [token][kPuRedPitch]
     auto put = [&](uint32_t m, uint32_t r, float v) {

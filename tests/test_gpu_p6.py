@@ -451,3 +451,39 @@ def test_p6_gemv_few_blocks(out_f, in_f, dense):
     y, ref = p6.gemv(x), (x.double() @ w.t()).bfloat16()
     assert torch.equal(y[1].nan_to_num(nan=7.0, posinf=1.0, neginf=-1.0), ref[1].nan_to_num(nan=7.0, posinf=1.0, neginf=-1.0))
     assert torch.equal(y[[0, 2, 3, 4, 5, 6, 7]], y8[[0, 2, 3, 4, 5, 6, 7]].bfloat16())
+
+
+@pytest.mark.parametrize("m", [16, 64])
+@pytest.mark.parametrize("out_f,in_f", [(256, 32768), (19000, 1280)])
+def test_p6_rows_behind_a_kernel_that_takes_long(out_f, in_f, m):
+    """Dependent launch: the kernel ahead (attention over four million positions by one CTA, a tenth of a second and more) lets the
+    launch begin at once, and however long it takes counts against none of the launch's bounded waits: the bits of a launch
+    with nothing ahead.  K split over a cluster and not, more stages than are in flight."""
+    from ixrun_b200.glue import AttnDecode
+    from ixrun_b200.p6 import P6Packed, set_pdl
+
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    codes = (torch.randn(out_f, in_f, generator=gen, device="cuda") * 12).round().clamp(-127, 127).to(torch.int8)
+    p6 = P6Packed(codes, torch.tensor(0.007, dtype=torch.bfloat16), out_f, in_f)
+    x = torch.randn(m, in_f, generator=gen, device="cuda").bfloat16()
+    n = 1 << 22
+    cache = torch.zeros(n, 1, 64, dtype=torch.bfloat16, device="cuda")
+    cache[-1] = 1
+    attn = AttnDecode(2, 1, 64, "cuda", splits=1)
+    q, pos = torch.ones(128, device="cuda").bfloat16(), torch.tensor([n - 1], dtype=torch.int32, device="cuda")
+    a, y = torch.empty(128, dtype=torch.bfloat16, device="cuda"), torch.empty(m, out_f, device="cuda")
+    torch.cuda.synchronize()
+    before = set_pdl(True)
+    try:
+        alone = p6.gemm(x, out_dtype=torch.float32)
+        torch.cuda.synchronize()
+        for _ in range(2):
+            y.zero_()
+            attn(q, cache, cache, pos, out=a)
+            p6.gemm(x, out=y)
+            torch.cuda.synchronize()
+            assert torch.equal(y, alone)
+    finally:
+        set_pdl(before)
+    ref = x.double() @ (codes.float() * p6.scale.float()).bfloat16().double().t()
+    assert float((alone.double() - ref).abs().max() / ref.abs().max()) < 2e-5
