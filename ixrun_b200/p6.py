@@ -94,7 +94,6 @@ class P6Packed:
         self._ref = C.byref(self.struct)             # (keeps the struct alive)
         self._index = index
         self._gemv_need = None                           # scratch bytes
-        self._call = None                                # the extension's object for this tensor
         self.resident_bytes = nb * BLOCK_BYTES + 4 * (nb + 1 + n_esc) + 2
         self.scratch = scratch if scratch is not None else GemvScratch.shared(dev)
 
@@ -131,6 +130,16 @@ class P6Packed:
                    total_bytes=sum(d.total_bytes for d in dps), **kw)
         self.sections = sections
         return self
+
+    @property
+    def scratch(self) -> GemvScratch:
+        """The scratch of this tensor's GEMV launches; may be replaced at any time, for the calls that follow."""
+        return self._scratch
+
+    @scratch.setter
+    def scratch(self, scratch: GemvScratch):
+        self._scratch = scratch
+        self._call = None                                # the extension's object for this tensor: it keeps the buffer's address
 
     def make_call(self):
         """The extension's call (x, bias, many) -> y, or None for what it leaves to `gemv`, `gemm` and the dense matmul."""

@@ -388,3 +388,23 @@ def test_call_through_the_extension_is_the_python_path(in_f, bias):
         with pytest.raises(Exception):
             lin(bad)
     assert lin(torch.randn(2, in_f, device="cuda")).dtype == torch.float32          # another type: the dense matmul
+
+
+def test_a_scratch_that_is_replaced_serves_the_next_call():
+    """Launches that may overlap need separate scratch instances: one that is set on a layer in use is the one that its next
+    call takes, through the module as through `gemv`."""
+    from ixrun_b200.engine import StreamingLinear
+    from ixrun_b200.p6 import GemvScratch
+
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    lin = StreamingLinear.from_weight((torch.randn(96, 8256, generator=gen, device="cuda") * 0.02).bfloat16())
+    x = torch.randn(2, 8256, generator=gen, device="cuda").bfloat16()
+    y = lin(x)
+    for _ in range(2):
+        own = lin._res.scratch = GemvScratch("cuda")
+        assert own.buf.numel() == 0 and lin._res.scratch is own
+        assert torch.equal(lin(x), y)
+        assert own.buf.numel() > 0                       # the call asked this one
+        torch.cuda.synchronize()
+        assert not bool(own.buf.any())                   # (zero between launches)
+        assert torch.equal(lin._res.gemv(x), y)
