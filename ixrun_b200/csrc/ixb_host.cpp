@@ -20,6 +20,15 @@ gemv_fn g_gemv = nullptr;
 rows_fn g_rows = nullptr;
 PyObject *g_check = nullptr;                             // raises the library's error for a status
 
+// The interpreter's lock, given up while torch allocates (which may wait for the device) and while a launch is made (which waits
+// where the queue is full): another thread may be the one that would end the wait.
+struct Unlocked {
+    PyThreadState *state = PyEval_SaveThread();
+    Unlocked() = default;
+    Unlocked(const Unlocked &) = delete;
+    ~Unlocked() { PyEval_RestoreThread(state); }
+};
+
 struct P6Call {
     PyObject_HEAD
     vectorcallfunc call;
@@ -41,29 +50,39 @@ PyObject *p6_call(PyObject *self_, PyObject *const *args, size_t nargsf, PyObjec
     }
     try {
         if (!THPVariable_Check(args[0])) Py_RETURN_NONE;
-        const at::Tensor &x = THPVariable_Unpack(args[0]);
+        const at::Tensor x = THPVariable_Unpack(args[0]);            // (held: other threads run below)
         if (x.scalar_type() != at::kBFloat16 || x.layout() != at::kStrided || !x.is_cuda() || x.get_device() != self->index ||
             at::isTensorSubclassLike(x) || x.is_neg() || x.dim() < 1 || x.size(-1) != self->in_f || !x.is_contiguous())
             Py_RETURN_NONE;
         const int64_t m = x.numel() / self->in_f;
         if (m < 1 || m > 64 || (m > 8 && (self->in_f % 64 || args[2] != Py_True))) Py_RETURN_NONE;
         const void *bias = nullptr;
+        at::Tensor b;
         if (args[1] != Py_None) {
             if (!THPVariable_Check(args[1])) Py_RETURN_NONE;
-            const at::Tensor &b = THPVariable_Unpack(args[1]);
+            b = THPVariable_Unpack(args[1]);
             if (b.scalar_type() != at::kBFloat16 || b.numel() != self->out_f || !b.is_cuda() || b.get_device() != self->index || !b.is_contiguous())
                 Py_RETURN_NONE;
             bias = b.data_ptr();
         }
-        c10::cuda::OptionalCUDAGuard guard;
-        if (c10::cuda::current_device() != self->index) guard.set_index((c10::DeviceIndex)self->index);
         at::DimVector shape(x.sizes().begin(), x.sizes().end());
         shape.back() = self->out_f;
-        at::Tensor y = at::empty(shape, at::TensorOptions().dtype(at::kBFloat16).device(at::Device(at::kCUDA, (c10::DeviceIndex)self->index)));
-        if (at::isTensorSubclassLike(y)) Py_RETURN_NONE;
-        void *stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)self->index).stream();
-        const int rc = m <= 8 ? g_gemv(self->tensor, x.data_ptr(), m, bias, y.data_ptr(), 0, self->scratch, self->scratch_bytes, stream)
-                              : g_rows(self->tensor, x.data_ptr(), m, bias, y.data_ptr(), 0, stream);
+        at::Tensor y;
+        int rc = 0;
+        bool plain;
+        {
+            const Unlocked unlocked;
+            c10::cuda::OptionalCUDAGuard guard;
+            if (c10::cuda::current_device() != self->index) guard.set_index((c10::DeviceIndex)self->index);
+            y = at::empty(shape, at::TensorOptions().dtype(at::kBFloat16).device(at::Device(at::kCUDA, (c10::DeviceIndex)self->index)));
+            plain = !at::isTensorSubclassLike(y);
+            if (plain) {
+                void *stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)self->index).stream();
+                rc = m <= 8 ? g_gemv(self->tensor, x.data_ptr(), m, bias, y.data_ptr(), 0, self->scratch, self->scratch_bytes, stream)
+                            : g_rows(self->tensor, x.data_ptr(), m, bias, y.data_ptr(), 0, stream);
+            }
+        }
+        if (!plain) Py_RETURN_NONE;
         if (rc) {
             PyObject *r = PyObject_CallFunction(g_check, "i", rc);
             Py_XDECREF(r);
@@ -152,7 +171,11 @@ PyObject *empty(PyObject *, PyObject *const *args, Py_ssize_t nargs)
             }
             const auto dt = type == 'B' ? at::kByte : type == 'b' ? at::kChar : type == 'i' ? at::kInt : at::kBFloat16;
             const int64_t size[1] = {n};
-            const at::Tensor t = at::empty(at::IntArrayRef(size, n < 0 ? 0 : 1), at::TensorOptions().dtype(dt).device(at::Device(at::kCUDA, (c10::DeviceIndex)index)));
+            at::Tensor t;
+            {
+                const Unlocked unlocked;
+                t = at::empty(at::IntArrayRef(size, n < 0 ? 0 : 1), at::TensorOptions().dtype(dt).device(at::Device(at::kCUDA, (c10::DeviceIndex)index)));
+            }
             PyObject *o = THPVariable_Wrap(t);
             if (!o) {
                 Py_DECREF(out);

@@ -408,3 +408,37 @@ def test_a_scratch_that_is_replaced_serves_the_next_call():
         torch.cuda.synchronize()
         assert not bool(own.buf.any())                   # (zero between launches)
         assert torch.equal(lin._res.gemv(x), y)
+
+
+def test_the_packed_call_lets_other_threads_run():
+    """The interpreter lock is free while the extension allocates and launches (a launch waits where the queue is full): the C
+    library's sleep takes the place of the launch, and another thread goes on meanwhile."""
+    import ctypes as C
+    import threading
+    import time
+
+    from ixrun_b200 import _lib
+
+    class Timespec(C.Structure):
+        _fields_ = [("s", C.c_long), ("ns", C.c_long)]
+
+    host, L = _lib.host(), _lib.lib()
+    sleep = C.cast(C.CDLL(None).nanosleep, C.c_void_p).value
+    for rows in (1, 64):
+        nap = Timespec(1, 0)                             # in the place of the tensor's structure: the first argument
+        call = host.p6(C.addressof(nap), 64, 128, 0, torch.zeros(1024, dtype=torch.uint8, device="cuda"))
+        x = torch.zeros(rows, 128, dtype=torch.bfloat16, device="cuda")
+        torch.cuda.synchronize()
+        done = []
+        host.bind(sleep, sleep, _lib.check)
+        try:
+            t = threading.Thread(target=lambda: (call(x, None, True), done.append(time.perf_counter())))
+            t0 = time.perf_counter()
+            t.start()
+            while time.perf_counter() - t0 < 0.3:        # (with the lock held: not before the sleep is over)
+                time.sleep(0.01)
+            seen = time.perf_counter() - t0
+            t.join()
+        finally:
+            host.bind(C.cast(L.ixb_p6_gemv, C.c_void_p).value, C.cast(L.ixb_p6_rows, C.c_void_p).value, _lib.check)
+        assert seen < 0.9 and done[0] - t0 >= 1.0
