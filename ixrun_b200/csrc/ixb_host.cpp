@@ -10,6 +10,7 @@
 #include <ATen/ops/empty.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 namespace {
@@ -90,8 +91,8 @@ PyObject *p6_call(PyObject *self_, PyObject *const *args, size_t nargsf, PyObjec
             return nullptr;
         }
         return THPVariable_Wrap(std::move(y));
-    } catch (const std::exception &e) {
-        if (!PyErr_Occurred()) PyErr_SetString(PyExc_RuntimeError, e.what());
+    } catch (...) {                                      // as torch's functions raise it: out of memory, an error of Python code
+        torch::translate_exception_to_python(std::current_exception());
         return nullptr;
     }
 }
@@ -183,9 +184,9 @@ PyObject *empty(PyObject *, PyObject *const *args, Py_ssize_t nargs)
             }
             PyTuple_SET_ITEM(out, i - 1, o);
         }
-    } catch (const std::exception &e) {
+    } catch (...) {
         Py_DECREF(out);
-        if (!PyErr_Occurred()) PyErr_SetString(PyExc_RuntimeError, e.what());
+        torch::translate_exception_to_python(std::current_exception());
         return nullptr;
     }
     return out;

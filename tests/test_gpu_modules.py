@@ -442,3 +442,21 @@ def test_the_packed_call_lets_other_threads_run():
         finally:
             host.bind(C.cast(L.ixb_p6_gemv, C.c_void_p).value, C.cast(L.ixb_p6_rows, C.c_void_p).value, _lib.check)
         assert seen < 0.9 and done[0] - t0 >= 1.0
+
+
+def test_errors_of_the_extension_keep_their_type():
+    """Memory that is not there and what a mode raises reach the caller as torch's functions raise them."""
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    from ixrun_b200 import _lib
+
+    class Refuse(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            raise KeyError("refused")
+
+    with pytest.raises(torch.OutOfMemoryError):
+        _lib.host().empty(0, (16, "i"), (1 << 50, "B"))
+    with Refuse(), pytest.raises(KeyError):
+        _lib.host().empty(0, (16, "i"))
+    a, b, c = _lib.host().empty(0, (16, "i"), (-1, "h"), (0, "b"))
+    assert (a.dtype, a.shape, b.dtype, b.shape, c.dtype, c.shape) == (torch.int32, (16,), torch.bfloat16, (), torch.int8, (0,))
