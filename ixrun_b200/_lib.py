@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import warnings
 
 import torch
 
@@ -177,17 +178,37 @@ def lib():
 _host = None
 
 
+class _PythonHost:
+    """What the extension does, for a machine on which it neither lies built nor can be built: allocations through torch, and
+    every packed linear's call left to the Python path."""
+
+    _TYPES = {"B": torch.uint8, "b": torch.int8, "i": torch.int32, "h": torch.bfloat16}
+
+    @classmethod
+    def empty(cls, index: int, *specs):
+        if index < 0:
+            raise ValueError("expected a CUDA device")
+        return tuple(torch.empty((n,) if n >= 0 else (), dtype=cls._TYPES[t], device=f"cuda:{index}") for n, t in specs)
+
+    @staticmethod
+    def p6(*_):
+        return lambda x, bias, many: None
+
+
 def host():
-    """The extension for the host side of a call (csrc/ixb_host.cpp), built first if it is missing or stale."""
+    """The extension for the host side of a call (csrc/ixb_host.cpp), built first if it is missing or stale; where that
+    cannot be done a stand-in without its speed."""
     global _host
     if _host is None:
-        if _build.host_is_stale():
-            try:
+        try:
+            if _build.host_is_stale():
                 _build.build_host()
-            except Exception as e:
-                raise IxbError(f"_ixbhost.so is missing or older than its source and cannot be built here: {e}") from e
-        from . import _ixbhost
-
+            from . import _ixbhost
+        except Exception as e:
+            warnings.warn(f"the host extension (_ixbhost.so) is missing or older than its source and cannot be built here, so packed "
+                          f"linears and deployment take their slower Python path: {e}", RuntimeWarning, stacklevel=2)
+            _host = _PythonHost
+            return _host
         L = lib()
         _ixbhost.bind(C.cast(L.ixb_p6_gemv, C.c_void_p).value, C.cast(L.ixb_p6_rows, C.c_void_p).value, check)
         _host = _ixbhost

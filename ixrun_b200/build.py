@@ -130,7 +130,10 @@ def build_host(force: bool = False) -> str:
                 return HOST_SO
             tmp, t = f"{HOST_SO}.tmp{os.getpid()}", _torch_dir()
             cuda = os.path.dirname(os.path.dirname(os.path.realpath(nvcc_path())))
-            r = subprocess.run(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-I{sysconfig.get_paths()['include']}",
+            import torch
+
+            abi = f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}"
+            r = subprocess.run(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", abi, f"-I{sysconfig.get_paths()['include']}",
                                 f"-I{t}/include", f"-I{t}/include/torch/csrc/api/include", f"-I{cuda}/include", HOST_SRC,
                                 "-o", tmp, f"-L{t}/lib", "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"],
                                capture_output=True, text=True)

@@ -460,3 +460,31 @@ def test_errors_of_the_extension_keep_their_type():
         _lib.host().empty(0, (16, "i"))
     a, b, c = _lib.host().empty(0, (16, "i"), (-1, "h"), (0, "b"))
     assert (a.dtype, a.shape, b.dtype, b.shape, c.dtype, c.shape) == (torch.int32, (16,), torch.bfloat16, (), torch.int8, (0,))
+
+
+@pytest.mark.filterwarnings("ignore:the host extension")
+def test_without_the_extension_the_python_path_serves(monkeypatch):
+    """No compiler and no built file: deployment and calls go through Python, with the same results."""
+    from ixrun_b200 import _lib
+    from ixrun_b200 import build as b
+    from ixrun_b200.engine import StreamingLinear
+
+    gen = torch.Generator(device="cuda").manual_seed(6)
+    w, bias = (torch.randn(96, 128, generator=gen, device="cuda") * 0.02).bfloat16(), torch.randn(96, device="cuda").bfloat16()
+    xs = [torch.randn(m, 128, generator=gen, device="cuda").bfloat16() for m in (1, 8, 23, 64, 65)]
+
+    def all_of():
+        lin = StreamingLinear.from_weight(w, bias=bias)
+        lin._set_shared_buf(torch.empty(96 * 128, dtype=torch.bfloat16, device="cuda"))
+        return [lin(x) for x in xs] + [lin._res.plane[:-960], lin._res.esc[:lin._res.n_esc], lin._res.blk_off]
+
+    want = all_of()
+
+    def refuse(force=False):
+        raise RuntimeError("no compiler")
+
+    monkeypatch.setattr(_lib, "_host", None)
+    monkeypatch.setattr(b, "host_is_stale", lambda: True)
+    monkeypatch.setattr(b, "build_host", refuse)
+    for got, ref in zip(all_of(), want):
+        assert torch.equal(got, ref)

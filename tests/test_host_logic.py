@@ -139,3 +139,22 @@ def test_on_device_refuses_a_tensor_that_is_on_no_gpu(monkeypatch):
     with pytest.raises(ValueError):
         with _lib.on_device(torch.zeros(1).get_device()):
             pass
+
+
+def test_a_machine_without_compiler_gets_the_python_path(monkeypatch):
+    """No built extension and no way to build it: a warning, and a stand-in that leaves every call to Python"""
+    from ixrun_b200 import _lib
+    from ixrun_b200 import build as b
+
+    def refuse(force=False):
+        raise RuntimeError("no compiler")
+
+    monkeypatch.setattr(_lib, "_host", None)
+    monkeypatch.setattr(b, "host_is_stale", lambda: True)
+    monkeypatch.setattr(b, "build_host", refuse)
+    with pytest.warns(RuntimeWarning, match="no compiler"):
+        host = _lib.host()
+    assert host.p6(0, 16, 64, 0, None)(torch.zeros(1, 64), None, True) is None
+    with pytest.raises(ValueError):
+        host.empty(-1, (4, "i"))
+    assert _lib.host() is host
