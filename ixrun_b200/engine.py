@@ -139,11 +139,11 @@ class StreamingLinear(nn.Module):
 
     def forward(self, x):
         res = self._res
-        if res is not None:
+        rows = x.numel() // self.in_features
+        if res is not None and rows <= TC_MAX_ROWS:
             y = (res._call or res.make_call())(x, self._bias_bf16, self._use_p6_gemm)
             if y is not None:
                 return y
-        rows = x.numel() // self.in_features
         if res is not None and x.dtype == torch.bfloat16 and x.shape[-1] == self.in_features and rows <= TC_MAX_ROWS:
             y = None
             if 1 <= rows <= FUSED_MAX_ROWS:

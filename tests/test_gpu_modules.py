@@ -488,3 +488,18 @@ def test_without_the_extension_the_python_path_serves(monkeypatch):
     monkeypatch.setattr(b, "build_host", refuse)
     for got, ref in zip(all_of(), want):
         assert torch.equal(got, ref)
+
+
+def test_a_prompt_asks_nothing_of_the_extension(monkeypatch):
+    """More rows than the fused kernels take: no object of the extension is made for the layer, and none is called."""
+    from ixrun_b200.engine import StreamingLinear
+    from ixrun_b200.p6 import P6Packed
+
+    lin = StreamingLinear.from_weight((torch.randn(96, 128, device="cuda") * 0.02).bfloat16())
+    lin._set_shared_buf(torch.empty(96 * 128, dtype=torch.bfloat16, device="cuda"))
+    calls = []
+    monkeypatch.setattr(P6Packed, "make_call", lambda self: calls.append(1) or (lambda *a: None))
+    for rows in (65, 1000):
+        assert lin(torch.randn(rows, 128, device="cuda").bfloat16()).shape == (rows, 96)
+    assert not calls and lin._res._call is None
+    assert lin(torch.randn(64, 128, device="cuda").bfloat16()).shape == (64, 96) and calls
