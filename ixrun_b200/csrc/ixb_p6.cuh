@@ -523,15 +523,24 @@ __device__ __forceinline__ uint32_t p6_image_at(uint32_t e)
     return (((c >> 4) * 32u + 4u * (r & 7u) + ((c >> 2) & 3u)) * 4u + 2u * ((c >> 1) & 1u) + (r >> 3)) * 4u + 2u * (c & 1u);
 }
 
-// layout -> bf16 weights in one pass, with the GEMV's own conversion.  Bound by memory (2.76 bytes per weight): the
-// plane is requested before the offsets, the block's weights go through a tile in shared memory (16-byte pieces swizzled) where
-// its outliers overwrite their placeholders, and every weight is stored once, a 32-byte sector per lane where the alignment
-// allows; eight CTAs per SM are in flight.  17408 x 5120 40.2 us (38.0 at the copy rate), 12288 x 2048 10.9, 2048 x 6144 6.0;
-// with the words dealt out over the quads by shuffles 40.5, 11.1 and 6.3, stored in 8-byte pieces 40.4, 11.5 and 7.3.
+// An outlier's register in k_p6_decode_bf16: row r, column c of the block sit in lane 4 (r & 7) + (c >> 4), register
+// 8 (r >> 3) + ((c & 15) >> 1), half c & 1.
+__device__ __forceinline__ uint32_t p6_row_lane(uint32_t e) { return 4u * ((e >> 12) & 7u) + ((e >> 4) & 3u); }
+__device__ __forceinline__ uint32_t p6_row_reg(uint32_t e) { return 8u * ((e >> 15) & 1u) + ((e >> 1) & 7u); }
+
+// layout -> bf16 weights in one pass, with the GEMV's own conversion.  Bound by memory (2.76 bytes per weight, the stores to an
+// output that stays in L2 faster than that).  The plane is requested before the offsets; the words of a quad's lanes are dealt out
+// while they are packed (8 shuffles; as weights it takes 16), so that a lane has 16 consecutive columns of two rows and every weight
+// is stored once, a 32-byte sector per lane and row where the alignment allows.  One or two outliers go straight into their
+// lane's register, more through an image of the lanes' registers in shared memory; eight CTAs per SM are in flight (six: 17408 x 5120
+// 40.7 us, 12288 x 2048 10.9).  In a graph, every launch to its own output / all to one that stays in L2, as a prompt's do: 17408 x
+// 5120 40.1 / 40.0 us, 12288 x 2048 13.5 / 10.3, 2048 x 6144 8.0 / 6.5, 4096 x 2048 5.9 / 4.7; with the weights turned round in a
+// tile of shared memory 39.8 / 39.8, 13.5 / 11.1, 8.0 / 6.8, 5.8 / 4.8; on the layout whose lanes held 16 columns as it was 39.8 /
+// 39.8, 13.2 / 10.3, 7.8 / 6.6, 6.0 / 4.5.
 // Needs in_f % 8 == 0 and a 16-byte aligned output.  One warp per block.
 __global__ void __launch_bounds__(256, 8) k_p6_decode_bf16(P6 p, __nv_bfloat16 *out)
 {
-    __shared__ uint4 tiles[8 * 128];
+    __shared__ uint4 images[8 * 128];
     const uint32_t b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (b >= p.rt * p.kb) return;                    // whole warps leave together
@@ -540,37 +549,63 @@ __global__ void __launch_bounds__(256, 8) k_p6_decode_bf16(P6 p, __nv_bfloat16 *
     const uint2 a2 = __ldg((const uint2 *)(blk + 512) + lane);
     const int32_t lo = __ldg(p.blk_off + b), hi = __ldg(p.blk_off + b + 1);
     const uint32_t R = b / p.kb, kbi = b - R * p.kb;
-    const uint32_t w[6] = {a.x, a.y, a.z, a.w, a2.x, a2.y};
-    uint32_t f[16];
-    p6_unpack(w, 0x43004300u, p6_scale2(p.scale[R * p.scale_stride]), f);
-    const uint32_t tile = (uint32_t)__cvta_generic_to_shared(tiles + (threadIdx.x >> 5) * 128);
-    auto piece = [&](uint32_t r, uint32_t c) { return tile + r * 128u + (c ^ (r & 7u)) * 16u; };     // columns 8 c .. 8 c + 7 of row r
-    const uint32_t g = (uint32_t)lane >> 2, t = (uint32_t)lane & 3u;
-    // pair 4 j + q: row g + 8 (q & 1), columns 16 j + 4 t + 2 (q >> 1) + {0, 1} of the block
+    const uint32_t s2 = p6_scale2(p.scale[R * p.scale_stride]);
+    // word j of u: pairs 4 j and 4 j + 1 of the lane (bits 0 / 16 and 6 / 22, as in words 0 .. 5), of v: 4 j + 2 and 4 j + 3
+    uint32_t u[4] = {a.x, a.z, a2.x, 0u}, v[4] = {a.y, a.w, a2.y, 0u};
+    u[3] = p6_and_or(a2.x >> 8, 0x00300030u, (a.x >> 12) & 0x000F000Fu) | p6_and_or(a2.x >> 4, 0x0C000C00u, (a.y >> 6) & 0x03C003C0u);
+    v[3] = p6_and_or(a2.y >> 8, 0x00300030u, (a.z >> 12) & 0x000F000Fu) | p6_and_or(a2.y >> 4, 0x0C000C00u, (a.w >> 6) & 0x03C003C0u);
+    p6_quad_transpose(u, lane);
+    p6_quad_transpose(v, lane);
+    uint32_t f[16];                                  // row g and row g + 8, columns 16 (lane & 3) .. + 15
 #pragma unroll
-    for (int s = 0; s < 2; ++s)
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-            asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(piece(g + 8u * s, 2u * j + (t >> 1)) + (t & 1u) * 8u), "r"(f[4 * j + s]), "r"(f[4 * j + 2 + s]) : "memory");
-    __syncwarp();
-    for (int32_t j = lo + lane; j < hi; j += 32) {
-        const uint32_t e = __ldg(p.esc + j), r = (e >> 12) & 15u, c = e & 63u;
-        asm volatile("st.shared.u16 [%0], %1;" ::"r"(piece(r, c >> 3) + (c & 7u) * 2u), "h"((unsigned short)(e >> 16)) : "memory");
+    for (int t = 0; t < 4; ++t) {
+        f[2 * t] = p6_weights(p6_and_or(u[t], 0x003F003Fu, 0x43004300u), s2);
+        f[2 * t + 1] = p6_weights(p6_and_or(v[t], 0x003F003Fu, 0x43004300u), s2);
+        f[8 + 2 * t] = p6_weights(p6_and_or(u[t] >> 6, 0x003F003Fu, 0x43004300u), s2);
+        f[8 + 2 * t + 1] = p6_weights(p6_and_or(v[t] >> 6, 0x003F003Fu, 0x43004300u), s2);
     }
-    __syncwarp();
-    const bool wide = (p.in_f & 15u) == 0 && ((uintptr_t)out & 31u) == 0;       // a lane's 32 bytes of a row are one sector
+    // placeholders are +0.0, so OR-ing the outlier weights in is exact
+    if (hi - lo <= 2) {
+        for (int32_t j = lo; j < hi; ++j) {
+            const uint32_t e = __ldg(p.esc + j), at = p6_row_reg(e);
+            const uint32_t w = (uint32_t)lane == p6_row_lane(e) ? ((e & 1u) ? e & 0xFFFF0000u : e >> 16) : 0u;
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {
-        const uint32_t r = 8u * k + g, c = 2u * t, row = R * kTileRows + r, col = kbi * kTileCols + 8u * c;
-        const uint4 v0 = p6_lds128(piece(r, c)), v1 = p6_lds128(piece(r, c + 1u));
-        if (row >= p.out_f || col >= p.in_f) continue;
-        __nv_bfloat16 *dst = out + (size_t)row * p.in_f + col;
+            for (int q = 0; q < 16; ++q)
+                if (at == (uint32_t)q) f[q] |= w;
+        }
+    } else {
+        uint4 *img = images + (threadIdx.x >> 5) * 128;                 // [4 quads of registers][32 lanes]
+#pragma unroll
+        for (int q = 0; q < 4; ++q) img[q * 32 + lane] = make_uint4(0, 0, 0, 0);
+        __syncwarp();
+        const uint32_t img_s = (uint32_t)__cvta_generic_to_shared(img);
+        for (int32_t j = lo + lane; j < hi; j += 32) {
+            const uint32_t e = __ldg(p.esc + j), at = p6_row_reg(e);
+            asm volatile("st.shared.u16 [%0], %1;" ::"r"(img_s + ((at >> 2) * 32u + p6_row_lane(e)) * 16u + (at & 3u) * 4u + (e & 1u) * 2u), "h"((unsigned short)(e >> 16)) : "memory");
+        }
+        __syncwarp();
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const uint4 w = img[q * 32 + lane];
+            f[4 * q] |= w.x;
+            f[4 * q + 1] |= w.y;
+            f[4 * q + 2] |= w.z;
+            f[4 * q + 3] |= w.w;
+        }
+    }
+    const bool wide = (p.in_f & 15u) == 0 && ((uintptr_t)out & 31u) == 0;       // a lane's 32 bytes of a row are one sector
+    const uint32_t col0 = kbi * kTileCols + 16u * (lane & 3);
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+        const uint32_t row = R * kTileRows + (lane >> 2) + 8u * s;
+        if (row >= p.out_f || col0 >= p.in_f) continue;
+        __nv_bfloat16 *dst = out + (size_t)row * p.in_f + col0;
         if (wide) {
-            const uint32_t v[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
-            st_sector(dst, v);
+            const uint32_t r[8] = {f[8 * s], f[8 * s + 1], f[8 * s + 2], f[8 * s + 3], f[8 * s + 4], f[8 * s + 5], f[8 * s + 6], f[8 * s + 7]};
+            st_sector(dst, r);
         } else {                                     // in_f % 8 == 0: eight columns or none
-            ((uint4 *)dst)[0] = v0;
-            if (col + 16u <= p.in_f) ((uint4 *)dst)[1] = v1;
+            ((uint4 *)dst)[0] = make_uint4(f[8 * s], f[8 * s + 1], f[8 * s + 2], f[8 * s + 3]);
+            if (col0 + 16u <= p.in_f) ((uint4 *)dst)[1] = make_uint4(f[8 * s + 4], f[8 * s + 5], f[8 * s + 6], f[8 * s + 7]);
         }
     }
 }
