@@ -24,7 +24,7 @@
 //           32 x uint2 (words 4, 5).  Word k holds pair 2k at bits 0 / 16 and
 //           pair 2k+1 at bits 6 / 22 (low / high element); the 4 + 4 spare
 //           bits of words 0..3 hold the low four bits of pairs 12..15, those of
-//           words 4, 5 their upper two bits (p6_get).
+//           words 4, 5 their upper two bits (p6_pair_words).
 //   esc     the outliers of every block as 32-bit entries
 //             bf16(code * s) << 16 | row_in_tile << 12 | (block & 63) << 6 | column_in_block
 //           sorted by block; blk_off[nb + 1] gives the first entry of every block.
@@ -91,15 +91,6 @@ struct P6 {
     uint32_t rt, kb;             // row tiles, column blocks per row tile; nb = rt * kb
     uint32_t scale_stride;
 };
-
-__host__ __device__ __forceinline__ int p6_code(uint32_t f) { return (int)f - 32; }
-
-__device__ __forceinline__ uint32_t p6_get(const uint32_t (&w)[6], int p, int h)
-{
-    if (p < 12) return (w[p >> 1] >> (6 * (p & 1) + 16 * h)) & 63u;
-    const int i = p - 12;
-    return ((w[i] >> (12 + 16 * h)) & 15u) | (((w[4 + (i >> 1)] >> (12 + 2 * (i & 1) + 16 * h)) & 3u) << 4);
-}
 
 // ------------------------------------------------------------------ build ---
 // word j of lane t of a quad <-> word t of lane j
@@ -185,7 +176,7 @@ k_p6_plane(const int8_t *__restrict__ codes, uint32_t out_f, uint32_t in_f, uint
         for (int v = 0; v < 2; ++v) {
             const uint32_t pair = __byte_perm(f, 0, v ? 0x4342 : 0x4140);          // fields at bits 0 and 16
             const int p = 4 * (k & 3) + 2 * v + (k >> 2);
-            if (p < 12) {                            // (see p6_get)
+            if (p < 12) {                            // (see p6_pair_words)
                 w[p >> 1] |= pair << (6 * (p & 1));
             } else {
                 const int i = p - 12;
@@ -236,8 +227,27 @@ k_p6_esc(const int8_t *__restrict__ codes, uint32_t out_f, uint32_t in_f, uint32
 }
 
 // ---------------------------------------------------------------- decode ----
+// A lane's plane words with the last four pairs put together: word j of u holds pair 4 j at bits 0 / 16 and 4 j + 1 at 6 / 22, of v
+// 4 j + 2 and 4 j + 3 (the other bits are anything).
+__device__ __forceinline__ void p6_pair_words(const uint4 &a, const uint2 &b, uint32_t (&u)[4], uint32_t (&v)[4])
+{
+    u[0] = a.x; u[1] = a.z; u[2] = b.x;
+    v[0] = a.y; v[1] = a.w; v[2] = b.y;
+    u[3] = p6_and_or(b.x >> 8, 0x00300030u, (a.x >> 12) & 0x000F000Fu) | p6_and_or(b.x >> 4, 0x0C000C00u, (a.y >> 6) & 0x03C003C0u);
+    v[3] = p6_and_or(b.y >> 8, 0x00300030u, (a.z >> 12) & 0x000F000Fu) | p6_and_or(b.y >> 4, 0x0C000C00u, (a.w >> 6) & 0x03C003C0u);
+}
+// the fields at bits 0 / 16 of u and v as four codes, the bytes of a word
+__device__ __forceinline__ uint32_t p6_codes4(uint32_t u, uint32_t v)
+{
+    const uint32_t t = __byte_perm(u & 0x003F003Fu, v & 0x003F003Fu, 0x6420) ^ 0x20202020u, sign = t & 0x20202020u;
+    return t | sign << 1 | sign << 2;
+}
+
 // plane -> int8 codes (OUT 0) or bf16 weights (OUT 1), row major [out_f, in_f]; outliers come out as 0 here.
-// A lane holds four times four consecutive columns of two rows: 4 or 8 bytes per store.
+// A lane holds four times four consecutive columns of two rows: 4 or 8 bytes per store; codes in aligned rows are dealt out over
+// the quad while packed, 16 bytes per store.
+// Codes, with the outliers' pass, in a graph: 17408 x 5120 40.5 us, 12288 x 2048 14.8, 8192 x 8200 39.8; 50.1, 16.9 and 40.5 with
+// four bytes per store and a code at a time; 39.3, 14.4 and 277 on the layout whose lanes held 16 columns.
 template <int OUT>
 __global__ void __launch_bounds__(256) k_p6_decode_plane(P6 p, void *out)
 {
@@ -247,32 +257,44 @@ __global__ void __launch_bounds__(256) k_p6_decode_plane(P6 p, void *out)
     uint32_t R = b / p.kb, kbi = b - R * p.kb;
     float sc = __bfloat162float(p.scale[R * p.scale_stride]);
     const unsigned char *blk = p.plane + (size_t)b * kP6BlockBytes;
-    const uint4 a = ((const uint4 *)blk)[lane];
-    const uint2 a2 = ((const uint2 *)(blk + 512))[lane];
-    uint32_t w[6] = {a.x, a.y, a.z, a.w, a2.x, a2.y};
+    uint32_t u[4], v[4];
+    p6_pair_words(((const uint4 *)blk)[lane], ((const uint2 *)(blk + 512))[lane], u, v);
     const bool vec = (p.in_f & 3u) == 0 && ((uintptr_t)out & (OUT == 0 ? 3u : 7u)) == 0;
+    const bool wide = OUT == 0 && ((p.in_f | (uint32_t)(uintptr_t)out) & 15u) == 0;
+    if (wide) {
+        p6_quad_transpose(u, lane);
+        p6_quad_transpose(v, lane);
+    }
 #pragma unroll
     for (int s = 0; s < 2; ++s) {                    // row g, row g + 8
         const uint32_t row = R * kTileRows + (lane >> 2) + 8 * s;
         if (row >= p.out_f) continue;
+        uint32_t r[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {                // columns col0 + c = pair 4 j + 2 (c >> 1) + s, half c & 1
+        for (int j = 0; j < 4; ++j) r[j] = p6_codes4(u[j] >> 6 * s, v[j] >> 6 * s);
+        if (wide) {                                  // columns 16 (lane & 3) .. + 15
+            const uint32_t col0 = kbi * kTileCols + 16 * (lane & 3);
+            if (col0 < p.in_f) *(uint4 *)((int8_t *)out + (size_t)row * p.in_f + col0) = make_uint4(r[0], r[1], r[2], r[3]);
+            continue;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {                // columns col0 .. col0 + 3
             const uint32_t col0 = kbi * kTileCols + 16 * j + 4 * (lane & 3);
-            uint32_t r[2] = {0u, 0u};
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const int code = p6_code(p6_get(w, 4 * j + 2 * (c >> 1) + s, c & 1));
-                if (OUT == 0) r[0] |= (uint32_t)(code & 0xff) << (8 * c);
-                else r[c >> 1] |= (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn((float)code * sc)) << (16 * (c & 1));
-            }
             const size_t o = (size_t)row * p.in_f + col0;
+            uint32_t w[2];
+            if (OUT == 1) {
+#pragma unroll
+                for (int k = 0; k < 2; ++k)
+                    w[k] = (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn((float)(int8_t)(r[j] >> 16 * k) * sc)) |
+                           (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn((float)(int8_t)(r[j] >> (16 * k + 8)) * sc)) << 16;
+            }
             if (vec && col0 < p.in_f) {
-                if (OUT == 0) *(uint32_t *)((char *)out + o) = r[0];
-                else *(uint2 *)((char *)out + 2 * o) = make_uint2(r[0], r[1]);
+                if (OUT == 0) *(uint32_t *)((char *)out + o) = r[j];
+                else *(uint2 *)((char *)out + 2 * o) = make_uint2(w[0], w[1]);
             } else {
                 for (uint32_t c = 0; c < 4u && col0 + c < p.in_f; ++c) {
-                    if (OUT == 0) ((int8_t *)out)[o + c] = (int8_t)((r[0] >> (8 * c)) & 0xff);
-                    else ((uint16_t *)out)[o + c] = (uint16_t)((r[c >> 1] >> (16 * (c & 1))) & 0xffff);
+                    if (OUT == 0) ((int8_t *)out)[o + c] = (int8_t)((r[j] >> (8 * c)) & 0xff);
+                    else ((uint16_t *)out)[o + c] = (uint16_t)((w[c >> 1] >> (16 * (c & 1))) & 0xffff);
                 }
             }
         }
@@ -550,10 +572,8 @@ __global__ void __launch_bounds__(256, 8) k_p6_decode_bf16(P6 p, __nv_bfloat16 *
     const int32_t lo = __ldg(p.blk_off + b), hi = __ldg(p.blk_off + b + 1);
     const uint32_t R = b / p.kb, kbi = b - R * p.kb;
     const uint32_t s2 = p6_scale2(p.scale[R * p.scale_stride]);
-    // word j of u: pairs 4 j and 4 j + 1 of the lane (bits 0 / 16 and 6 / 22, as in words 0 .. 5), of v: 4 j + 2 and 4 j + 3
-    uint32_t u[4] = {a.x, a.z, a2.x, 0u}, v[4] = {a.y, a.w, a2.y, 0u};
-    u[3] = p6_and_or(a2.x >> 8, 0x00300030u, (a.x >> 12) & 0x000F000Fu) | p6_and_or(a2.x >> 4, 0x0C000C00u, (a.y >> 6) & 0x03C003C0u);
-    v[3] = p6_and_or(a2.y >> 8, 0x00300030u, (a.z >> 12) & 0x000F000Fu) | p6_and_or(a2.y >> 4, 0x0C000C00u, (a.w >> 6) & 0x03C003C0u);
+    uint32_t u[4], v[4];
+    p6_pair_words(a, a2, u, v);
     p6_quad_transpose(u, lane);
     p6_quad_transpose(v, lane);
     uint32_t f[16];                                  // row g and row g + 8, columns 16 (lane & 3) .. + 15
