@@ -82,6 +82,21 @@ static cudaError_t opt_in_smem(K kernel, bool (&done)[64], int bytes)
     return cudaSuccess;
 }
 
+// CTAs of a kernel without dynamic shared memory that fit an SM of the current device, looked up once per instantiation and device
+template <class K>
+static cudaError_t ctas_per_sm(K kernel, int threads, std::atomic<int> (&known)[64], int *ctas)
+{
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+    *ctas = known[dev].load(std::memory_order_relaxed);
+    if (*ctas) return cudaSuccess;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctas, kernel, threads, 0);
+    if (e == cudaSuccess) known[dev].store(*ctas = std::max(1, *ctas), std::memory_order_relaxed);
+    return e;
+}
+
 static int to_streams(const ixb_packed *w, Streams *s)
 {
     if (!w) return fail(IXB_E_ARG, "packed tensor is NULL");
@@ -1449,24 +1464,38 @@ static cudaError_t launch_attn(int64_t hq, int64_t hkv, int64_t splits, cudaStre
     auto ctas = [&](int64_t groups) {
         return (unsigned)std::max<int64_t>(1, std::min<int64_t>(splits, (2 * num_sms() + groups * batch - 1) / (groups * batch)));
     };
-    // One CTA for all parts of a group and sequence from where there are 240 of them: 16 / 8 heads of 128, sequences of 150 to
-    // 300 and of 500 to 1000 positions, many CTAs against one, us: 192 of them (24 sequences) 19.0 / 15.8 and 37.6 / 43.9, 240
-    // 22.6 / 17.2 and 47.6 / 47.9, 320 26.8 / 18.9 and 65 / 52, 1024 69 / 40 and 163 / 115; of 3000 positions 115 / 115 for 240
-    // and 161 / 123 for 320.  Not eight heads to a group: too many registers for two CTAs of 64 (240 of 3000 positions:
-    // 173 / 185).
-    auto local = [&](int64_t groups, int64_t g) { return join.tickets && g < 8 && groups * batch >= 240; };
+    // kAttnOne from where the groups of all sequences fill the chip without being cut: from two per SM on, what the form with many
+    // CTAs has beside one another, or from 240 on where that form's registers leave room for one CTA only.  16 / 8 heads of 128,
+    // many CTAs against one, us, for sequences of 150 to 300 / 500 to 1000 / 1500 to 3000 positions: 192 groups 15.1 / 13.7,
+    // 32.6 / 38.3, 77 / 92; 288 19.0 / 15.8, 36.7 / 42.7, 87 / 101; 304 19.7 / 16.7, 47.5 / 46.7, 126 / 112; 512 24.7 / 23.3,
+    // 60 / 63, 156 / 155; 1024 46 / 37, 110 / 103, 288 / 253.  16 / 4 heads of 128 (one CTA an SM): 192 23.4 / 19.2, 50 / 53,
+    // 124 / 124; 240 28.7 / 19.2, 63 / 55, 157 / 128.  Not heads of 256 (6 / 2 heads, 304 groups 39 / 43, 101 / 109, 263 / 287),
+    // nor eight heads to a group: too many registers.
+    // kAttnMany instead of kAttnWide where the grid has more CTAs than there are SMs and two of them fit one.  (Asked only then: the
+    // question makes the driver load that form, and where it lay among a step's kernels cost the step of one sequence 0.6 %.)
 #define IXB_ATTN(G)                                                                                                            \
     do {                                                                                                                       \
-        const bool one = local(hq / G, G);                                                                                     \
-        constexpr bool LOCAL = G < 8;                                                                                          \
-        const size_t ring = one && D <= 128 ? 2u * (D / 32 + (size_t)kAttnChunk * D / 2048) * 4096u : 0u;                      \
-        if (ring) {                                                                                                            \
+        constexpr AttnForm ONE = D <= 128 && G < 8 ? kAttnOne : kAttnWide;                                                     \
+        const int64_t groups = hq / G, pairs = groups * batch;                                                                 \
+        unsigned cut = ctas(groups);                                                                                           \
+        int per_sm = 1;                                                                                                        \
+        if (pairs * cut > num_sms()) {                                                                                         \
+            static std::atomic<int> known[64];                                                                                 \
+            const cudaError_t oc = ctas_per_sm(k_attn_decode<D, G, kAttnMany>, 256, known, &per_sm);                           \
+            if (oc != cudaSuccess) return oc;                                                                                  \
+        }                                                                                                                      \
+        const bool one = ONE == kAttnOne && join.tickets && pairs >= (per_sm > 1 ? 2 * num_sms() : 240);                       \
+        if (one) cut = 1u;                                                                                                     \
+        const size_t ring = one ? 2u * (D / 32 + (size_t)kAttnChunk * D / 2048) * 4096u : 0u;                                  \
+        if (one) {                                                                                                             \
             static bool attr_set[64] = {false};                                                                                \
-            const cudaError_t oe = opt_in_smem(k_attn_decode<D, G, LOCAL>, attr_set, (int)ring);                               \
+            const cudaError_t oe = opt_in_smem(k_attn_decode<D, G, ONE>, attr_set, (int)ring);                                 \
             if (oe != cudaSuccess) return oe;                                                                                  \
         }                                                                                                                      \
-        return launch_glue_smem(one ? k_attn_decode<D, G, LOCAL> : k_attn_decode<D, G, false>,                                 \
-                                dim3((unsigned)(hq / G), one ? 1u : ctas(hq / G), (unsigned)batch), dim3(256), ring, st,       \
+        return launch_glue_smem(one          ? k_attn_decode<D, G, ONE>                                                        \
+                                : per_sm > 1 ? k_attn_decode<D, G, kAttnMany>                                                  \
+                                             : k_attn_decode<D, G, kAttnWide>,                                                 \
+                                dim3((unsigned)groups, cut, (unsigned)batch), dim3(256), ring, st,                             \
                                 (const __nv_bfloat16 *)q, (const __nv_bfloat16 *)k_cache, (const __nv_bfloat16 *)v_cache, pos, \
                                 (float *)scratch, (uint32_t)hq, (uint32_t)hkv, scale, (uint32_t)q_stride, (size_t)batch_stride,\
                                 (uint32_t)splits, (uint32_t)max_seq, join);                                                    \

@@ -346,16 +346,21 @@ __device__ __forceinline__ uint32_t attn_parts(uint32_t n_ctx, uint32_t splits)
 {
     return min(splits, (n_ctx + kAttnChunk - 1u) / kAttnChunk);
 }
-// LOCAL: one CTA per group and sequence takes all of its parts.  Their sums stay in shared memory (as many as six kilobytes
+// Three forms with the same sums in the same order, so the same bits (launch_attn has the rule and what it was measured on):
+// kAttnWide  the grid has at most a CTA for every SM, which may have all registers: everything a chunk needs is in flight at once.
+//            16 / 8 heads of 128, one sequence of 1100 positions: 5.5 us a launch, 6.2 with two CTAs' registers.
+// kAttnMany  more CTAs than SMs: registers as they fall (two CTAs an SM for most sizes).  Five rows of 705 positions verified 9.7
+//            us, 11.6 with one CTA's registers; eight sequences of 500 to 1000 positions 15 and 18.5.
+// kAttnOne   (heads of 64 and 128) one CTA per group and sequence takes all of its parts.  Their sums stay in shared memory (as many as six kilobytes
 // hold; the rest go through the scratch) and nothing is published: the same sums in the same order as by many CTAs, so the same
 // bits.  Bound by the chain of a chunk, not by its bytes (a fifth to a half of the copy rate), so three CTAs of an SM run it
-// side by side.  Heads of 64 and 128 have two chunks in flight through shared memory, a thread's own pieces (nobody else reads
+// side by side.  Two chunks are in flight through shared memory, a thread's own pieces (nobody else reads
 // them, so no barrier waits for them); the warps' sums take the place of the chunk that was taken last, without which only two
-// CTAs fit.  Forty sequences of 150 to 300 positions, 16 / 8 heads of 128: 26.8 us by many CTAs, 17.9 with the next chunk in
-// registers, 18.9 with two in shared memory; of 500 to 1000 positions 65, 49 and 52, and thirty of them 48, 49 and 48.  (One
-// running softmax over all chunks instead of parts: 14.7 and 38, but other bits than the sequence's own.)
+// CTAs fit.  Forty sequences of 150 to 300 positions, 16 / 8 heads of 128: 20.9 us by many CTAs, 17.7 so; of 500 to 1000 positions
+// 49 and 48.  (One running softmax over all chunks instead of parts: 14.7 and 38, but other bits than the sequence's own.)
+enum AttnForm { kAttnWide, kAttnMany, kAttnOne };
 __host__ __device__ constexpr int attn_keep(int d, int g) { return 1536 / (g * d) > 0 ? 1536 / (g * d) : 1; }
-__host__ __device__ constexpr int attn_local_ctas(int d, int g) { return g * d <= 256 ? 3 : g * d <= 512 ? 2 : 1; }       // per SM: registers
+__host__ __device__ constexpr int attn_one_ctas(int d, int g) { return g * d <= 256 ? 3 : g * d <= 512 ? 2 : 1; }       // per SM: registers
 struct AttnJoin {
     uint32_t *tickets;
     __nv_bfloat16 *out;
@@ -363,8 +368,8 @@ struct AttnJoin {
     uint32_t gate_stride, gate_row_stride;
 };
 
-template <int D, int G, bool LOCAL>
-__global__ void __launch_bounds__(256, LOCAL ? attn_local_ctas(D, G) : 1)
+template <int D, int G, AttnForm FORM>
+__global__ void __launch_bounds__(256, FORM == kAttnOne ? attn_one_ctas(D, G) : FORM == kAttnWide ? 1 : 0)     // 0: no minimum
 k_attn_decode(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat16 *__restrict__ k_cache,
               const __nv_bfloat16 *__restrict__ v_cache, const int32_t *pos, float *part, uint32_t hq, uint32_t hkv,
               float scale, uint32_t q_stride, size_t batch_stride, uint32_t splits, uint32_t max_seq, AttnJoin join)
@@ -390,16 +395,17 @@ k_attn_decode(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat16 *__restri
     static_assert(PG * G * D <= NR * HG * D && NW <= NR, "sums of the join fit");
     __shared__ __align__(16) float sm_q[G][D];         // scaled queries
     __shared__ float sm_s[G][C], sm_c[G];              // a chunk's scores, then weights; the sums' rescaling
-    constexpr bool RING = LOCAL && D <= 128;
-    __shared__ __align__(16) float sm_acc_own[RING ? 1 : NR * HG * D];
+    constexpr bool ONE = FORM == kAttnOne;
+    static_assert(!ONE || D <= 128, "two chunks of 256 dimensions do not fit beside one another");
+    __shared__ __align__(16) float sm_acc_own[ONE ? 1 : NR * HG * D];
     __shared__ float sm_w[G][kAttnMaxSplits], sm_sum[G];
     __shared__ uint32_t sm_last;
-    constexpr int KEEP = LOCAL ? attn_keep(D, G) : 1;
-    __shared__ __align__(16) float sm_part[LOCAL ? KEEP : 1][LOCAL ? G * D : 4];
-    __shared__ float2 sm_ml[LOCAL ? G : 1][KEEP];
+    constexpr int KEEP = ONE ? attn_keep(D, G) : 1;
+    __shared__ __align__(16) float sm_part[ONE ? KEEP : 1][ONE ? G * D : 4];
+    __shared__ float2 sm_ml[ONE ? G : 1][KEEP];
     extern __shared__ __align__(16) uint4 sm_ring[];   // [2][KC + VP][256 threads]
     // the warps' sums: [NR][HG][D], with a ring in the half of the chunk that was taken last
-    static_assert(!RING || NR * HG * D * 4 <= (KC + VP) * 4096, "fits");
+    static_assert(!ONE || NR * HG * D * 4 <= (KC + VP) * 4096, "fits");
     float *sm_acc = sm_acc_own;
     auto acc_at = [&](int w, int h, int d) -> float & { return sm_acc[(w * HG + h) * D + d]; };
     asm volatile("griddepcontrol.launch_dependents;");
@@ -413,7 +419,7 @@ k_attn_decode(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat16 *__restri
     const __nv_bfloat16 *kb = k_cache + (size_t)kvh * D + kt * 8, *vb = v_cache + (size_t)kvh * D + vd;
     const uint32_t last = (uint32_t)pos[0];
     uint4 kr[KC], vr[VP];
-    const uint32_t ring = RING ? (uint32_t)__cvta_generic_to_shared(sm_ring) + tid * 16u : 0u;
+    const uint32_t ring = ONE ? (uint32_t)__cvta_generic_to_shared(sm_ring) + tid * 16u : 0u;
     uint32_t visit = 0;                                // chunks taken so far; even ones lie in the first half of the ring
     auto piece = [&](uint32_t i, int j) { return ring + ((i & 1u) * (KC + VP) + j) * 4096u; };
     auto request = [&](uint32_t c, uint32_t i, uint32_t limit) {       // chunk c as the i-th to be taken
@@ -448,8 +454,8 @@ k_attn_decode(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat16 *__restri
         }
         join.out[((size_t)blockIdx.z * hq + head0 + h) * D + d] = __float2bfloat16_rn(o);
     };
-    if (RING) {
-        request(0u, 0u, max_seq - 1u);                 // (LOCAL has max_seq)
+    if (ONE) {
+        request(0u, 0u, max_seq - 1u);                 // (ONE has max_seq)
     } else if (max_seq) {
         fetch_k(blockIdx.y, max_seq - 1u);
         fetch_v(blockIdx.y, max_seq - 1u);
@@ -461,7 +467,7 @@ k_attn_decode(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat16 *__restri
             join.out[((size_t)blockIdx.z * hq + head0 + i / D) * D + i % D] = __float2bfloat16_rn(__int_as_float(0x7FFFFFFF));
     }
     if (blockIdx.y >= used) {
-        if (RING) cp_async_wait<0>();
+        if (ONE) cp_async_wait<0>();
         return;
     }
     uint32_t ps = 0, pc = 0;                           // part and chunk requested last
@@ -470,7 +476,7 @@ k_attn_decode(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat16 *__restri
         if (ps < used) request(pc, i, n_ctx - 1u);
         else cp_async_commit();
     };
-    if (RING) request_next(1u);
+    if (ONE) request_next(1u);
     __syncthreads();
     if (!max_seq) {
         fetch_k(blockIdx.y, n_ctx - 1u);
@@ -490,7 +496,7 @@ k_attn_decode(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat16 *__restri
             float sc[G];
 #pragma unroll
             for (int h = 0; h < G; ++h) sc[h] = 0.f;
-            if (RING) {
+            if (ONE) {
                 cp_async_wait<1>();                    // the chunk is there, the next one may be on its way
 #pragma unroll
                 for (int j = 0; j < KC; ++j) kr[j] = taken(piece(visit, j));
@@ -506,7 +512,7 @@ k_attn_decode(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat16 *__restri
                     sc[h] = fmaf(kf[7], q1.w, fmaf(kf[6], q1.z, fmaf(kf[5], q1.y, fmaf(kf[4], q1.x, sc[h]))));
                 }
             }
-            if (!RING && ahead) fetch_k(nxt, n_ctx - 1u);
+            if (!ONE && ahead) fetch_k(nxt, n_ctx - 1u);
             const bool live = c * kAttnChunk + kp < n_ctx;
 #pragma unroll
             for (int h = 0; h < G; ++h) {
@@ -539,7 +545,7 @@ k_attn_decode(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat16 *__restri
 #pragma unroll
             for (int j = 0; j < VP; ++j) {
                 float vf[8];
-                if (RING) vr[j] = taken(piece(visit, KC + j));
+                if (ONE) vr[j] = taken(piece(visit, KC + j));
                 unpack8(vr[j], vf);
                 if (c * kAttnChunk + vg + j * VG >= n_ctx) continue;       // (not read, or rows beyond the position)
 #pragma unroll
@@ -549,22 +555,22 @@ k_attn_decode(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat16 *__restri
                     for (int k = 0; k < 8; ++k) acc[h][k] = fmaf(p, vf[k], acc[h][k]);
                 }
             }
-            if (!RING && ahead) fetch_v(nxt, n_ctx - 1u);
-            if (RING && more) {
+            if (!ONE && ahead) fetch_v(nxt, n_ctx - 1u);
+            if (ONE && more) {
                 request_next(visit + 2u);              // into the pieces that this thread has just taken
                 ++visit;
             }
             if (more) __syncthreads();                 // the weights are read: the next chunk's scores may follow
         }
         // join: the warp's groups of threads by shuffles, the warps in shared memory, HG heads at a time
-        if (RING) {
+        if (ONE) {
             sm_acc = (float *)(sm_ring + (visit & 1u) * (KC + VP) * 256u);
             __syncthreads();                           // nobody takes pieces of it any more
         }
         float *dst = part + ((size_t)head0 * splits + s) * D;
 #pragma unroll
         for (int h0 = 0; h0 < G; h0 += HG) {
-            if (h0 || (!RING && s != blockIdx.y)) __syncthreads();  // sm_acc is free
+            if (h0 || (!ONE && s != blockIdx.y)) __syncthreads();  // sm_acc is free
 #pragma unroll
             for (int hh = 0; hh < HG; ++hh) {
                 if (h0 + hh >= G) break;
@@ -583,29 +589,29 @@ k_attn_decode(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat16 *__restri
                 float a = 0.f;
 #pragma unroll
                 for (int w = 0; w < NW; ++w) a += acc_at(w, i / D, i % D);
-                if (LOCAL && s < (uint32_t)KEEP) sm_part[s][h0 * D + i] = a;
+                if (ONE && s < (uint32_t)KEEP) sm_part[s][h0 * D + i] = a;
                 else dst[(size_t)(h0 + i / D) * splits * D + i % D] = a;
             }
         }
-        if (RING && s + 1u < used) {
+        if (ONE && s + 1u < used) {
             __syncthreads();                           // the sums are read
             request_next(visit + 2u);
             ++visit;
         }
         if (wid < G && lane == 0) {
-            if (LOCAL && s < (uint32_t)KEEP) sm_ml[wid][s] = make_float2(M, L);
+            if (ONE && s < (uint32_t)KEEP) sm_ml[wid][s] = make_float2(M, L);
             else part_ml[(size_t)(head0 + wid) * splits + s] = make_float2(M, L);
         }
     }
-    if (!LOCAL && !join.tickets) return;
+    if (!ONE && !join.tickets) return;
     // ---- the last CTA of the group joins the parts.  The CTAs with work add numbers whose sum is zero to the ticket, the first
     // one 1 - ctas and the others 1: it is zero again exactly when all of them have come.  So nobody resets it, and it is zero
     // after launches that overlapped too (whose own results are lost).
     const uint32_t ctas = min(gridDim.y, used);
     uint32_t *ticket = join.tickets + (size_t)blockIdx.z * gridDim.x + blockIdx.x;
-    if (!LOCAL) __threadfence();                       // this thread's share of the parts, before the ticket
+    if (!ONE) __threadfence();                       // this thread's share of the parts, before the ticket
     __syncthreads();
-    if (!LOCAL && ctas > 1u) {
+    if (!ONE && ctas > 1u) {
         const uint32_t mine = blockIdx.y ? 1u : 1u - ctas;
         if (threadIdx.x == 0) sm_last = atomicAdd(ticket, mine) + mine == 0u;
         __syncthreads();
@@ -615,11 +621,11 @@ k_attn_decode(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat16 *__restri
     // all of the group's sums are requested at once, as far as registers go: a thread takes four dimensions of a head and
     // every PG-th part (rounds of eight dependent loads of one value: 29 us a launch at a 4097-token context, not 16.5)
     constexpr int MAXQ = (QD + 255) / 256;             // quads per thread
-    constexpr int UN = LOCAL ? 1 : 16;
+    constexpr int UN = ONE ? 1 : 16;
     const int pg = QD >= 256 ? 0 : tid / QD, q0 = QD >= 256 ? tid : tid % QD;
     float4 first[UN];
     auto sums = [&](int qd, uint32_t s) -> float4 {
-        if (LOCAL && s < (uint32_t)KEEP) return *(const float4 *)&sm_part[s][qd * 4];
+        if (ONE && s < (uint32_t)KEEP) return *(const float4 *)&sm_part[s][qd * 4];
         return __ldcg((const float4 *)(part + ((size_t)(head0 + qd * 4 / D) * splits + s) * D + qd * 4 % D));
     };
 #pragma unroll
@@ -629,7 +635,7 @@ k_attn_decode(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat16 *__restri
     }
     if (wid < G) {                                     // a warp per head: the parts' weights and their sum
         const float2 *p = part_ml + (size_t)(head0 + wid) * splits;
-        auto max_sum = [&](uint32_t s) { return LOCAL && s < (uint32_t)KEEP ? sm_ml[wid][s] : __ldcg(p + s); };
+        auto max_sum = [&](uint32_t s) { return ONE && s < (uint32_t)KEEP ? sm_ml[wid][s] : __ldcg(p + s); };
         float mx = -INFINITY, sum = 0.f;
         for (uint32_t s = lane; s < used; s += 32) mx = fmaxf(mx, max_sum(s).x);
 #pragma unroll

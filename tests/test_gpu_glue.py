@@ -138,14 +138,16 @@ def test_attn_decode_parts(hq, hkv, d, splits, ctx):
     assert not bool(one.tickets.any())
 
 
+@pytest.mark.parametrize("groups", [40, 200, 240, 300])
 @pytest.mark.parametrize("hq,hkv,d,splits", [(2, 1, 64, 18), (16, 8, 128, 18), (16, 8, 128, 3), (12, 4, 128, 65), (16, 4, 128, 9),
                                              (12, 2, 64, 18), (3, 3, 128, 1), (6, 2, 256, 9), (8, 2, 256, 2)])
-def test_attn_decode_one_cta_per_group(hq, hkv, d, splits):
-    """So many sequences that one CTA takes all parts of a group: no position (NaN), one, the edges of a chunk and of a part,
-    more parts than are kept in shared memory, the whole cache.  Each sequence has the bits that it has alone."""
+def test_attn_decode_one_cta_per_group(hq, hkv, d, splits, groups):
+    """From a few sequences to so many that one CTA takes all parts of a group, through all forms of the kernel: no position
+    (NaN), one, the edges of a chunk and of a part, more parts than are kept in shared memory, the whole cache.  Each sequence has
+    the bits that it has alone."""
     from ixrun_b200.glue import AttnDecode
 
-    dev, max_seq, b = "cuda", 1300, -(-240 // hkv)
+    dev, max_seq, b = "cuda", 1300, -(-groups // hkv)
     gen = torch.Generator(device=dev).manual_seed(hq)
     kc = torch.randn(b, max_seq, hkv, d, generator=gen, device=dev).bfloat16()
     vc = torch.randn(b, max_seq, hkv, d, generator=gen, device=dev).bfloat16()
@@ -161,7 +163,7 @@ def test_attn_decode_one_cta_per_group(hq, hkv, d, splits):
     for g in (None, gate):
         out = many(q, kc, vc, pos, gate=g, gate_row_stride=hq * d if g is not None else 0)
         assert not bool(many.tickets.any())
-        for r in list(range(len(edges))) + [b - 1]:
+        for r in [*range(min(b, len(edges))), b - 1]:
             alone = one(q[r], kc[r], vc[r], pos[r:r + 1], gate=None if g is None else g[r])
             assert torch.equal(alone.view(torch.int16), out[r].view(torch.int16))
 
