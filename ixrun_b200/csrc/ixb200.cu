@@ -1807,14 +1807,14 @@ static int pu_rooms(const int **rooms)
     *rooms = table[dev].n;
     return IXB_OK;
 }
-// K splits (CTAs of a cluster): the least time, counted in column blocks (0.255 us each).  Beside its blocks a launch takes 2, or
-// 4 + splits where sums are joined; and where it fills more than 0.43 of the places for its clusters, up to 18 more, because the
-// launch behind it then finds no room to begin in (dependent launches in a graph).  Fitted to fourteen layers of 320 x 512 to
-// 17408 x 17408, 1 to 16 splits each: the choice is within 0.2 us of the best everywhere.  Without dependent launches a launch
-// takes about 20 blocks longer whatever it fills (5000 x 2176, 23 rows: 2 splits 10.9 us, 3 10.1; dependent 8.1 and 8.3).
+// K splits (CTAs of a cluster): the least time, counted in column blocks (0.27 us each).  Beside its blocks a launch takes 2, or
+// 4 + splits where sums are joined, 10 for each of several rounds; and where it fills more than half of the places for its clusters,
+// 5 to 10, because the launch behind it then finds no room to begin in.  For dependent launches, as captured steps make them:
+// the best choice within 0.1 us on eighteen layers of 320 x 512 to 17408 x 17408 with 16 and 64 rows, 1 to 16 splits each.  Launches
+// that do not overlap would rather have more splits on the small ones (4096 x 2048: 2 splits 6.0 us dependent and 10.1 alone, 4 7.2
+// and 7.9), but a plan that looked at the switch gave a layer other bits in a captured step than in a call.
 static int pu_plan(uint32_t rt, uint32_t kb, uint32_t *splits)
 {
-    const bool dependent = g_p6_pdl.load() != 0;
     const uint32_t groups = (rt + kPuTiles - 1) / kPuTiles;
     const int *rooms;
     const int rc = pu_rooms(&rooms);
@@ -1824,9 +1824,8 @@ static int pu_plan(uint32_t rt, uint32_t kb, uint32_t *splits)
         if (rooms[s] <= 0) continue;
         const uint32_t room = (uint32_t)rooms[s], rounds = (groups + room - 1) / room;
         const float used = (float)groups / (float)room;
-        const float blocks = (float)(rounds * ((kb + s - 1) / s));
-        const float cost = dependent ? blocks + (s == 1u ? 2.f : 4.f + (float)s) + (rounds > 1u ? 10.f * (float)rounds : used > 0.43f ? 31.f * (used - 0.43f) : 0.f)
-                                     : blocks + (s == 1u ? 0.f : 5.f) + 20.f * (float)(rounds - 1u);
+        const float cost = (float)(rounds * ((kb + s - 1) / s)) + (s == 1u ? 2.f : 4.f + (float)s) +
+                           (rounds > 1u ? 10.f * (float)rounds : used > 0.5f ? 10.f * used : 0.f);
         if (best == 0.f || cost < best) {
             best = cost;
             *splits = s;

@@ -22,7 +22,7 @@ def set_pdl(on: bool) -> bool:
     """Programmatic dependent launch for the P6 GEMV (process-wide; returns the previous setting).
 
     When on, a GEMV launch may begin fetching its weights while the kernel ahead of it in the stream finishes; it
-    still waits for that kernel before touching activations, output or scratch.  Turn it on after deployment, once
+    still waits for that kernel before touching activations, output or scratch.  Results do not depend on it.  Turn it on after deployment, once
     the device has been synchronised: a layout still being built would be read too early."""
     return bool(_lib.lib().ixb_set_pdl(1 if on else 0))
 

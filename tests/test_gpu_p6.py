@@ -487,3 +487,40 @@ def test_p6_rows_behind_a_kernel_that_takes_long(out_f, in_f, m):
         set_pdl(before)
     ref = x.double() @ (codes.float() * p6.scale.float()).bfloat16().double().t()
     assert float((alone.double() - ref).abs().max() / ref.abs().max()) < 2e-5
+
+
+@pytest.mark.parametrize("m", [9, 23, 48, 64])
+@pytest.mark.parametrize("out_f,in_f", [(4096, 2048), (2048, 6144), (1024, 5120), (640, 1536), (320, 512), (8224, 200)])
+def test_p6_rows_have_the_same_bits_with_dependent_launches(out_f, in_f, m):
+    """9..64 rows called one by one, with dependent launches and in a captured chain of them: the same bits of every layer,
+    whatever its K splits; the second launch of the chain reads what the first one wrote.  (9 rows: hardly an outlier a block,
+    the other kernel than at 23.)"""
+    from ixrun_b200.p6 import P6Packed, set_pdl
+
+    gen = torch.Generator(device="cuda").manual_seed(out_f + m)
+    codes = (torch.randn(out_f, in_f, generator=gen, device="cuda") * (8 if m == 9 else 12)).round().clamp(-127, 127).to(torch.int8)
+    a = P6Packed(codes, torch.tensor(0.007, dtype=torch.bfloat16), out_f, in_f)
+    b = P6Packed(codes.t().contiguous(), torch.tensor(0.004, dtype=torch.bfloat16), in_f, out_f)
+    x = torch.randn(m, in_f, generator=gen, device="cuda").bfloat16()
+    call = (lambda p, t: p.gemm(t)) if in_f % 64 == 0 else (lambda p, t: p.rows(t))
+    h = call(a, x)
+    y = call(b, h)
+    torch.cuda.synchronize()
+    before = set_pdl(True)
+    try:
+        h1 = call(a, x)
+        y1 = call(b, h1)
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            for _ in range(3):
+                h2 = call(a, x)
+                y2 = call(b, h2)
+        graph.replay()
+        torch.cuda.synchronize()
+    finally:
+        set_pdl(before)
+    for got in (h1, h2):
+        assert torch.equal(got, h)
+    for got in (y1, y2):
+        assert torch.equal(got, y)
