@@ -1775,7 +1775,6 @@ static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder()
     return fn;
 }
 
-constexpr int kPuMaxSplits = 16;                         // CTAs of a cluster (above 8 by opt-in)
 // clusters of 1 .. kPuMaxSplits CTAs that run at once on the current device (0: none of that size), and the kernel made ready
 static int pu_rooms(const int **rooms)
 {

@@ -5,8 +5,8 @@
 //   Y[t][n] = sum_k X[t][k] * bf16(code[n][k] * scale)        t < m_tok <= NTOK
 //
 //   CTA      = 128 weight rows (8 row tiles, the MMA's M) x a contiguous range of column blocks; K is split over the CTAs of a
-//              cluster as far as it takes to fill the chip, and the splits' sums are added in rank order through distributed
-//              shared memory: no scratch, no second launch, reproducible.
+//              cluster as far as it takes to fill the chip, and the splits' sums are added in pairs, pairs of pairs and so on
+//              through distributed shared memory: no scratch, no second launch, reproducible.
 //   stage    = two column blocks (128 k): the packed weights of 8 row tiles arrive by one three-dimensional TMA copy (eight
 //              stages ahead), the activations [tokens rounded up to 16] by one two-dimensional copy per block (four stages,
 //              rows of 128 bytes, 128-byte swizzle); the converted weights are 64 columns of tensor memory (four stages).
@@ -43,6 +43,7 @@ namespace ixb {
 constexpr int kPuTiles = 8;                              // row tiles per CTA
 constexpr int kPuRows = kPuTiles * kTileRows;            // 128, the MMA's M
 constexpr int kPuMaxRows = 64;
+constexpr int kPuMaxSplits = 16;                         // CTAs of a cluster (above 8 by opt-in)
 constexpr int kPuPhases = 3;                             // converter warps per row tile
 constexpr int kPuConv = kPuTiles * kPuPhases;            // warps 0..23
 constexpr int kPuMmaWarp = kPuConv;                      // 24
@@ -59,7 +60,8 @@ constexpr int kPuRedPitch = kPuRows + 4;                 // floats of one token 
 constexpr int32_t kPuEntries = 128;                      // outlier entries of its run that a converter warp stages
 
 // Column block b adds into accumulator b % pu_accs: the tensor core cuts the low bits of what it adds to a large sum, so many
-// short chains lose less than one long one.
+// short chains lose less than one long one.  They are joined in pairs for the same reason: 2-norm error of fp32 outputs against 64
+// bits, one after the other / in pairs, 300 x 16384 (16 splits) 0.86e-7 / 0.65e-7, 2048 x 6144 with 16 rows 0.60e-7 / 0.55e-7.
 __host__ __device__ __forceinline__ uint32_t pu_accs(uint32_t n_pad)
 {
     const uint32_t n = 256u / n_pad;
@@ -378,17 +380,39 @@ k_p6_umma(P6 p, const __grid_constant__ CUtensorMap wmap, const __grid_constant_
     // warp: its quarter of the rows (lane = row), every sixth run of eight tokens
     const uint32_t r0 = 32u * quarter + (uint32_t)lane;
     for (uint32_t c0 = ((uint32_t)warp >> 2) * 8u; warp < kPuConv && c0 < m_tok; c0 += (kPuConv / 4) * 8u) {
-        float v[8];
+        // the accumulators in pairs, pairs of pairs and so on (one without a block was never written: zero)
+        const uint32_t accs = min(nk, pu_accs(n_pad));
+        auto load = [&](uint32_t q, uint32_t (&r)[8]) {
+            if (q < accs) {                                             // (uniform)
+                asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                             : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                             : "r"(tmem + ((32u * quarter) << 16) + q * n_pad + c0) : "memory");
+            } else {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = 0.f;
-        for (uint32_t q = 0; q < min(nk, pu_accs(n_pad)); ++q) {        // (an accumulator without a block was never written)
-            uint32_t r[8];
-            asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                         : "r"(tmem + ((32u * quarter) << 16) + q * n_pad + c0) : "memory");
+                for (int j = 0; j < 8; ++j) r[j] = 0u;
+            }
+        };
+        float v[8], four[8];
+#pragma unroll
+        for (uint32_t q = 0; q < 8u; q += 2u) {
+            if (q >= 4u && q >= accs) break;
+            uint32_t a[8], b[8];
+            load(q, a);
+            load(q + 1u, b);
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-            for (int j = 0; j < 8; ++j) v[j] += __uint_as_float(r[j]);
+            for (int j = 0; j < 8; ++j) {
+                asm volatile("" : "+r"(a[j]), "+r"(b[j]));              // (not before the wait)
+                const float two = __uint_as_float(a[j]) + __uint_as_float(b[j]);
+                if (q == 0u) v[j] = two;
+                else if (q == 4u) four[j] = two;
+                else if (q == 2u) v[j] += two;
+                else four[j] += two;
+            }
+        }
+        if (accs > 4u) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[j] += four[j];
         }
 #pragma unroll
         for (uint32_t j = 0; j < 8u; ++j) {
@@ -403,8 +427,20 @@ k_p6_umma(P6 p, const __grid_constant__ CUtensorMap wmap, const __grid_constant_
         pr_cluster_sync();
         for (uint32_t i = split * (uint32_t)kPuThreads + tid; i < m_tok * kPuRows; i += splits * (uint32_t)kPuThreads) {
             const uint32_t m = i / kPuRows, r = i % kPuRows, a = smem0 + (m * kPuRedPitch + r) * 4u;
-            float v = pr_ld_cluster(a, 0);
-            for (uint32_t c = 1; c < splits; ++c) v += pr_ld_cluster(a, c);
+            // the splits in pairs, pairs of pairs and so on (uniform branches: most launches have two to six)
+            auto quad = [&](uint32_t c) {
+                const float v0 = pr_ld_cluster(a, c), v1 = c + 1u < splits ? pr_ld_cluster(a, c + 1u) : 0.f;
+                if (c + 2u >= splits) return v0 + v1;
+                const float v2 = pr_ld_cluster(a, c + 2u), v3 = c + 3u < splits ? pr_ld_cluster(a, c + 3u) : 0.f;
+                return (v0 + v1) + (v2 + v3);
+            };
+            float v = quad(0u);
+            if (splits > 4u) v += quad(4u);
+            if (splits > 8u) {
+                float w = quad(8u);
+                if (splits > 12u) w += quad(12u);
+                v += w;
+            }
             put(m, r, v);
         }
         pr_cluster_sync();                             // no CTA leaves while another reads its sums

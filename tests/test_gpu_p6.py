@@ -524,3 +524,19 @@ def test_p6_rows_have_the_same_bits_with_dependent_launches(out_f, in_f, m):
         assert torch.equal(got, h)
     for got in (y1, y2):
         assert torch.equal(got, y)
+
+
+@pytest.mark.parametrize("m", [9, 32, 64])
+def test_p6_rows_join_many_sums_in_pairs(m):
+    """A layer of few rows and many columns: its fp32 outputs are 64 to 128 partial sums.  A rounding to the nearest has a relative
+    error of 0.25e-7 (2^-23 / sqrt(12), the mantissa's mean 0.72), and so has each of the seven levels of a sum in pairs, as random
+    partial sums keep their 2-norm from level to level: sqrt(7) of it, 0.66e-7.  Two levels' worth more for the short chains in the
+    tensor core; one after the other the sums lose sqrt(12.8) of it."""
+    from ixrun_b200.p6 import P6Packed
+
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    codes = (torch.randn(300, 16384, generator=gen, device="cuda") * 6).round().clamp(-31, 31).to(torch.int8)
+    p6 = P6Packed(codes, torch.tensor(2.0 ** -9, dtype=torch.bfloat16), 300, 16384)
+    x = torch.randn(m, 16384, generator=gen, device="cuda").bfloat16()
+    ref = x.double() @ (codes.double() * 2.0 ** -9).t()
+    assert float((p6.gemm(x, out_dtype=torch.float32).double() - ref).norm() / ref.norm()) < 0.75e-7
