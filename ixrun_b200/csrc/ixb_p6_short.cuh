@@ -6,16 +6,16 @@
 //   CTA   = a contiguous range of whole row tiles, so that nothing is joined across CTAs; 16 warps.
 //   warp  = a contiguous part of K, the same one in every tile of the CTA: its activations are its own (no CTA barrier between
 //           their arrival and the first product) and are fetched once for all tiles.
-//   Ahead of griddepcontrol.wait: the warp's first blocks are in registers, two of them already as weights with their outliers
-//   OR-ed over the placeholders (+0.0) from an image of the lanes' registers in shared memory; further ones are requested kPsAhead
-//   ahead.  Behind it: activations (cp.async), four mma.sync per block, partial tiles to shared memory, one barrier, sums of
+//   Ahead of griddepcontrol.wait: all of the warp's blocks (eight at most, which is what the kernel is taken for) are requested into
+//   registers, two of them are already weights with their outliers OR-ed over the placeholders (+0.0) from an image of the lanes'
+//   registers in shared memory.  Behind it: activations (cp.async), four mma.sync per block, partial tiles to shared memory, one barrier, sums of
 //   the 16 parts by shuffles in a fixed tree, outputs.
 //
 // What bounds it: one chain of latencies: launch, activations from L2, two to eight blocks, the barrier, the sums, the stores.  In a
-// graph with dependent launch, k_p6_mma and this kernel at 1 / 8 rows: 2048 x 2048 5.3 -> 2.9, 7.1 -> 4.1 us; 4096 x 2048 6.0 -> 4.0,
-// 7.7 -> 5.3; 2048 x 6144 6.7 -> 5.0, 8.7 -> 6.7; 1024 x 3072 5.0 -> 2.1, 7.0 -> 3.3.  There, joining the parts of 24 warps through
+// graph with dependent launch, k_p6_mma and this kernel at 1 / 8 rows: 2048 x 2048 5.3 -> 2.9, 7.1 -> 4.2 us; 4096 x 2048 6.0 -> 4.1,
+// 7.7 -> 5.4; 2048 x 6144 6.7 -> 5.0, 8.7 -> 6.7; 1024 x 3072 5.0 -> 2.1, 7.0 -> 3.5.  There, joining the parts of 24 warps through
 // arrival counters took 1.75 us of the 5.3, the outliers' own pass 0.45 at one row and 1.5 at five, the CTA-wide staging of
-// activations the rest.  With more blocks per warp than are requested ahead it is the slower one: 10240 x 2048 (10 blocks) 7.6
+// activations the rest.  With more blocks per warp, the rest requested one by one, it was the slower one: 10240 x 2048 (10 blocks) 7.6
 // and 7.7 us, 9.1 and 10.0; 12288 x 2048 (12) 7.8 and 9.2.
 #pragma once
 #include "ixb_p6.cuh"
@@ -26,7 +26,7 @@ constexpr int kPsWarps = 16;
 constexpr int kPsThreads = kPsWarps * 32;
 constexpr int kPsReady = 2;                              // blocks converted ahead of the dependency wait
 constexpr int kPsAhead = 6;                              // packed blocks in registers behind those
-constexpr uint32_t kPsMaxBlocks = kPsReady + kPsAhead;   // blocks of a warp
+constexpr uint32_t kPsMaxBlocks = kPsReady + kPsAhead;   // blocks of a warp: all are requested at once, none later
 
 struct PsPlan {
     uint32_t grid, tiles, slice;                         // CTAs; most tiles of a CTA; most column blocks of a warp
@@ -171,16 +171,13 @@ k_p6_short(P6 p, const __nv_bfloat16 *__restrict__ x, uint32_t m_rows, const __n
 #pragma unroll
     for (int i = 0; i < kPsReady; ++i)
         if ((uint32_t)i < n) multiply(fr[i]);
-    for (uint32_t i = kPsReady; i < n; i += kPsAhead) {
 #pragma unroll
-        for (uint32_t q = 0; q < (uint32_t)kPsAhead; ++q) {
-            if (i + q >= n) break;
-            fetch_entry(ahead[(q + 2u) % kPsAhead]);     // of the block after the next
-            uint32_t f[16];
-            convert(ahead[q], s_cur, f);
-            fetch(ahead[q]);
-            multiply(f);
-        }
+    for (int q = 0; q < kPsAhead; ++q) {
+        if ((uint32_t)(kPsReady + q) >= n) break;
+        if (q + 2 < kPsAhead) fetch_entry(ahead[q + 2]);  // of the block after the next
+        uint32_t f[16];
+        convert(ahead[q], s_cur, f);
+        multiply(f);
     }
     if (!nk) {                                           // fewer column blocks than warps: zeros
         for (uint32_t i = 0; i < tiles * ps_part(MULTI); i += 32u)
