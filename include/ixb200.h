@@ -225,7 +225,7 @@ int ixb_p6_gemv(const ixb_p6 *t, const void *x_device, int64_t m_rows, const voi
  * fixed order (reproducible).  Takes the place of the reference's decode + dense matmul for 9..64 rows
  * (ixrun/engine.py:171-173; precedent for a fused kernel: ixrun/tpab_gemm.py:34-94).
  * ixb_p6_rows: in_f a multiple of 8, no scratch (splits are joined inside a cluster of CTAs).
- * ixb_p6_gemm: the same for in_f a multiple of 64; a scratch of at least 256 bytes, 256-byte aligned, is asked for (its
+ * ixb_p6_gemm: the same for in_f a multiple of 64; a scratch of 256 bytes, 256-byte aligned, is asked for (its
  *   kernels once kept partial sums there) and left alone.
  * Waits inside the kernels are bounded and count their own work only, not a kernel ahead that they wait for; a launch in which
  * one runs out leaves NaN in its outputs. */

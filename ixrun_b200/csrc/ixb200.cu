@@ -1898,7 +1898,7 @@ static int p6_rows_any(const P6 &p, int64_t n_esc, const void *x, int64_t m_rows
 extern "C" size_t ixb_p6_gemm_scratch_bytes(int64_t out_f, int64_t in_f, int64_t m_rows)
 {
     if (out_f <= 0 || in_f <= 0 || m_rows < 1 || m_rows > kPuMaxRows || out_f * in_f > 800000000LL) return 0;
-    return m_rows <= 32 ? 256 : 512;      // no kernel uses it; more than 32 rows have always been told to bring more than the 256 that are enough
+    return 256;                           // what ixb_p6_gemm asks for; no kernel uses it
 }
 
 extern "C" int ixb_p6_gemm(const ixb_p6 *t, const void *x, int64_t m_rows, const void *bias, void *y, int y_is_f32,
