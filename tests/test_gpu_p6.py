@@ -136,12 +136,13 @@ def test_p6_full_size_against_the_oracle(out_f, in_f):
     assert p6.resident_bytes < 1.2 * dp.total_bytes
 
 
-def test_p6_programmatic_dependent_launch_gives_the_same_result():
+@pytest.mark.parametrize("out_f,in_f", [(512, 5120), (512, 8256), (2400, 5120), (100, 2052)])
+def test_p6_programmatic_dependent_launch_gives_the_same_result(out_f, in_f):
     """Back-to-back launches with programmatic dependent launch on (eagerly and replayed from a CUDA graph):
-    every launch must still see the activations written just before it and produce the bits of a plain launch."""
+    every launch must still see the activations written just before it and produce the bits of a plain launch.  Two layers of few
+    blocks per warp, one of many between such ones, two of many (tiles shared by CTAs), and two whose rows are no multiple of 16 bytes."""
     from ixrun_b200.p6 import set_pdl
 
-    out_f, in_f = 512, 5120
     _, _, a = make(out_f, in_f, 11)
     _, _, b = make(in_f, out_f, 12)
     x = torch.randn(1, in_f, device="cuda").bfloat16()
@@ -297,11 +298,14 @@ def test_p6_gemm_few_row_groups(out_f, in_f, outliers, m):
     assert torch.equal(out, p6.rows(x)) and bool((small == 7).all())
 
 
-@pytest.mark.parametrize("out_f,in_f,dense", [(48, 6464, False), (48, 6464, True), (16, 64, True), (2500, 96, True), (5120, 320, False)])
+@pytest.mark.parametrize("out_f,in_f,dense", [(48, 6464, False), (48, 6464, True), (16, 64, True), (2500, 96, True), (5120, 320, False),
+                                              (48, 16448, False), (48, 16448, True), (2500, 4200, True), (2500, 100, True),
+                                              (5120, 2180, False), (14800, 16448, False)])
 def test_p6_gemv_rows_get_the_bits_they_get_alone(out_f, in_f, dense):
-    """Outliers go through the tensor core 32 at a time for all activation rows: runs of more than 64 blocks, more steps
-    than blocks (every second code an outlier), segments shorter than the pipeline, several row tiles per run; up to 8
-    rows, with activations in shared memory and (wide rows) from global memory.  Against float64 sums of exact products."""
+    """Layers of few blocks per warp (the first five) and of many.  There outliers go through the tensor core 32 at a time for all
+    activation rows: more steps than blocks (every second code an outlier), segments shorter than the pipeline, several row tiles
+    per run, runs of more than 64 blocks (the last); up to 8 rows, with activations in shared memory and (eight wide rows) from
+    global memory.  Against float64 sums of exact products."""
     from ixrun_b200.p6 import P6Packed
 
     gen = torch.Generator(device="cuda").manual_seed(out_f + in_f)
@@ -309,19 +313,21 @@ def test_p6_gemv_rows_get_the_bits_they_get_alone(out_f, in_f, dense):
     p6 = P6Packed(codes, torch.tensor(0.007, dtype=torch.bfloat16), out_f, in_f)
     x = torch.randn(8, in_f, generator=gen, device="cuda").bfloat16()
     ref = x.double() @ (codes.float() * p6.scale.float()).bfloat16().double().t()
-    alone = torch.cat([p6.gemv(x[i:i + 1], out_dtype=torch.float32) for i in range(8)])
+    alone = torch.cat([p6.gemv(x[i:i + 1].clone(), out_dtype=torch.float32) for i in range(8)])      # (16-byte aligned)
     assert float((alone.double() - ref).abs().max() / ref.abs().max()) < 2e-5
     for m in (2, 3, 7, 8):
         assert torch.equal(p6.gemv(x[:m], out_dtype=torch.float32), alone[:m])
 
 
-def test_p6_gemv_infinite_activation_reaches_only_its_rows():
+@pytest.mark.parametrize("in_f", [256, 8264, 100])
+def test_p6_gemv_infinite_activation_reaches_only_its_rows(in_f):
     """An infinite activation in one of three rows: the other rows keep their bits, and a weight row without an outlier in
-    that column gets what the dense product gives (an infinity of the weight's sign, NaN for weight 0)."""
+    that column gets what the dense product gives (an infinity of the weight's sign, NaN for weight 0).  On the kernel for few
+    blocks per warp (256 columns) and on the other one."""
     from ixrun_b200.p6 import P6Packed
 
     gen = torch.Generator(device="cuda").manual_seed(2)
-    out_f, in_f, col = 64, 256, 77
+    out_f, col = 64, 77
     codes = torch.randint(1, 32, (out_f, in_f), generator=gen, device="cuda").to(torch.int8)
     codes[::2] = -torch.randint(1, 17, (out_f // 2, in_f), generator=gen, device="cuda").to(torch.int8)
     codes[5, col], codes[21, col], codes[3, 5], codes[8, col] = 100, -90, 120, 0
@@ -331,7 +337,7 @@ def test_p6_gemv_infinite_activation_reaches_only_its_rows():
     x[1, col] = float("inf")
     y = p6.gemv(x)
     assert torch.equal(y[0], clean[0]) and torch.equal(y[2], clean[2])
-    for got in (y[1], p6.gemv(x[1:2])[0]):
+    for got in (y[1], p6.gemv(x[1:2].clone())[0]):
         for r in range(out_f):
             if r in (5, 21):
                 assert not bool(torch.isfinite(got[r]))               # an outlier there: not finite either
@@ -446,7 +452,7 @@ def test_p6_gemv_few_blocks(out_f, in_f, dense):
         assert torch.equal(p6.gemv(x[:m], out_dtype=torch.float32), y8[:m])
     assert torch.equal(p6.gemv(x[:3], bias=bias), y8[:3].bfloat16() + bias)
     if (out_f, in_f) in ((2048, 8256), (19000, 512)):
-        return                                       # the other kernel: an infinity that meets an outlier is NaN there
+        return                                       # the other kernel: an infinity that meets an outlier is NaN there (see above)
     x[1, in_f // 2] = float("-inf")
     y, ref = p6.gemv(x), (x.double() @ w.t()).bfloat16()
     assert torch.equal(y[1].nan_to_num(nan=7.0, posinf=1.0, neginf=-1.0), ref[1].nan_to_num(nan=7.0, posinf=1.0, neginf=-1.0))
