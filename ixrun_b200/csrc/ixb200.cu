@@ -1881,9 +1881,13 @@ static int p6_rows_any(const P6 &p, int64_t n_esc, const void *x, int64_t m_rows
     if (p.in_f % 8u) return fail(IXB_E_UNSUPPORTED, "in_f=%u is not a multiple of 8", p.in_f);
     if ((uintptr_t)x & 15u) return fail(IXB_E_ARG, "x is not 16-byte aligned");
     int rc;
-    // Blocks with several outliers cost k_p6_umma more: its converters are what a stage waits for.  17408 x 5120 at 16 rows with
-    // 1.4 / 3.8 / 7.9 / 23 / 47 / 112 outliers per block, k_p6_rows and k_p6_umma: 28.1 and 26.9 us / 29.3, 29.9 / 29.5, 32.3 / 30.8, 36.2 /
-    // 45.2, 46.4 / 72.3, 63.7; at 32 rows and more k_p6_umma is the faster one of all.
+    // Blocks with several outliers cost k_p6_umma more: its converters are what a stage waits for.  16 rows, dependent launches, with
+    // 0.7 / 3 / 5 / 8 / 20 / 45 / 70 outliers per block, k_p6_rows and k_p6_umma: 17408 x 5120 27.1 and 25.5 us / 29.6, 29.5 / 30.0,
+    // 31.2 / 30.0, 32.8 / 30.4, 35.4 / 45.3, 44.8 / 62.3, 52.9; 6144 x 5120 15.6, 14.4 / 17.0, 15.7 / 17.1, 16.4 / 17.2, 17.5 / 17.4,
+    // 19.3 / 24.3, 23.9 / 32.8, 27.8; 5000 x 2176 7.6, 8.1 / 8.2, 8.6 / 8.2, 8.6 / 8.2, 8.6 / 8.4, 9.1 / 10.5, 10.8 / 13.0, 12.6.
+    // With 24 rows the two are closer (17408 x 5120: 33.6, 31.4 with 5, 34.0, 35.7 with 20); from 32 on k_p6_umma is the faster one of
+    // all.  On layers of few column blocks a CTA it would be so in dependent launches at any density, but not alone (2048 x 2048
+    // with 8: 6.0 and 4.8; 7.3 and 8.0).
     const float density = (float)n_esc / ((float)p.rt * (float)p.kb);
     if (m_rows <= kPrMaxRows && density > 3.f && density < 50.f) {
         PrPlan plan = {1, 1, 1};
