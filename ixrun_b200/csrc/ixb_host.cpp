@@ -10,6 +10,7 @@
 #include <ATen/ops/empty.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <c10/util/SmallVector.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
@@ -160,36 +161,37 @@ PyObject *empty(PyObject *, PyObject *const *args, Py_ssize_t nargs)
         if (!PyErr_Occurred()) PyErr_SetString(PyExc_ValueError, "expected a CUDA device");
         return nullptr;
     }
-    PyObject *out = PyTuple_New(nargs - 1);
-    if (!out) return nullptr;
+    struct Spec {
+        long long n;
+        int type;
+    };
     try {
-        for (Py_ssize_t i = 1; i < nargs; ++i) {
-            long long n;
-            int type;
-            if (!PyArg_ParseTuple(args[i], "LC", &n, &type)) {
-                Py_DECREF(out);
-                return nullptr;
+        c10::SmallVector<Spec, 8> specs((size_t)(nargs - 1));
+        c10::SmallVector<at::Tensor, 8> tensors;
+        for (Py_ssize_t i = 1; i < nargs; ++i)
+            if (!PyArg_ParseTuple(args[i], "LC", &specs[i - 1].n, &specs[i - 1].type)) return nullptr;
+        {
+            const Unlocked unlocked;
+            for (const Spec &s : specs) {
+                const auto dt = s.type == 'B' ? at::kByte : s.type == 'b' ? at::kChar : s.type == 'i' ? at::kInt : at::kBFloat16;
+                const int64_t size[1] = {s.n};
+                tensors.push_back(at::empty(at::IntArrayRef(size, s.n < 0 ? 0 : 1), at::TensorOptions().dtype(dt).device(at::Device(at::kCUDA, (c10::DeviceIndex)index))));
             }
-            const auto dt = type == 'B' ? at::kByte : type == 'b' ? at::kChar : type == 'i' ? at::kInt : at::kBFloat16;
-            const int64_t size[1] = {n};
-            at::Tensor t;
-            {
-                const Unlocked unlocked;
-                t = at::empty(at::IntArrayRef(size, n < 0 ? 0 : 1), at::TensorOptions().dtype(dt).device(at::Device(at::kCUDA, (c10::DeviceIndex)index)));
-            }
-            PyObject *o = THPVariable_Wrap(t);
+        }
+        PyObject *out = PyTuple_New(nargs - 1);
+        for (Py_ssize_t i = 0; out && i < nargs - 1; ++i) {
+            PyObject *o = THPVariable_Wrap(std::move(tensors[i]));
             if (!o) {
                 Py_DECREF(out);
                 return nullptr;
             }
-            PyTuple_SET_ITEM(out, i - 1, o);
+            PyTuple_SET_ITEM(out, i, o);
         }
+        return out;
     } catch (...) {
-        Py_DECREF(out);
         torch::translate_exception_to_python(std::current_exception());
         return nullptr;
     }
-    return out;
 }
 
 PyMethodDef methods[] = {{"p6", new_p6, METH_VARARGS, nullptr},
