@@ -139,9 +139,14 @@ class StreamingLinear(nn.Module):
 
     def forward(self, x):
         res = self._res
+        call = None if res is None else res._call
+        if call is not None:
+            y = call(x, self._bias_bf16, self._use_p6_gemm)
+            if y is not None:
+                return y
         rows = x.numel() // self.in_features
-        if res is not None and rows <= TC_MAX_ROWS:
-            y = (res._call or res.make_call())(x, self._bias_bf16, self._use_p6_gemm)
+        if call is None and res is not None and rows <= TC_MAX_ROWS:      # (a prompt has no use for the extension's object)
+            y = res.make_call()(x, self._bias_bf16, self._use_p6_gemm)
             if y is not None:
                 return y
         if res is not None and x.dtype == torch.bfloat16 and x.shape[-1] == self.in_features and rows <= TC_MAX_ROWS:
