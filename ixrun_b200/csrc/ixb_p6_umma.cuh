@@ -19,13 +19,14 @@
 //            epilogue: tcgen05.ld of the accumulators by warps 0..23, outputs (or a split's sums) from there
 //
 // What bounds it: the conversion's instructions (66 per 1024 weights and lane, about 130 with outliers and hand-over); the rows
-// cost next to nothing (17408 x 5120: 25.5 us at 16 rows, 26.8 at 64, k_p6_rows 27.0 and 49.3 on the same box).  Without the conversion
-// it takes 16.0 us, HBM alone would take 10.5.  How it came there, on that layer at 64 rows of another box: mma.sync with the weights in registers (k_p6_rows) 48.6, bound
-// by its rate of 540 TFLOP/s and a barrier per block; the weights through shared memory to tcgen05 59.7, by the hand-over; weights
-// in tensor memory 35.3, by the chain of instructions of the one thread that issues the MMAs (hence uniform addresses, unrolled
-// slots, two blocks per hand-over); activations by cp.async 39 to 52 (16-byte pieces of core matrices are half a sector each),
-// by TMA 30.3; packed weights by TMA instead of registers, so that the loads of outliers and weights wait for nobody, 25.4 (by
-// eight one-dimensional bulk copies a stage 27.5).
+// cost next to nothing (17408 x 5120: 25.5 us at 16 rows, 26.8 at 64; k_p6_rows beside it 26.9 and 48.9).  Without the conversion it
+// takes 16.0 us, HBM alone would take 10.5.  How it came there, on that layer at 64 rows: mma.sync with the weights in registers
+// (k_p6_rows) 48.6, bound by its rate of 540 TFLOP/s and a barrier per block; the weights through shared memory to tcgen05 59.7, by
+// the hand-over; weights in tensor memory 35.3, by the chain of instructions of the one thread that issues the MMAs (hence uniform
+// addresses, unrolled slots, two blocks per hand-over); activations by cp.async 39 to 52 (16-byte pieces of core matrices are half a
+// sector each), by TMA 30.3; packed weights by TMA instead of registers, so that the loads of outliers and weights wait for nobody,
+// 25.4 (by eight one-dimensional bulk copies a stage 27.5).  That chain of instructions still counts: the vote on the waits of
+// a stage is the cheapest form of them (17408 x 5120 at 16 rows 25.5; without it 26.7, with the MMAs predicated on them 28.7).
 //
 // Every wait on an mbarrier is bounded, and no thread begins one that depends on the activations before the kernel ahead is
 // complete: such a wait counts this CTA's own copies, conversions and MMAs only, however long that kernel takes.  A thread whose
