@@ -496,7 +496,7 @@ DEFAULT_LAYOUT = "p6"
 LAYOUT_KERNEL = {"p6": "k_p6_mma<1>", "streams": "k_gemv<1>"}
 LAYOUT_TEXT = {
     "p6": ("resident P6 re-layout of the same int8 codes (6-bit plane in mma fragment order whose fields are part of "
-           "the bf16 number 96 + code, + a weight list for codes outside -32..31), built on the GPU at deploy time "
+           "the bf16 number 160 + code, + a weight list for codes outside -32..31), built on the GPU at deploy time "
            "from the reference's packed streams"),
     "streams": "the reference's (3,5,8) streams read directly",
 }

@@ -169,8 +169,8 @@ int ixb_group_scale(const int8_t *codes_device, const void *group_scales_fp16_de
  * addressed by rank:
  *   plane    a 6-bit field per element, blocks of 16 rows x 64 columns (ragged
  *            edges padded), 768 contiguous bytes per block, block b =
- *            row_tile * ceil(in_f / 64) + column_block.  The field is bits 6..1
- *            of the low byte of the bf16 number 96 + code (codes -32 .. 31),
+ *            row_tile * ceil(in_f / 64) + column_block.  The field is the low
+ *            six bits of the bf16 number 160 + code (codes -32 .. 31),
  *            so the GEMV needs a shift, a mask, a subtraction and a multiplication
  *            per pair of weights to obtain bf16(code * scale) -- the reference's
  *            dequantised weight (ixrun/quantize.py:182, ixrun/fused.py:169-170),
